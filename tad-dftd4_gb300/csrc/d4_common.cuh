@@ -73,6 +73,17 @@ constexpr int ATM_SPARSE_DMAX = 2048;
 constexpr int ATM_ORDER_MAX = 16384;
 
 
+// One pair of the register-tiled FP64 ATM (d4_atm64.cu): everything a triple
+// needs of a pair, 32 bytes.
+struct alignas(32) PairRec {
+  double x, u;  // r^2, 1 / r^2
+  double t;     // (R0/r)^(alp/3), at most PAIR_T_MAX
+  double q;     // sqrt(C6 at q = 0) / r^3
+};
+// (R0/r)^(alp/3) above this (R0/r beyond 1e18 for alp = 16) damps a triple
+// to below 1e-100 of its energy anyway; three such factors stay finite.
+constexpr double PAIR_T_MAX = 1e100;
+
 struct Workspace {
   int *status;      // [1]
   float *eeq_final; // [B][2] final EEQ refinement residual (forward, adjoint); fixed offset
@@ -104,9 +115,14 @@ struct Workspace {
   double *pr_ir;    // [B*N*N] 1/distance
   double *pr_L;     // [B*N*N] log(R0/r) of the ATM damping
   double *pr_c;     // [B*N*N] sqrt(C6 at q = 0)
+  PairRec *pr4;     // [B*N*N] the four above as one record per pair (register-tiled
+                    // FP64 ATM, in their place; only the entries i < j)
+  double *rowmax;   // [B*N] largest r^2 of each atom (register-tiled FP64 ATM; in the
+                    // place of dEdcnq, which is written after it)
   double *pr_S;     // [B*N*N] dE_ATM/d(r^2) (atomics)
   double *pr_P;     // [B*N*N] sum of weighted triple energies (atomics)
-  double *pr_da1;   // [B*N*N] d log R0 / d a1 (parameter gradients only)
+  double *pr_da1;   // [B*N*N] d log R0 / d a1 (parameter gradients only; register-tiled
+                    // FP64 ATM: entries i < j, and log(R0/r) in the entries i > j)
   double *pr_da2;   // [B*N*N] d log R0 / d a2 (parameter gradients only)
   // exact C9 (D4_FLAG_EXACT_C9, FP64 method only)
   double *ax;       // [B*N*23] polarisabilities a_i(iw) of the exact C9
@@ -225,10 +241,14 @@ inline Workspace carve_workspace(void *base, int B, int N, int S, uint32_t flags
   w.dA0_dcn = (grad && !mixed) ? (double *)take(8 * BNS23) : nullptr;
   w.G = (grad && !mixed) ? (double *)take(8 * BNS23) : nullptr;
   w.G0 = (grad && !mixed) ? (double *)take(8 * BNS23) : nullptr;
-  w.pr_r = mixed ? nullptr : (double *)take(8 * BNN);
-  w.pr_ir = mixed ? nullptr : (double *)take(8 * BNN);
-  w.pr_L = mixed ? nullptr : (double *)take(8 * BNN);
-  w.pr_c = mixed ? nullptr : (double *)take(8 * BNN);
+  const size_t plane = align_up(8 * BNN, 256);
+  char *pr = mixed ? nullptr : (char *)take(4 * plane);
+  w.pr4 = (PairRec *)pr;
+  w.pr_r = (double *)pr;
+  w.pr_ir = pr ? (double *)(pr + plane) : nullptr;
+  w.pr_L = pr ? (double *)(pr + 2 * plane) : nullptr;
+  w.pr_c = pr ? (double *)(pr + 3 * plane) : nullptr;
+  w.rowmax = w.dEdcnq;
   w.pr_S = (grad && !mixed) ? (double *)take(8 * BNN) : nullptr;
   w.pr_P = (grad && !mixed) ? (double *)take(8 * BNN) : nullptr;
   const bool pgrad = (flags & D4_FLAG_PARAM_GRAD) != 0;
@@ -322,6 +342,8 @@ struct Ctx {
   int B, N, S;
   uint32_t flags;
   int atm_tiled;  // the register-tiled ATM runs (set by the precision form's launcher)
+  int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
+  double cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp3 (set by launch_fp64)
   Workspace w;
   d4_outputs_t out;
 };

@@ -5,9 +5,10 @@
 // quantities live in dense per-structure N x N blocks, only the leading
 // n_eff x n_eff part of which is touched.  Every "atom-owned" kernel maps one
 // warp to one atom i and loops its lanes over partners j, so per-atom sums
-// need no atomics.  The ATM kernel maps a CTA to a tile of pairs (j, k) and
-// loops over the third atom i < j.
+// need no atomics.  The general ATM kernel maps a CTA to a tile of pairs (j, k)
+// and loops over the third atom i < j.
 #include <float.h>
+#include <math.h>
 
 #include "d4_common.cuh"
 #include "d4_kernels.cuh"
@@ -528,6 +529,11 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
     }
     if (grad && lane < NFREQ)
       for (int s = 0; s < c.S; ++s) c.w.G[(ai * c.S + s) * NFREQ + lane] = 0.0;
+    if (c.atm64 && i < n) {  // padding below the last atom: empty pair records
+      if (lane == 0) c.w.rowmax[ai] = 0.0;
+      for (int j = i + 1 + lane; j < n; j += 32)
+        c.w.pr4[ai * N + j] = PairRec{0.0, 0.0, 0.0, 0.0};
+    }
     return;
   }
   const d4_params_t &p = c.par;
@@ -542,6 +548,11 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
   // s6, s8, s10, a1, a2, -, alp, rs6, rs8, bet (slots of d_param_grad)
   double pg[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const double *rvdw_row = c.rvdw_in ? c.rvdw_in + ai * N : nullptr;
+  const double alp3 = p.alp / 3.0;
+  double rmax = 0.0;
+  if (c.atm64)
+    for (int j = i + 1 + lane; j < n; j += 32)
+      if (c.w.z[(size_t)b * N + j] == 0) c.w.pr4[ai * N + j] = PairRec{0.0, 0.0, 0.0, 0.0};
   for (int s = 0; s < nslot; ++s) {
     if (lane < NFREQ) {
       const size_t o = (ai * c.S + s) * NFREQ + lane;
@@ -571,13 +582,28 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
       const double sqq = sqrt(qq);
       const double R0 = p.a1 * sqq + p.a2;
       const size_t pij = ((size_t)b * N + i) * N + j;
-      c.w.pr_r[pij] = r;
-      c.w.pr_ir[pij] = 1.0 / r;
-      c.w.pr_L[pij] = log(R0 / r);
-      c.w.pr_c[pij] = sqrt(c60);
-      if (c.w.pr_da1) {
-        c.w.pr_da1[pij] = sqq / R0;
-        c.w.pr_da2[pij] = 1.0 / R0;
+      if (c.atm64) {
+        rmax = fmax(rmax, r2);
+        if (j > i) {
+          const double ir = 1.0 / r, u = ir * ir;
+          c.w.pr4[pij] = PairRec{r2, u, fmin(exp(alp3 * log(R0 * ir)), PAIR_T_MAX),
+                                 sqrt(c60) * (u * ir)};
+          if (c.w.pr_da1) {
+            c.w.pr_da1[pij] = sqq / R0;
+            c.w.pr_da2[pij] = 1.0 / R0;
+          }
+        } else if (c.w.pr_da1) {
+          c.w.pr_da1[pij] = log(R0 / r);
+        }
+      } else {
+        c.w.pr_r[pij] = r;
+        c.w.pr_ir[pij] = 1.0 / r;
+        c.w.pr_L[pij] = log(R0 / r);
+        c.w.pr_c[pij] = sqrt(c60);
+        if (c.w.pr_da1) {
+          c.w.pr_da1[pij] = sqq / R0;
+          c.w.pr_da2[pij] = 1.0 / R0;
+        }
       }
       if (r <= p.cut_disp2 && p.damping != D4_DAMP_RATIONAL) {
         // D3-family damping: e = s6 c6 t6 + s8 c8 t8 (dispersion2,
@@ -687,6 +713,11 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
   gx = warp_sum(gx);
   gy = warp_sum(gy);
   gz = warp_sum(gz);
+  if (c.atm64) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    if (lane == 0) c.w.rowmax[ai] = rmax;
+  }
   if (c.flags & D4_FLAG_PARAM_GRAD) {
     const int npg = p.damping != D4_DAMP_RATIONAL ? 10 : 5;
 #pragma unroll
@@ -716,7 +747,8 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
 
 // ---------------------------------------------------------------- ATM
 
-// Axilrod-Teller-Muto energy over triples i < j < k.  A CTA owns a tile of
+// The general FP64 ATM (energy weights, unusual exponents; the common case
+// is d4_atm64.cu).  Axilrod-Teller-Muto energy over triples i < j < k.  A CTA owns a tile of
 // pairs (j, k) -- 8 rows j (one per warp) by 32 columns k (one per lane) --
 // and loops over i < j.  Everything a triple needs is a per-pair scalar:
 // r, 1/r, log(R0/r), sqrt(C6(q=0)).  With GRAD, it accumulates per pair
@@ -915,7 +947,7 @@ __global__ void __launch_bounds__(256) pair_atm_bwd_kernel(Ctx c) {
   const int slot_x = c.w.slot[ax];
   const size_t base = (size_t)b * N * N;
   const double *fw = c.tab.freq_weights;
-  double gx = 0.0, gy = 0.0, gz = 0.0;
+  double gx = 0.0, gy = 0.0, gz = 0.0, psum = 0.0;
   for (int s = 0; s < nslot; ++s) {
     double gacc[NFREQ];
 #pragma unroll
@@ -931,8 +963,16 @@ __global__ void __launch_bounds__(256) pair_atm_bwd_kernel(Ctx c) {
       gy += 2.0 * S * (py - P[3 * y + 1]);
       gz += 2.0 * S * (pz - P[3 * y + 2]);
       if (Pv != 0.0) {
-        const double cc = c.w.pr_c[base + (size_t)x * N + y];
-        const double D = Pv / (2.0 * cc * cc);
+        double c60;
+        if (c.atm64) {
+          const PairRec &pr = c.w.pr4[o];
+          c60 = (pr.q * pr.q) * (pr.x * pr.x * pr.x);
+          psum += Pv;
+        } else {
+          const double cc = c.w.pr_c[base + (size_t)x * N + y];
+          c60 = cc * cc;
+        }
+        const double D = Pv / (2.0 * c60);
         const double *A0y = c.w.A0 + (ay * c.S + slot_x) * NFREQ;
 #pragma unroll
         for (int w = 0; w < NFREQ; ++w) gacc[w] += D * A0y[w];
@@ -955,6 +995,7 @@ __global__ void __launch_bounds__(256) pair_atm_bwd_kernel(Ctx c) {
   gx = warp_sum(gx);
   gy = warp_sum(gy);
   gz = warp_sum(gz);
+  if (c.atm64) psum = warp_sum(psum);
   if (c.w.f3x) {  // exact C9: the ATM force of atom x from its own warp
     gx += c.w.f3x[3 * ax];
     gy += c.w.f3x[3 * ax + 1];
@@ -978,7 +1019,10 @@ __global__ void __launch_bounds__(256) pair_atm_bwd_kernel(Ctx c) {
     c.out.d_gradient[3 * ax] += gx;
     c.out.d_gradient[3 * ax + 1] += gy;
     c.out.d_gradient[3 * ax + 2] += gz;
-    c.out.d_energy[ax] += c.w.e3[ax];
+    // (register-tiled ATM: every triple reaches the atom through two of its
+    // pair sums, a third of its energy each atom; e3 holds the corrections of
+    // the triples with a side beyond the cutoff)
+    c.out.d_energy[ax] += c.w.e3[ax] + psum * (1.0 / 6.0);
   }
 }
 
@@ -1089,8 +1133,26 @@ __global__ void prepare_alpha_kernel(d4_tables_t tab, d4_model_cfg_t cfg,
 
 // ---------------------------------------------------------------- launch
 
-int launch_fp64(const Ctx &c, cudaStream_t st) {
+// The largest x with sqrt(x) <= cut, so that comparing r^2 decides as
+// comparing r does (a negative or NaN cutoff: no pair).
+static double cutoff_sq(double cut) {
+  if (!(cut >= 0.0)) return -1.0;
+  double x = cut * cut;
+  for (int k = 0; k < 4 && sqrt(x) > cut; ++k) x = nextafter(x, 0.0);
+  for (int k = 0; k < 4 && isfinite(x) && sqrt(nextafter(x, INFINITY)) <= cut; ++k)
+    x = nextafter(x, INFINITY);
+  return x;
+}
+
+int launch_fp64(const Ctx &c_in, cudaStream_t st) {
+  Ctx c = c_in;
   const int B = c.B, N = c.N;
+  // The register-tiled ATM takes unit energy weights and the approximate C9;
+  // alp beyond 100 (16 in the method) could clip (R0/r)^(alp/3) at ratios
+  // that another factor of the triple makes up for.
+  c.atm64 = c.weights == nullptr && !(c.flags & D4_FLAG_EXACT_C9) && c.par.alp >= 0.0 &&
+            c.par.alp <= 100.0;
+  c.cut3_sq = cutoff_sq(c.par.cut_disp3);
   const dim3 atoms((N + 7) / 8, B);
   const bool grad = (c.flags & D4_FLAG_GRADIENT) != 0;
   const bool eeq = (c.flags & D4_FLAG_CHARGES_IN) == 0;
@@ -1128,6 +1190,8 @@ int launch_fp64(const Ctx &c, cudaStream_t st) {
   stage_begin(ST_ATM, st);
   if (c.flags & D4_FLAG_EXACT_C9) {
     launch_atm_exact(c, st);
+  } else if (c.atm64) {
+    launch_atm_tiled64(c, st);
   } else if (grad) {
     if (c.flags & D4_FLAG_PARAM_GRAD)
       atm_kernel<true, true><<<tiles, 256, 0, st>>>(c);
