@@ -96,7 +96,7 @@ struct Workspace {
   double *cnq;      // [B*N] capped EEQ coordination number
   double *dcnq;     // [B*N] d(capped)/d(raw)
   double *q;        // [B*N] atomic charges
-  double *eeq_y;    // [B*N] A^-1 1
+  double *eeq_y;    // [B*N] A^-1 1 by atom (precision form); L^-1 1 in compact order (FP64)
   double *eeq_w;    // [B*N] adjoint charges
   double *eeq_sum;  // [B*2] (sum y, lambda)
   double *dEdcn;    // [B*N]

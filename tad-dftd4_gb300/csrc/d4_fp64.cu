@@ -103,212 +103,6 @@ __global__ void __launch_bounds__(256) cn_kernel(Ctx c) {
   }
 }
 
-// ---------------------------------------------------------------- EEQ
-
-// Row-oriented triangular solves with one warp.  L is packed lower.
-// forward: L z = v (in place); backward: L^T x = z (in place).
-template <int NRHS>
-__device__ void warp_forward_solve(const double *L, double *v, int ldv, int m) {
-  const int lane = threadIdx.x & 31;
-  for (int i = 0; i < m; ++i) {
-    const double *row = L + tri_index(i, 0);
-    double s[NRHS];
-#pragma unroll
-    for (int r = 0; r < NRHS; ++r) s[r] = 0.0;
-    for (int k = lane; k < i; k += 32) {
-      const double l = row[k];
-#pragma unroll
-      for (int r = 0; r < NRHS; ++r) s[r] += l * v[r * ldv + k];
-    }
-#pragma unroll
-    for (int r = 0; r < NRHS; ++r) s[r] = warp_sum(s[r]);
-    if (lane == 0) {
-      const double inv = 1.0 / row[i];
-#pragma unroll
-      for (int r = 0; r < NRHS; ++r) v[r * ldv + i] = (v[r * ldv + i] - s[r]) * inv;
-    }
-    __syncwarp();
-  }
-}
-
-template <int NRHS>
-__device__ void warp_backward_solve(const double *L, double *v, int ldv, int m) {
-  const int lane = threadIdx.x & 31;
-  for (int i = m - 1; i >= 0; --i) {
-    double s[NRHS];
-#pragma unroll
-    for (int r = 0; r < NRHS; ++r) s[r] = 0.0;
-    for (int k = i + 1 + lane; k < m; k += 32) {
-      const double l = L[tri_index(k, i)];
-#pragma unroll
-      for (int r = 0; r < NRHS; ++r) s[r] += l * v[r * ldv + k];
-    }
-#pragma unroll
-    for (int r = 0; r < NRHS; ++r) s[r] = warp_sum(s[r]);
-    if (lane == 0) {
-      const double inv = 1.0 / L[tri_index(i, i)];
-#pragma unroll
-      for (int r = 0; r < NRHS; ++r) v[r * ldv + i] = (v[r * ldv + i] - s[r]) * inv;
-    }
-    __syncwarp();
-  }
-}
-
-// EEQ charges of one structure per CTA: build the (real-atom) Coulomb matrix
-// in packed form, Cholesky-factorise it, solve for A^-1 b and A^-1 1, apply
-// the total-charge constraint.  The factor is kept in the workspace for the
-// adjoint solve.  ``SMEM``: factorise in shared memory, else in place in the
-// workspace.
-template <bool SMEM>
-__global__ void __launch_bounds__(256) eeq_kernel(Ctx c) {
-  extern __shared__ double s_dyn[];
-  const int b = blockIdx.x;
-  const int N = c.N;
-  const int n = c.w.n_eff[b];
-  __shared__ int s_m;
-  __shared__ double s_inv;
-  // shared scratch: idx[N] (int), vectors rhs[2*N]
-  int *s_idx = reinterpret_cast<int *>(s_dyn);
-  double *vec = s_dyn + (N + 1) / 2 + 1;  // 2 * N doubles
-  double *L = SMEM ? vec + 2 * N : c.w.eeq_L + (size_t)b * ((size_t)N * (N + 1) / 2);
-  const int m = compact_real_atoms(c, b, n, s_idx, &s_m);
-  const double *P = c.positions + (size_t)b * N * 3;
-  const int *Zb = c.w.z + (size_t)b * N;
-  const size_t tri_m = (size_t)m * (m + 1) / 2;
-  // build
-  for (size_t t = threadIdx.x; t < tri_m; t += blockDim.x) {
-    // invert t -> (ii, jj) with jj <= ii
-    int ii = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while (tri_index(ii + 1, 0) <= t) ++ii;
-    while (tri_index(ii, 0) > t) --ii;
-    const int jj = (int)(t - tri_index(ii, 0));
-    const int ia = s_idx[ii], ja = s_idx[jj];
-    const int za = Zb[ia], zb = Zb[ja];
-    double v;
-    if (ii == jj) {
-      v = c.tab.eeq_eta[za] + SQRT_2_OVER_PI / c.tab.eeq_rad[za];
-    } else {
-      const double dx = P[3 * ia] - P[3 * ja], dy = P[3 * ia + 1] - P[3 * ja + 1],
-                   dz = P[3 * ia + 2] - P[3 * ja + 2];
-      const double r = sqrt(dx * dx + dy * dy + dz * dz);
-      const double ra = c.tab.eeq_rad[za], rb = c.tab.eeq_rad[zb];
-      const double g = 1.0 / sqrt(ra * ra + rb * rb);
-      v = erf(g * r) / r;
-    }
-    L[t] = v;
-  }
-  for (int k = threadIdx.x; k < m; k += blockDim.x) {
-    const int ia = s_idx[k];
-    const int z = Zb[ia];
-    const double cq = c.w.cnq[(size_t)b * N + ia];
-    const double sq = cq > 0.0 ? sqrt(cq) : 0.0;
-    vec[k] = -c.tab.eeq_chi[z] + c.tab.eeq_kcn[z] * sq;
-    vec[N + k] = 1.0;
-  }
-  __syncthreads();
-  // right-looking Cholesky, packed lower
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int k = 0; k < m; ++k) {
-    if (threadIdx.x == 0) {
-      double d = L[tri_index(k, k)];
-      if (!(d > 0.0)) {
-        set_status(c.w.status, D4_ERR_EEQ_SINGULAR);
-        d = 1.0;
-      }
-      d = sqrt(d);
-      L[tri_index(k, k)] = d;
-      s_inv = 1.0 / d;
-    }
-    __syncthreads();
-    const double inv = s_inv;
-    for (int i = k + 1 + threadIdx.x; i < m; i += blockDim.x) L[tri_index(i, k)] *= inv;
-    __syncthreads();
-    for (int i = k + 1 + warp; i < m; i += nw) {
-      const double lik = L[tri_index(i, k)];
-      double *row = L + tri_index(i, 0);
-      for (int j = k + 1 + lane; j <= i; j += 32) row[j] -= lik * L[tri_index(j, k)];
-    }
-    __syncthreads();
-  }
-  if (warp == 0) {
-    warp_forward_solve<2>(L, vec, N, m);
-    warp_backward_solve<2>(L, vec, N, m);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    double sx = 0.0, sy = 0.0;
-    for (int k = lane; k < m; k += 32) {
-      sx += vec[k];
-      sy += vec[N + k];
-    }
-    sx = warp_sum(sx);
-    sy = warp_sum(sy);
-    if (lane == 0) {
-      const double lam = m > 0 ? (sx - c.charge[b]) / sy : 0.0;
-      c.w.eeq_sum[2 * b] = sy;
-      c.w.eeq_sum[2 * b + 1] = lam;
-      s_inv = lam;
-    }
-  }
-  __syncthreads();
-  const double lam = s_inv;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    c.w.q[(size_t)b * N + i] = 0.0;
-    c.w.eeq_y[(size_t)b * N + i] = 0.0;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < m; k += blockDim.x) {
-    const size_t a = (size_t)b * N + s_idx[k];
-    c.w.q[a] = vec[k] - lam * vec[N + k];
-    c.w.eeq_y[a] = vec[N + k];
-  }
-  if (SMEM) {
-    double *G = c.w.eeq_L + (size_t)b * ((size_t)N * (N + 1) / 2);
-    for (size_t t = threadIdx.x; t < tri_m; t += blockDim.x) G[t] = L[t];
-  }
-}
-
-// Adjoint of the constrained EEQ solve: w = A^-1 g - nu A^-1 1 with
-// sum(w) = 0, g = dE/dq.  Then dE/d(raw EEQ CN) = w kcn / (2 sqrt(cn)) dcap.
-__global__ void __launch_bounds__(256) eeq_adjoint_kernel(Ctx c) {
-  extern __shared__ double s_dyn[];
-  const int b = blockIdx.x;
-  const int N = c.N;
-  const int n = c.w.n_eff[b];
-  __shared__ int s_m;
-  __shared__ double s_nu;
-  int *s_idx = reinterpret_cast<int *>(s_dyn);
-  double *vec = s_dyn + (N + 1) / 2 + 1;
-  const int m = compact_real_atoms(c, b, n, s_idx, &s_m);
-  const double *L = c.w.eeq_L + (size_t)b * ((size_t)N * (N + 1) / 2);
-  for (int k = threadIdx.x; k < m; k += blockDim.x) vec[k] = c.w.dEdq[(size_t)b * N + s_idx[k]];
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {
-    warp_forward_solve<1>(L, vec, N, m);
-    warp_backward_solve<1>(L, vec, N, m);
-    double su = 0.0;
-    for (int k = lane; k < m; k += 32) su += vec[k];
-    su = warp_sum(su);
-    if (lane == 0) s_nu = m > 0 ? su / c.w.eeq_sum[2 * b] : 0.0;
-  }
-  __syncthreads();
-  const double nu = s_nu;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    c.w.eeq_w[(size_t)b * N + i] = 0.0;
-    c.w.dEdcnq[(size_t)b * N + i] = 0.0;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < m; k += blockDim.x) {
-    const size_t a = (size_t)b * N + s_idx[k];
-    const double w = vec[k] - nu * c.w.eeq_y[a];
-    c.w.eeq_w[a] = w;
-    const double cq = c.w.cnq[a];
-    const int z = c.w.z[a];
-    c.w.dEdcnq[a] = cq > 0.0 ? w * c.tab.eeq_kcn[z] * 0.5 / sqrt(cq) * c.w.dcnq[a] : 0.0;
-  }
-}
-
 // ---------------------------------------------------------------- weights
 
 constexpr int WU = 4;  // (atom, slot) units per warp of weights_kernel
@@ -1163,17 +957,9 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   stage_begin(ST_CN, st);
   cn_kernel<<<atoms, 256, 0, st>>>(c);
   stage_end(ST_CN, st);
-  const size_t vec_bytes = (size_t)8 * ((N + 1) / 2 + 1 + 2 * N);
-  const size_t tri_bytes = (size_t)8 * ((size_t)N * (N + 1) / 2);
   stage_begin(ST_EEQ, st);
   if (eeq) {
-    if (vec_bytes + tri_bytes <= 220 * 1024) {
-      ensure_smem(eeq_kernel<true>, (int)(vec_bytes + tri_bytes));
-      eeq_kernel<true><<<B, 256, vec_bytes + tri_bytes, st>>>(c);
-    } else {
-      ensure_smem(eeq_kernel<false>, (int)vec_bytes);
-      eeq_kernel<false><<<B, 256, vec_bytes, st>>>(c);
-    }
+    launch_eeq64(c, st);
   } else {
     const size_t total = (size_t)B * N;
     charges_in_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(c);
@@ -1207,8 +993,7 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
     stage_end(ST_PAIR_ATM_BWD, st);
     if (eeq) {
       stage_begin(ST_EEQ_ADJ, st);
-      ensure_smem(eeq_adjoint_kernel, (int)vec_bytes);
-      eeq_adjoint_kernel<<<B, 256, vec_bytes, st>>>(c);
+      launch_eeq64_adjoint(c, st);
       stage_end(ST_EEQ_ADJ, st);
     }
     stage_begin(ST_PAIR_CN_BWD, st);
@@ -1269,15 +1054,7 @@ int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_
   const dim3 atoms((N + 7) / 8, B);
   launch_prep(c, st);
   cn_kernel<<<atoms, 256, 0, st>>>(c);
-  const size_t vec_bytes = (size_t)8 * ((N + 1) / 2 + 1 + 2 * N);
-  const size_t tri_bytes = (size_t)8 * ((size_t)N * (N + 1) / 2);
-  if (vec_bytes + tri_bytes <= 220 * 1024) {
-    ensure_smem(eeq_kernel<true>, (int)(vec_bytes + tri_bytes));
-    eeq_kernel<true><<<B, 256, vec_bytes + tri_bytes, st>>>(c);
-  } else {
-    ensure_smem(eeq_kernel<false>, (int)vec_bytes);
-    eeq_kernel<false><<<B, 256, vec_bytes, st>>>(c);
-  }
+  launch_eeq64(c, st);
   launch_weights(c, st);
   props_kernel<<<atoms, 256, 0, st>>>(c, c6out, alpha_out, q_out);
   return 0;

@@ -45,6 +45,8 @@ void launch_pair_fwd_tc(const Ctx &c, cudaStream_t st);  // D4, precision form (
 bool pair_atm_bwd_tc_ok(const Ctx &c);
 void launch_pair_atm_bwd_tc(const Ctx &c, cudaStream_t st);
 void launch_atm_tiled64(const Ctx &c, cudaStream_t st);  // FP64 (d4_atm64.cu)
+void launch_eeq64(const Ctx &c, cudaStream_t st);  // FP64 EEQ charges (d4_eeq64.cu)
+void launch_eeq64_adjoint(const Ctx &c, cudaStream_t st);
 void launch_atm_exact(const Ctx &c, cudaStream_t st);  // exact C9, FP64 (d4_exact.cu)
 int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_out,
                       cudaStream_t st);
