@@ -1,9 +1,9 @@
 // Register-tiled FP64 ATM of the plain method: all triples i < j < k of
 // structures with unit energy weights (any size, padding atoms anywhere).
 //
-// GB300 issues two FP64 lanes per clock and SM, so a warp instruction on the
-// FP64 pipe takes 16 cycles and everything else (loads, shuffles, integer
-// work, reductions at L2) hides behind it: the kernel is built for the
+// A warp instruction occupies its sub-partition's FP64 pipe for 64 cycles, so
+// everything else (loads, shuffles, integer work, reductions at L2) hides
+// behind the FP64 instructions: the kernel is built for the
 // fewest FP64 instructions per triple.  The pair records carry r^2, 1/r^2,
 // (R0/r)^(alp/3) and sqrt(C6(q=0)) / r^3, so that damping and C9 / R^3 are
 // products (no exp per triple), the atom energies follow from the pair
@@ -15,6 +15,7 @@
 // ms, 301 atoms 4.82 -> 0.52 ms, 57 atoms 0.48 -> 0.019 ms (energy +
 // gradient); 32 atoms, energy only, 0.125 -> 0.016 ms.
 #include "d4_common.cuh"
+#include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
 
 namespace d4 {
@@ -22,17 +23,6 @@ namespace d4 {
 namespace {
 
 constexpr int A6_K = 8;  // outer atoms per task (lanes of a group)
-
-// 1 / d for d >= 1: the PTX approximation (20 bits and more) and one
-// third-order step y (1 + e + e^2), e = 1 - d y (Householder's method for
-// 1/x), whose error e^3 is below the rounding of the two FMAs.  d = inf does
-// not occur (PAIR_T_MAX), d beyond 2^1022 gives 0.
-__device__ __forceinline__ double rcp_pos(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 
 // Sum of two lanes' values, split: the lane whose bit h is clear keeps the
 // sum of the pair's a, the other the sum of the pair's b.

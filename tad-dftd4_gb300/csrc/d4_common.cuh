@@ -343,7 +343,8 @@ struct Ctx {
   uint32_t flags;
   int atm_tiled;  // the register-tiled ATM runs (set by the precision form's launcher)
   int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
-  double cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp3 (set by launch_fp64)
+  int pair64;     // the pair stages of d4_pair64.cu run (set by launch_fp64)
+  double cut2_sq, cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp2, cut_disp3 (likewise)
   Workspace w;
   d4_outputs_t out;
 };
@@ -419,6 +420,21 @@ __device__ __forceinline__ void zeta_and_deriv(double gam, double qref, double q
     *z = exp(ga);
     *dz = 0.0;
   }
+}
+
+// (R0/r)^(alp/3) from its logarithm, clipped for the pair records (NaN stays).
+__device__ __forceinline__ double pair_t(double log_t) {
+  const double t = exp(log_t);
+  return t > PAIR_T_MAX ? PAIR_T_MAX : t;
+}
+
+// (row, col), col <= row, of entry t of a packed lower triangle
+__device__ __forceinline__ void tri_entry(long long t, int &row, int &col) {
+  int r = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while ((long long)(r + 1) * (r + 2) / 2 <= t) ++r;
+  while ((long long)r * (r + 1) / 2 > t) --r;
+  row = r;
+  col = (int)(t - (long long)r * (r + 1) / 2);
 }
 
 __host__ __device__ inline size_t tri_index(int i, int j) {  // packed lower, j <= i

@@ -24,6 +24,7 @@
 // eliminated column by column (three barriers each) and one warp solved row
 // by row.
 #include "d4_common.cuh"
+#include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
 
 namespace d4 {
@@ -92,9 +93,7 @@ struct PanelSmem {
 };
 
 // Pivot of column c, whose entries (a lane per row) are `a`: the scaled column
-// and 1 / sqrt(d) to shared memory.  1 / sqrt(d) by the PTX approximation y
-// (20 bits and more) and one third-order step y (1 + e / 2 + 3 e^2 / 8), e =
-// 1 - d y^2 (the binomial series of (1 - e)^(-1/2)).
+// and 1 / sqrt(d) to shared memory.
 __device__ __forceinline__ void eeq64_pivot(double a, int c, PanelSmem &sm, int *status) {
   const int lane = threadIdx.x & 31;
   double d = __shfl_sync(FULL, a, c);
@@ -105,10 +104,7 @@ __device__ __forceinline__ void eeq64_pivot(double a, int c, PanelSmem &sm, int 
     d = 1.0;
   }
   if (lane == c) a = d;
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-(d * y), y, 1.0);
-  const double inv = fma(y * e, fma(0.375, e, 0.5), y);
+  const double inv = rsqrt_pos(d);
   sm.L[c * EB + lane] = lane >= c ? a * inv : 0.0;
   if (lane == c) sm.inv[c] = inv;
 }
@@ -249,13 +245,6 @@ __device__ __forceinline__ void eeq64_update_tile(double *L, const double *sj, d
   }
 }
 
-__device__ __forceinline__ void eeq64_tile_of(int t, int &ti, int &tj) {  // packed lower tiles
-  ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-  while (ti > 0 && ti * (ti + 1) / 2 > t) --ti;
-  tj = t - ti * (ti + 1) / 2;
-}
-
 // Block inverse X of block kk: from the packed factor or the scratch of the
 // panel kernel.
 struct InvAt {
@@ -375,42 +364,106 @@ __device__ void eeq64_charges(const Ctx &c, int b, const double *L, const InvAt 
 
 }  // namespace
 
-// Coulomb matrix of the real atoms (packed lower rows) and the right-hand
-// sides.  A thread per pair of the flattened triangle, so that small
-// structures fill their warps (a warp per row took 1.4x as long for 30
-// atoms); a pair with g r >= 6 has erf = 1 to the last bit.
-__global__ void __launch_bounds__(128) eeq64_build_kernel(Ctx c) {
+// Off-diagonal Coulomb matrix of the real atoms (packed lower rows).  A thread
+// per pair of the flattened triangle, so that small structures fill their
+// warps; pairs with g r < 6.6 (beyond, erf = 1 to the last bit) are queued per
+// warp and evaluated 32 at a time, so that erf runs with full warps.
+__global__ void __launch_bounds__(128) eeq64_build_kernel(Ctx c, int rounds) {
+  __shared__ int s_i[4][64], s_j[4][64];
   const int b = blockIdx.y;
   const int N = c.N, n = c.w.n_eff[b];
-  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
-  if (t >= (long long)n * (n + 1) / 2) return;
-  int i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-  while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
-  while ((long long)i * (i + 1) / 2 > t) --i;
-  const int j = (int)(t - (long long)i * (i + 1) / 2);
-  const int *C = c.w.cidx + (size_t)b * N, *Z = c.w.z + (size_t)b * N;
-  const int ci = C[i], cj = C[j];
-  if (ci < 0 || cj < 0) return;
-  const double ra = c.tab.eeq_rad[Z[i]];
-  double *out = eeq64_factor(c, b) + tri_index(ci, cj);
-  if (i == j) {
-    *out = c.tab.eeq_eta[Z[i]] + SQRT_2_OVER_PI / ra;
-    const double cq = c.w.cnq[(size_t)b * N + i];
-    eeq64_rhs(c, b, 0)[ci] =
-        -c.tab.eeq_chi[Z[i]] + c.tab.eeq_kcn[Z[i]] * (cq > 0.0 ? sqrt(cq) : 0.0);
-    eeq64_rhs(c, b, 1)[ci] = 1.0;
-    return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long pairs = (long long)n * (n - 1) / 2;
+  long long t = ((long long)blockIdx.x * 4 + warp) * 32 * rounds + lane;
+  if (t - lane >= pairs) return;
+  const size_t ab = (size_t)b * N;
+  const int *C = c.w.cidx + ab, *Z = c.w.z + ab;
+  const double *P = c.positions + 3 * ab;
+  double *L = eeq64_factor(c, b);
+  auto pair = [&](int i, int j, bool near) {
+    const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
+                 dz = P[3 * i + 2] - P[3 * j + 2];
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    double v = rsqrt(r2);
+    if (near) {
+      const double ra = c.tab.eeq_rad[Z[i]], rb = c.tab.eeq_rad[Z[j]];
+      v *= erf(r2 * v * rsqrt(ra * ra + rb * rb));
+      if (!(r2 > 0.0)) v = nan("");  // coincident atoms: erf(0) / 0
+    }
+    L[tri_index(C[i], C[j])] = v;
+  };
+  int queued = 0;
+  for (int k = 0; k < rounds; ++k, t += 32) {
+    int i = 0, j = 0;
+    bool near = false;
+    if (t < pairs) {
+      tri_entry(t, i, j);
+      ++i;  // j < i
+      if (Z[i] != 0 && Z[j] != 0) {
+        const float4 pi = c.w.pos32[ab + i], pj = c.w.pos32[ab + j];
+        const float ra = c.w.aux32[ab + i].z, rb = c.w.aux32[ab + j].z;
+        const float ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
+        near = !(ex * ex + ey * ey + ez * ez > 44.0f * (ra * ra + rb * rb));
+        if (!near) pair(i, j, false);
+      }
+    }
+    const unsigned m = __ballot_sync(FULL, near);
+    if (near) {
+      const int at = queued + __popc(m & ((1u << lane) - 1u));
+      s_i[warp][at] = i;
+      s_j[warp][at] = j;
+    }
+    queued += __popc(m);
+    __syncwarp();
+    if (queued >= 32) {
+      pair(s_i[warp][lane], s_j[warp][lane], true);
+      queued -= 32;
+      __syncwarp();
+      if (lane < queued) {
+        s_i[warp][lane] = s_i[warp][32 + lane];
+        s_j[warp][lane] = s_j[warp][32 + lane];
+      }
+      __syncwarp();
+    }
   }
-  const double *P = c.positions + (size_t)b * N * 3;
-  const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
-               dz = P[3 * i + 2] - P[3 * j + 2];
-  const double r2 = dx * dx + dy * dy + dz * dz;
-  const double rb = c.tab.eeq_rad[Z[j]];
-  const double ir = rsqrt(r2);
-  const double g2 = ra * ra + rb * rb;  // 1 / gamma^2
-  double v = ir;
-  if (r2 < 36.0 * g2) v *= erf(r2 * ir * rsqrt(g2));
-  *out = r2 > 0.0 ? v : nan("");  // coincident atoms: erf(0) / 0
+  if (lane < queued) pair(s_i[warp][lane], s_j[warp][lane], true);
+}
+
+namespace {
+
+// The smooth cap of atom a's EEQ coordination number (and its derivative), in
+// place of the raw count; returns the EEQ right-hand side -chi + kcn sqrt(cn).
+//   log(1 + e^m) - log(1 + e^(m - cn)) as log1p(expm1(cn) / (1 + e^(cn - m))):
+// the same function without the cancellation of the two logarithms, so that
+// nearly isolated atoms (cn << 1) keep a relative accuracy (the right-hand
+// side takes sqrt(cn), which magnifies absolute noise there).
+__device__ __forceinline__ double eeq64_cap(const Ctx &c, size_t a) {
+  const double cn = c.w.cnq[a];
+  const double f = 1.0 / (1.0 + exp(cn - c.par.cn_eeq_max));
+  const double cq = log1p(expm1(cn) * f);
+  c.w.cnq[a] = cq;
+  c.w.dcnq[a] = f;
+  const int z = c.w.z[a];
+  return -c.tab.eeq_chi[z] + c.tab.eeq_kcn[z] * (cq > 0.0 ? sqrt(cq) : 0.0);
+}
+
+__device__ __forceinline__ double eeq64_diagonal(const Ctx &c, int z) {
+  return c.tab.eeq_eta[z] + SQRT_2_OVER_PI / c.tab.eeq_rad[z];
+}
+
+}  // namespace
+
+// Capped EEQ coordination numbers of all atoms; with the EEQ, right-hand
+// sides and diagonal of its matrix (structures of the multi-CTA path).
+__global__ void __launch_bounds__(128) eeq64_rhs_kernel(Ctx c, bool eeq) {
+  const size_t a = (size_t)blockIdx.x * 128 + threadIdx.x;
+  if (a >= (size_t)c.B * c.N || c.w.z[a] == 0) return;
+  const double v = eeq64_cap(c, a);
+  if (!eeq) return;
+  const int b = (int)(a / c.N), k = c.w.cidx[a];
+  eeq64_rhs(c, b, 0)[k] = v;
+  eeq64_rhs(c, b, 1)[k] = 1.0;
+  eeq64_factor(c, b)[tri_index(k, k)] = eeq64_diagonal(c, c.w.z[a]);
 }
 
 // One structure per CTA in shared memory (N <= EEQ64_SMALL, at most 32 S rows
@@ -427,10 +480,15 @@ __global__ void __launch_bounds__(256) eeq64_small_kernel(Ctx c) {
   double *L = s_dyn + 2 * N;    // packed
   const int tri_m = m * (m + 1) / 2;
   double *G = eeq64_factor(c, b);
-  for (int t = threadIdx.x; t < tri_m; t += blockDim.x) L[t] = G[t];
-  for (int t = threadIdx.x; t < m; t += blockDim.x) {
-    v[t] = eeq64_rhs(c, b, 0)[t];
-    v[N + t] = eeq64_rhs(c, b, 1)[t];
+  for (int t = threadIdx.x; t < tri_m; t += blockDim.x) L[t] = G[t];  // (diagonal: below)
+  __syncthreads();
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const size_t a = (size_t)b * N + i;
+    const int k = c.w.cidx[a];
+    if (k < 0) continue;
+    v[k] = eeq64_cap(c, a);
+    v[N + k] = 1.0;
+    L[tri_index(k, k)] = eeq64_diagonal(c, c.w.z[a]);
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -442,7 +500,7 @@ __global__ void __launch_bounds__(256) eeq64_small_kernel(Ctx c) {
     constexpr int PARTS = EB / CW;
     for (int t = warp; t < T * (T + 1) / 2 * PARTS; t += nw) {
       int ti, tj;
-      eeq64_tile_of(t / PARTS, ti, tj);
+      tri_entry(t / PARTS, ti, tj);
       eeq64_update_tile<CW>(L, nullptr, v, v + N, ti, tj, t % PARTS, k0, t0, m);
     }
     __syncthreads();
@@ -480,7 +538,7 @@ __global__ void __launch_bounds__(128) eeq64_update_kernel(Ctx c, int k0) {
   const int t = blockIdx.x * 4 + warp;
   if (t >= T * (T + 1) / 2 * PARTS) return;
   int ti, tj;
-  eeq64_tile_of(t / PARTS, ti, tj);
+  tri_entry(t / PARTS, ti, tj);
   double *L = eeq64_factor(c, b);
   double *sj = s_j[warp];
 #pragma unroll
@@ -555,10 +613,19 @@ static void launch_small(const Ctx &c, cudaStream_t st) {
   eeq64_small_kernel<S><<<c.B, ES_THREADS, bytes, st>>>(c);
 }
 
+void launch_eeq64_cap(const Ctx &c, cudaStream_t st, bool eeq) {
+  const size_t total = (size_t)c.B * c.N;
+  eeq64_rhs_kernel<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(c, eeq);
+}
+
 void launch_eeq64(const Ctx &c, cudaStream_t st) {
   const int B = c.B, N = c.N;
-  const long long pairs = (long long)N * (N + 1) / 2;
-  eeq64_build_kernel<<<dim3((unsigned)((pairs + 127) / 128), B), 128, 0, st>>>(c);
+  const long long pairs = (long long)N * (N - 1) / 2;
+  // eight pairs per thread fill the queues of a batch, one spreads few pairs
+  const int rounds = B * pairs <= 4LL * 152 * 128 ? 1 : 8;
+  if (pairs > 0)
+    eeq64_build_kernel<<<dim3((unsigned)((pairs + 128 * rounds - 1) / (128 * rounds)), B), 128, 0,
+                         st>>>(c, rounds);
   if (N <= EEQ64_SMALL) {
     const int rows = EB + 2 + (N > EB ? N - EB : 0);  // beside the first diagonal block
     if (rows <= 64)
@@ -569,6 +636,7 @@ void launch_eeq64(const Ctx &c, cudaStream_t st) {
       launch_small<4>(c, st);
     return;
   }
+  launch_eeq64_cap(c, st, true);
   for (int k0 = 0; k0 < N; k0 += EB) {
     const int left = N > k0 + EB ? N - k0 - EB : 0, rows = EB + 2 + left;
     const int T = (left + 31) / 32;

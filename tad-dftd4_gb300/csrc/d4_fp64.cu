@@ -23,8 +23,8 @@ __global__ void __launch_bounds__(256) prep_kernel(Ctx c) { prep_structure(c, bl
 
 // ---------------------------------------------------------------- CN
 
-// D4 coordination number (EN weighted, cut_cn) and the EEQ coordination
-// number (plain count, cut_cn_eeq, smooth cap) in one pass over the pairs.
+// D4 coordination number (EN weighted, cut_cn) and the raw EEQ coordination
+// number (plain count, cut_cn_eeq) in one pass over the pairs.
 // A pair whose FP32 estimate of x exceeds 9 (1/2 erfc(x) < 1e-36) is dropped
 // before any FP64 work.  The surviving partners of the warp's
 // atom are queued in shared memory and evaluated 32 at a time, so the FP64
@@ -92,13 +92,7 @@ __global__ void __launch_bounds__(256) cn_kernel(Ctx c) {
   s_q4 = warp_sum(s_q4);
   if (lane == 0) {
     c.w.cn[ai] = s_d4;
-    const double m = c.par.cn_eeq_max;
-    // log(1 + e^m) - log(1 + e^(m - cn)) as log1p(expm1(cn) / (1 + e^(cn - m))):
-    // the same function without the cancellation of the two logarithms, so
-    // that nearly isolated atoms (cn << 1) keep a relative accuracy (the EEQ
-    // right-hand side takes sqrt(cn), which magnifies absolute noise there)
-    c.w.cnq[ai] = log1p(expm1(s_q4) / (1.0 + exp(s_q4 - m)));
-    c.w.dcnq[ai] = 1.0 / (1.0 + exp(s_q4 - m));
+    c.w.cnq[ai] = s_q4;  // capped with the EEQ right-hand sides (eeq64_cap)
     if (c.out.d_cn) c.out.d_cn[ai] = s_d4;
   }
 }
@@ -380,7 +374,7 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
         rmax = fmax(rmax, r2);
         if (j > i) {
           const double ir = 1.0 / r, u = ir * ir;
-          c.w.pr4[pij] = PairRec{r2, u, fmin(exp(alp3 * log(R0 * ir)), PAIR_T_MAX),
+          c.w.pr4[pij] = PairRec{r2, u, pair_t(alp3 * log(R0 * ir)),
                                  sqrt(c60) * (u * ir)};
           if (c.w.pr_da1) {
             c.w.pr_da1[pij] = sqq / R0;
@@ -878,7 +872,7 @@ __global__ void finish_kernel(Ctx c) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)c.B * c.N;
   if (t >= total) return;
-  if (!(c.flags & D4_FLAG_GRADIENT)) c.out.d_energy[t] += c.w.e3[t];
+  if (!(c.flags & D4_FLAG_GRADIENT) && !c.pair64) c.out.d_energy[t] += c.w.e3[t];
   if (c.out.d_charges) c.out.d_charges[t] = c.w.q[t];
   if (c.out.d_cn_eeq) c.out.d_cn_eeq[t] = c.w.cnq[t];
 }
@@ -946,7 +940,15 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   // that another factor of the triple makes up for.
   c.atm64 = c.weights == nullptr && !(c.flags & D4_FLAG_EXACT_C9) && c.par.alp >= 0.0 &&
             c.par.alp <= 100.0;
+  c.cut2_sq = cutoff_sq(c.par.cut_disp2);
   c.cut3_sq = cutoff_sq(c.par.cut_disp3);
+  // With the rational damping on top, the pair stages of d4_pair64.cu, which
+  // write the energies and parameter gradients to the outputs directly.
+  c.pair64 = c.atm64 && c.par.damping == D4_DAMP_RATIONAL;
+  if (c.pair64) {
+    c.w.e3 = c.out.d_energy;
+    if (c.flags & D4_FLAG_PARAM_GRAD) c.w.pgrad = c.out.d_param_grad;
+  }
   const dim3 atoms((N + 7) / 8, B);
   const bool grad = (c.flags & D4_FLAG_GRADIENT) != 0;
   const bool eeq = (c.flags & D4_FLAG_CHARGES_IN) == 0;
@@ -963,6 +965,7 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   } else {
     const size_t total = (size_t)B * N;
     charges_in_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(c);
+    if (c.out.d_cn_eeq) launch_eeq64_cap(c, st, false);
   }
   stage_end(ST_EEQ, st);
   stage_begin(ST_WEIGHTS, st);
@@ -970,7 +973,10 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   weights_kernel<<<units, 256, 0, st>>>(c);
   stage_end(ST_WEIGHTS, st);
   stage_begin(ST_PAIR_FWD, st);
-  pair_fwd_kernel<<<atoms, 256, 0, st>>>(c);
+  if (c.pair64)
+    launch_pair64(c, st);
+  else
+    pair_fwd_kernel<<<atoms, 256, 0, st>>>(c);
   stage_end(ST_PAIR_FWD, st);
   const dim3 tiles(((N + 7) / 8) * ((N + 31) / 32), B);
   stage_begin(ST_ATM, st);
@@ -989,7 +995,10 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   stage_end(ST_ATM, st);
   if (grad) {
     stage_begin(ST_PAIR_ATM_BWD, st);
-    pair_atm_bwd_kernel<<<atoms, 256, 0, st>>>(c);
+    if (c.pair64)
+      launch_pair64_bwd(c, st);
+    else
+      pair_atm_bwd_kernel<<<atoms, 256, 0, st>>>(c);
     stage_end(ST_PAIR_ATM_BWD, st);
     if (eeq) {
       stage_begin(ST_EEQ_ADJ, st);
@@ -997,13 +1006,17 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
       stage_end(ST_EEQ_ADJ, st);
     }
     stage_begin(ST_PAIR_CN_BWD, st);
-    pair_cn_bwd_kernel<<<atoms, 256, 0, st>>>(c);
+    if (c.pair64)
+      launch_pair64_forces(c, st);
+    else
+      pair_cn_bwd_kernel<<<atoms, 256, 0, st>>>(c);
     stage_end(ST_PAIR_CN_BWD, st);
   }
+  if (c.pair64 && !c.out.d_charges && !c.out.d_cn_eeq) return 0;
   stage_begin(ST_FINISH, st);
   const size_t total = (size_t)B * N;
   finish_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(c);
-  if (c.flags & D4_FLAG_PARAM_GRAD)
+  if ((c.flags & D4_FLAG_PARAM_GRAD) && !c.pair64)
     param_grad_finish_kernel<<<(D4_PARAM_GRAD_STRIDE * B + 255) / 256, 256, 0, st>>>(c);
   stage_end(ST_FINISH, st);
   return 0;
@@ -1069,16 +1082,12 @@ void launch_prep_memsets(const Ctx &c, cudaStream_t st) {
   cudaMemsetAsync(c.w.status, 0, sizeof(int), st);
   if (c.N > PREP_ZERO_MAX_N) {  // the pair accumulators of large structures: plain memsets
     const size_t bnn = (size_t)c.B * c.N * c.N;
-    if (c.w.pr_S) cudaMemsetAsync(c.w.pr_S, 0, 8 * bnn, st);
-    if (c.w.pr_P) cudaMemsetAsync(c.w.pr_P, 0, 8 * bnn, st);
+    if (c.w.pr_S && !c.pair64) cudaMemsetAsync(c.w.pr_S, 0, 8 * bnn, st);
+    if (c.w.pr_P && !c.pair64) cudaMemsetAsync(c.w.pr_P, 0, 8 * bnn, st);
     if (c.w.prS32) cudaMemsetAsync(c.w.prS32, 0, 4 * bnn, st);
     if (c.w.prP32) cudaMemsetAsync(c.w.prP32, 0, 4 * bnn, st);
   }
   if (c.w.atm_cnt) cudaMemsetAsync(c.w.atm_cnt, 0, 8 * 2 * (size_t)c.B, st);
-}
-
-void launch_cn(const Ctx &c, cudaStream_t st) {
-  cn_kernel<<<dim3((c.N + 7) / 8, c.B), 256, 0, st>>>(c);
 }
 
 void launch_weights(const Ctx &c, cudaStream_t st) {

@@ -45,7 +45,11 @@ void launch_pair_fwd_tc(const Ctx &c, cudaStream_t st);  // D4, precision form (
 bool pair_atm_bwd_tc_ok(const Ctx &c);
 void launch_pair_atm_bwd_tc(const Ctx &c, cudaStream_t st);
 void launch_atm_tiled64(const Ctx &c, cudaStream_t st);  // FP64 (d4_atm64.cu)
+void launch_pair64(const Ctx &c, cudaStream_t st);  // FP64 pair stages (d4_pair64.cu)
+void launch_pair64_bwd(const Ctx &c, cudaStream_t st);
+void launch_pair64_forces(const Ctx &c, cudaStream_t st);
 void launch_eeq64(const Ctx &c, cudaStream_t st);  // FP64 EEQ charges (d4_eeq64.cu)
+void launch_eeq64_cap(const Ctx &c, cudaStream_t st, bool eeq);
 void launch_eeq64_adjoint(const Ctx &c, cudaStream_t st);
 void launch_atm_exact(const Ctx &c, cudaStream_t st);  // exact C9, FP64 (d4_exact.cu)
 int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_out,
@@ -54,7 +58,6 @@ int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_
 // stages shared by the FP64 method and the precision form (d4_fp64.cu)
 void launch_prep(const Ctx &c, cudaStream_t st);
 void launch_prep_memsets(const Ctx &c, cudaStream_t st);  // the memsets of launch_prep
-void launch_cn(const Ctx &c, cudaStream_t st);
 void launch_weights(const Ctx &c, cudaStream_t st);
 void launch_charges_in(const Ctx &c, cudaStream_t st);
 void launch_finish(const Ctx &c, cudaStream_t st);

@@ -75,6 +75,7 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
     c.w.w32[a] = c.weights ? (float)c.weights[a] : 1.0f;
     c.w.slot[a] = s < c.S ? s : c.S - 1;
     c.w.e3[a] = 0.0;
+    if (c.pair64) c.w.rowmax[a] = 0.0;
     if (ok) {
       const double *p = c.positions + 3 * a;
       const double dx = p[0] - p0[0], dy = p[1] - p0[1], dz = p[2] - p0[2];
@@ -111,7 +112,7 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
   if (threadIdx.x < D4_PARAM_GRAD_STRIDE) c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + threadIdx.x] = 0.0;
   if (b == 0 && threadIdx.x < NFREQ)
     c.w.fw32[threadIdx.x] = (float)(THOPI * c.tab.freq_weights[threadIdx.x]);
-  if (c.w.pr_S && c.N <= PREP_ZERO_MAX_N) {
+  if (c.w.pr_S && c.N <= PREP_ZERO_MAX_N && !c.pair64) {
     for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
       const int i = t / n, j = t % n;
       const size_t o = ((size_t)b * N + i) * N + j;
