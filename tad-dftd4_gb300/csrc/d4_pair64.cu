@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(PT) pair64_kernel(Ctx c, int per, int parts) {
     if (c.w.z[ab + i] == 0 || c.w.z[ab + j] == 0) {  // padding: a pair of nothing
       c.w.pr4[up] = PairRec{0.0, 0.0, 0.0, 0.0};
       if (grad) c.w.pr_S[up] = c.w.pr_S[lo] = c.w.pr_P[up] = c.w.pr_P[lo] = 0.0;
+      if (pgrad) c.w.pr_da1[up] = c.w.pr_da1[lo] = c.w.pr_da2[up] = 0.0;
       continue;
     }
     const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
