@@ -1,0 +1,557 @@
+// Register-tiled ATM of the precision form: all triples i < j < k of
+// structures with unit energy weights (any size; padding atoms anywhere) that
+// do not run over neighbour triples.  Energy weights run the per-triple kernel
+// (d4_mixed.cu, atm_mixed_kernel).
+//
+// Bound by FP32 issue and latency (512 structures of 8..200 atoms: 0.70 of the
+// issue slots at 16 warps per SM, 409 million warp instructions, 476 us).  The
+// pair sums leave by 8-byte reductions at L2 instead of shared-memory atomics
+// (compare-and-swap loops), so no structure size is special and the sums of
+// the parameter gradients fit beside them; the (i, j) sums cross lanes through
+// shared memory (24 instructions per step; halving exchanges took 56).  Lanes
+// holding 4 middle x 2 outer atoms (fewer exchanges, more tasks) were slower,
+// 664 us, and so were direct loads instead of staged copies, 563.
+// Measured, ATM stage, against a tile kernel with the sums in shared memory
+// (N <= 234; no parameter gradients) and the per-triple kernel elsewhere: 512
+// structures of 8..200 atoms 572 -> 526 us; 256 of 20..150 with parameter
+// gradients 793 -> 258; 997 atoms 2115 -> 576; 1000 of 5..60, energies only,
+// 110 -> 55.
+#include "d4_atm.cuh"
+#include "d4_common.cuh"
+#include "d4_kernels.cuh"
+
+namespace d4 {
+
+namespace {
+
+constexpr int A3 = 8;             // middle atoms per lane, and outer atoms per task
+constexpr int A3_THREADS = 128;
+constexpr int A3_ROW = 10;        // row and group strides of the (i, j) sums in shared memory
+constexpr int A3_GROUP = 88;      // (float2; no bank conflicts)
+constexpr int A3_STAGES = 3;      // staged chunks of eight inner atoms per warp
+
+// Halving exchanges over the lane bits H, H/2, ... (STEPS of them): v[p]
+// for p < NV >> STEPS ends as the sum over the 2^STEPS lanes that differ in
+// those bits of the value with index p + (NV/2) bit(H) + (NV/4) bit(H/2) + ...
+template <int NV, int H, int STEPS>
+__device__ __forceinline__ void halving(float (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    const int m = NV >> (s + 1), h = H >> s;
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int q = 0; q < m; ++q) {
+      const float keep = up ? v[q + m] : v[q];
+      const float send = up ? v[q] : v[q + m];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
+}
+
+// 16 bytes of global memory to shared memory, or zeros.
+__device__ __forceinline__ void copy16(float4 *dst, const float4 *src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src),
+               "r"(ok ? 16 : 0) : "memory");
+}
+
+struct A3Pair {
+  const float4 *__restrict__ T;
+  const float4 *__restrict__ Tda;  // PGRAD: (dlogR0/da1, dlogR0/da2, log(R0/r), -)
+  float2 *SP;
+  double *e3;
+  double esc;  // factor of the energies added to e3 directly
+  float cut2, alp3h;
+  int N;
+};
+
+struct A3Pg {
+  float s9 = 0.f, alp = 0.f, a1 = 0.f, a2 = 0.f;
+  __device__ __forceinline__ void add(float w, const float4 &d) {
+    a1 = fmaf(w, d.x, a1);
+    a2 = fmaf(w, d.y, a2);
+    alp = fmaf(w, d.z, alp);
+  }
+};
+
+// One step: inner atom i of this lane's group against the eight middle atoms
+// j0 .. j0 + 7 and the lane's outer atom k.  rec: the staged records (i, j) and
+// (i, k) of the group's row, zeros where that is not a pair of the task (whose
+// triples then vanish).  MASK: an atom of the step has a pair beyond the
+// cutoff, so each triple takes its weight, (f_ij f_ik + f_ij f_jk + f_ik f_jk)
+// / 3 (f: pair inside; 1, 1/3 or 0).  Of a 1/3 triple (weighted energy e_w)
+// the atom of both inside pairs gets nothing and the other two e_w / 2 each
+// (the reference's attribution): the row sums give the latter e_w / 6 through
+// their inside pair and e_w / 3 through the outside one (atm_mirror_kernel),
+// the former 2 e_w / 6, which leaves here as -e_w / 3 (Eik, Ek, s_cj).
+template <bool GRAD, bool PGRAD, bool MASK>
+__device__ __forceinline__ void a3_step(const A3Pair &a, const float4 *rec, int j0,
+                                        unsigned jmask, int k, bool kok, int i, bool iok,
+                                        const float (&zjk)[A3], const float (&izjk)[A3],
+                                        const float (&ejk)[A3], const float (&qjk)[A3],
+                                        float (&Sjk)[A3], float (&Pjk)[A3], float (&Wjk)[A3],
+                                        float &Ek, float *s_cj, float2 *s_red, A3Pg &pg) {
+  const int l = threadIdx.x & 7;
+  const size_t row = (size_t)i * a.N;
+  const float4 pik = rec[A3 + l];
+  const float y = pik.x, iy38 = 0.375f * pik.y;
+  const bool fik = !MASK || y <= a.cut2;
+  float Sik = 0.f, Pik = 0.f, Wik = 0.f, Eik = 0.f, ei = 0.f;
+  float wij[PGRAD ? A3 : 1];
+  if (GRAD) __syncwarp();  // s_red: the last step's sums have been read
+#pragma unroll
+  for (int t = 0; t < A3; ++t) {
+    const float4 pij = rec[t];
+    const float x = pij.x, z = zjk[t];
+    bool fij = true, fjk = true;
+    int m = 3;
+    float qij = pij.w;
+    if (MASK) {
+      fij = x <= a.cut2;
+      fjk = z <= a.cut2;
+      m = (int)fij + (int)fik + (int)fjk;
+      if (GRAD) qij *= m == 3 ? 1.f : (m == 2 ? (1.0f / 3.0f) : 0.f);
+      else qij = m >= 2 ? qij : 0.f;
+    }
+    // atm_triple (d4_atm.cuh) with its sums in place
+    const float u = x - y, A = u + z, B = fmaf(2.0f, x, -A), C = z - u;
+    const float AB = A * B, h = pij.y * (iy38 * izjk[t]);
+    const float w = fmaf(AB * C, h, 1.0f);
+    const float fd = sfu_rcp(fmaf(pij.z, pik.z * ejk[t], 1.0f));
+    const float Q = qij * (pik.w * qjk[t]);
+    const float cq = Q * fd;
+    const float eu = cq * w;
+    if (!GRAD) {
+      // atom energies in units of eu / 3: all inside gives every atom 1, else
+      // nothing to the atom of both inside pairs and 1/2 to the other two
+      if (MASK && m == 2) {
+        const float e2 = 0.5f * eu;
+        ei += fjk ? e2 : 0.f;
+        Eik += fij ? e2 : 0.f;  // (of atom k)
+        Pjk[t] += fik ? e2 : 0.f;
+      } else {
+        ei += eu;
+        Eik += eu;
+        Pjk[t] += eu;
+      }
+      continue;
+    }
+    if (MASK) {  // energies of the 1/3 triples, for the atom of their inside pairs
+      const float e2 = m == 2 ? eu : 0.f;
+      ei += fjk ? 0.f : e2;
+      Ek += fij ? 0.f : e2;
+      if (!fik) s_cj[32 * t] += e2;
+    }
+    const float U = cq * h;
+    const float V = cq * fmaf(w, fmaf(-a.alp3h, fd, a.alp3h - 2.5f), 1.0f);
+    const float AC = A * C, BC = B * C;
+    const float Sg = AB + AC + BC;
+    Sik = fmaf(U, fmaf(-2.0f, BC, Sg), fmaf(V, pik.y, Sik));
+    Sjk[t] = fmaf(U, fmaf(-2.0f, AC, Sg), fmaf(V, izjk[t], Sjk[t]));
+    Pik += eu;
+    Pjk[t] += eu;
+    s_red[A3_ROW * t + l] = make_float2(fmaf(U, fmaf(-2.0f, AB, Sg), V * pij.y), eu);
+    if (PGRAD) {
+      const float wv = Q * w * fmaf(-fd, fd, fd);
+      Wik += wv;
+      Wjk[t] += wv;
+      wij[t] = wv;
+    }
+  }
+  if (!GRAD || MASK) {  // energies of atom i over the group's lanes
+    ei += __shfl_xor_sync(0xffffffffu, ei, 1);
+    ei += __shfl_xor_sync(0xffffffffu, ei, 2);
+    ei += __shfl_xor_sync(0xffffffffu, ei, 4);
+    if (iok && l == 0 && ei != 0.f) atomicAdd(&a.e3[i], (double)ei * a.esc);
+  }
+  if (!GRAD) {
+    Ek += Eik;
+  } else {
+    if (iok && kok && k > i) {
+      red2(&a.SP[row + k], Sik, Pik);
+      if (PGRAD) {
+        pg.s9 += Pik;
+        pg.add(Wik, a.Tda[row + k]);
+      }
+    }
+    // the (i, j) sums over the eight lanes: lane l adds up row l of s_red
+    __syncwarp();
+    float s = 0.f, e = 0.f;
+    const float4 *r4 = reinterpret_cast<const float4 *>(s_red + A3_ROW * l);
+#pragma unroll
+    for (int t = 0; t < A3 / 2; ++t) {
+      const float4 r = r4[t];
+      s += r.x + r.z;
+      e += r.y + r.w;
+    }
+    const bool ok = iok && j0 + l > i && ((jmask >> l) & 1u);
+    if (ok) red2(&a.SP[row + j0 + l], s, e);
+    if (PGRAD) {
+      float (&wv)[A3] = *reinterpret_cast<float(*)[A3]>(&wij[0]);
+      halving<A3, 4, 3>(wv);  // lane l: value l
+      if (ok) pg.add(wv[0], a.Tda[row + j0 + l]);
+    }
+  }
+}
+
+// Number of tasks of a structure of n atoms whose tasks cover 8 s inner atoms
+// each: tiles g (middle atoms 1 + 8 g ..) have NG - g chunks of outer atoms
+// and g / s + 1 ranges of inner atoms.
+__device__ __forceinline__ long long a3_tasks(int n, int s) {
+  const long long ng = n < 3 ? 0 : (n - 2 + A3 - 1) / A3;
+  long long t = 0;
+  for (long long m = ng; m > 0; m -= s) t += m * (m + 1) / 2;
+  return t;
+}
+
+}  // namespace
+
+// Running task counts of the structures in launch order (largest first),
+// [0] = 0 .. [B], and the task counter behind them; in the room of dEdcn,
+// which is written after the ATM.  One CTA.
+__global__ void __launch_bounds__(1024) atm32_plan_kernel(Ctx c, int s) {
+  __shared__ long long s_sum[32];
+  long long *first = reinterpret_cast<long long *>(c.w.dEdcn);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  long long base = 0;
+  for (int b0 = 0; b0 < c.B; b0 += 1024) {
+    long long v = 0;
+    if (b0 + tid < c.B) {
+      const int b = c.w.sorder[b0 + tid], n = c.w.n_eff[b];
+      v = atm_sparse_mode(c, b, n) ? 0 : a3_tasks(n, s);
+    }
+    long long x = v;  // inclusive scan over the CTA
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_sum[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      long long y = s_sum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long z = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) y += z;
+      }
+      s_sum[lane] = y;
+    }
+    __syncthreads();
+    x += base + (warp > 0 ? s_sum[warp - 1] : 0);
+    if (b0 + tid < c.B) first[b0 + tid + 1] = x;
+    base += s_sum[31];
+    __syncthreads();
+  }
+  if (tid == 0) {
+    first[0] = 0;
+    first[c.B + 1] = 0;  // the task counter
+  }
+}
+
+// A warp task is a tile of eight consecutive middle atoms j, eight outer atoms
+// k > j and 8 s consecutive inner atoms i < j: lane (q, l) takes k = kc + l,
+// keeps the eight (j, k) records and sums in registers and walks every fourth
+// i of the range (group q).  The (i, j) and (i, k) records are copied to shared
+// memory two chunks of eight i ahead.  Per i a lane evaluates eight triples
+// from one (i, k) record and eight broadcast (i, j) records, adds its (i, k)
+// sums with one reduction at L2, and the group's (i, j) sums change lanes
+// through shared memory for another.  Warps take tasks from a counter, largest structures
+// first.
+template <bool GRAD, bool PGRAD>
+__global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c, int s) {
+  __shared__ float s_c[A3_THREADS / 32][A3 * 32];
+  __shared__ float4 s_rec[A3_THREADS / 32][A3_STAGES][8 * 2 * A3];
+  __shared__ __align__(16) float2 s_sum[A3_THREADS / 32][4 * A3_GROUP];
+  const int lane = threadIdx.x & 31, q = lane >> 3;
+  const int N = c.N;
+  const long long *first = reinterpret_cast<const long long *>(c.w.dEdcn);
+  unsigned long long *next =
+      reinterpret_cast<unsigned long long *>(c.w.dEdcn) + c.B + 1;
+  const long long total = first[c.B];
+  auto take = [&]() {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(next, 1ull);
+    return (long long)__shfl_sync(0xffffffffu, t, 0);
+  };
+  int at = 0;  // position in launch order of the last task's structure
+  for (long long task = take(); task < total;) {
+    const long long following = take();  // on its way while this task runs
+    // the structure: tasks come in order, so search on from the last one
+    if (task >= first[at + 1]) {
+      int lo = at + 1, hi = c.B - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (task >= first[mid + 1])
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      at = lo;
+    }
+    const int b = c.w.sorder[at];
+    const int n = c.w.n_eff[b];
+    // tile, chunk and inner range
+    const int ng = (n - 2 + A3 - 1) / A3;
+    int t = (int)(task - first[at]);
+    int ip = 0, m = ng;
+    while (t >= m * (m + 1) / 2) {
+      t -= m * (m + 1) / 2;
+      m -= s;
+      ++ip;
+    }
+    int u, ch;
+    tri_entry(t, u, ch);
+    const int j0 = 1 + A3 * (ng - 1 - u), kc = j0 + 1 + A3 * ch;
+    const int jend = min(j0 + A3, n - 1);
+    const int ib0 = ip * A3 * s, iend = min(ib0 + A3 * s, jend - 1);
+    const size_t bN = (size_t)b * N;
+    A3Pair a;
+    a.T = c.w.ptf + bN * N;
+    a.Tda = PGRAD ? c.w.ptf_da + bN * N : nullptr;
+    a.SP = GRAD ? c.w.prSP32 + bN * N : nullptr;
+    a.e3 = c.w.e3 + bN;
+    a.esc = GRAD ? (PGRAD ? c.par.s9 : 1.0) * (-1.0 / 3.0) : c.par.s9 / 3.0;
+    a.cut2 = c.pf.cut3 * c.pf.cut3;
+    a.alp3h = 0.5f * c.pf.alp3;
+    a.N = N;
+    const bool gaps = c.w.n_real[b] != n;
+    const int *Z = c.w.z + bN;
+    const float *far2 = reinterpret_cast<const float *>(c.w.atm_rowmax) + bN;
+    const int k = kc + (lane & 7);
+    const bool kok = k < n && (!gaps || Z[k] != 0);
+    // s9 goes into the (j, k) records; parameter gradients and energies
+    // without gradient apply it at the end
+    const float s9q = (GRAD && !PGRAD) ? c.pf.s9 : 1.f;
+    float zjk[A3], izjk[A3], ejk[A3], qjk[A3], Sjk[A3], Pjk[A3], Wjk[A3];
+    unsigned jmask = 0u;
+    bool far = kok && far2[k] > a.cut2;
+#pragma unroll
+    for (int tt = 0; tt < A3; ++tt) {
+      const int jt = j0 + tt;
+      const bool jok = jt < jend && (!gaps || Z[jt] != 0);
+      jmask |= (unsigned)jok << tt;
+      float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kok && jok && jt < k) r = a.T[(size_t)jt * N + k];
+      zjk[tt] = r.x;
+      izjk[tt] = r.y;
+      ejk[tt] = 6.0f * r.z;  // prescaled for atm_triple<., true>
+      qjk[tt] = s9q * r.w;   // 0 where (j, k) is not a pair: every product vanishes
+      Sjk[tt] = Pjk[tt] = Wjk[tt] = 0.f;
+      far |= jok && far2[jt] > a.cut2;
+    }
+    const bool task_far = __any_sync(0xffffffffu, far);
+    for (int ib = ib0 + lane; ib < iend; ib += 32) far |= far2[ib] > a.cut2;
+    const bool any_far = __any_sync(0xffffffffu, far);
+    float Ek = 0.f;
+    float *cj = s_c[threadIdx.x >> 5] + lane;
+    if (GRAD && any_far) {
+#pragma unroll
+      for (int tt = 0; tt < A3; ++tt) cj[32 * tt] = 0.f;
+    }
+    A3Pg pg;
+    // records of eight inner atoms at a time: entry 16 r + t is (i, j0 + t),
+    // 16 r + 8 + t is (i, kc + t), i = first + r; copied two chunks ahead
+    float4(*stage)[8 * 2 * A3] = s_rec[threadIdx.x >> 5];
+    float2 *red = s_sum[threadIdx.x >> 5] + A3_GROUP * q;
+    auto fetch = [&](int first_i, int st) {
+      if (first_i < iend) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int slot = lane + 32 * e, r = slot >> 4, col = slot & 15;
+          const int i = first_i + r, x = col < A3 ? j0 + col : kc + col - A3;
+          const bool ok = i < iend && x > i && (col < A3 ? ((jmask >> col) & 1u) != 0u : x < n) &&
+                          (!gaps || (Z[i] != 0 && Z[x] != 0));
+          copy16(&stage[st][slot], a.T + (ok ? (size_t)i * N + x : 0), ok);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncwarp();  // every lane is done with the last task's records
+    fetch(ib0, 0);
+    fetch(ib0 + 8, 1);
+    int st = 0;
+    for (int ib = ib0; ib < iend; ib += 8) {
+      fetch(ib + 16, st >= A3_STAGES - 2 ? st - (A3_STAGES - 2) : st + 2);
+      asm volatile("cp.async.wait_group 2;" ::: "memory");
+      __syncwarp();
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        const int i = ib + 4 * half + q;
+        if (ib + 4 * half >= iend) break;
+        const bool iok = i < iend && (!gaps || Z[i] != 0);
+        const float4 *rec = stage[st] + 2 * A3 * (4 * half + q);
+        const bool mask =
+            task_far || (any_far && __any_sync(0xffffffffu, iok && far2[i] > a.cut2));
+        if (mask)
+          a3_step<GRAD, PGRAD, true>(a, rec, j0, jmask, k, kok, i, iok, zjk, izjk, ejk, qjk, Sjk,
+                                     Pjk, Wjk, Ek, cj, red, pg);
+        else
+          a3_step<GRAD, PGRAD, false>(a, rec, j0, jmask, k, kok, i, iok, zjk, izjk, ejk, qjk, Sjk,
+                                      Pjk, Wjk, Ek, cj, red, pg);
+      }
+      __syncwarp();
+      if (++st == A3_STAGES) st = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // the four groups' (j, k) sums: two exchanges leave group q the pairs of
+    // middle atoms 2 q and 2 q + 1
+    constexpr int K = GRAD ? (PGRAD ? 3 : 2) : 1, NV = K * A3;
+    float v[NV];
+#pragma unroll
+    for (int tt = 0; tt < A3; ++tt) {
+      if (GRAD) {
+        v[tt * K] = Sjk[tt];
+        v[tt * K + 1] = Pjk[tt];
+        if (PGRAD) v[tt * K + K - 1] = Wjk[tt];
+      } else {
+        v[tt] = Pjk[tt];
+      }
+    }
+    halving<NV, 16, 2>(v);
+    if (GRAD) {
+      if (any_far) {  // the 1/3 triples' common middle and outer atoms
+#pragma unroll
+        for (int tt = 0; tt < A3; ++tt) {
+          const float e = warp_sumf(cj[32 * tt]);
+          if (lane == 0 && e != 0.f) atomicAdd(&a.e3[j0 + tt], (double)e * a.esc);
+        }
+        Ek += __shfl_xor_sync(0xffffffffu, Ek, 8);
+        Ek += __shfl_xor_sync(0xffffffffu, Ek, 16);
+        if (q == 0 && kok && Ek != 0.f) atomicAdd(&a.e3[k], (double)Ek * a.esc);
+      }
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int jt = j0 + 2 * q + p;
+        if (kok && jt < k && ((jmask >> (2 * q + p)) & 1u)) {
+          red2(&a.SP[(size_t)jt * N + k], v[p * K], v[p * K + 1]);
+          if (PGRAD) pg.add(v[p * K + K - 1], a.Tda[(size_t)jt * N + k]);
+        }
+      }
+    } else {
+      // energies: of the middle atoms over the outer ones, of the outer atoms
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        float ej = v[p];
+        ej += __shfl_xor_sync(0xffffffffu, ej, 1);
+        ej += __shfl_xor_sync(0xffffffffu, ej, 2);
+        ej += __shfl_xor_sync(0xffffffffu, ej, 4);
+        if ((lane & 7) == 0 && ej != 0.f) atomicAdd(&a.e3[j0 + 2 * q + p], (double)ej * a.esc);
+      }
+      Ek += __shfl_xor_sync(0xffffffffu, Ek, 8);
+      Ek += __shfl_xor_sync(0xffffffffu, Ek, 16);
+      if (q == 0 && kok && Ek != 0.f) atomicAdd(&a.e3[k], (double)Ek * a.esc);
+    }
+    if (PGRAD) {
+      pg.s9 = warp_sumf(pg.s9);
+      pg.alp = warp_sumf(pg.alp);
+      pg.a1 = warp_sumf(pg.a1);
+      pg.a2 = warp_sumf(pg.a2);
+      if (lane == 0) {  // d fd / d(alp/3 sum log(R0/r)) = -fd (1 - fd)
+        double *o = c.w.pgrad + (size_t)b * D4_PARAM_GRAD_STRIDE;
+        const double s9 = c.par.s9, w = -s9 * (c.par.alp / 3.0);
+        atomicAdd(&o[3], w * (double)pg.a1);
+        atomicAdd(&o[4], w * (double)pg.a2);
+        atomicAdd(&o[5], (double)pg.s9);
+        atomicAdd(&o[6], -s9 * (1.0 / 3.0) * (double)pg.alp);
+      }
+    }
+    task = following;
+  }
+}
+
+// The lower half of the ATM pair sums from the upper one, 32 x 32 tiles through
+// shared memory.  After atm32_kernel also the atom energies from the row sums
+// (every triple reaches an atom through two of its pairs, a third of its
+// energy each; a pair beyond the cutoff counts twice, see a3_step) and, with
+// parameter gradients, the factor s9.
+__global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float s9) {
+  __shared__ float2 s_t[32][33];
+  __shared__ float s_e[32][33];
+  const int b = blockIdx.y, N = c.N, n = c.w.n_eff[b];
+  int ti, tj;  // rows ti, columns tj >= ti
+  tri_entry(blockIdx.x, tj, ti);
+  if (tj * 32 >= n) return;
+  if (atm_sparse_mode(c, b, n)) {  // atm_sparse_kernel did both itself
+    rows = false;
+    s9 = 1.f;
+  }
+  float2 *SP = c.w.prSP32 + (size_t)b * N * N;
+  double *e3 = c.w.e3 + (size_t)b * N;
+  const float cut2 = c.pf.cut3 * c.pf.cut3;
+  const float *far2 = reinterpret_cast<const float *>(c.w.atm_rowmax) + (size_t)b * N;
+  const float4 *T = c.w.ptf + (size_t)b * N * N;
+  const int *Z = c.w.z + (size_t)b * N;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int jr = tj * 32 + tx;
+  const bool jok = jr < n && Z[jr] != 0;
+  const bool far_j = rows && jok && far2[jr] > cut2;
+#pragma unroll
+  for (int r = ty; r < 32; r += 8) {
+    const int i = ti * 32 + r;
+    float2 v = make_float2(0.f, 0.f);
+    if (jok && jr > i && Z[i] != 0) {
+      v = SP[(size_t)i * N + jr];
+      if (s9 != 1.f) {
+        v.x *= s9;
+        v.y *= s9;
+        SP[(size_t)i * N + jr] = v;
+      }
+    }
+    float ev = v.y;
+    if (far_j && ev != 0.f && T[(size_t)i * N + jr].x > cut2) ev += ev;
+    s_t[r][tx] = v;
+    s_e[r][tx] = ev;
+    if (rows) {
+      const float e = warp_sumf(ev);
+      if (tx == 0 && e != 0.f) atomicAdd(&e3[i], (double)e * (1.0 / 6.0));
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = ty; r < 32; r += 8) {
+    const int i = tj * 32 + r, j = ti * 32 + tx;  // destination (i > j)
+    const float2 v = s_t[tx][r];
+    if (i < n && j < n && i > j) SP[(size_t)i * N + j] = v;
+    if (rows) {
+      const float e = warp_sumf(s_e[tx][r]);
+      if (tx == 0 && e != 0.f) atomicAdd(&e3[i], (double)e * (1.0 / 6.0));
+    }
+  }
+}
+
+void launch_atm_mirror(const Ctx &c, cudaStream_t st, bool rows, float s9) {
+  const unsigned T = (unsigned)(c.N + 31) / 32;
+  atm_mirror_kernel<<<dim3(T * (T + 1) / 2, c.B), 256, 0, st>>>(c, rows, s9);
+}
+
+void launch_atm32(const Ctx &c, cudaStream_t st) {
+  if (c.N < 3) return;
+  static int sms[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int &nsm = sms[dev & 63];
+  if (nsm == 0) {
+    int v = 0;
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    nsm = v > 0 ? v : 1;
+  }
+  const bool grad = (c.flags & D4_FLAG_GRADIENT) != 0;
+  const bool pgrad = (c.flags & D4_FLAG_PARAM_GRAD) != 0;
+  // inner atoms per task: 128 (finding, loading and flushing a task takes as
+  // long as 1.5 of its steps: 8-atom steps 16 against 4 per task 559 to 652 us
+  // for 512 structures of 8..200 atoms), fewer where a wave of warps would not
+  // get two such tasks each
+  const double triples = (double)c.B * c.N * c.N * c.N / 6.0;
+  int s = 16;
+  while (s > 1 && triples < 2.0 * 64 * 8 * s * 16.0 * nsm) s >>= 1;
+  atm32_plan_kernel<<<1, 1024, 0, st>>>(c, s);
+  const unsigned grid = (unsigned)((pgrad ? 3 : 4) * nsm);
+  if (pgrad)
+    atm32_kernel<true, true><<<grid, A3_THREADS, 0, st>>>(c, s);
+  else if (grad)
+    atm32_kernel<true, false><<<grid, A3_THREADS, 0, st>>>(c, s);
+  else
+    atm32_kernel<false, false><<<grid, A3_THREADS, 0, st>>>(c, s);
+}
+
+}  // namespace d4

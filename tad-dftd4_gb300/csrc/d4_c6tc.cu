@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) pair_fwd_tc_kernel(Ctx c) {
   const float4 li = real ? PL[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float wi = real ? c.w.w32[ai] : 0.f;
   float4 *Tt = c.w.ptf + bN * N;  // written transposed: T[j][i], coalesced over i
+  float2 *SPt = GRAD ? c.w.prSP32 + bN * N : nullptr;
   float4 *Tdat = PGRAD ? c.w.ptf_da + bN * N : nullptr;
   const float alp3 = c.pf.alp3;
   const bool tabled = c.r4r2_in == nullptr;
@@ -336,6 +337,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) pair_fwd_tc_kernel(Ctx c) {
         const float ir2 = __frcp_rn(r2);
         Tt[(size_t)j * N + i] = make_float4(r2, ir2, expf(alp3 * lnR0r),
                                             sqrtf(fmaxf(c60, 0.f)) * (ir * ir2));
+        if (GRAD && j < i) SPt[(size_t)j * N + i] = make_float2(0.f, 0.f);  // ATM sums
         r2mx = fmaxf(r2mx, r2);
         if (PGRAD)
           Tdat[(size_t)j * N + i] = make_float4(sqq * iR0, iR0, lnR0r, 0.f);
@@ -623,8 +625,7 @@ __global__ void __launch_bounds__(BW_THREADS) pair_atm_bwd_tc_kernel(Ctx c) {
   const float4 *PL = c.w.pos32lo + bN;
   const float4 px = real ? P[x] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 lx = real ? PL[x] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float *Sxy = c.w.prS32 + bN * N;
-  const float *Pxy = c.w.prP32 + bN * N;
+  const float2 *SPxy = c.w.prSP32 + bN * N;
   const float4 *T = c.w.ptf + bN * N;
   const float *A032 = c.w.A032 + bN * NFREQ;  // [w][N] of structure b
   constexpr uint32_t IDESC = tc::idesc_tf32(TC_M, 32);
@@ -657,8 +658,9 @@ __global__ void __launch_bounds__(BW_THREADS) pair_atm_bwd_tc_kernel(Ctx c) {
         const int q = q0 + u, y = y0 + q;
         const bool ok = real && y < n && y != x && S.zy[q] != 0;
         const size_t o = (size_t)(ok ? y : 0) * N + x;  // the pair arrays are symmetric
-        sv[u] = ok ? Sxy[o] : 0.f;
-        pv[u] = ok ? Pxy[o] : 0.f;
+        const float2 sp = ok ? SPxy[o] : make_float2(0.f, 0.f);
+        sv[u] = sp.x;
+        pv[u] = sp.y;
         cv[u] = ok ? T[o].w : 0.f;
       }
 #pragma unroll

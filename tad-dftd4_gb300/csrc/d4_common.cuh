@@ -139,8 +139,7 @@ struct Workspace {
   float *fw32;      // [23] (3/pi) times the Casimir-Polder weights, FP32
   // precision form only
   float4 *adj32;    // [B*N] (dE/dCN, dE/dCN_EEQ, q, EEQ adjoint w) in FP32
-  float *prS32;     // [B*N*N] ATM dE/d(r^2), FP32 accumulation
-  float *prP32;     // [B*N*N] ATM weighted triple energies, FP32 accumulation
+  float2 *prSP32;   // [B*N*N] ATM (dE/d(r^2), weighted triple energies), FP32 accumulation
   float *eeq_hi;    // [B*N*N] dense EEQ matrix of the real atoms (compact order) as the
   float *eeq_lo;    //         double-float hi + lo
   int *ridx;        // [B*N] atom index of the k-th real atom
@@ -269,8 +268,7 @@ inline Workspace carve_workspace(void *base, int B, int N, int S, uint32_t flags
     w.adj32 = (float4 *)take(16 * BN);
     w.sorder = (int *)take(sizeof(int) * (size_t)B);
     w.atm_rowmax = (unsigned *)take(sizeof(unsigned) * BN);
-    w.prS32 = grad ? (float *)take(4 * BNN) : nullptr;
-    w.prP32 = grad ? (float *)take(4 * BNN) : nullptr;
+    w.prSP32 = grad ? (float2 *)take(8 * BNN) : nullptr;
     w.eeq_hi = (float *)take(4 * BNN);
     w.eeq_lo = (float *)take(4 * BNN);
     w.ridx = (int *)take(sizeof(int) * BN);
@@ -341,7 +339,6 @@ struct Ctx {
   const double *rvdw_in;  // [B*N*N] pairwise radii of the zero / modified-zero damping
   int B, N, S;
   uint32_t flags;
-  int atm_tiled;  // the register-tiled ATM runs (set by the precision form's launcher)
   int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
   int pair64;     // the pair stages of d4_pair64.cu run (set by launch_fp64)
   double cut2_sq, cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp2, cut_disp3 (likewise)
@@ -353,19 +350,6 @@ struct Ctx {
 // ---------------------------------------------------------------- helpers
 
 constexpr int ATM_KMAX = 8;  // CTAs per structure at most (ATM kernels of the precision form)
-
-// CTAs of the register-tiled ATM for a structure of n atoms in a batch of B:
-// 1.2M triples per CTA for batches of 512 structures and more (measured on
-// batch512 at 512 threads: 600000 -> 12 % slower, 900000 -> 3 %, 1800000 ->
-// 13 %: fewer CTAs per structure mean fewer masked edge steps per task and
-// fewer flushes, until the largest structures' CTAs set the makespan), fewer
-// for smaller batches so that they still fill the GPU.
-__host__ __device__ inline int atm_tiled_ctas(int n, int B) {
-  const long long per = B >= 512 ? 1200000 : (B <= 64 ? 75000 : 1200000LL * B / 512);
-  const long long work = (long long)n * n * n / 6;
-  const int K = (int)((work + per - 1) / per);
-  return K < 1 ? 1 : (K > ATM_KMAX ? ATM_KMAX : K);
-}
 
 __device__ __forceinline__ double atom_r4r2(const Ctx &c, size_t a, int64_t z) {
   return c.r4r2_in ? c.r4r2_in[a] : c.tab.r4r2[z];

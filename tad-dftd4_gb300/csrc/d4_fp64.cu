@@ -291,6 +291,14 @@ __device__ __forceinline__ DampD3 damp_d3(int kind, int n, double r, double R0, 
   return d;
 }
 
+// The entries of the register-tiled ATM for a pair i < j with a padding atom.
+__device__ __forceinline__ void clear_pair64(const Ctx &c, int b, int i, int j) {
+  const size_t base = (size_t)b * c.N * c.N;
+  const size_t up = base + (size_t)i * c.N + j, lo = base + (size_t)j * c.N + i;
+  c.w.pr4[up] = PairRec{0.0, 0.0, 0.0, 0.0};
+  if (c.w.pr_da1) c.w.pr_da1[up] = c.w.pr_da1[lo] = c.w.pr_da2[up] = 0.0;
+}
+
 // Fused C6 + rational (BJ) two-body energy, its direct gradient and its C6
 // adjoint, and the per-pair tables the ATM kernel consumes.  One warp per
 // atom i; lanes over partners j.  C6 is never stored.
@@ -319,8 +327,7 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
       for (int s = 0; s < c.S; ++s) c.w.G[(ai * c.S + s) * NFREQ + lane] = 0.0;
     if (c.atm64 && i < n) {  // padding below the last atom: empty pair records
       if (lane == 0) c.w.rowmax[ai] = 0.0;
-      for (int j = i + 1 + lane; j < n; j += 32)
-        c.w.pr4[ai * N + j] = PairRec{0.0, 0.0, 0.0, 0.0};
+      for (int j = i + 1 + lane; j < n; j += 32) clear_pair64(c, b, i, j);
     }
     return;
   }
@@ -340,7 +347,7 @@ __global__ void __launch_bounds__(256) pair_fwd_kernel(Ctx c) {
   double rmax = 0.0;
   if (c.atm64)
     for (int j = i + 1 + lane; j < n; j += 32)
-      if (c.w.z[(size_t)b * N + j] == 0) c.w.pr4[ai * N + j] = PairRec{0.0, 0.0, 0.0, 0.0};
+      if (c.w.z[(size_t)b * N + j] == 0) clear_pair64(c, b, i, j);
   for (int s = 0; s < nslot; ++s) {
     if (lane < NFREQ) {
       const size_t o = (ai * c.S + s) * NFREQ + lane;
@@ -1084,8 +1091,6 @@ void launch_prep_memsets(const Ctx &c, cudaStream_t st) {
     const size_t bnn = (size_t)c.B * c.N * c.N;
     if (c.w.pr_S && !c.pair64) cudaMemsetAsync(c.w.pr_S, 0, 8 * bnn, st);
     if (c.w.pr_P && !c.pair64) cudaMemsetAsync(c.w.pr_P, 0, 8 * bnn, st);
-    if (c.w.prS32) cudaMemsetAsync(c.w.prS32, 0, 4 * bnn, st);
-    if (c.w.prP32) cudaMemsetAsync(c.w.prP32, 0, 4 * bnn, st);
   }
   if (c.w.atm_cnt) cudaMemsetAsync(c.w.atm_cnt, 0, 8 * 2 * (size_t)c.B, st);
 }

@@ -7,6 +7,7 @@
 // Shared stages (prep, finish) are the FP64 ones.
 #include <float.h>
 
+#include "d4_atm.cuh"
 #include "d4_common.cuh"
 #include "d4_chol.cuh"
 #include "d4_kernels.cuh"
@@ -489,6 +490,7 @@ __global__ void __launch_bounds__(256, 2) pair_fwd_mixed_kernel(Ctx c) {
       const float lnR0r = logf(R0 * ir) + R0d.lo / R0;
       const float ir2 = __frcp_rn(r2);
       T[j] = make_float4(r2, ir2, expf(c.pf.alp3 * lnR0r), sqrtf(c60) * (ir * ir2));
+      if (GRAD && i < j) c.w.prSP32[(size_t)ai * N + j] = make_float2(0.f, 0.f);  // ATM sums
       r2mx = fmaxf(r2mx, r2);
       if (PGRAD) Tda[j] = make_float4(sqq / R0, 1.0f / R0, lnR0r, 0.f);
       if (r <= cut2) {
@@ -617,22 +619,6 @@ __global__ void __launch_bounds__(1024) size_order_kernel(Ctx c) {
 
 // ---------------------------------------------------------------- ATM
 
-// 2^x on the special-function unit (ex2.approx.ftz: relative error about
-// 2^-22, results below 2^-126 flushed to 0); the ATM damping
-// 1 / (1 + 6 * 2^x) needs no more.
-__device__ __forceinline__ float sfu_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// 1 / x to the SFU's ~1 ulp (x >= 1 here: the ATM damping)
-__device__ __forceinline__ float sfu_rcp(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 __device__ __forceinline__ int tri_u(int j, int k, int n) {  // j < k, upper triangle
   return j * n - j * (j + 1) / 2 + (k - j - 1);
 }
@@ -652,7 +638,7 @@ __device__ __forceinline__ int atm_ctas(int n) {
 template <bool SMEM>
 struct AtmAcc {
   float *sS, *sP, *sE;  // shared (SMEM): upper triangle and atoms
-  float *gS, *gP;       // global pair blocks [N][N]
+  float2 *gSP;          // global pair block [N][N]
   double *gE;           // atom energies
   double escale;        // s9 / 6: energies arrive in units of (triple energy without s9) / 6
   int n, N;
@@ -662,8 +648,7 @@ struct AtmAcc {
       atomicAdd(&sS[t], S);
       atomicAdd(&sP[t], P);
     } else {
-      atomicAdd(&gS[(size_t)j * N + k], S);
-      atomicAdd(&gP[(size_t)j * N + k], P);
+      red2(&gSP[(size_t)j * N + k], S, P);
     }
   }
   __device__ __forceinline__ void energy(int x, float e) const {
@@ -681,7 +666,8 @@ struct AtmAcc {
     } else if (what == 2) {
       atomicAdd(&gE[j], (double)v * escale);
     } else {
-      atomicAdd((what == 1 ? gP : gS) + (size_t)j * N + k, v);
+      float2 *o = &gSP[(size_t)j * N + k];
+      atomicAdd(what == 1 ? &o->y : &o->x, v);
     }
   }
 };
@@ -702,56 +688,6 @@ __device__ __forceinline__ float warp_sum3_scatter(float a, float b, float c) {
   k += __shfl_xor_sync(0xffffffffu, k, 2);
   k += __shfl_xor_sync(0xffffffffu, k, 1);
   return k;
-}
-
-// ATM triple (i, j, k) of the precision form from its three pair records
-// (r^2, 1/r^2, (R0/r)^(alp/3), sqrt(C6(q=0)) / r^3) of the pairs ij, ik,
-// jk (x, y, z = their r^2).  With R = r_ij r_ik r_jk, the angular factor is
-// w / R^3, w = 1 + 3/8 (x - y + z)(x + y - z)(y + z - x) / R^2, and C9 / R^3
-// is the product Q of the records' fourth entries, so the energy without s9
-// is eu = Q fd w with fd = 1 / (1 + 6 prod (R0/r)^(alp/3)) (the reference's
-// damping, model/d4.py three-body term through damping/atm.py).  dex, dey,
-// dez: d eu / d(x, y, z); qwg = Q w fd (1 - fd), for the parameter gradients.
-struct AtmTri {
-  float eu, dex, dey, dez, qwg;
-};
-
-// EZ6: ez arrives multiplied by 6 (a caller that holds the (j, k) record for
-// many triples scales it once).
-template <bool GRAD, bool EZ6 = false>
-__device__ __forceinline__ AtmTri atm_triple(float x, float ix2, float ex, float qx, float y,
-                                             float iy2, float ey, float qy, float z, float iz2,
-                                             float ez, float qz, float alp3h) {
-  AtmTri r;
-  const float ir2 = ix2 * (iy2 * iz2);
-  const float h = 0.375f * ir2;
-  const float u = x - y;
-  const float A = u + z, Bv = (x + y) - z, Cv = z - u;
-  const float AB = A * Bv;
-  const float w = fmaf(AB * Cv, h, 1.0f);
-  // (rounding 1 + 6 prod drops its small values at distant triples alike;
-  // measured on 16000 atoms the three-body energy stays within 1e-8 Eh of
-  // the FP64 reference, and a Newton-corrected fd costs 3 % of the kernel)
-  const float fd = EZ6 ? sfu_rcp(fmaf(ex, ey * ez, 1.0f))
-                      : sfu_rcp(fmaf(6.0f, ex * (ey * ez), 1.0f));
-  const float Q = qx * (qy * qz);
-  const float cq = Q * fd;
-  r.eu = cq * w;
-  if (GRAD) {
-    // U = 3/8 C9 fd / R^5, V = C9 / (2 R^3) (fd (2 - 5 w) + w alp/3 fd (1 - fd))
-    //   = C9 fd / R^3 (1 + w (alp/6 (1 - fd) - 5/2))
-    const float U = cq * h;
-    const float V = cq * fmaf(w, fmaf(-alp3h, fd, alp3h - 2.5f), 1.0f);
-    const float AC = A * Cv, BC = Bv * Cv;
-    const float Sg = AB + AC + BC;
-    r.dex = fmaf(U, fmaf(-2.0f, AB, Sg), V * ix2);
-    r.dey = fmaf(U, fmaf(-2.0f, BC, Sg), V * iy2);
-    r.dez = fmaf(U, fmaf(-2.0f, AC, Sg), V * iz2);
-    r.qwg = Q * w * fmaf(-fd, fd, fd);
-  } else {
-    r.dex = r.dey = r.dez = r.qwg = 0.f;
-  }
-  return r;
 }
 
 // Constant inputs of the ATM triple loop of one structure.
@@ -874,20 +810,6 @@ __device__ __forceinline__ void atm_task(const AtmIn &in, const AtmAcc<SMEM> &ac
   if (kok && Ek != 0.f) acc.energy(k, Ek);
 }
 
-// Whether the ATM of structure b runs over neighbour triples (centre-atom
-// enumeration, atm_sparse_kernel) instead of all triples i < j < k: when
-// every centre's neighbour list fits the kernel's shared memory and the
-// centre-pair visits, sum_j deg_j (deg_j - 1) / 2, are fewer than half the
-// n (n - 1) (n - 2) / 6 triples.  Counts come from atm_nbr_kernel; only
-// structures of the global-accumulation path (N > 234) have them.
-__device__ __forceinline__ bool atm_sparse_mode(const Ctx &c, int b, int n) {
-  if (c.w.atm_cnt == nullptr) return false;
-  const unsigned long long visits = c.w.atm_cnt[2 * b], dmax = c.w.atm_cnt[2 * b + 1];
-  const unsigned long long nn = (unsigned long long)n;
-  const unsigned long long all = nn * (nn - 1) * (nn - 2) / 6;
-  return dmax <= (unsigned long long)ATM_SPARSE_DMAX && 2 * visits < all;
-}
-
 // CTAs per structure of the global-accumulation ATM (large structures):
 // about ATM_BIG_TRIPLES triples each, at most ATM_BIG_KMAX.
 constexpr long long ATM_BIG_TRIPLES = 250000;
@@ -898,8 +820,8 @@ __host__ __device__ inline int atm_ctas_big(int n) {
   return K < 1 ? 1 : (K > ATM_BIG_KMAX ? ATM_BIG_KMAX : (int)K);
 }
 
-// ATM energy and adjoint over triples i < j < k of one structure.  A warp
-// takes a task (j, 32 consecutive k > j) and loops over i: lanes hold the
+// The general ATM (energy weights; the common case is d4_atm32.cu): energy and
+// adjoint over triples i < j < k of one structure.  A warp takes a task (j, 32 consecutive k > j) and loops over i: lanes hold the
 // (j, k) pair record in registers and read the (i, j) (broadcast) and (i, k)
 // (coalesced 128-bit) records.  A pair record holds r^2, 1/r^2,
 // (R0/r)^(alp/3) and sqrt(C6(q=0)) / r^3, so the damping factor and
@@ -932,8 +854,7 @@ __global__ void __launch_bounds__(PGRAD ? ATM_THREADS_PGRAD : ATM_THREADS)
   acc.sS = s_acc;
   acc.sP = s_acc + P;
   acc.sE = s_acc + 2 * P;
-  acc.gS = GRAD ? c.w.prS32 + (size_t)b * N * N : nullptr;
-  acc.gP = GRAD ? c.w.prP32 + (size_t)b * N * N : nullptr;
+  acc.gSP = GRAD ? c.w.prSP32 + (size_t)b * N * N : nullptr;
   acc.gE = c.w.e3 + (size_t)b * N;
   acc.escale = c.par.s9 / 6.0;
   if (SMEM) {
@@ -999,11 +920,8 @@ __global__ void __launch_bounds__(PGRAD ? ATM_THREADS_PGRAD : ATM_THREADS)
         if (GRAD) {
           const float sv = acc.sS[t] * s9, pv = acc.sP[t] * s9;
           if (sv != 0.f || pv != 0.f) {
-            const size_t base = (size_t)b * N * N;
-            atomicAdd(&c.w.prS32[base + (size_t)j * N + k], sv);
-            atomicAdd(&c.w.prP32[base + (size_t)j * N + k], pv);
-            atomicAdd(&c.w.prS32[base + (size_t)k * N + j], sv);
-            atomicAdd(&c.w.prP32[base + (size_t)k * N + j], pv);
+            red2(&acc.gSP[(size_t)j * N + k], sv, pv);
+            red2(&acc.gSP[(size_t)k * N + j], sv, pv);
           }
         }
       }
@@ -1011,436 +929,6 @@ __global__ void __launch_bounds__(PGRAD ? ATM_THREADS_PGRAD : ATM_THREADS)
     for (int x = threadIdx.x; x < n; x += blockDim.x) {
       const float ev = acc.sE[x];
       if (ev != 0.f) atomicAdd(&c.w.e3[(size_t)b * N + x], (double)ev * acc.escale);
-    }
-  }
-}
-
-// ---------------------------------------------------------------- ATM, register-tiled
-
-// Shared-memory ATM (n <= 234) for structures with no padding below the
-// last real atom and unit atom weights.  A triple whose three pairs lie
-// inside the three-body cutoff has attribution weight 1, and the atom
-// energies follow from the pair sums, E_x = sum_y P(x, y) (each triple
-// reaches x through two pairs; the same total as the per-triple attribution
-// eu / 3 per atom).  Triples with a pair beyond the cutoff are only possible
-// where one of the three atoms is "far" (its largest pair r^2, recorded by
-// the pair kernels, exceeds the cutoff): steps and tasks that touch a far
-// atom run the masked variant, which weights each triple by
-// (f_ij f_ik + f_ij f_jk + f_ik f_jk) / 3 (f: pair inside the cutoff; 1, 1/3
-// or 0) and corrects the atom energies of the 1/3 triples, whose pair sums
-// alone do not give the reference attribution (in these units the atom of
-// both inside pairs gets 0, the other two eu each, while the pair sums give
-// each 2 eu / 3): -2 eu / 3 to the common atom and +eu / 3 to the other two,
-// accumulated beside the row sums.
-//
-// A warp task is a tile of AT_C = 8 consecutive middle atoms j (j0 .. j0+7)
-// and a chunk of 8 outer atoms k > j.  Lane (q, l) = (lane / 8, lane % 8)
-// takes k = kc + l and keeps the eight (j, k) pair records and their
-// dE/dr^2 and energy sums in registers; the four lane groups q walk the
-// inner atoms i < j in step (group q takes every fourth i of the CTA's
-// sequence).  Per i a lane reads the (i, k) record and the eight (i, j)
-// records (one row segment per group), evaluates eight triples, adds its
-// (i, k) sums to shared memory once, and the group reduce-scatters its
-// sixteen (i, j) sums over its eight lanes.  8 x 8 tiles keep the triples
-// evaluated outside i < j < k at ~22 % for sizes 8..200 (8 x 32: ~50 %).
-// The triple arithmetic is that of atm_task with unit atom weights.
-// Structures outside these conditions run atm_task in the same kernel.
-constexpr int AT_C = 8;             // middle atoms per task (and outer atoms per chunk)
-constexpr int AT_THREADS = 512;     // 16 warps at 128 registers, no spills (measured on
-                                    // batch512: 768 threads at 80 registers spill and run
-                                    // 13 % slower, 640 at 96 registers 10 % slower)
-constexpr int AT_TASKS_MAX = 900;   // tiles x chunks for n <= 237 (30 x 30)
-constexpr int AT_FAR_WORDS = 8;     // far-atom bits for n <= 256
-__host__ __device__ inline size_t atm_tiled_smem_bytes(int N) {
-  return atm_smem_bytes(N) + sizeof(int) * AT_TASKS_MAX;
-}
-
-// tri_u(i, x, n) = tri_row(i, n) + x for x > i
-__device__ __forceinline__ int tri_row(int i, int n) { return i * n - i * (i + 1) / 2 - i - 1; }
-
-// Halving exchanges over the lane bits H, H/2, ... (STEPS of them): v[p]
-// for p < NV >> STEPS ends as the sum over the 2^STEPS lanes that differ in
-// those bits of the value with index p + (NV/2) bit(H) + (NV/4) bit(H/2) + ...
-template <int NV, int H, int STEPS>
-__device__ __forceinline__ void lane_halving(float (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int s = 0; s < STEPS; ++s) {
-    const int m = NV >> (s + 1), h = H >> s;
-    const bool up = (lane & h) != 0;
-#pragma unroll
-    for (int q = 0; q < m; ++q) {
-      const float keep = up ? v[q + m] : v[q];
-      const float send = up ? v[q] : v[q + m];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, h);
-    }
-  }
-}
-
-// Per-structure state of the tiled ATM: shared accumulators, the far-atom
-// bit set, the cutoff and the damping exponent.
-struct AtTile {
-  const float4 *__restrict__ T;
-  float *sS, *sP, *sE;
-  const unsigned *far;  // bit x: atom x has a pair beyond the three-body cutoff
-  float cut2, alp3h;
-  int n, N;
-  __device__ __forceinline__ bool is_far(int x) const {
-    return x < n && ((far[x >> 5] >> (x & 31)) & 1u) != 0u;
-  }
-};
-
-// One step of a tile task: inner atom i of this lane's group.  GUARD: some
-// (i, j) of the step are not pairs (i >= j, j beyond the structure, i
-// beyond the task's range).  MASK: a far atom takes part, so each triple
-// carries its cutoff weight and the 1/3 triples their energy corrections.
-template <bool GRAD, bool GUARD, bool MASK>
-__device__ __forceinline__ void atm_tile_step(const AtTile &a, int j0, int jend, int k, bool kok,
-                                              int i, const float (&zjk)[AT_C],
-                                              const float (&izjk)[AT_C],
-                                              const float (&ejk)[AT_C],
-                                              const float (&qjk)[AT_C], float (&Sjk)[AT_C],
-                                              float (&Pjk)[AT_C]) {
-  const int l = threadIdx.x & 7;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool iok = !GUARD || i < jend - 1;
-  const float4 *Ti = a.T + (size_t)(iok ? i : 0) * a.N;
-  const bool lk = iok && kok && k > i;
-  const float4 pik = lk ? Ti[k] : zero4;
-  const bool fik = !MASK || pik.x <= a.cut2;
-  float Sik = 0.f, Pik = 0.f;
-  constexpr int NV = GRAD ? 2 * AT_C : AT_C;
-  float v[NV];  // (i, j) sums: dE/dr^2 (GRAD) then energies
-#pragma unroll
-  for (int t = 0; t < AT_C; ++t) {
-    float4 pij;
-    if (GUARD) {
-      const int jt = j0 + t;
-      const bool ok = iok && jt > i && jt < jend;
-      pij = ok ? Ti[ok ? jt : 0] : zero4;
-    } else {
-      pij = Ti[j0 + t];
-    }
-    bool fij = true, fjk = true;
-    float qij = pij.w;
-    if (MASK) {  // cutoff weight 1, 1/3 or 0, folded into C9 / R^3
-      fij = pij.x <= a.cut2;
-      fjk = zjk[t] <= a.cut2;
-      const int m = (int)fij + (int)fik + (int)fjk;
-      qij *= m == 3 ? 1.f : (m == 2 ? (1.0f / 3.0f) : 0.f);
-    }
-    const AtmTri tr = atm_triple<GRAD, true>(pij.x, pij.y, pij.z, qij, pik.x, pik.y, pik.z,
-                                             pik.w, zjk[t], izjk[t], ejk[t], qjk[t], a.alp3h);
-    if (MASK && !(fij & fik & fjk) && tr.eu != 0.f) {
-      // a 1/3 triple: -2 eu_w to the atom of both inside pairs, +eu_w to the others
-      atomicAdd(&a.sE[i], fjk ? tr.eu : -2.f * tr.eu);
-      atomicAdd(&a.sE[j0 + t], fik ? tr.eu : -2.f * tr.eu);
-      atomicAdd(&a.sE[k], fij ? tr.eu : -2.f * tr.eu);
-    }
-    Pik += tr.eu;
-    Pjk[t] += tr.eu;
-    if (GRAD) {
-      Sik += tr.dey;
-      Sjk[t] += tr.dez;
-      v[t] = tr.dex;
-      v[AT_C + t] = tr.eu;
-    } else {
-      v[t] = tr.eu;
-    }
-  }
-  const int rb = tri_row(i, a.n);
-  if (lk) {
-    if (GRAD) atomicAdd(&a.sS[rb + k], Sik);
-    atomicAdd(&a.sP[rb + k], Pik);
-  }
-  // group sums over the eight lanes: lane l keeps values NV/8 l .. NV/8 l + NV/8 - 1
-  lane_halving<NV, 4, 3>(v);
-#pragma unroll
-  for (int p = 0; p < NV / 8; ++p) {
-    const int idx = (NV / 8) * l + p;
-    const int jt = j0 + idx % AT_C;
-    if (!GUARD || (iok && jt > i && jt < jend && v[p] != 0.f))
-      atomicAdd(&((GRAD && idx < AT_C) ? a.sS : a.sP)[rb + jt], v[p]);
-  }
-}
-
-// The steps of a task over inner atoms i, i running from ib in steps of st4
-// while i < ilim: the masked step where a far atom takes part
-// (warp-uniform: any of the four groups' i), the plain one elsewhere.
-template <bool GRAD, bool GUARD>
-__device__ __forceinline__ int atm_tile_steps(const AtTile &a, bool any_far, bool task_far,
-                                              int ib, int ilim, int st4, int istep, int j0,
-                                              int jend, int k, bool kok,
-                                              const float (&zjk)[AT_C],
-                                              const float (&izjk)[AT_C],
-                                              const float (&ejk)[AT_C],
-                                              const float (&qjk)[AT_C], float (&Sjk)[AT_C],
-                                              float (&Pjk)[AT_C]) {
-  const int i_off = ((threadIdx.x & 31) >> 3) * istep;
-  for (; ib < ilim; ib += st4) {
-    const int i = ib + i_off;
-    if (any_far && (task_far || __any_sync(0xffffffffu, a.is_far(i))))
-      atm_tile_step<GRAD, GUARD, true>(a, j0, jend, k, kok, i, zjk, izjk, ejk, qjk, Sjk, Pjk);
-    else
-      atm_tile_step<GRAD, GUARD, false>(a, j0, jend, k, kok, i, zjk, izjk, ejk, qjk, Sjk, Pjk);
-  }
-  return ib;
-}
-
-template <bool GRAD>
-__device__ __forceinline__ void atm_tile_task(const AtTile &a, bool any_far, int j0, int kc,
-                                              int i0, int istep) {
-  const int lane = threadIdx.x & 31;
-  const int q = lane >> 3;
-  const int n = a.n;
-  const int k = kc + (lane & 7);
-  const bool kok = k < n;
-  float zjk[AT_C], izjk[AT_C], ejk[AT_C], qjk[AT_C], Sjk[AT_C], Pjk[AT_C];
-#pragma unroll
-  for (int t = 0; t < AT_C; ++t) {
-    const int jt = j0 + t;
-    const bool ok = kok && jt < k;  // then also jt <= n - 2
-    const float4 r = ok ? a.T[(size_t)jt * a.N + k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    zjk[t] = r.x;
-    izjk[t] = r.y;
-    ejk[t] = 6.0f * r.z;  // prescaled for atm_triple<., true>
-    qjk[t] = r.w;  // 0 also zeroes every product of a (j, k) that is not a pair
-    Sjk[t] = 0.f;
-    Pjk[t] = 0.f;
-  }
-  const int jend = min(j0 + AT_C, n - 1);  // middle atoms j0 .. jend - 1
-  // a far middle or outer atom makes every step of the task a masked one
-  bool task_far = false;
-  if (any_far) {
-    bool mine = a.is_far(k);
-#pragma unroll
-    for (int t = 0; t < AT_C; ++t) mine |= a.is_far(j0 + t);
-    task_far = __any_sync(0xffffffffu, mine);
-  }
-  // group q takes i = i0 + (4 s + q) istep, s = 0, 1, ...
-  const int st4 = 4 * istep;
-  int ib = i0;  // i of group 0 in this step
-  if (j0 + AT_C <= n - 1) {
-    // plain steps while all four groups' i are below j0: ib + 3 istep < j0
-    const int ilim = j0 - 3 * istep;
-    ib = atm_tile_steps<GRAD, false>(a, any_far, task_far, ib, ilim, st4, istep, j0, jend, k,
-                                     kok, zjk, izjk, ejk, qjk, Sjk, Pjk);
-  }
-  atm_tile_steps<GRAD, true>(a, any_far, task_far, ib, jend - 1, st4, istep, j0, jend, k, kok,
-                             zjk, izjk, ejk, qjk, Sjk, Pjk);
-  // (j, k) sums of the four groups: group q keeps values NV/4 q .. NV/4 q + NV/4 - 1
-  constexpr int NV = GRAD ? 2 * AT_C : AT_C;
-  float v[NV];
-#pragma unroll
-  for (int t = 0; t < AT_C; ++t) {
-    if (GRAD) {
-      v[t] = Sjk[t];
-      v[AT_C + t] = Pjk[t];
-    } else {
-      v[t] = Pjk[t];
-    }
-  }
-  lane_halving<NV, 16, 2>(v);
-#pragma unroll
-  for (int p = 0; p < NV / 4; ++p) {
-    const int idx = (NV / 4) * q + p;
-    const int jt = j0 + idx % AT_C;
-    if (kok && jt < k && v[p] != 0.f)
-      atomicAdd(&((GRAD && idx < AT_C) ? a.sS : a.sP)[tri_u(jt, k, n)], v[p]);
-  }
-}
-
-template <bool GRAD>
-__global__ void __launch_bounds__(AT_THREADS, 1) atm_tiled_kernel(Ctx c) {
-  extern __shared__ float s_acc[];
-  __shared__ int s_next, s_ntask, s_any_far;
-  __shared__ unsigned s_far[AT_FAR_WORDS];
-  const int b = c.w.sorder[blockIdx.y];
-  const int cta = blockIdx.x;
-  const int N = c.N;
-  const int n = c.w.n_eff[b];
-  if (n < 3) return;
-  const int K = atm_tiled_ctas(n, c.B);
-  if (cta >= K) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nwarps = blockDim.x >> 5;
-  const int P = n * (n - 1) / 2;
-  float *sS = s_acc, *sP = s_acc + P, *sE = s_acc + 2 * P;
-  int *s_task = reinterpret_cast<int *>(s_acc + 2 * P + n);
-  const float cut2 = c.pf.cut3 * c.pf.cut3;
-  const bool tiled = c.w.n_real[b] == n;
-  for (int t = threadIdx.x; t < 2 * P + n; t += blockDim.x) s_acc[t] = 0.f;
-  if (threadIdx.x == 0) s_any_far = 0;
-  if (warp < AT_FAR_WORDS) {  // far atoms: largest pair r^2 beyond the cutoff
-    const int x = 32 * warp + lane;
-    const bool far = x < n && __uint_as_float(c.w.atm_rowmax[(size_t)b * N + x]) > cut2;
-    const unsigned m = __ballot_sync(0xffffffffu, far);
-    if (lane == 0) s_far[warp] = m;
-  }
-  const int NT = (n - 2 + AT_C - 1) / AT_C;  // tiles of middle atoms 1 .. n - 2
-  if (tiled && threadIdx.x < NT) {
-    // task table: tiles from the last (longest i range) to the first, the
-    // chunks of eight outer atoms of each in order
-    auto nch = [&](int ti) { return (n - 1 - (1 + AT_C * ti) + AT_C - 1) / AT_C; };
-    const int ti = threadIdx.x;
-    int off = 0;
-    for (int u = NT - 1; u > ti; --u) off += nch(u);
-    for (int ch = 0; ch < nch(ti); ++ch) s_task[off + ch] = (ti << 8) | ch;
-    if (ti == 0) {
-      s_ntask = off + nch(0);
-      s_next = nwarps;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < AT_FAR_WORDS && s_far[threadIdx.x] != 0u) s_any_far = 1;
-  __syncthreads();
-  const float4 *T = c.w.ptf + (size_t)b * N * N;
-  if (tiled) {
-    AtTile a;
-    a.T = T;
-    a.sS = sS;
-    a.sP = sP;
-    a.sE = sE;
-    a.far = s_far;
-    a.cut2 = cut2;
-    a.alp3h = 0.5f * c.pf.alp3;
-    a.n = n;
-    a.N = N;
-    const bool any_far = s_any_far != 0;
-    const int ntask = s_ntask;
-    for (int task = warp; task < ntask;) {
-      const int e = s_task[task];
-      const int j0 = 1 + AT_C * (e >> 8);
-      atm_tile_task<GRAD>(a, any_far, j0, j0 + 1 + AT_C * (e & 255), cta, K);
-      int nx = 0;
-      if (lane == 0) nx = atomicAdd(&s_next, 1);
-      task = __shfl_sync(0xffffffffu, nx, 0);
-    }
-  } else {
-    AtmAcc<true> acc;
-    acc.n = n;
-    acc.N = N;
-    acc.sS = sS;
-    acc.sP = sP;
-    acc.sE = sE;
-    acc.gS = acc.gP = nullptr;
-    acc.gE = nullptr;
-    acc.escale = c.par.s9 / 6.0;
-    AtmIn in;
-    in.Zb = c.w.z + (size_t)b * N;
-    in.gaps = c.w.n_real[b] != n;
-    in.T = T;
-    in.Tda = nullptr;
-    in.W = c.w.w32 + (size_t)b * N;
-    in.cut2 = cut2;
-    in.alp3 = c.pf.alp3;
-    in.s9 = c.pf.s9;
-    in.s9m = 1.f;
-    in.weighted = false;
-    in.N = N;
-    AtmPg pg;
-    int j = 1, jbase = 0, nch = (n - 2 + 31) >> 5;
-    for (int t = warp;; t += nwarps) {
-      while (j < n - 1 && t >= jbase + nch) {
-        jbase += nch;
-        ++j;
-        nch = (n - 1 - j + 31) >> 5;
-      }
-      if (j >= n - 1) break;
-      if (in.gaps && in.Zb[j] == 0) continue;
-      atm_task<true, GRAD, false>(in, acc, n, j, j + 1 + 32 * (t - jbase), cta, K, pg);
-    }
-  }
-  __syncthreads();
-  // Flush: the upper half of the pair sums row by row (lanes over k > j),
-  // then the lower half row by row (lanes over j < k), both coalesced in
-  // global memory; a structure with one CTA stores, several CTAs add.  The
-  // tiled path's atom energies are the row sums of P: the part over y > x
-  // in the first pass (parked in sE), the part over y < x in the second.
-  const float s9 = c.pf.s9;
-  float *gS = GRAD ? c.w.prS32 + (size_t)b * N * N : nullptr;
-  float *gP = GRAD ? c.w.prP32 + (size_t)b * N * N : nullptr;
-  const bool solo = K == 1;
-  const double escale = c.par.s9 / 6.0;
-  for (int j = warp; j < n; j += nwarps) {
-    const int rb = tri_row(j, n);
-    float er = 0.f;
-    for (int k = j + 1 + lane; k < n; k += 32) {
-      const float pv = sP[rb + k];
-      er += pv;
-      if (GRAD) {
-        const float sv = sS[rb + k];
-        float *ds = gS + (size_t)j * N + k, *dp = gP + (size_t)j * N + k;
-        if (solo) {
-          *ds = sv * s9;
-          *dp = pv * s9;
-        } else if (sv != 0.f || pv != 0.f) {
-          atomicAdd(ds, sv * s9);
-          atomicAdd(dp, pv * s9);
-        }
-      }
-    }
-    if (tiled) {
-      er = warp_sumf(er);
-      if (lane == 0) sE[j] += er;  // beside the 1/3-triple corrections
-    }
-  }
-  __syncthreads();
-  for (int k = warp; k < n; k += nwarps) {
-    float ec = 0.f;
-    for (int j = lane; j < k; j += 32) {
-      const int t = tri_u(j, k, n);
-      const float pv = sP[t];
-      ec += pv;
-      if (GRAD) {
-        const float sv = sS[t];
-        float *ds = gS + (size_t)k * N + j, *dp = gP + (size_t)k * N + j;
-        if (solo) {
-          *ds = sv * s9;
-          *dp = pv * s9;
-        } else if (sv != 0.f || pv != 0.f) {
-          atomicAdd(ds, sv * s9);
-          atomicAdd(dp, pv * s9);
-        }
-      }
-    }
-    if (tiled) {
-      ec = warp_sumf(ec);
-      const float ev = ec + sE[k];  // E_k = sum_y P(k, y)
-      if (lane == 0 && ev != 0.f) atomicAdd(&c.w.e3[(size_t)b * N + k], (double)ev * escale);
-    }
-  }
-  if (!tiled)
-    for (int x = threadIdx.x; x < n; x += blockDim.x) {
-      const float ev = sE[x];
-      if (ev != 0.f) atomicAdd(&c.w.e3[(size_t)b * N + x], (double)ev * escale);
-    }
-}
-
-// Lower half of the ATM pair accumulators from the upper half (global
-// accumulation), 32 x 32 tiles through shared memory.
-__global__ void atm_mirror_kernel(Ctx c) {
-  __shared__ float sS[32][33], sP[32][33];
-  const int b = blockIdx.z;
-  const int N = c.N;
-  const int n = c.w.n_eff[b];
-  const int ti = blockIdx.y, tj = blockIdx.x;  // source tile (rows ti, columns tj), tj >= ti
-  if (tj < ti || ti * 32 >= n || tj * 32 >= n) return;
-  float *S = c.w.prS32 + (size_t)b * N * N;
-  float *P = c.w.prP32 + (size_t)b * N * N;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int r = ty; r < 32; r += blockDim.x >> 5) {
-    const int i = ti * 32 + r, j = tj * 32 + tx;
-    const bool ok = i < n && j < n && j > i;
-    sS[r][tx] = ok ? S[(size_t)i * N + j] : 0.f;
-    sP[r][tx] = ok ? P[(size_t)i * N + j] : 0.f;
-  }
-  __syncthreads();
-  for (int r = ty; r < 32; r += blockDim.x >> 5) {
-    const int i = tj * 32 + r, j = ti * 32 + tx;  // destination (i > j)
-    if (i < n && j < n && i > j) {
-      S[(size_t)i * N + j] = sS[tx][r];
-      P[(size_t)i * N + j] = sP[tx][r];
     }
   }
 }
@@ -1632,8 +1120,7 @@ __global__ void __launch_bounds__(ATM_SPARSE_THREADS, 2) atm_sparse_kernel(Ctx c
   const bool weighted = c.weights != nullptr;
   const float cut2 = c.pf.cut3 * c.pf.cut3, alp3 = c.pf.alp3, s9 = c.pf.s9;
   const float alp3h = 0.5f * alp3;
-  float *gS = GRAD ? c.w.prS32 + bN * N : nullptr;
-  float *gP = GRAD ? c.w.prP32 + bN * N : nullptr;
+  float2 *gSP = GRAD ? c.w.prSP32 + bN * N : nullptr;
   const float wj = W[j];
   float Ej = 0.f;
   AtmPg pg;
@@ -1675,8 +1162,7 @@ __global__ void __launch_bounds__(ATM_SPARSE_THREADS, 2) atm_sparse_kernel(Ctx c
         pe += we;
         atomicAdd(&s_S[e], ws * tr.dez);
         atomicAdd(&s_P[e], we);
-        atomicAdd(&gS[(size_t)i * N + k], ws * tr.dey);  // i < k: upper half
-        atomicAdd(&gP[(size_t)i * N + k], we);
+        red2(&gSP[(size_t)i * N + k], ws * tr.dey, we);  // i < k: upper half
         if (PGRAD) {
           const float4 daik = Tda[(size_t)i * N + k];
           const float4 dajk = Tda[(size_t)j * N + k];
@@ -1731,8 +1217,7 @@ __global__ void __launch_bounds__(ATM_SPARSE_THREADS, 2) atm_sparse_kernel(Ctx c
       const float sv = s_S[t], pv = s_P[t];
       if (sv != 0.f || pv != 0.f) {
         const size_t o = j < k ? (size_t)j * N + k : (size_t)k * N + j;  // upper half
-        atomicAdd(&gS[o], sv);
-        atomicAdd(&gP[o], pv);
+        red2(&gSP[o], sv, pv);
       }
     }
   }
@@ -1773,8 +1258,8 @@ __global__ void __launch_bounds__(256) pair_atm_bwd_mixed_kernel(Ctx c) {
       const size_t ay = (size_t)b * N + y;
       if (y == x || c.w.z[ay] == 0 || c.w.slot[ay] != s) continue;
       const size_t o = base + (size_t)x * N + y;
-      const float S = c.w.prS32[o];
-      const float Pv = c.w.prP32[o];
+      const float2 sp = c.w.prSP32[o];
+      const float S = sp.x, Pv = sp.y;
       const float3 d = pos_diff(px, lx, P[y], PL[y]);
       gx.add(2.0f * S * d.x);
       gy.add(2.0f * S * d.y);
@@ -2307,13 +1792,22 @@ static unsigned build_blocks(const Ctx &c) {
   return (unsigned)(tiles < want ? (tiles > 0 ? tiles : 1) : want);
 }
 
+// The per-triple ATM (energy weights): shared-memory accumulation, or global.
 template <bool SMEM, bool GRAD, bool PGRAD>
-static void launch_atm(const Ctx &c, cudaStream_t st, size_t smem) {
-  if (SMEM)
-    ensure_smem(atm_mixed_kernel<SMEM, GRAD, PGRAD>, (int)smem);
+static void launch_atm_general(const Ctx &c, cudaStream_t st) {
+  const size_t smem = SMEM ? atm_smem_bytes(c.N) : 0;
+  if (SMEM && GRAD)  // adds to both halves; the pair kernels clear the upper one
+    cudaMemsetAsync(c.w.prSP32, 0, 8 * (size_t)c.B * c.N * c.N, st);
+  if (SMEM) ensure_smem(atm_mixed_kernel<SMEM, GRAD, PGRAD>, (int)smem);
   const int threads = PGRAD ? ATM_THREADS_PGRAD : ATM_THREADS;
   const int K = SMEM ? ATM_KMAX : atm_ctas_big(c.N);
-  if (!SMEM) {
+  atm_mixed_kernel<SMEM, GRAD, PGRAD><<<dim3(K, c.B), threads, smem, st>>>(c);
+}
+
+template <bool GRAD, bool PGRAD>
+static void launch_atm(const Ctx &c, cudaStream_t st) {
+  const bool big = !atm_smem_fits(c.N);  // these can run over neighbour triples
+  if (big) {
     atm_nbr_kernel<<<dim3((c.N + 7) / 8, c.B), 256, 0, st>>>(c);
     int P = 1;
     while (P < c.N && P < ATM_ORDER_MAX) P <<= 1;
@@ -2321,16 +1815,20 @@ static void launch_atm(const Ctx &c, cudaStream_t st, size_t smem) {
     ensure_smem(atm_order_kernel, osm);
     atm_order_kernel<<<c.B, 1024, osm, st>>>(c);
   }
-  atm_mixed_kernel<SMEM, GRAD, PGRAD><<<dim3(K, c.B), threads, smem, st>>>(c);
-  if (!SMEM) {  // neighbour-triple variant; returns at once for dense structures
+  const bool tiled = c.weights == nullptr;
+  if (tiled)
+    launch_atm32(c, st);
+  else if (big)
+    launch_atm_general<false, GRAD, PGRAD>(c, st);
+  else
+    launch_atm_general<true, GRAD, PGRAD>(c, st);
+  if (big) {  // returns at once for dense structures
     const int sp = ATM_SPARSE_DMAX * (16 + 4 * 4);
     ensure_smem(atm_sparse_kernel<GRAD, PGRAD>, sp);
     atm_sparse_kernel<GRAD, PGRAD><<<dim3(c.N, c.B), ATM_SPARSE_THREADS, sp, st>>>(c);
   }
-  if (!SMEM && GRAD) {
-    const int T = (c.N + 31) / 32;
-    atm_mirror_kernel<<<dim3(T, T, c.B), 256, 0, st>>>(c);
-  }
+  if (GRAD && (big || tiled))
+    launch_atm_mirror(c, st, tiled, tiled && PGRAD ? c.pf.s9 : 1.f);
 }
 
 int launch_mixed(const Ctx &c_in, cudaStream_t st) {
@@ -2340,8 +1838,6 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   const bool grad = (c.flags & D4_FLAG_GRADIENT) != 0;
   const bool pgrad = (c.flags & D4_FLAG_PARAM_GRAD) != 0;
   const bool eeq = (c.flags & D4_FLAG_CHARGES_IN) == 0;
-  const bool atm_tiled = atm_smem_fits(N) && !pgrad && c.weights == nullptr;
-  c.atm_tiled = atm_tiled ? 1 : 0;  // (the prep skips zeroing what that kernel stores)
   timing_next_call();
   stage_begin(ST_PREP, st);
   launch_prep_memsets(c, st);
@@ -2388,34 +1884,13 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   else
     pair_fwd_mixed_kernel<false, false><<<atoms, 256, 0, st>>>(c);
   stage_end(ST_PAIR_FWD, st);
-  // ATM: shared-memory accumulation when the largest structure fits
-  const size_t atm_smem = atm_smem_bytes(N);
-  const bool atm_sm = atm_smem_fits(N);
   stage_begin(ST_ATM, st);
-  if (atm_tiled) {  // register-tiled triples
-    const size_t sm = atm_tiled_smem_bytes(N);
-    if (grad) {
-      ensure_smem(atm_tiled_kernel<true>, (int)sm);
-      atm_tiled_kernel<true><<<dim3(ATM_KMAX, B), AT_THREADS, sm, st>>>(c);
-    } else {
-      ensure_smem(atm_tiled_kernel<false>, (int)sm);
-      atm_tiled_kernel<false><<<dim3(ATM_KMAX, B), AT_THREADS, sm, st>>>(c);
-    }
-  } else if (atm_sm) {
-    if (pgrad)
-      launch_atm<true, true, true>(c, st, atm_smem);
-    else if (grad)
-      launch_atm<true, true, false>(c, st, atm_smem);
-    else
-      launch_atm<true, false, false>(c, st, atm_smem);
-  } else {
-    if (pgrad)
-      launch_atm<false, true, true>(c, st, 0);
-    else if (grad)
-      launch_atm<false, true, false>(c, st, 0);
-    else
-      launch_atm<false, false, false>(c, st, 0);
-  }
+  if (pgrad)
+    launch_atm<true, true>(c, st);
+  else if (grad)
+    launch_atm<true, false>(c, st);
+  else
+    launch_atm<false, false>(c, st);
   stage_end(ST_ATM, st);
   if (grad) {
     stage_begin(ST_PAIR_ATM_BWD, st);

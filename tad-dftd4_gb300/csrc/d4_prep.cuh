@@ -120,16 +120,6 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
       c.w.pr_P[o] = 0.0;
     }
   }
-  // (the register-tiled ATM stores every pair sum of a structure it covers
-  // with one CTA, so those structures need no zeroing)
-  if (c.w.prS32 && c.N <= PREP_ZERO_MAX_N && !(c.atm_tiled && atm_tiled_ctas(n, c.B) == 1)) {
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      const int i = t / n, j = t % n;
-      const size_t o = ((size_t)b * N + i) * N + j;
-      c.w.prS32[o] = 0.f;
-      c.w.prP32[o] = 0.f;
-    }
-  }
 }
 
 }  // namespace d4
