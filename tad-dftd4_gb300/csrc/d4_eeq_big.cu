@@ -1242,7 +1242,11 @@ void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint) {
       else eeq_big_residual_kernel<1, false><<<rg, 256, 0, st>>>(c, it);
     }
   }
-  eeq_big_finish_kernel<<<dim3(FIN_CTAS, B), 1024, 0, st>>>(c, adjoint ? 1 : 0);
+  launch_eeq_big_finish(c, st, adjoint);
+}
+
+void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint) {
+  eeq_big_finish_kernel<<<dim3(FIN_CTAS, c.B), 1024, 0, st>>>(c, adjoint ? 1 : 0);
 }
 
 }  // namespace d4

@@ -821,9 +821,10 @@ __host__ __device__ inline int atm_ctas_big(int n) {
 }
 
 // The general ATM (energy weights; the common case is d4_atm32.cu): energy and
-// adjoint over triples i < j < k of one structure.  A warp takes a task (j, 32 consecutive k > j) and loops over i: lanes hold the
-// (j, k) pair record in registers and read the (i, j) (broadcast) and (i, k)
-// (coalesced 128-bit) records.  A pair record holds r^2, 1/r^2,
+// adjoint over triples i < j < k of one structure.  A warp takes a task (j, 32
+// consecutive k > j) and loops over i: lanes hold the (j, k) pair record in
+// registers and read the (i, j) (broadcast) and (i, k) (coalesced 128-bit)
+// records.  A pair record holds r^2, 1/r^2,
 // (R0/r)^(alp/3) and sqrt(C6(q=0)) / r^3, so the damping factor and
 // C9 / (r_ij r_ik r_jk)^3 are two products each (atm_triple).
 //   SMEM (n <= 234): K <= 8 CTAs share a structure, interleaving i; per-pair
@@ -1865,7 +1866,7 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
       ensure_smem(eeq_mixed_kernel<true>, (int)(vec_bytes + pt_bytes + tri_bytes));
       eeq_mixed_kernel<true><<<B, EEQ_THREADS, vec_bytes + pt_bytes + tri_bytes, st>>>(c);
     } else {
-      launch_eeq_big(c, st, false);
+      if (!eeq_cg_takes(c) || !launch_eeq_cg(c, st, false)) launch_eeq_big(c, st, false);
     }
   } else {
     launch_charges_in(c, st);
@@ -1905,7 +1906,12 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
         ensure_smem(eeq_adjoint_mixed_kernel<true>, (int)(vec_bytes + tri_bytes));
         eeq_adjoint_mixed_kernel<true><<<B, EEQ_THREADS, vec_bytes + tri_bytes, st>>>(c);
       } else {
-        launch_eeq_big(c, st, true);
+        if (!eeq_cg_takes(c)) {
+          launch_eeq_big(c, st, true);
+        } else if (!launch_eeq_cg(c, st, true)) {  // the factor is needed after all
+          launch_eeq_big(c, st, false);
+          launch_eeq_big(c, st, true);
+        }
       }
       stage_end(ST_EEQ_ADJ, st);
     }
