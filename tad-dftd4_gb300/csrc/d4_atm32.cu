@@ -459,8 +459,205 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
   }
 }
 
+// ATM over the neighbour triples of structures in sparse mode (atm_sparse_mode;
+// unit energy weights): a CTA per centre atom j, whose neighbours L (ascending;
+// runs of consecutive atoms where the structure is in spatial order) form the
+// triples (i, j, k), i < k, with r_ij and r_jk inside the cutoff.  A triple
+// with r_ik outside has no other centre; one with all sides inside is taken at
+// its smallest atom (j < i).  A warp task is 32 neighbours k, a lane each with
+// its (j, k) record and sums in registers, against up to 64 neighbours i, four
+// rows' (i, k) records in flight: the (i, k) sums leave by one reduction at L2
+// each, the (i, j) sums of four rows cross lanes through shared memory.  Atom
+// energies come from the pair sums (atm_mirror_kernel); only the energies e_w
+// of the centre's 1/3 triples, which it gets nothing of, leave here as -e_w /
+// 3 (see a3_step).  Energies without gradient have no pair sums and add up
+// atom energies instead, in units of eu / 6.
+constexpr int SP_THREADS = 512, SP_ROWS = 4, SP_BLOCK = 64;
+constexpr int SP_ROW = 40;  // float2 stride of the row sums (8 lanes and 2 of padding each)
+
+// Tasks of the first m chunks: chunk ec has ec / 2 + 1 blocks of rows.
+__device__ __forceinline__ int sp_tasks(int m) { return (m + 1) * (m + 1) / 4; }
+
+template <bool GRAD, bool PGRAD>
+__global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
+  extern __shared__ float4 s_rec[];  // [ATM_SPARSE_DMAX] records (j, L[t])
+  float2 *s_SP = reinterpret_cast<float2 *>(s_rec + ATM_SPARSE_DMAX);  // their sums
+  int *s_L = reinterpret_cast<int *>(s_SP + ATM_SPARSE_DMAX);
+  float *s_W = reinterpret_cast<float *>(s_L + ATM_SPARSE_DMAX);  // PGRAD: damping sums
+  __shared__ __align__(16) float2 s_row[SP_THREADS / 32][SP_ROWS * SP_ROW];
+  __shared__ float s_red[SP_THREADS / 32];
+  __shared__ int s_next;
+  const int b = blockIdx.y, N = c.N, n = c.w.n_eff[b];
+  if ((int)blockIdx.x >= n || n < 3 || !atm_sparse_mode(c, b, n)) return;
+  const size_t bN = (size_t)b * N;
+  const int j = c.zsorted ? (int)blockIdx.x : c.w.atm_order[bN + blockIdx.x];
+  if (c.w.z[bN + j] == 0) return;
+  const int d = c.w.nbr_deg[bN + j];  // <= ATM_SPARSE_DMAX in sparse mode
+  if (d < 2) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float4 *T = c.w.ptf + bN * N;
+  const float4 *Tda = PGRAD ? c.w.ptf_da + bN * N : nullptr;
+  float2 *SP = GRAD ? c.w.prSP32 + bN * N : nullptr;
+  const int *L = c.w.nbr + (bN + j) * N;
+  for (int t = tid; t < d; t += SP_THREADS) {
+    const int k = L[t];
+    s_L[t] = k;
+    s_rec[t] = T[(size_t)j * N + k];
+    s_SP[t] = make_float2(0.f, 0.f);
+    if (PGRAD) s_W[t] = 0.f;
+  }
+  if (tid == 0) s_next = SP_THREADS / 32;
+  __syncthreads();
+  const float cut2 = c.pf.cut3 * c.pf.cut3, alp3h = 0.5f * c.pf.alp3;
+  const float s9 = (GRAD && !PGRAD) ? c.pf.s9 : 1.f;  // PGRAD, energies: at the end
+  float2 *rowbuf = s_row[warp];
+  float Cj = 0.f;
+  A3Pg pg;
+  const int nch = (d + 31) / 32, tasks = sp_tasks(nch);
+  for (int task = warp; task < tasks;) {
+    // chunk ec of 32 neighbours k has ec / 2 + 1 blocks of 64 rows i
+    int ec = (int)(2.0f * sqrtf((float)task));
+    while (sp_tasks(ec + 1) <= task) ++ec;
+    while (ec > 0 && sp_tasks(ec) > task) --ec;
+    const int a_beg = SP_BLOCK * (task - sp_tasks(ec));
+    const int a_end = min(min(a_beg + SP_BLOCK, d - 1), 32 * ec + 31);  // rows a < e
+    const int e = 32 * ec + lane;
+    const bool eok = e < d;
+    const int k = eok ? s_L[e] : 0;
+    const float4 pjk = eok ? s_rec[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float z = pjk.x, ejk = 6.0f * pjk.z, qjk = s9 * pjk.w;
+    float Sjk = 0.f, Pjk = 0.f, Wjk = 0.f;
+    for (int a0 = a_beg; a0 < a_end; a0 += SP_ROWS) {
+      float4 pik[SP_ROWS];
+#pragma unroll
+      for (int r = 0; r < SP_ROWS; ++r) {
+        const int a = a0 + r;
+        const bool ok = a < a_end && eok && e > a;
+        pik[r] = ok ? T[(size_t)s_L[ok ? a : 0] * N + k] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      float wij[PGRAD ? SP_ROWS : 1];
+#pragma unroll
+      for (int r = 0; r < SP_ROWS; ++r) {
+        const int a = a0 + r;
+        const int i = s_L[a < a_end ? a : 0];
+        const bool in = pik[r].x <= cut2;
+        const bool use = a < a_end && eok && e > a && (j < i || !in);
+        float2 out = make_float2(0.f, 0.f);
+        float wv = 0.f;
+        if (__any_sync(0xffffffffu, use)) {
+          // atm_triple (d4_atm.cuh) with its sums in place
+          const float4 pij = s_rec[a];
+          const float x = pij.x, y = pik[r].x;
+          const float u = x - y, A = u + z, B = fmaf(2.0f, x, -A), C = z - u;
+          const float AB = A * B, h = pij.y * (0.375f * pik[r].y * pjk.y);
+          const float w = fmaf(AB * C, h, 1.0f);
+          const float fd = sfu_rcp(fmaf(pij.z, pik[r].z * ejk, 1.0f));
+          float qij = use ? pij.w : 0.f;
+          if (GRAD && !in) qij *= 1.0f / 3.0f;
+          const float Q = qij * (pik[r].w * qjk);
+          const float cq = Q * fd, eu = cq * w;
+          if (GRAD) {
+            const float U = cq * h;
+            const float V = cq * fmaf(w, fmaf(-alp3h, fd, alp3h - 2.5f), 1.0f);
+            const float AC = A * C, BC = B * C;
+            const float Sg = AB + AC + BC;
+            out = make_float2(fmaf(U, fmaf(-2.0f, AB, Sg), V * pij.y), eu);
+            Sjk = fmaf(U, fmaf(-2.0f, AC, Sg), fmaf(V, pjk.y, Sjk));
+            Pjk += eu;
+            Cj += in ? 0.f : eu;
+            if (use)
+              red2(&SP[(size_t)i * N + k], fmaf(U, fmaf(-2.0f, BC, Sg), V * pik[r].y), eu);
+            if (PGRAD) {
+              wv = Q * w * fmaf(-fd, fd, fd);
+              Wjk += wv;
+              pg.s9 += eu;
+              if (use) pg.add(wv, Tda[(size_t)i * N + k]);
+            }
+          } else {
+            // all sides inside: a third to each atom; else half to i and to k
+            out.x = in ? 2.0f * eu : eu;
+            Pjk += out.x;
+            Cj += in ? 2.0f * eu : 0.f;
+          }
+        }
+        rowbuf[SP_ROW * r + lane + 2 * (lane >> 3)] = out;
+        if (PGRAD) wij[r] = wv;
+      }
+      __syncwarp();
+      // (i, j) sums: eight lanes per row, four entries each
+      {
+        const int r = lane >> 3, q = lane & 7;  // entries 4 q .. 4 q + 3
+        const float4 *p4 =
+            reinterpret_cast<const float4 *>(rowbuf + SP_ROW * r + 4 * q + 2 * (q >> 1));
+        const float4 v0 = p4[0], v1 = p4[1];
+        float sv = (v0.x + v0.z) + (v1.x + v1.z), ev = (v0.y + v0.w) + (v1.y + v1.w);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+          sv += __shfl_xor_sync(0xffffffffu, sv, o);
+          if (GRAD) ev += __shfl_xor_sync(0xffffffffu, ev, o);
+        }
+        if (q == 0 && a0 + r < a_end) {
+          if (sv != 0.f) atomicAdd(&s_SP[a0 + r].x, sv);
+          if (GRAD && ev != 0.f) atomicAdd(&s_SP[a0 + r].y, ev);
+        }
+      }
+      if (PGRAD) {
+#pragma unroll
+        for (int r = 0; r < SP_ROWS; ++r) {
+          const float wv = warp_sumf(wij[r]);
+          if (lane == 0 && wv != 0.f) atomicAdd(&s_W[a0 + r], wv);
+        }
+      }
+      __syncwarp();
+    }
+    if (eok) {
+      if (GRAD && Sjk != 0.f) atomicAdd(&s_SP[e].x, Sjk);
+      if (Pjk != 0.f) atomicAdd(GRAD ? &s_SP[e].y : &s_SP[e].x, Pjk);
+      if (PGRAD && Wjk != 0.f) atomicAdd(&s_W[e], Wjk);
+    }
+    int nx = 0;
+    if (lane == 0) nx = atomicAdd(&s_next, 1);
+    task = __shfl_sync(0xffffffffu, nx, 0);
+  }
+  Cj = warp_sumf(Cj);
+  if (lane == 0) s_red[warp] = Cj;
+  __syncthreads();
+  double *e3 = c.w.e3 + bN;
+  if (tid == 0) {
+    float t = 0.f;
+    for (int w = 0; w < SP_THREADS / 32; ++w) t += s_red[w];
+    const double f = GRAD ? (PGRAD ? c.par.s9 : 1.0) * (-1.0 / 3.0) : c.par.s9 / 6.0;
+    if (t != 0.f) atomicAdd(&e3[j], (double)t * f);
+  }
+  for (int t = tid; t < d; t += SP_THREADS) {
+    const int k = s_L[t];
+    const float2 v = s_SP[t];
+    if (GRAD) {
+      if (v.x != 0.f || v.y != 0.f)
+        red2(&SP[j < k ? (size_t)j * N + k : (size_t)k * N + j], v.x, v.y);
+      if (PGRAD) pg.add(s_W[t], Tda[(size_t)j * N + k]);
+    } else if (v.x != 0.f) {
+      atomicAdd(&e3[k], (double)v.x * (c.par.s9 / 6.0));
+    }
+  }
+  if (PGRAD) {  // d fd / d(alp/3 sum log(R0/r)) = -fd (1 - fd)
+    pg.s9 = warp_sumf(pg.s9);
+    pg.alp = warp_sumf(pg.alp);
+    pg.a1 = warp_sumf(pg.a1);
+    pg.a2 = warp_sumf(pg.a2);
+    if (lane == 0) {
+      double *o = c.w.pgrad + (size_t)b * D4_PARAM_GRAD_STRIDE;
+      const double s9d = c.par.s9, w = -s9d * (c.par.alp / 3.0);
+      atomicAdd(&o[3], w * (double)pg.a1);
+      atomicAdd(&o[4], w * (double)pg.a2);
+      atomicAdd(&o[5], (double)pg.s9);
+      atomicAdd(&o[6], -s9d * (1.0 / 3.0) * (double)pg.alp);
+    }
+  }
+}
+
 // The lower half of the ATM pair sums from the upper one, 32 x 32 tiles through
-// shared memory.  After atm32_kernel also the atom energies from the row sums
+// shared memory.  After the unit-weight kernels also the atom energies from the row sums
 // (every triple reaches an atom through two of its pairs, a third of its
 // energy each; a pair beyond the cutoff counts twice, see a3_step) and, with
 // parameter gradients, the factor s9.
@@ -471,10 +668,6 @@ __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float
   int ti, tj;  // rows ti, columns tj >= ti
   tri_entry(blockIdx.x, tj, ti);
   if (tj * 32 >= n) return;
-  if (atm_sparse_mode(c, b, n)) {  // atm_sparse_kernel did both itself
-    rows = false;
-    s9 = 1.f;
-  }
   float2 *SP = c.w.prSP32 + (size_t)b * N * N;
   double *e3 = c.w.e3 + (size_t)b * N;
   const float cut2 = c.pf.cut3 * c.pf.cut3;
@@ -522,6 +715,22 @@ __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float
 void launch_atm_mirror(const Ctx &c, cudaStream_t st, bool rows, float s9) {
   const unsigned T = (unsigned)(c.N + 31) / 32;
   atm_mirror_kernel<<<dim3(T * (T + 1) / 2, c.B), 256, 0, st>>>(c, rows, s9);
+}
+
+template <bool GRAD, bool PGRAD>
+static void launch_sparse32(const Ctx &c, cudaStream_t st) {
+  const int bytes = ATM_SPARSE_DMAX * (16 + 8 + 4 + (PGRAD ? 4 : 0));
+  ensure_smem(atm_sparse32_kernel<GRAD, PGRAD>, bytes);
+  atm_sparse32_kernel<GRAD, PGRAD><<<dim3(c.N, c.B), SP_THREADS, bytes, st>>>(c);
+}
+
+void launch_atm_sparse32(const Ctx &c, cudaStream_t st) {
+  if (c.flags & D4_FLAG_PARAM_GRAD)
+    launch_sparse32<true, true>(c, st);
+  else if (c.flags & D4_FLAG_GRADIENT)
+    launch_sparse32<true, false>(c, st);
+  else
+    launch_sparse32<false, false>(c, st);
 }
 
 void launch_atm32(const Ctx &c, cudaStream_t st) {

@@ -71,6 +71,10 @@ constexpr int ATM_SPARSE_DMAX = 2048;
 // Structures up to this size get their ATM centres in spatial (Z-) order
 // (one shared-memory sort per structure); larger ones keep index order.
 constexpr int ATM_ORDER_MAX = 16384;
+// The precision form takes structures of this size range in spatial order
+// throughout (d4_mixed.cu, zsort_kernel).
+constexpr int ZSORT_MIN = 1536;
+__host__ __device__ inline bool zsort_fits(int N) { return N >= ZSORT_MIN && N <= ATM_ORDER_MAX; }
 
 
 // One pair of the register-tiled FP64 ATM (d4_atm64.cu): everything a triple
@@ -179,6 +183,12 @@ struct Workspace {
   unsigned long long *atm_cnt;  // [B*2] (sum_j deg_j (deg_j - 1) / 2, max_j deg_j)
   int *atm_order;   // [B*N] atoms in Z-order of their positions (centre order of the
                     // neighbour-triple ATM)
+  // spatially sorted copies (precision form, zsort_fits(N)): perm[k] = input
+  // index of sorted atom k, then inputs and outputs in sorted order
+  int *zs_perm;       // [B*N]
+  int64_t *zs_num;    // [B*N]
+  double *zs_pos, *zs_q, *zs_r4, *zs_w;           // [B*N*3], [B*N] each
+  double *zs_e, *zs_g, *zs_oq, *zs_ocn, *zs_ocnq;  // [B*N], [B*N*3], [B*N] each
   int *sorder;      // [B] structures by decreasing n_eff (launch order of the
                     // per-structure kernels of the precision form)
   unsigned *atm_rowmax;  // [B*N] largest r^2 over the real pairs of each atom (FP32
@@ -305,6 +315,19 @@ inline Workspace carve_workspace(void *base, int B, int N, int S, uint32_t flags
       w.eeq_Y = (float *)take(4 * 2 * BN);
       w.eeq_Xd = (float *)take(4 * (size_t)B * eeq_nsb(N) * EEQ_SB * EEQ_SB);
     }
+    if (zsort_fits(N)) {
+      w.zs_perm = (int *)take(sizeof(int) * BN);
+      w.zs_num = (int64_t *)take(8 * BN);
+      w.zs_pos = (double *)take(24 * BN);
+      w.zs_q = (double *)take(8 * BN);
+      w.zs_r4 = (double *)take(8 * BN);
+      w.zs_w = (double *)take(8 * BN);
+      w.zs_e = (double *)take(8 * BN);
+      w.zs_g = (double *)take(24 * BN);
+      w.zs_oq = (double *)take(8 * BN);
+      w.zs_ocn = (double *)take(8 * BN);
+      w.zs_ocnq = (double *)take(8 * BN);
+    }
     if (!atm_smem_fits(N)) {
       w.nbr = (int *)take(sizeof(int) * BNN);
       w.nbr_deg = (int *)take(sizeof(int) * BN);
@@ -339,6 +362,7 @@ struct Ctx {
   const double *rvdw_in;  // [B*N*N] pairwise radii of the zero / modified-zero damping
   int B, N, S;
   uint32_t flags;
+  int zsorted;    // the atoms are in spatial order (set by launch_mixed)
   int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
   int pair64;     // the pair stages of d4_pair64.cu run (set by launch_fp64)
   double cut2_sq, cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp2, cut_disp3 (likewise)

@@ -49,6 +49,7 @@ bool pair_atm_bwd_tc_ok(const Ctx &c);
 void launch_pair_atm_bwd_tc(const Ctx &c, cudaStream_t st);
 void launch_atm_tiled64(const Ctx &c, cudaStream_t st);  // FP64 (d4_atm64.cu)
 void launch_atm32(const Ctx &c, cudaStream_t st);  // precision form (d4_atm32.cu)
+void launch_atm_sparse32(const Ctx &c, cudaStream_t st);
 void launch_atm_mirror(const Ctx &c, cudaStream_t st, bool rows, float s9);
 void launch_pair64(const Ctx &c, cudaStream_t st);  // FP64 pair stages (d4_pair64.cu)
 void launch_pair64_bwd(const Ctx &c, cudaStream_t st);

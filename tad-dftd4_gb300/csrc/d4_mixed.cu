@@ -974,12 +974,11 @@ __global__ void __launch_bounds__(256) atm_nbr_kernel(Ctx c) {
   }
 }
 
-// Centre order of the neighbour-triple ATM: the real atoms of a structure
-// sorted by the Z-order (Morton) code of their positions on a 1024^3 grid
-// over the structure's bounding box, so that CTAs running at the same time
-// work on nearby centres and share their neighbourhoods' pair records in L2.
-// One CTA per structure: bitonic sort of (code << 32 | atom) keys in shared
-// memory (padding last); n <= ATM_ORDER_MAX, else index order.
+// The atoms of structure b in Z-order: sorted by the Morton code of their
+// positions on a 1024^3 grid over the structure's bounding box, padding last.
+// One CTA of 1024 threads: bitonic sort of (code << 32 | atom) keys in shared
+// memory (n <= ATM_ORDER_MAX); s_key[t] & 0xFFFFFFFF is the t-th atom.
+// ``at(t)`` gives a position, ``real(t)`` whether atom t < n is one.
 __device__ __forceinline__ unsigned spread_bits10(unsigned v) {  // 10 bits -> every third bit
   v &= 0x3FFu;
   v = (v | (v << 16)) & 0x030000FFu;
@@ -989,24 +988,16 @@ __device__ __forceinline__ unsigned spread_bits10(unsigned v) {  // 10 bits -> e
   return v;
 }
 
-__global__ void __launch_bounds__(1024) atm_order_kernel(Ctx c) {
-  extern __shared__ unsigned long long s_key[];
+template <typename At, typename Real>
+__device__ __forceinline__ void morton_sort(unsigned long long *s_key, int n, At at, Real real) {
   __shared__ float s_lo[3][32], s_hi[3][32];
-  const int b = blockIdx.x;
-  const int N = c.N;
-  const int n = c.w.n_eff[b];
-  const size_t bN = (size_t)b * N;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (n > ATM_ORDER_MAX) {
-    for (int t = tid; t < n; t += blockDim.x) c.w.atm_order[bN + t] = t;
-    return;
-  }
   int P = 1;
   while (P < n) P <<= 1;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   for (int t = tid; t < n; t += blockDim.x) {
-    if (c.w.z[bN + t] == 0) continue;
-    const float4 p = c.w.pos32[bN + t];
+    if (!real(t)) continue;
+    const float3 p = at(t);
     const float v[3] = {p.x, p.y, p.z};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -1039,8 +1030,8 @@ __global__ void __launch_bounds__(1024) atm_order_kernel(Ctx c) {
   }
   for (int t = tid; t < P; t += blockDim.x) {
     unsigned code = 0xFFFFFFFFu;  // padding and beyond n: last
-    if (t < n && c.w.z[bN + t] != 0) {
-      const float4 p = c.w.pos32[bN + t];
+    if (t < n && real(t)) {
+      const float3 p = at(t);
       const float v[3] = {p.x, p.y, p.z};
       unsigned q[3];
 #pragma unroll
@@ -1069,7 +1060,70 @@ __global__ void __launch_bounds__(1024) atm_order_kernel(Ctx c) {
       __syncthreads();
     }
   }
-  for (int t = tid; t < n; t += blockDim.x) c.w.atm_order[bN + t] = (int)(s_key[t] & 0xFFFFFFFFu);
+}
+
+// Centre order of the neighbour-triple ATM where the atoms themselves are not
+// in spatial order: CTAs running at the same time then work on nearby centres
+// and share their neighbourhoods' pair records in L2.
+__global__ void __launch_bounds__(1024) atm_order_kernel(Ctx c) {
+  extern __shared__ unsigned long long s_key[];
+  const int b = blockIdx.x;
+  const int n = c.w.n_eff[b];
+  const size_t bN = (size_t)b * c.N;
+  if (n > ATM_ORDER_MAX) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) c.w.atm_order[bN + t] = t;
+    return;
+  }
+  morton_sort(
+      s_key, n,
+      [&](int t) {
+        const float4 p = c.w.pos32[bN + t];
+        return make_float3(p.x, p.y, p.z);
+      },
+      [&](int t) { return c.w.z[bN + t] != 0; });
+  for (int t = threadIdx.x; t < n; t += blockDim.x)
+    c.w.atm_order[bN + t] = (int)(s_key[t] & 0xFFFFFFFFu);
+}
+
+// Large structures run in spatial order from the start: their inputs are
+// gathered in Z-order and the outputs scattered back at the end.  Neighbour
+// lists then hold runs of consecutive atoms, so that the gathers and
+// reductions of the neighbour triples, which bound that kernel at the L1
+// (86 % of its wavefronts in index order), fall into shared sectors, and
+// lanes over partners agree on cutoffs.
+__global__ void __launch_bounds__(1024) zsort_kernel(Ctx c) {
+  extern __shared__ unsigned long long s_key[];
+  const int N = c.N;
+  const size_t bN = (size_t)blockIdx.x * N;
+  const double *P = c.positions + 3 * bN;
+  morton_sort(
+      s_key, N,
+      [&](int t) {
+        return make_float3((float)P[3 * t], (float)P[3 * t + 1], (float)P[3 * t + 2]);
+      },
+      [&](int t) { return c.numbers[bN + t] != 0; });
+  for (int t = threadIdx.x; t < N; t += blockDim.x) {
+    const int a = (int)(s_key[t] & 0xFFFFFFFFu);
+    c.w.zs_perm[bN + t] = a;
+    c.w.zs_num[bN + t] = c.numbers[bN + a];
+    for (int d = 0; d < 3; ++d) c.w.zs_pos[3 * (bN + t) + d] = P[3 * a + d];
+    if (c.charges_in) c.w.zs_q[bN + t] = c.charges_in[bN + a];
+    if (c.r4r2_in) c.w.zs_r4[bN + t] = c.r4r2_in[bN + a];
+    if (c.weights) c.w.zs_w[bN + t] = c.weights[bN + a];
+  }
+}
+
+// Outputs of sorted structures back in input order.
+__global__ void zsort_out_kernel(Ctx c, d4_outputs_t out) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)c.B * c.N) return;
+  const size_t a = t / c.N * c.N + c.w.zs_perm[t];
+  out.d_energy[a] = c.w.zs_e[t];
+  if (c.flags & D4_FLAG_GRADIENT)
+    for (int d = 0; d < 3; ++d) out.d_gradient[3 * a + d] = c.w.zs_g[3 * t + d];
+  if (out.d_charges) out.d_charges[a] = c.w.zs_oq[t];
+  if (out.d_cn) out.d_cn[a] = c.w.zs_ocn[t];
+  if (out.d_cn_eeq) out.d_cn_eeq[a] = c.w.zs_ocnq[t];
 }
 
 constexpr int ATM_SPARSE_THREADS = 512;
@@ -1099,7 +1153,7 @@ __global__ void __launch_bounds__(ATM_SPARSE_THREADS, 2) atm_sparse_kernel(Ctx c
   const int n = c.w.n_eff[b];
   if ((int)blockIdx.x >= n || n < 3 || !atm_sparse_mode(c, b, n)) return;
   const size_t bN = (size_t)b * N;
-  const int j = c.w.atm_order[bN + blockIdx.x];  // centres in spatial order
+  const int j = c.zsorted ? (int)blockIdx.x : c.w.atm_order[bN + blockIdx.x];  // in spatial order
   if (c.w.z[bN + j] == 0) return;
   const int d = c.w.nbr_deg[bN + j];  // <= ATM_SPARSE_DMAX in sparse mode
   if (d < 2) return;
@@ -1793,6 +1847,12 @@ static unsigned build_blocks(const Ctx &c) {
   return (unsigned)(tiles < want ? (tiles > 0 ? tiles : 1) : want);
 }
 
+static int morton_smem(int N) {
+  int P = 1;
+  while (P < N && P < ATM_ORDER_MAX) P <<= 1;
+  return 8 * P;
+}
+
 // The per-triple ATM (energy weights): shared-memory accumulation, or global.
 template <bool SMEM, bool GRAD, bool PGRAD>
 static void launch_atm_general(const Ctx &c, cudaStream_t st) {
@@ -1810,11 +1870,11 @@ static void launch_atm(const Ctx &c, cudaStream_t st) {
   const bool big = !atm_smem_fits(c.N);  // these can run over neighbour triples
   if (big) {
     atm_nbr_kernel<<<dim3((c.N + 7) / 8, c.B), 256, 0, st>>>(c);
-    int P = 1;
-    while (P < c.N && P < ATM_ORDER_MAX) P <<= 1;
-    const int osm = 8 * P;
-    ensure_smem(atm_order_kernel, osm);
-    atm_order_kernel<<<c.B, 1024, osm, st>>>(c);
+    if (!c.zsorted) {
+      const int osm = morton_smem(c.N);
+      ensure_smem(atm_order_kernel, osm);
+      atm_order_kernel<<<c.B, 1024, osm, st>>>(c);
+    }
   }
   const bool tiled = c.weights == nullptr;
   if (tiled)
@@ -1823,7 +1883,9 @@ static void launch_atm(const Ctx &c, cudaStream_t st) {
     launch_atm_general<false, GRAD, PGRAD>(c, st);
   else
     launch_atm_general<true, GRAD, PGRAD>(c, st);
-  if (big) {  // returns at once for dense structures
+  if (big && tiled) {  // (returns at once for dense structures)
+    launch_atm_sparse32(c, st);
+  } else if (big) {
     const int sp = ATM_SPARSE_DMAX * (16 + 4 * 4);
     ensure_smem(atm_sparse_kernel<GRAD, PGRAD>, sp);
     atm_sparse_kernel<GRAD, PGRAD><<<dim3(c.N, c.B), ATM_SPARSE_THREADS, sp, st>>>(c);
@@ -1842,6 +1904,22 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   timing_next_call();
   stage_begin(ST_PREP, st);
   launch_prep_memsets(c, st);
+  const d4_outputs_t out = c.out;
+  if (zsort_fits(N)) {
+    ensure_smem(zsort_kernel, morton_smem(N));
+    zsort_kernel<<<B, 1024, morton_smem(N), st>>>(c);
+    c.zsorted = 1;
+    c.numbers = c.w.zs_num;
+    c.positions = c.w.zs_pos;
+    if (c.charges_in) c.charges_in = c.w.zs_q;
+    if (c.r4r2_in) c.r4r2_in = c.w.zs_r4;
+    if (c.weights) c.weights = c.w.zs_w;
+    c.out.d_energy = c.w.zs_e;
+    if (out.d_gradient) c.out.d_gradient = c.w.zs_g;
+    if (out.d_charges) c.out.d_charges = c.w.zs_oq;
+    if (out.d_cn) c.out.d_cn = c.w.zs_ocn;
+    if (out.d_cn_eeq) c.out.d_cn_eeq = c.w.zs_ocnq;
+  }
   prep_tables_kernel<<<B + TABLES32_THREADS / 256, 256, 0, st>>>(c);
   {
     int P = 1;
@@ -1921,6 +1999,8 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   }
   stage_begin(ST_FINISH, st);
   launch_finish(c, st);
+  if (c.zsorted)
+    zsort_out_kernel<<<(unsigned)(((size_t)B * N + 255) / 256), 256, 0, st>>>(c, out);
   stage_end(ST_FINISH, st);
   return 0;
 }

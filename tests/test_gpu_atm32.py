@@ -82,3 +82,32 @@ def test_parameter_gradients_match_fp64(d4, sizes, width, cut3):
     assert np.abs(mixed[1] - plain[1]).max() <= F_TOL
     gm, gp = mixed[2][:, :7], plain[2][:, :7]
     assert np.abs(gm - gp).max() <= 1e-6 * max(1.0, np.abs(gp).max())
+
+
+@pytest.mark.parametrize("cut3", [12.0, 60.0])
+def test_spatial_order_and_neighbour_triples_match_fp64(d4, cut3):
+    """Structures that run in spatial order: every per-atom input and output
+    (r4r2 and energy weights in; energies, forces, charges, both CNs out) keeps
+    its atom; 12 Bohr takes the neighbour triples, 60 Bohr all triples."""
+    disp = import_module("tad-dftd4_gb300.disp")
+    batch = _batch((1536, 300), 1540)
+    dev = batch[1].device
+    g = torch.Generator().manual_seed(5)
+    real = (batch[0] != 0).cpu()
+    r4r2 = ((2.0 + 3.0 * torch.rand(real.shape, generator=g, dtype=torch.float64)) * real).to(dev)
+    weights = (torch.rand(real.shape, generator=g, dtype=torch.float64) * real).to(dev)
+    out = []
+    for precision in ("mixed", "fp64"):
+        runner, _, _ = disp._prepare(*batch, PARAM, "d4", None, r4r2, None, None,
+                                     d4.Cutoff(disp3=cut3), None, None, None, precision)
+        out.append((runner.run(batch[1], gradient=True, param_grad=True, charges_out=True,
+                               cn_out=True, cn_eeq_out=True),
+                    runner.run(batch[1], gradient=True, weights=weights)[1],
+                    runner.run(batch[1])[0]))
+    (mixed, mw, me), (plain, pw, pe) = out
+    for k, tol in ((0, E_TOL), (1, F_TOL), (3, 1e-7), (4, 1e-6), (5, 1e-6)):
+        assert (mixed[k] - plain[k]).abs().max().item() <= tol, k
+    assert (mw - pw).abs().max().item() <= F_TOL
+    assert (me - pe).abs().max().item() <= E_TOL
+    gm, gp = mixed[2][:, :7].cpu().numpy(), plain[2][:, :7].cpu().numpy()
+    assert np.abs(gm - gp).max() <= 1e-6 * max(1.0, np.abs(gp).max())
