@@ -122,6 +122,21 @@ def _value(v) -> float:
     return float(v)
 
 
+def _on_host(param: Param) -> Param:
+    """``param`` with its tensors as Python floats, read with one copy: a wait
+    for the device per parameter costs more than the rest of a call."""
+    keys = [k for k in PARAM_ORDER if isinstance(param.get(k), torch.Tensor)]
+    if not keys:
+        return param
+    with torch.no_grad():
+        tensors = [param[k].detach().reshape(()) for k in keys]
+        if len(tensors) == 1 or len({(t.dtype, t.device) for t in tensors}) > 1:
+            values = [_value(t) for t in tensors]
+        else:
+            values = torch.stack(tensors).tolist()
+    return {**param, **{k: float(v) for k, v in zip(keys, values)}}
+
+
 def _given(param: Param, key: str):
     """The call's value of ``key``: the parameter dict's entry, else the
     reference's call default (None when there is none)."""
@@ -138,6 +153,7 @@ def resolve(param: Param, damping: Damping | None = None) -> dict:
     (order 6, 8, then 10).
     """
     damping = damping if damping is not None else RationalDamping()
+    param = _on_host(param)
     has_t8 = _given(param, "s8") is not None or _given(param, "rs8") is not None
     has_s10 = param.get("s10") is not None
     orders = [6] + ([8] if has_t8 else []) + ([10] if "s10" in param and has_s10 else [])

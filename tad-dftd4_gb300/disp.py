@@ -88,8 +88,36 @@ def _drain_pending() -> None:
 
 def _as_tensor(x, device, dtype):
     if isinstance(x, torch.Tensor):
-        return x.to(device=device, dtype=dtype)
+        return x if x.dtype is dtype and x.device == device else x.to(device=device, dtype=dtype)
     return torch.tensor(x, device=device, dtype=dtype)
+
+
+# A tensor operation that changes nothing still costs 3 to 5 microseconds of
+# host time, and a call on a small structure is bound by the host (energy and
+# forces of 57 atoms: 227 us of kernels in 441 us, 394 us without them): these
+# skip such operations.
+def _plain(x: torch.Tensor, dtype) -> torch.Tensor:
+    """``x.detach().to(dtype).contiguous()`` for reading its data."""
+    if x.dtype is dtype and x.is_contiguous():
+        return x
+    return x.detach().to(dtype).contiguous()
+
+
+def _atoms(numbers: torch.Tensor, N: int, device) -> torch.Tensor:
+    """Atomic numbers as a contiguous (B, N) int64 tensor on ``device``."""
+    if (numbers.dim() == 2 and numbers.dtype is torch.int64 and numbers.is_contiguous()
+            and numbers.device == device):
+        return numbers
+    return numbers.reshape(-1, N).to(device=device, dtype=torch.int64).contiguous()
+
+
+def _structures(positions: torch.Tensor, N: int) -> torch.Tensor:
+    """Positions as (B, N, 3)."""
+    return positions if positions.dim() == 3 else positions.reshape(-1, N, 3)
+
+
+def _cast(x: torch.Tensor, dtype) -> torch.Tensor:
+    return x if x.dtype is dtype else x.to(dtype)
 
 
 def _resolve_model(model, numbers) -> BaseModel:
@@ -155,7 +183,7 @@ class Runner:
         lib = _lib.load()
         device = positions.device
         B, N = self.numbers.shape
-        pos = positions.detach().to(torch.float64).contiguous()
+        pos = _plain(positions, torch.float64)
         flags = 0
         if gradient or param_grad:
             flags |= _lib.FLAG_GRADIENT
@@ -192,20 +220,20 @@ class Runner:
         params, cfg = self.ct_params, self.ct_cfg
         batch = _lib.Batch(
             n_struct=B, n_pad=N, d_numbers=self.numbers.data_ptr(), d_positions=pos.data_ptr(),
-            d_charge=self.charge.data_ptr(),
-            d_charges_in=self.q.data_ptr() if self.q is not None else None,
-            d_r4r2_in=self.r4r2.data_ptr() if self.r4r2 is not None else None,
-            d_energy_weights=w.data_ptr() if w is not None else None,
-            d_rvdw_in=self.rvdw.data_ptr() if self.rvdw is not None else None,
-        )
-        outs = _lib.Outputs(
-            d_energy=energy.data_ptr(),
-            d_gradient=grad.data_ptr() if grad is not None else None,
-            d_charges=qout.data_ptr() if qout is not None else None,
-            d_cn=cnout.data_ptr() if cnout is not None else None,
-            d_param_grad=pgrad.data_ptr() if pgrad is not None else None,
-            d_cn_eeq=cnqout.data_ptr() if cnqout is not None else None,
-        )
+            d_charge=self.charge.data_ptr())
+        if self.q is not None:
+            batch.d_charges_in = self.q.data_ptr()
+        if self.r4r2 is not None:
+            batch.d_r4r2_in = self.r4r2.data_ptr()
+        if w is not None:
+            batch.d_energy_weights = w.data_ptr()
+        if self.rvdw is not None:
+            batch.d_rvdw_in = self.rvdw.data_ptr()
+        outs = _lib.Outputs(d_energy=energy.data_ptr())
+        for field, t in (("d_gradient", grad), ("d_charges", qout), ("d_cn", cnout),
+                         ("d_param_grad", pgrad), ("d_cn_eeq", cnqout)):
+            if t is not None:
+                setattr(outs, field, t.data_ptr())
         cur = torch.cuda.current_stream(device)
         stream = cur.cuda_stream
         with _on_device(device):
@@ -224,8 +252,11 @@ class Runner:
                                         f"({B} structures x {N} atoms)")
                 _PENDING.append(self.token)
             elif CHECK_STATUS:
-                _raise_status(lib.d4_read_status(work.data_ptr(), stream),
-                              "d4_dispersion (device status)")
+                word = torch.empty(1, dtype=torch.int32, pin_memory=True)
+                _lib.check(lib.d4_status_async(work.data_ptr(), word.data_ptr(), stream),
+                           "d4_status_async")
+                cur.synchronize()
+                _raise_status(int(word[0]), "d4_dispersion (device status)")
         if cn_eeq_out:
             return energy, grad, pgrad, qout, cnout, cnqout
         return energy, grad, pgrad, qout, cnout
@@ -257,19 +288,20 @@ class _D4Function(torch.autograd.Function):
                                                defer_status=need_pos or need_par)
         ctx.token = runner.token
         ctx.runner = runner
-        ctx.positions = positions.detach()
-        ctx.save_for_backward(grad if grad is not None else torch.empty(0),
-                              pgrad if pgrad is not None else torch.empty(0))
-        return energy.to(positions.dtype)
+        if grad is not None:
+            ctx.positions = positions.detach()
+            ctx.save_for_backward(*((grad,) if pgrad is None else (grad, pgrad)))
+        return _cast(energy, positions.dtype)
 
     @staticmethod
     def backward(ctx, go):
-        grad, pgrad = ctx.saved_tensors
+        grad, *rest = ctx.saved_tensors
+        pgrad = rest[0] if rest else None
         runner: Runner = ctx.runner
         if go.numel() > 0 and all(st == 0 for st in go.stride()):
             # one value broadcast over all atoms (the gradient of energy.sum()):
             # uniform, no need to look at it on the host
-            w0 = go.reshape(-1)[:1].to(torch.float64).reshape(1, 1)
+            w0 = _cast(go[:1, :1], torch.float64)
             uniform = True
         else:
             go = go.to(torch.float64)
@@ -284,7 +316,7 @@ class _D4Function(torch.autograd.Function):
             w0 = torch.ones_like(w0)
         gpos = gpar = None
         if ctx.needs_input_grad[0]:
-            gpos = (w0.unsqueeze(-1) * grad).to(ctx.positions.dtype)
+            gpos = _cast(w0.unsqueeze(-1) * grad, ctx.positions.dtype)
         if ctx.needs_input_grad[1]:
             gpar = (w0 * pgrad).sum(0)[: len(PARAM_ORDER)]
         # the forward's status word: read here if the forward has finished,
@@ -374,13 +406,13 @@ def _prepare(numbers, positions, charge, param, model, rcov, r4r2, rvdw, q, cuto
                 )
             shape = numbers.shape
             N = shape[-1]
-            nums = numbers.reshape(-1, N).to(device=device, dtype=torch.int64).contiguous()
+            nums = _atoms(numbers, N, device)
             B = nums.shape[0]
             charge = _as_tensor(charge, device, dtype)
             if charge.dim() == 0:
                 chg = charge.to(torch.float64).expand(B).contiguous()
             else:
-                chg = charge.reshape(-1).to(torch.float64).contiguous()
+                chg = _plain(charge if charge.dim() == 1 else charge.reshape(-1), torch.float64)
                 if chg.numel() != B:
                     raise ValueError(f"charge of shape {tuple(charge.shape)} for {B} structures")
             runner = Runner(numbers=nums, charge=chg, tables=tab, model=mdl, params=resolved,
@@ -426,12 +458,12 @@ def _prepare(numbers, positions, charge, param, model, rcov, r4r2, rvdw, q, cuto
 
     shape = numbers.shape
     N = shape[-1]
-    nums = numbers.reshape(-1, N).to(device=device, dtype=torch.int64).contiguous()
+    nums = _atoms(numbers, N, device)
     B = nums.shape[0]
     if charge.dim() == 0:
         chg = charge.to(torch.float64).expand(B).contiguous()
     else:
-        chg = charge.reshape(-1).to(torch.float64).contiguous()
+        chg = _plain(charge if charge.dim() == 1 else charge.reshape(-1), torch.float64)
         if chg.numel() != B:
             raise ValueError(f"charge of shape {tuple(charge.shape)} for {B} structures")
     tab = _tables.device_tables(device, mdl.ref_charges, mdl.ga, mdl.gc)
@@ -461,14 +493,18 @@ def _prepare(numbers, positions, charge, param, model, rcov, r4r2, rvdw, q, cuto
         n_slots=n_slots, mixed=precision == "mixed", rvdw=rv, exact_c9=exact_c9,
     )
     if any(isinstance(param.get(k), torch.Tensor) for k in PARAM_ORDER):
-        pvec = []
-        for key in PARAM_ORDER:
-            v = param.get(key)
-            if isinstance(v, torch.Tensor):
-                pvec.append(v.reshape(()).to(device=device, dtype=torch.float64))
-            else:
-                pvec.append(torch.tensor(resolved[key], dtype=torch.float64, device=device))
-        pvec = torch.stack(pvec)
+        # a vector for autograd only (the values are ``resolved``): the tensors
+        # in their slots, a cached zero elsewhere
+        given = [param.get(k) for k in PARAM_ORDER]
+        kinds = {(t.dtype, t.device) for t in given if isinstance(t, torch.Tensor)}
+        to = (torch.float64, device) if len(kinds) > 1 else kinds.pop()
+        zero = _PVEC.get(to)
+        if zero is None:
+            zero = _PVEC[to] = torch.zeros((), dtype=to[0], device=to[1])
+        pvec = torch.stack([zero if not isinstance(t, torch.Tensor) else
+                            t.reshape(()) if (t.dtype, t.device) == to else
+                            t.reshape(()).to(device=to[1], dtype=to[0]) for t in given])
+        pvec = pvec.to(device=device, dtype=torch.float64)
     else:  # plain numbers: a cached constant vector (no copy per call)
         key = (device, tuple(float(resolved[k]) for k in PARAM_ORDER))
         pvec = _PVEC.get(key)
@@ -528,9 +564,8 @@ def _evaluate(numbers, positions, charge, param, *, model, rcov, r4r2, rvdw, q, 
     runner, pvec, shape = _prepare(numbers, positions, charge, param, model, rcov, r4r2,
                                    rvdw, q, cutoff, cn_function, counting_function,
                                    damping_function, precision, exact_c9)
-    pos = positions.reshape(-1, shape[-1], 3)
-    energy = _D4Function.apply(pos, pvec, runner)
-    return energy.reshape(shape)
+    energy = _D4Function.apply(_structures(positions, shape[-1]), pvec, runner)
+    return energy if energy.shape == shape else energy.reshape(shape)
 
 
 def dispersion_energy_gradient(numbers, positions, charge, param, **kw):
@@ -547,10 +582,9 @@ def dispersion_energy_gradient(numbers, positions, charge, param, **kw):
                                 kw.pop("precision", None), kw.pop("exact_c9", False))
     if kw:
         raise TypeError(f"unexpected arguments {sorted(kw)}")
-    pos = positions.reshape(-1, shape[-1], 3)
-    energy, grad, _, _, _ = runner.run(pos, gradient=True)
-    return (energy.reshape(shape).to(positions.dtype),
-            grad.reshape(*shape, 3).to(positions.dtype))
+    energy, grad, _, _, _ = runner.run(_structures(positions, shape[-1]), gradient=True)
+    return (_cast(energy.reshape(shape), positions.dtype),
+            _cast(grad.reshape(*shape, 3), positions.dtype))
 
 
 def _fd_hessian(grad_fn, numbers: torch.Tensor, positions: torch.Tensor,
