@@ -21,7 +21,9 @@
 // Bound by the barrier and the L2 round trips of the exchange.
 //
 // Measured, charges / adjoint, against the factorisation (d4_eeq_big.cu):
-// 997 atoms 1099 / 184 -> 251 / 186 us; the rule below has other sizes.
+// 997 atoms 1099 / 184 -> 223 / 167 us; the rule below has other sizes.  Of an
+// iteration's 8200 cycles there, 2700 go to the barrier, 1450 to the product,
+// 1480 to reading the exchanged rows and 2500 to the updates and reductions.
 #include "d4_common.cuh"
 #include "d4_kernels.cuh"
 
@@ -29,8 +31,12 @@ namespace d4 {
 
 namespace {
 
-constexpr int CG_THREADS = 512;
-constexpr int CG_WARPS = CG_THREADS / 32;
+// Threads per CTA: reductions and barriers cost per warp, the product of many
+// rows wants more of them.  256 against 512 threads, charges / adjoint in us by
+// rows per CTA: 8 (1 x 300) 139 / 102 and 148 / 109, 8 (1 x 997) 223 / 167 and
+// 251 / 186, 11 (4 x 400) 173 / 125 and 174 / 123, 14 (1 x 2000) 404 / 329 and
+// 392 / 302, 57 (16 x 512) 293 / 227 and 266 / 192.
+constexpr int CG_FEW = 256, CG_MANY = 512, CG_FEW_ROWS = 10;
 constexpr float CG_TOL = 1e-10f;     // max |b - A x|
 constexpr float CG_GAIN = 1e-12f;    // of (r, r / diag) per FP32 solve
 constexpr int CG_OUTER = 16;         // refinements at most
@@ -50,7 +56,7 @@ __device__ __forceinline__ unsigned *cg_counter(const Ctx &c, int b) {
 }
 
 struct CgSmem {
-  float red[2][CG_WARPS][4];
+  __align__(16) float red[2][4][CG_MANY / 32];  // [turn][value][warp]
   int dead;
 };
 
@@ -73,9 +79,10 @@ __device__ bool cg_barrier(unsigned *counter, unsigned target, CgSmem &sm, int *
   return sm.dead == 0;
 }
 
-// Sums (or maxima from index NS on) of V values over the CTA, the same in all
-// threads.  The buffers alternate, so one synchronisation is enough.
-template <int V, int NS>
+// Sums (or maxima from index NS on) of V values over the NT threads of the CTA,
+// the same in all threads.  The buffers alternate, so one synchronisation is
+// enough.
+template <int NT, int V, int NS>
 __device__ __forceinline__ void cg_reduce(float (&v)[V], CgSmem &sm, int &turn) {
 #pragma unroll
   for (int q = 0; q < V; ++q) v[q] = q < NS ? warp_sumf(v[q]) : warp_maxf(v[q]);
@@ -83,14 +90,18 @@ __device__ __forceinline__ void cg_reduce(float (&v)[V], CgSmem &sm, int &turn) 
   turn ^= 1;
   if ((threadIdx.x & 31) == 0)
 #pragma unroll
-    for (int q = 0; q < V; ++q) sm.red[turn][warp][q] = v[q];
+    for (int q = 0; q < V; ++q) sm.red[turn][q][warp] = v[q];
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < V; ++q) {
-    float a = sm.red[turn][0][q];
+    const float4 *r = reinterpret_cast<const float4 *>(sm.red[turn][q]);
+    float a = 0.f;  // (the maxima are of absolute values)
 #pragma unroll
-    for (int w = 1; w < CG_WARPS; ++w)
-      a = q < NS ? a + sm.red[turn][w][q] : fmaxf(a, sm.red[turn][w][q]);
+    for (int w = 0; w < NT / 128; ++w) {
+      const float4 x = r[w];
+      a = q < NS ? a + ((x.x + x.y) + (x.z + x.w))
+                 : fmaxf(a, fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)));
+    }
     v[q] = a;
   }
 }
@@ -146,8 +157,8 @@ __global__ void cg_rhs_kernel(Ctx c, int adjoint) {
 
 // X = A^-1 B for NR right-hand sides of every structure.  ROWS: a CTA's rows
 // of the matrix in shared memory.
-template <int NR, bool ROWS>
-__global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int groups) {
+template <int NT, int NR, bool ROWS>
+__global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups) {
   extern __shared__ __align__(16) float s_dyn[];
   __shared__ CgSmem sm;
   const int N = c.N;
@@ -174,16 +185,16 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
     int par = 0;
     float res = 0.f;
     __syncthreads();  // the last structure's shared memory is free
-    for (int k = tid; k < ms; k += CG_THREADS) {
+    for (int k = tid; k < ms; k += NT) {
       dinv[k] = k < m ? 1.0f / Hi[(size_t)k * N + k] : 0.f;
 #pragma unroll
       for (int q = 0; q < NR; ++q) r[q * ms + k] = k < m ? B[q * N + k].x : 0.f;
     }
     if (ROWS)
-      for (int i = warp; i < R; i += CG_WARPS)
+      for (int i = warp; i < R; i += (NT / 32))
         for (int k = lane; k < ms; k += 32)
           rows[(size_t)i * ms + k] = k < m ? Hi[(size_t)(row0 + i) * N + k] : 0.f;
-    for (int t = tid; t < NR * RS; t += CG_THREADS) x[t] = make_float2(0.f, 0.f);
+    for (int t = tid; t < NR * RS; t += NT) x[t] = make_float2(0.f, 0.f);
     __syncthreads();
     bool alive = true;
     for (int outer = 0;; ++outer) {
@@ -193,7 +204,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
         float v[2 * NR];
 #pragma unroll
         for (int q = 0; q < 2 * NR; ++q) v[q] = 0.f;
-        for (int k = tid; k < ms; k += CG_THREADS)
+        for (int k = tid; k < ms; k += NT)
 #pragma unroll
           for (int q = 0; q < NR; ++q) {
             const float rv = r[q * ms + k], uv = dinv[k] * rv;
@@ -202,8 +213,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
             v[q] = fmaf(rv, uv, v[q]);
             v[NR + q] = fmaxf(v[NR + q], fabsf(rv));
           }
-        for (int t = tid; t < NR * RS; t += CG_THREADS) p[t] = d[t] = 0.f;
-        cg_reduce<2 * NR, NR>(v, sm, turn);
+        for (int t = tid; t < NR * RS; t += NT) p[t] = d[t] = 0.f;
+        cg_reduce<NT, 2 * NR, NR>(v, sm, turn);
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
           g[q] = v[q];
@@ -224,7 +235,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
       for (int it = 0; it < CG_INNER; ++it) {
         // own rows of A u
         float *w = cg_exchange(c, b, par);
-        for (int i = warp; i < R; i += CG_WARPS) {
+        for (int i = warp; i < R; i += (NT / 32)) {
           float a[NR];
 #pragma unroll
           for (int q = 0; q < NR; ++q) a[q] = 0.f;
@@ -268,19 +279,19 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
         float v[NR];
 #pragma unroll
         for (int q = 0; q < NR; ++q) v[q] = 0.f;
-        for (int t = tid; t < NR * R; t += CG_THREADS) {
-          const int q = t / R, i = t % R;
+        for (int t = tid; t < NR * R; t += NT) {
+          const int q = NR == 2 && t >= R, i = t - q * R;
           p[q * RS + i] = fmaf(beta[q], p[q * RS + i], u[q * ms + row0 + i]);
         }
 #pragma unroll 4
-        for (int k = tid; k < m; k += CG_THREADS)
+        for (int k = tid; k < m; k += NT)
 #pragma unroll
           for (int q = 0; q < NR; ++q) {
             const float wv = __ldcg(&w[q * N + k]);
             v[q] = fmaf(wv, u[q * ms + k], v[q]);
             s[q * ms + k] = fmaf(beta[q], s[q * ms + k], wv);
           }
-        cg_reduce<NR, NR>(v, sm, turn);
+        cg_reduce<NT, NR, NR>(v, sm, turn);
         bool bad = false, definite = true;
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -303,14 +314,14 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
           break;
         }
         // d += alpha p (own rows), r -= alpha s, u = r / diag
-        for (int t = tid; t < NR * R; t += CG_THREADS) {
-          const int q = t / R, i = t % R;
+        for (int t = tid; t < NR * R; t += NT) {
+          const int q = NR == 2 && t >= R, i = t - q * R;
           d[q * RS + i] = fmaf(alpha[q], p[q * RS + i], d[q * RS + i]);
         }
         float n[2 * NR];
 #pragma unroll
         for (int q = 0; q < 2 * NR; ++q) n[q] = 0.f;
-        for (int k = tid; k < m; k += CG_THREADS)
+        for (int k = tid; k < m; k += NT)
 #pragma unroll
           for (int q = 0; q < NR; ++q) {
             const float rv = fmaf(-alpha[q], s[q * ms + k], r[q * ms + k]);
@@ -320,7 +331,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
             n[q] = fmaf(rv, uv, n[q]);
             n[NR + q] = fmaxf(n[NR + q], fabsf(rv));
           }
-        cg_reduce<2 * NR, NR>(n, sm, turn);
+        cg_reduce<NT, 2 * NR, NR>(n, sm, turn);
         bool more = false;
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -334,8 +345,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
       if (!alive) break;
       // x += d; the residual in double-float
       __syncthreads();
-      for (int t = tid; t < NR * R; t += CG_THREADS) {
-        const int q = t / R, i = t % R;
+      for (int t = tid; t < NR * R; t += NT) {
+        const int q = NR == 2 && t >= R, i = t - q * R;
         const float2 o = x[q * RS + i];
         const dfl v = df_add(dfl{o.x, o.y}, dfl{d[q * RS + i], 0.f});
         x[q * RS + i] = make_float2(v.hi, v.lo);
@@ -344,12 +355,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
       alive = cg_barrier(counter, (unsigned)G * ++passed, sm, c.w.status);
       if (!alive) break;
       float2 *xs = reinterpret_cast<float2 *>(s);  // [NR][ms], over s and u
-      for (int k = tid; k < m; k += CG_THREADS)
+      for (int k = tid; k < m; k += NT)
 #pragma unroll
         for (int q = 0; q < NR; ++q) xs[q * ms + k] = __ldcg(&X[q * N + k]);
       __syncthreads();
       float *w = cg_exchange(c, b, par);
-      for (int i = warp; i < R; i += CG_WARPS) {
+      for (int i = warp; i < R; i += (NT / 32)) {
         const int row = row0 + i;
         dfl a[NR];
 #pragma unroll
@@ -373,7 +384,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) eeq_cg_kernel(Ctx c, int G, int
       alive = cg_barrier(counter, (unsigned)G * ++passed, sm, c.w.status);
       if (!alive) break;
       par ^= 1;
-      for (int k = tid; k < ms; k += CG_THREADS)
+      for (int k = tid; k < ms; k += NT)
 #pragma unroll
         for (int q = 0; q < NR; ++q) r[q * ms + k] = k < m ? __ldcg(&w[q * N + k]) : 0.f;
       __syncthreads();
@@ -420,11 +431,16 @@ bool launch_cg(const Ctx &c, cudaStream_t st) {
   const size_t smem = rows ? p.full : p.vec;
   Ctx cc = c;
   void *args[] = {&cc, &p.G, &p.groups};
-  const void *f = rows ? reinterpret_cast<const void *>(&eeq_cg_kernel<NR, true>)
-                       : reinterpret_cast<const void *>(&eeq_cg_kernel<NR, false>);
+  const bool few = (c.N + p.G - 1) / p.G <= CG_FEW_ROWS;
+  auto pick = [&](auto *many_rows, auto *many, auto *few_rows, auto *few_) {
+    return few ? reinterpret_cast<const void *>(rows ? few_rows : few_)
+               : reinterpret_cast<const void *>(rows ? many_rows : many);
+  };
+  const void *f = pick(&eeq_cg_kernel<CG_MANY, NR, true>, &eeq_cg_kernel<CG_MANY, NR, false>,
+                       &eeq_cg_kernel<CG_FEW, NR, true>, &eeq_cg_kernel<CG_FEW, NR, false>);
   ensure_smem_impl(f, smem);
-  if (cudaLaunchCooperativeKernel(f, dim3((unsigned)(p.G * p.groups)), dim3(CG_THREADS), args,
-                                  smem, st) != cudaSuccess) {
+  if (cudaLaunchCooperativeKernel(f, dim3((unsigned)(p.G * p.groups)),
+                                  dim3(few ? CG_FEW : CG_MANY), args, smem, st) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -436,7 +452,7 @@ bool launch_cg(const Ctx &c, cudaStream_t st) {
 // Whether conjugate gradients solve the batch: when every CTA holds its matrix
 // rows in shared memory, or when all SMs share few structures whose matrices
 // stay in L2.  Charges + adjoint against the factorisation, us: 1 x 300 atoms
-// 258 / 600, 1 x 2000 694 / 2184, 1 x 4000 1710 / 3621, 16 x 512 458 / 937;
+// 241 / 600, 1 x 2000 694 / 2184, 1 x 4000 1710 / 3621, 16 x 512 458 / 937;
 // but 1 x 6001 7429 / 5621 (matrix from HBM) and 160 x 320 2875 / 1779 (a CTA
 // per structure, matrix from L2).
 bool eeq_cg_takes(const Ctx &c) {
