@@ -4,7 +4,7 @@
 // (d4_mixed.cu, atm_mixed_kernel).
 //
 // Bound by FP32 issue and latency (512 structures of 8..200 atoms: 0.70 of the
-// issue slots at 16 warps per SM, 409 million warp instructions, 476 us).  The
+// issue slots at 16 warps per SM).  The
 // pair sums leave by 8-byte reductions at L2 instead of shared-memory atomics
 // (compare-and-swap loops), so no structure size is special and the sums of
 // the parameter gradients fit beside them; the (i, j) sums cross lanes through
@@ -13,8 +13,8 @@
 // 664 us, and so were direct loads instead of staged copies, 563.
 // Measured, ATM stage, against a tile kernel with the sums in shared memory
 // (N <= 234; no parameter gradients) and the per-triple kernel elsewhere: 512
-// structures of 8..200 atoms 572 -> 526 us; 256 of 20..150 with parameter
-// gradients 793 -> 258; 997 atoms 2115 -> 576; 1000 of 5..60, energies only,
+// structures of 8..200 atoms 572 -> 503 us; 256 of 20..150 with parameter
+// gradients 793 -> 249; 997 atoms 2115 -> 562; 1000 of 5..60, energies only,
 // 110 -> 55.
 #include "d4_atm.cuh"
 #include "d4_common.cuh"
@@ -144,16 +144,15 @@ __device__ __forceinline__ void a3_step(const A3Pair &a, const float4 *rec, int 
       if (!fik) s_cj[32 * t] += e2;
     }
     const float U = cq * h;
-    const float V = cq * fmaf(w, fmaf(-a.alp3h, fd, a.alp3h - 2.5f), 1.0f);
-    const float AC = A * C, BC = B * C;
-    const float Sg = AB + AC + BC;
-    Sik = fmaf(U, fmaf(-2.0f, BC, Sg), fmaf(V, pik.y, Sik));
-    Sjk[t] = fmaf(U, fmaf(-2.0f, AC, Sg), fmaf(V, izjk[t], Sjk[t]));
+    const float V = fmaf(eu, fmaf(-a.alp3h, fd, a.alp3h - 2.5f), cq);
+    const float sm = fmaf(A, C, AB), df = fmaf(-A, C, AB);
+    Sik = fmaf(U, fmaf(-B, C, sm), fmaf(V, pik.y, Sik));
+    Sjk[t] = fmaf(U, fmaf(B, C, df), fmaf(V, izjk[t], Sjk[t]));
     Pik += eu;
     Pjk[t] += eu;
-    s_red[A3_ROW * t + l] = make_float2(fmaf(U, fmaf(-2.0f, AB, Sg), V * pij.y), eu);
+    s_red[A3_ROW * t + l] = make_float2(fmaf(U, fmaf(B, C, -df), V * pij.y), eu);
     if (PGRAD) {
-      const float wv = Q * w * fmaf(-fd, fd, fd);
+      const float wv = fmaf(-eu, fd, eu);
       Wik += wv;
       Wjk[t] += wv;
       wij[t] = wv;
@@ -196,8 +195,11 @@ __device__ __forceinline__ void a3_step(const A3Pair &a, const float4 *rec, int 
 }
 
 // Number of tasks of a structure of n atoms whose tasks cover 8 s inner atoms
-// each: tiles g (middle atoms 1 + 8 g ..) have NG - g chunks of outer atoms
-// and g / s + 1 ranges of inner atoms.
+// each.  Tiles of middle atoms are counted from the last (n - 9 .. n - 2), so
+// that all chunks of outer atoms are full and the lowest tile, with the fewest
+// inner atoms, takes what does not divide by eight (its first j may be < 1).
+// Tile g from below has NG - g chunks of outer atoms and g / s + 1 ranges of
+// inner atoms.
 __device__ __forceinline__ long long a3_tasks(int n, int s) {
   const long long ng = n < 3 ? 0 : (n - 2 + A3 - 1) / A3;
   long long t = 0;
@@ -301,8 +303,7 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
     }
     int u, ch;
     tri_entry(t, u, ch);
-    const int j0 = 1 + A3 * (ng - 1 - u), kc = j0 + 1 + A3 * ch;
-    const int jend = min(j0 + A3, n - 1);
+    const int j0 = n - 1 - A3 * (u + 1), kc = j0 + 1 + A3 * ch, jend = j0 + A3;
     const int ib0 = ip * A3 * s, iend = min(ib0 + A3 * s, jend - 1);
     const size_t bN = (size_t)b * N;
     A3Pair a;
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
 #pragma unroll
     for (int tt = 0; tt < A3; ++tt) {
       const int jt = j0 + tt;
-      const bool jok = jt < jend && (!gaps || Z[jt] != 0);
+      const bool jok = jt > 0 && (!gaps || Z[jt] != 0);
       jmask |= (unsigned)jok << tt;
       float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
       if (kok && jok && jt < k) r = a.T[(size_t)jt * N + k];
@@ -413,7 +414,8 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
 #pragma unroll
         for (int tt = 0; tt < A3; ++tt) {
           const float e = warp_sumf(cj[32 * tt]);
-          if (lane == 0 && e != 0.f) atomicAdd(&a.e3[j0 + tt], (double)e * a.esc);
+          if (lane == 0 && ((jmask >> tt) & 1u) && e != 0.f)
+            atomicAdd(&a.e3[j0 + tt], (double)e * a.esc);
         }
         Ek += __shfl_xor_sync(0xffffffffu, Ek, 8);
         Ek += __shfl_xor_sync(0xffffffffu, Ek, 16);
@@ -435,7 +437,8 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
         ej += __shfl_xor_sync(0xffffffffu, ej, 1);
         ej += __shfl_xor_sync(0xffffffffu, ej, 2);
         ej += __shfl_xor_sync(0xffffffffu, ej, 4);
-        if ((lane & 7) == 0 && ej != 0.f) atomicAdd(&a.e3[j0 + 2 * q + p], (double)ej * a.esc);
+        if ((lane & 7) == 0 && ((jmask >> (2 * q + p)) & 1u) && ej != 0.f)
+          atomicAdd(&a.e3[j0 + 2 * q + p], (double)ej * a.esc);
       }
       Ek += __shfl_xor_sync(0xffffffffu, Ek, 8);
       Ek += __shfl_xor_sync(0xffffffffu, Ek, 16);
@@ -558,17 +561,16 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
           const float cq = Q * fd, eu = cq * w;
           if (GRAD) {
             const float U = cq * h;
-            const float V = cq * fmaf(w, fmaf(-alp3h, fd, alp3h - 2.5f), 1.0f);
-            const float AC = A * C, BC = B * C;
-            const float Sg = AB + AC + BC;
-            out = make_float2(fmaf(U, fmaf(-2.0f, AB, Sg), V * pij.y), eu);
-            Sjk = fmaf(U, fmaf(-2.0f, AC, Sg), fmaf(V, pjk.y, Sjk));
+            const float V = fmaf(eu, fmaf(-alp3h, fd, alp3h - 2.5f), cq);
+            const float sm = fmaf(A, C, AB), df = fmaf(-A, C, AB);
+            out = make_float2(fmaf(U, fmaf(B, C, -df), V * pij.y), eu);
+            Sjk = fmaf(U, fmaf(B, C, df), fmaf(V, pjk.y, Sjk));
             Pjk += eu;
             Cj += in ? 0.f : eu;
             if (use)
-              red2(&SP[(size_t)i * N + k], fmaf(U, fmaf(-2.0f, BC, Sg), V * pik[r].y), eu);
+              red2(&SP[(size_t)i * N + k], fmaf(U, fmaf(-B, C, sm), V * pik[r].y), eu);
             if (PGRAD) {
-              wv = Q * w * fmaf(-fd, fd, fd);
+              wv = fmaf(-eu, fd, eu);
               Wjk += wv;
               pg.s9 += eu;
               if (use) pg.add(wv, Tda[(size_t)i * N + k]);

@@ -11,9 +11,12 @@
 // instructions per triple with its gradient against ~186 of the per-triple
 // kernel (d4_fp64.cu, atm_kernel: one pair (j, k) per lane, an exp, a
 // division and full warp sums per triple).  Measured, ATM stage: 64
-// structures of 8..200 atoms 11.06 -> 1.96 ms, 360 of 30 atoms 1.36 -> 0.31
-// ms, 301 atoms 4.82 -> 0.52 ms, 57 atoms 0.48 -> 0.019 ms (energy +
-// gradient); 32 atoms, energy only, 0.125 -> 0.016 ms.
+// structures of 8..200 atoms 11.06 -> 1.76 ms, 360 of 30 atoms 1.36 -> 0.22
+// ms, 301 atoms 4.82 -> 0.43 ms, 57 atoms 0.48 -> 0.018 ms (energy +
+// gradient); 32 atoms, energy only, 0.125 -> 0.016 ms.  Of the middle atoms'
+// order: tiles counted from the last atom instead of the first, and steps
+// without the middle atoms below all inner ones, took 1.96 -> 1.76 ms and 0.31
+// -> 0.22 ms.
 #include "d4_common.cuh"
 #include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
@@ -88,12 +91,13 @@ struct A6Pg {
 };
 
 // One step: inner atom i of this lane's group against the J middle atoms
-// j0 .. of the task and the lane's outer atom k.  GUARD: some (i, j) are not
-// pairs of the task (i >= j, j or i beyond the range).  MASK: an atom of the
+// j0 .. of the task and the lane's outer atom k.  ib: the first group's inner
+// atom.  GUARD: some (i, j) are not pairs of the task (i >= j, i beyond the
+// range).  MASK: an atom of the
 // step has a pair beyond the cutoff, so each triple takes its weight
 // (1, 1/3 or 0) and the 1/3 triples their energy attribution.
 template <int J, bool GRAD, bool PGRAD, bool GUARD, bool MASK>
-__device__ __forceinline__ void a6_step(const A6 &a, int j0, int jend, int k, bool kok, int i,
+__device__ __forceinline__ void a6_step(const A6 &a, int j0, int k, bool kok, int ib, int i,
                                         bool iok, const double (&zjk)[J], const double (&ujk)[J],
                                         const double (&tjk)[J], const double (&qjk)[J],
                                         double (&Sjk)[J], double (&Pjk)[J], double (&Wjk)[J],
@@ -109,10 +113,18 @@ __device__ __forceinline__ void a6_step(const A6 &a, int j0, int jend, int k, bo
 #pragma unroll
   for (int s = 0; s < J; ++s) {
     const int t = GroupSum<J>::ord(s);
+    if (GUARD && j0 + t <= ib) {  // no lane of the warp has a triple
+      if (GRAD) {
+        gS.put(s, 0.0);
+        gP.put(s, 0.0);
+        if (PGRAD) gW.put(s, 0.0);
+      }
+      continue;
+    }
     PairRec ij;
     if (GUARD) {
       const int jt = j0 + t;
-      const bool ok = iok && jt > i && jt < jend;
+      const bool ok = iok && jt > i;
       ij = ok ? Ti[ok ? jt : 0] : zero;
     } else {
       ij = Ti[j0 + t];
@@ -165,7 +177,7 @@ __device__ __forceinline__ void a6_step(const A6 &a, int j0, int jend, int k, bo
     const double AC = A * C, BC = B * C;
     const double sm = AB + AC, df = AB - AC;
     const double U = D * w;
-    const double V = D * fma(g, fma(-a.alp6, fd, a.alp6 - 2.5), 1.0);
+    const double V = fma(e, fma(-a.alp6, fd, a.alp6 - 2.5), D);
     Sik = fma(V, ik.u, fma(U, sm - BC, Sik));
     Sjk[t] = fma(V, ujk[t], fma(U, df + BC, Sjk[t]));
     Pik += e;
@@ -201,7 +213,7 @@ __device__ __forceinline__ void a6_step(const A6 &a, int j0, int jend, int k, bo
     }
   }
   const int jt = j0 + GroupSum<J>::mine();
-  if (GroupSum<J>::owner() && (!GUARD || (iok && jt > i && jt < jend))) {
+  if (GroupSum<J>::owner() && (!GUARD || (iok && jt > i))) {
     atomicAdd(&a.S[row + jt], sc * gS.a);
     atomicAdd(&a.P[row + jt], sc * gP.a);
     if (PGRAD) {
@@ -226,11 +238,11 @@ template <int J, bool GRAD, bool PGRAD>
 __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
   const int b = blockIdx.z;
   const int n = c.w.n_eff[b];
-  const int NT = n < 3 ? 0 : (n - 2 + J - 1) / J;  // tiles of middle atoms 1 .. n - 2
   const int lane = threadIdx.x & 31;
   const int task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  // tiles have ceil((n - 1 - j0) / 8) chunks; walk J / 8-row groups so that
-  // the chunk count is linear in the group index
+  // groups of eight middle atoms, the top one n - 9 .. n - 2, so that all
+  // chunks of outer atoms are full and what does not divide by eight is left to
+  // the lowest group, which has the fewest inner atoms (its first j may be < 1)
   constexpr int R = A6_K / J;  // tiles per eight middle atoms
   const int NG = n < 3 ? 0 : (n - 2 + A6_K - 1) / A6_K;
   if (task >= R * (NG * (NG + 1) / 2)) return;
@@ -239,10 +251,10 @@ __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
   while ((u + 1) * (u + 2) / 2 <= pt) ++u;
   while (u > 0 && u * (u + 1) / 2 > pt) --u;
   const int ch = pt - u * (u + 1) / 2;
-  const int j0 = 1 + A6_K * (NG - 1 - u) + J * sub;
-  if (j0 > n - 2 || NT == 0) return;
-  const int kc = 1 + A6_K * (NG - 1 - u) + 1 + A6_K * ch;
-  const int jend = min(j0 + J, n - 1);
+  const int jg = n - 1 - A6_K * (u + 1), j0 = jg + J * sub;
+  const int kc = jg + 1 + A6_K * ch;
+  const int jend = j0 + J;
+  if (jend < 2) return;
   const int ib0 = blockIdx.y * il;
   const int iend = min(ib0 + il, jend - 1);  // i < j <= jend - 1
   if (ib0 >= iend) return;
@@ -270,13 +282,13 @@ __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
   for (int t = 0; t < J; ++t) {
     const int jt = j0 + t;
     PairRec r{0.0, 0.0, 0.0, 0.0};
-    if (kok && jt < k) r = a.T[(size_t)jt * N + k];
+    if (jt > 0 && kok && jt < k) r = a.T[(size_t)jt * N + k];
     zjk[t] = r.x;
     ujk[t] = r.u;
     tjk[t] = 6.0 * r.t;
     qjk[t] = s9q * r.q;  // 0 where (j, k) is not a pair: every product vanishes
     Sjk[t] = Pjk[t] = Wjk[t] = 0.0;
-    far |= jt < jend && far2[jt] > a.cut2;
+    far |= jt > 0 && far2[jt] > a.cut2;
   }
   const bool task_far = __any_sync(0xffffffffu, far);
   double Ek = 0.0;
@@ -285,15 +297,15 @@ __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
     const int i = ib + (lane >> 3);
     const bool iok = i < iend;
     const bool mask = task_far || __any_sync(0xffffffffu, iok && far2[i] > a.cut2);
-    const bool guard = ib + 4 > iend || ib + 4 > j0 || j0 + J > n - 1;
+    const bool guard = ib + 4 > iend || ib + 4 > j0;
     if (mask)
-      a6_step<J, GRAD, PGRAD, true, true>(a, j0, jend, k, kok, i, iok, zjk, ujk, tjk, qjk, Sjk,
-                                          Pjk, Wjk, Ek, pg);
+      a6_step<J, GRAD, PGRAD, true, true>(a, j0, k, kok, ib, i, iok, zjk, ujk, tjk, qjk, Sjk, Pjk,
+                                          Wjk, Ek, pg);
     else if (guard)
-      a6_step<J, GRAD, PGRAD, true, false>(a, j0, jend, k, kok, i, iok, zjk, ujk, tjk, qjk, Sjk,
-                                           Pjk, Wjk, Ek, pg);
+      a6_step<J, GRAD, PGRAD, true, false>(a, j0, k, kok, ib, i, iok, zjk, ujk, tjk, qjk, Sjk, Pjk,
+                                           Wjk, Ek, pg);
     else
-      a6_step<J, GRAD, PGRAD, false, false>(a, j0, jend, k, kok, i, iok, zjk, ujk, tjk, qjk, Sjk,
+      a6_step<J, GRAD, PGRAD, false, false>(a, j0, k, kok, ib, i, iok, zjk, ujk, tjk, qjk, Sjk,
                                             Pjk, Wjk, Ek, pg);
   }
   // the four groups' (j, k) sums: two exchanges leave each lane J / 4 of them
@@ -310,7 +322,7 @@ __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
       };
       const double sv = join(Sjk), pv = join(Pjk);
       const double wv = PGRAD ? join(Wjk) : 0.0;
-      if (kok && jt < k && jt < jend) {
+      if (jt > 0 && kok && jt < k) {
         const size_t o = (size_t)jt * N + k;
         atomicAdd(&a.S[o], sc * sv);
         atomicAdd(&a.P[o], sc * pv);
@@ -329,7 +341,7 @@ __global__ void __launch_bounds__(128) atm_tiled64_kernel(Ctx c, int il) {
 #pragma unroll
     for (int t = 0; t < J; ++t) {
       const double ej = warp_sum(Pjk[t]);
-      if (lane == 0 && ej != 0.0) atomicAdd(&a.e3[j0 + t], ej * third);
+      if (lane == 0 && j0 + t > 0 && ej != 0.0) atomicAdd(&a.e3[j0 + t], ej * third);
     }
   }
   if (PGRAD) {
@@ -356,11 +368,15 @@ static void launch_tiled64(const Ctx &c, cudaStream_t st) {
   const long long tasks = (A6_K / J) * NG * (NG + 1) / 2;
   // inner atoms per task: 32 (the ends of a task cost 1 % of eight steps, and
   // a task of 200 inner atoms alone on its SM would outlast the rest of a
-  // batch), fewer where the batch would give an SM fewer than 32 tasks
+  // batch), down to 8 where an SM would get fewer than 128 tasks (301 atoms
+  // 564 -> 463 us, 360 x 30 271 -> 254), 4 where it would get fewer than 32
+  // (57 atoms 30 -> 20; 360 x 30, which has more, loses by it: 325)
   int il = 32;
-  while (il > 4 && tasks * c.B * ((N + il - 1) / il) < 2LL * 152 * 16) il >>= 1;
+  auto count = [&]() { return tasks * c.B * ((N + il - 1) / il); };
+  while (il > 8 && count() < 128LL * 152) il >>= 1;
+  if (count() < 32LL * 152) il = 4;
   // one warp per CTA spreads few tasks over the SMs; four where there are many
-  const int warps = tasks * c.B * ((N + il - 1) / il) < 152LL * 64 ? 1 : 4;
+  const int warps = count() < 64LL * 152 ? 1 : 4;
   const dim3 grid((unsigned)((tasks + warps - 1) / warps), (unsigned)((N + il - 1) / il),
                   (unsigned)c.B);
   atm_tiled64_kernel<J, GRAD, PGRAD><<<grid, 32 * warps, 0, st>>>(c, il);
