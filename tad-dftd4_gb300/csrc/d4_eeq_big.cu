@@ -1214,7 +1214,7 @@ void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint) {
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cap = cudaStreamCaptureStatusActive;
   const bool host_check =
       nsb >= 8 && cap == cudaStreamCaptureStatusNone && !(c.flags & D4_FLAG_NO_HOST_WAIT);
-  eeq_big_rhs_kernel<<<dim3((N + 255) / 256, B), 256, 0, st>>>(c, adjoint ? 1 : 0);
+  launch_eeq_big_rhs(c, st, adjoint);
   for (int it = 0; it < EEQ_BIG_REFINE; ++it) {
     if (host_check && it >= 2 && converged_on_host(c, st, it - 1)) break;
     // V = L^-T L^-1 V: forward sweep into Y, backward sweep into V
@@ -1232,17 +1232,27 @@ void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint) {
         eeq_sweep_above_kernel<<<dim3((s0 + AB_COLS - 1) / AB_COLS, B), 256, 0, st>>>(c, sb, it,
                                                                                      nr);
     }
-    eeq_big_update_kernel<<<dim3((N + 255) / 256, B), 256, 0, st>>>(c, it, nr);
-    const dim3 rg((N + 8 * RS_ROWS - 1) / (8 * RS_ROWS), B);
-    if (N % 4 == 0) {
-      if (nr == 2) eeq_big_residual_kernel<2, true><<<rg, 256, 0, st>>>(c, it);
-      else eeq_big_residual_kernel<1, true><<<rg, 256, 0, st>>>(c, it);
-    } else {
-      if (nr == 2) eeq_big_residual_kernel<2, false><<<rg, 256, 0, st>>>(c, it);
-      else eeq_big_residual_kernel<1, false><<<rg, 256, 0, st>>>(c, it);
-    }
+    launch_eeq_big_refine(c, st, it, adjoint);
   }
   launch_eeq_big_finish(c, st, adjoint);
+}
+
+void launch_eeq_big_rhs(const Ctx &c, cudaStream_t st, bool adjoint) {
+  eeq_big_rhs_kernel<<<dim3((c.N + 255) / 256, c.B), 256, 0, st>>>(c, adjoint ? 1 : 0);
+}
+
+// x += v and the residual of refinement iteration ``it``.
+void launch_eeq_big_refine(const Ctx &c, cudaStream_t st, int it, bool adjoint) {
+  const int B = c.B, N = c.N;
+  eeq_big_update_kernel<<<dim3((N + 255) / 256, B), 256, 0, st>>>(c, it, adjoint ? 1 : 2);
+  const dim3 rg((N + 8 * RS_ROWS - 1) / (8 * RS_ROWS), B);
+  if (N % 4 == 0) {
+    if (!adjoint) eeq_big_residual_kernel<2, true><<<rg, 256, 0, st>>>(c, it);
+    else eeq_big_residual_kernel<1, true><<<rg, 256, 0, st>>>(c, it);
+  } else {
+    if (!adjoint) eeq_big_residual_kernel<2, false><<<rg, 256, 0, st>>>(c, it);
+    else eeq_big_residual_kernel<1, false><<<rg, 256, 0, st>>>(c, it);
+  }
 }
 
 void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint) {

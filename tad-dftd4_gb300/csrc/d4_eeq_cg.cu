@@ -25,6 +25,7 @@
 // iteration's 8200 cycles there, 2700 go to the barrier, 1450 to the product,
 // 1480 to reading the exchanged rows and 2500 to the updates and reductions.
 #include "d4_common.cuh"
+#include "d4_group.cuh"
 #include "d4_kernels.cuh"
 
 namespace d4 {
@@ -41,7 +42,6 @@ constexpr float CG_TOL = 1e-10f;     // max |b - A x|
 constexpr float CG_GAIN = 1e-12f;    // of (r, r / diag) per FP32 solve
 constexpr int CG_OUTER = 16;         // refinements at most
 constexpr int CG_INNER = 500;        // iterations of one FP32 solve at most
-constexpr unsigned CG_POLLS = 1u << 22;  // of a barrier (about two seconds)
 constexpr size_t CG_SMEM = 200 * 1024;
 
 // Rows of A u (and residuals) in turn: two buffers, alternating, so that a CTA
@@ -59,25 +59,6 @@ struct CgSmem {
   __align__(16) float red[2][4][CG_MANY / 32];  // [turn][value][warp]
   int dead;
 };
-
-// Barrier of the group's G CTAs; false after CG_POLLS polls (the status word
-// then reports it and every CTA leaves).
-__device__ bool cg_barrier(unsigned *counter, unsigned target, CgSmem &sm, int *status) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-    unsigned v = 0, k = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-    } while (v < target && ++k < CG_POLLS);
-    if (v < target) {
-      set_status(status, D4_ERR_DEVICE_TIMEOUT);
-      sm.dead = 1;
-    }
-  }
-  __syncthreads();
-  return sm.dead == 0;
-}
 
 // Sums (or maxima from index NS on) of V values over the NT threads of the CTA,
 // the same in all threads.  The buffers alternate, so one synchronisation is
@@ -272,7 +253,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
           for (int q = 0; q < NR; ++q) a[q] = warp_sumf(a[q]);
           if (lane < NR) __stcg(&w[lane * N + row0 + i], lane == 0 ? a[0] : a[NR - 1]);
         }
-        alive = cg_barrier(counter, (unsigned)G * ++passed, sm, c.w.status);
+        alive = group_barrier(counter, (unsigned)G * ++passed, sm.dead, c.w.status);
         if (!alive) break;
         par ^= 1;
         // p = u + beta p (own rows), s = A u + beta s, (A u, u)
@@ -352,7 +333,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
         x[q * RS + i] = make_float2(v.hi, v.lo);
         __stcg(&X[q * N + row0 + i], make_float2(v.hi, v.lo));
       }
-      alive = cg_barrier(counter, (unsigned)G * ++passed, sm, c.w.status);
+      alive = group_barrier(counter, (unsigned)G * ++passed, sm.dead, c.w.status);
       if (!alive) break;
       float2 *xs = reinterpret_cast<float2 *>(s);  // [NR][ms], over s and u
       for (int k = tid; k < m; k += NT)
@@ -381,7 +362,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
           if (lane == 0) __stcg(&w[q * N + row], v.hi);
         }
       }
-      alive = cg_barrier(counter, (unsigned)G * ++passed, sm, c.w.status);
+      alive = group_barrier(counter, (unsigned)G * ++passed, sm.dead, c.w.status);
       if (!alive) break;
       par ^= 1;
       for (int k = tid; k < ms; k += NT)

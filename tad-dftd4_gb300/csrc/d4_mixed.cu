@@ -1423,10 +1423,10 @@ __global__ void __launch_bounds__(256) pair_cn_bwd_mixed_kernel(Ctx c) {
 // 1/g and the diagonal from per-element tables; no FP64 instruction.
 // Persistent blocks loop over the 32 x 32 tiles of the lower triangles of
 // all structures; a tile and its mirror are both stored coalesced (the
-// mirror through shared memory).  The lower tiles' hi part also goes to the
-// multi-CTA factorisation's matrix F (row stride eeq_ldf(N)), which reads
-// nothing above the diagonal.
-__global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c) {
+// mirror through shared memory).  ``factor``: the lower tiles' hi part also goes
+// to the multi-CTA factorisation's matrix F (row stride eeq_ldf(N)), which
+// reads nothing above the diagonal.
+__global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c, bool factor) {
   __shared__ float4 s_erf[ERF_TAB];
   __shared__ float s_hi[32][33], s_lo[32][33];
   for (int k = threadIdx.x; k < ERF_TAB; k += blockDim.x) s_erf[k] = c.w.erf_tab[k];
@@ -1483,7 +1483,7 @@ __global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c) {
         }
         Hi[(size_t)k * N + l] = v.hi;
         Lo[(size_t)k * N + l] = v.lo;
-        F[(size_t)k * NF + l] = v.hi;  // the factorisation's input (lower part)
+        if (factor) F[(size_t)k * NF + l] = v.hi;  // the factorisation's input (lower part)
       }
       s_hi[rr][tx] = v.hi;
       s_lo[rr][tx] = v.lo;
@@ -1831,6 +1831,10 @@ __global__ void __launch_bounds__(EEQ_THREADS, 2) eeq_adjoint_mixed_kernel(Ctx c
 // ---------------------------------------------------------------- launch
 
 // persistent grid of the EEQ build: 4 blocks per SM, at most one per tile
+static bool launch_eeq_iterative(const Ctx &c, cudaStream_t st, bool adjoint) {
+  return eeq_dcg_takes(c) ? launch_eeq_dcg(c, st, adjoint) : launch_eeq_cg(c, st, adjoint);
+}
+
 static unsigned build_blocks(const Ctx &c) {
   static int sms[64] = {0};
   int dev = 0;
@@ -1939,12 +1943,16 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   const bool eeq_smem = eeq_small_fits(N);
   stage_begin(ST_EEQ, st);
   if (eeq) {
-    if (!eeq_smem) eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c);
     if (eeq_smem) {  // builds its matrix itself
       ensure_smem(eeq_mixed_kernel<true>, (int)(vec_bytes + pt_bytes + tri_bytes));
       eeq_mixed_kernel<true><<<B, EEQ_THREADS, vec_bytes + pt_bytes + tri_bytes, st>>>(c);
     } else {
-      if (!eeq_cg_takes(c) || !launch_eeq_cg(c, st, false)) launch_eeq_big(c, st, false);
+      const bool iterate = eeq_dcg_takes(c) || eeq_cg_takes(c);
+      eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, !iterate);
+      if (!iterate || !launch_eeq_iterative(c, st, false)) {
+        if (iterate) eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true);
+        launch_eeq_big(c, st, false);
+      }
     }
   } else {
     launch_charges_in(c, st);
@@ -1984,9 +1992,10 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
         ensure_smem(eeq_adjoint_mixed_kernel<true>, (int)(vec_bytes + tri_bytes));
         eeq_adjoint_mixed_kernel<true><<<B, EEQ_THREADS, vec_bytes + tri_bytes, st>>>(c);
       } else {
-        if (!eeq_cg_takes(c)) {
+        if (!eeq_dcg_takes(c) && !eeq_cg_takes(c)) {
           launch_eeq_big(c, st, true);
-        } else if (!launch_eeq_cg(c, st, true)) {  // the factor is needed after all
+        } else if (!launch_eeq_iterative(c, st, true)) {  // the factor is needed after all
+          eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true);
           launch_eeq_big(c, st, false);
           launch_eeq_big(c, st, true);
         }
