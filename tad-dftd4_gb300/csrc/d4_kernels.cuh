@@ -49,6 +49,8 @@ bool launch_eeq_cg(const Ctx &c, cudaStream_t st, bool adjoint);
 bool eeq_dcg_takes(const Ctx &c);  // deflated, large structures (d4_eeq_dcg.cu)
 bool launch_eeq_dcg(const Ctx &c, cudaStream_t st, bool adjoint);
 void launch_pair_fwd_tc(const Ctx &c, cudaStream_t st);  // D4, precision form (d4_c6tc.cu)
+void launch_pair_fwd_d4s32(const Ctx &c, cudaStream_t st);  // D4S, precision form (d4_d4s32.cu)
+void launch_pair_bwd_d4s32(const Ctx &c, cudaStream_t st);
 bool pair_atm_bwd_tc_ok(const Ctx &c);
 void launch_pair_atm_bwd_tc(const Ctx &c, cudaStream_t st);
 void launch_atm_tiled64(const Ctx &c, cudaStream_t st);  // FP64 (d4_atm64.cu)

@@ -385,197 +385,6 @@ __global__ void __launch_bounds__(256) cn_mixed_kernel(Ctx c) {
   }
 }
 
-// ---------------------------------------------------------------- pairs
-
-// Fused C6 + BJ two-body term in FP32, the per-pair ATM table (float4:
-// r^2, 1/r^2, (R0/r)^(alp/3), sqrt(C6(q=0)) / r^3), the direct gradient and
-// the C6 adjoint.  One warp per atom i, lanes over partners j.
-template <bool GRAD, bool PGRAD>
-__global__ void __launch_bounds__(256, 2) pair_fwd_mixed_kernel(Ctx c) {
-  const int b = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 8 + warp;
-  const int N = c.N;
-  __shared__ float s_wa[8][NFREQ];
-  __shared__ float s_wa0[8][NFREQ];
-  if (i >= N) return;
-  const size_t ai = (size_t)b * N + i;
-  const int zi = c.w.z[ai];
-  const int n = c.w.n_eff[b];
-  if (i >= n || zi == 0) {
-    if (lane == 0) {
-      c.out.d_energy[ai] = 0.0;
-      if (GRAD) {
-        c.out.d_gradient[3 * ai] = 0.0;
-        c.out.d_gradient[3 * ai + 1] = 0.0;
-        c.out.d_gradient[3 * ai + 2] = 0.0;
-      }
-    }
-    if (GRAD && lane < NFREQ)
-      for (int s = 0; s < c.S; ++s) c.w.G32[(ai * c.S + s) * NFREQ + lane] = 0.f;
-    return;
-  }
-  const d4_params_t &p = c.par;
-  const float s6 = c.pf.s6, s8 = c.pf.s8, s10 = c.pf.s10;
-  const float cut2 = c.pf.cut2;
-  const float4 *P = c.w.pos32 + (size_t)b * N;
-  const float4 *PL = c.w.pos32lo + (size_t)b * N;
-  const float4 pi = P[i], li = PL[i];
-  const float wi = c.w.w32[ai];
-  const int nslot = c.w.n_slots[b];
-  const int slot_i = c.w.slot[ai];
-  float4 *T = c.w.ptf + (size_t)ai * N;
-  float4 *Tda = PGRAD ? c.w.ptf_da + (size_t)ai * N : nullptr;
-  // R0 = a1 sqrt(qq) + a2, qq = 3 r4r2_i r4r2_j, R0^6 and R0^8 as
-  // double-floats, so that no FP32 rounding of a per-element-pair constant
-  // biases every pair of that element pair the same way: from the per-call
-  // element-pair table, or (per-atom r4r2 given) per pair from u_i = a1
-  // sqrt(3) s_i, v_i = sqrt(3) s_i (FP64 per atom) and s_j = pos32.w + pos32lo.w
-  const bool tabled = c.r4r2_in == nullptr;
-  // compensated sums of c6 t6 (with (s10/s6) c10 t10 folded in) and of
-  // c8 t8; s6 and s8 are applied in FP64 at the end (one FP32 sum of both
-  // orders, with s8/s6 as a double-float, measured 4x less accurate)
-  const double sref = p.s6 != 0.0 ? p.s6 : 1.0;
-  const dfl rho10 = df_from(p.has_s10 ? p.s10 / sref : 0.0);
-  const float rho6 = p.s6 != 0.0 ? 1.f : 0.f;
-  Acc32 e_acc, e8_acc, gx, gy, gz;
-  float pg[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  float r2mx = 0.f;  // largest r^2 of this atom's pairs (the ATM's far-atom test)
-  for (int s = 0; s < nslot; ++s) {
-    if (lane < NFREQ) {  // A' already carries sqrt((3/pi) w): C6 = sum_w A'_i A'_j
-      const size_t o = a32_index(b, i, s, lane, N, c.S);
-      s_wa[warp][lane] = c.w.A32[o];
-      s_wa0[warp][lane] = c.w.A032[o];
-    }
-    __syncwarp();
-    float gacc[NFREQ];
-#pragma unroll
-    for (int w = 0; w < NFREQ; ++w) gacc[w] = 0.f;
-    for (int j = lane; j < n; j += 32) {
-      const size_t aj = (size_t)b * N + j;
-      const int zj = c.w.z[aj];
-      if (j == i || zj == 0 || c.w.slot[aj] != s) continue;
-      const float4 pj = P[j];
-      const float3 d = pos_diff(pi, li, pj, PL[j]);
-      const float dx = d.x, dy = d.y, dz = d.z;
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      const float ir = __frcp_rn(sqrtf(r2));  // correctly rounded: no bias in the ATM records
-      const float r = r2 * ir;
-      const float *Aj = c.w.A32 + a32_index(b, j, slot_i, 0, N, c.S);
-      const float *A0j = c.w.A032 + a32_index(b, j, slot_i, 0, N, c.S);
-      float c6 = 0.f, c60 = 0.f;
-#pragma unroll
-      for (int w = 0; w < NFREQ; ++w) {
-        c6 = fmaf(s_wa[warp][w], Aj[(size_t)w * N], c6);
-        c60 = fmaf(s_wa0[warp][w], A0j[(size_t)w * N], c60);
-      }
-      dfl R0d, qqd, R06d, R08d;
-      if (tabled) {  // per element pair, from the table r4r2 values
-        const float4 A = c.w.pairA[zi * MAX_ELEM_ID + zj], Bq = c.w.pairB[zi * MAX_ELEM_ID + zj];
-        R0d = {A.x, A.y};
-        qqd = {A.z, A.w};
-        R06d = {Bq.x, Bq.y};
-        R08d = {Bq.z, Bq.w};
-      } else {  // per-atom r4r2 given (rare): FP64 per pair
-        const double si = (double)pi.w + (double)li.w, sj = (double)pj.w + (double)PL[j].w;
-        const double qq = 3.0 * si * si * sj * sj;
-        const double R0 = p.a1 * sqrt(qq) + p.a2;
-        const double R02 = R0 * R0, R06 = R02 * R02 * R02;
-        R0d = df_from(R0);
-        qqd = df_from(qq);
-        R06d = df_from(R06);
-        R08d = df_from(R06 * R02);
-      }
-      const float R0 = R0d.hi, sqq = sqrtf(qqd.hi);
-      const float lnR0r = logf(R0 * ir) + R0d.lo / R0;
-      const float ir2 = __frcp_rn(r2);
-      T[j] = make_float4(r2, ir2, expf(c.pf.alp3 * lnR0r), sqrtf(c60) * (ir * ir2));
-      if (GRAD && i < j) c.w.prSP32[(size_t)ai * N + j] = make_float2(0.f, 0.f);  // ATM sums
-      r2mx = fmaxf(r2mx, r2);
-      if (PGRAD) Tda[j] = make_float4(sqq / R0, 1.0f / R0, lnR0r, 0.f);
-      if (r <= cut2) {
-        const float r6 = r2 * r2 * r2, R02 = R0 * R0, R06 = R06d.hi;
-        const float t6 = 1.0f / ((r6 + R06) + R06d.lo);
-        float eterm = rho6 * c6 * t6;
-        float dEdr = 6.0f * s6 * c6 * (r6 * ir) * t6 * t6;
-        float K = -s6 * t6;
-        float dE_dR0 = 6.0f * s6 * c6 * (R06 / R0) * t6 * t6;
-        pg[0] -= wi * c6 * t6;
-        if (p.has_s8) {
-          const float r8 = r6 * r2, R08 = R08d.hi, qq = qqd.hi;
-          const float t8 = 1.0f / ((r8 + R08) + R08d.lo);
-          const float c8 = fmaf(c6, qqd.hi, c6 * qqd.lo);
-          const float e8 = c8 * t8;
-          e8_acc.add(e8);
-          dEdr += 8.0f * s8 * c8 * (r8 * ir) * t8 * t8;
-          K -= s8 * qq * t8;
-          dE_dR0 += 8.0f * s8 * c8 * (R08 / R0) * t8 * t8;
-          pg[1] -= wi * c8 * t8;
-        }
-        if (p.has_s10) {  // rare: FP32 powers
-          const float qq = sqq * sqq;
-          const float r10 = r6 * r2 * r2, R010 = R06 * R02 * R02;
-          const float t10 = 1.0f / (r10 + R010);
-          const float q2 = qq * qq * (49.0f / 40.0f);
-          const float c10 = c6 * q2;
-          const float e10 = c10 * t10;
-          eterm = fmaf(rho10.hi, e10, fmaf(rho10.lo, e10, eterm));
-          dEdr += 10.0f * s10 * c10 * (r10 * ir) * t10 * t10;
-          K -= s10 * q2 * t10;
-          dE_dR0 += 10.0f * s10 * c10 * (R010 / R0) * t10 * t10;
-          pg[2] -= wi * c10 * t10;
-        }
-        e_acc.add(eterm);
-        const float phi = 0.5f * (wi + c.w.w32[aj]);
-        dEdr *= phi;
-        K *= phi;
-        pg[3] += wi * 0.5f * dE_dR0 * sqq;
-        pg[4] += wi * 0.5f * dE_dR0;
-        const float f = dEdr * ir;
-        gx.add(f * dx);
-        gy.add(f * dy);
-        gz.add(f * dz);
-        if (GRAD) {
-#pragma unroll
-          for (int w = 0; w < NFREQ; ++w) gacc[w] = fmaf(K, Aj[(size_t)w * N], gacc[w]);
-        }
-      }
-    }
-    if (GRAD) {
-      const float mine = warp_reduce_scatter32(gacc);  // lane w: sum of gacc[w]
-      if (lane < NFREQ) c.w.G32[(ai * c.S + s) * NFREQ + lane] = mine;  // dE/dA'_i
-    }
-    __syncwarp();
-  }
-  if (GRAD && lane < NFREQ)
-    for (int s = nslot; s < c.S; ++s) c.w.G32[(ai * c.S + s) * NFREQ + lane] = 0.f;
-  const Acc32 ea = warp_sum_acc(e_acc), ea8 = warp_sum_acc(e8_acc);
-  r2mx = warp_maxf(r2mx);
-  if (lane == 0 && r2mx > 0.f) atomicMax(&c.w.atm_rowmax[ai], __float_as_uint(r2mx));
-  if (PGRAD) {
-    float v[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] = warp_sumf(pg[k]);
-    if (lane == 0) {
-      atomicAdd(&c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + 0], 0.5 * (double)v[0]);
-      atomicAdd(&c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + 1], 0.5 * (double)v[1]);
-      atomicAdd(&c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + 2], 0.5 * (double)v[2]);
-      atomicAdd(&c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + 3], (double)v[3]);
-      atomicAdd(&c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + 4], (double)v[4]);
-    }
-  }
-  if (GRAD) {
-    const Acc32 g0 = warp_sum_acc(gx), g1 = warp_sum_acc(gy), g2 = warp_sum_acc(gz);
-    if (lane == 0) {
-      c.out.d_gradient[3 * ai] = g0.value();
-      c.out.d_gradient[3 * ai + 1] = g1.value();
-      c.out.d_gradient[3 * ai + 2] = g2.value();
-    }
-  }
-  if (lane == 0)
-    c.out.d_energy[ai] = -0.5 * (sref * ea.value() + (p.has_s8 ? p.s8 * ea8.value() : 0.0));
-}
-
 // ---------------------------------------------------------------- launch order
 
 // Structures by decreasing size (n_eff), ties by index: the per-structure
@@ -1278,81 +1087,6 @@ __global__ void __launch_bounds__(ATM_SPARSE_THREADS, 2) atm_sparse_kernel(Ctx c
   }
 }
 
-// ATM forces, C6(q=0) adjoint, chain rule to dE/dCN and dE/dq, E2 + E3.
-__global__ void __launch_bounds__(256) pair_atm_bwd_mixed_kernel(Ctx c) {
-  const int b = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int x = blockIdx.x * 8 + warp;
-  const int N = c.N;
-  if (x >= N) return;
-  const size_t ax = (size_t)b * N + x;
-  const int zx = c.w.z[ax];
-  const int n = c.w.n_eff[b];
-  if (x >= n || zx == 0) {
-    if (lane == 0) {
-      c.w.dEdcn[ax] = 0.0;
-      c.w.dEdq[ax] = 0.0;
-      c.w.adj32[ax] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    return;
-  }
-  const float4 *P = c.w.pos32 + (size_t)b * N;
-  const float4 *PL = c.w.pos32lo + (size_t)b * N;
-  const float4 px = P[x], lx = PL[x];
-  const int nslot = c.w.n_slots[b];
-  const int slot_x = c.w.slot[ax];
-  const size_t base = (size_t)b * N * N;
-  const float4 *T = c.w.ptf + base + (size_t)x * N;
-  Acc32 gx, gy, gz;
-  Acc32 dcn_acc, dq_acc;
-  for (int s = 0; s < nslot; ++s) {
-    float gacc[NFREQ];
-#pragma unroll
-    for (int w = 0; w < NFREQ; ++w) gacc[w] = 0.f;
-    for (int y = lane; y < n; y += 32) {
-      const size_t ay = (size_t)b * N + y;
-      if (y == x || c.w.z[ay] == 0 || c.w.slot[ay] != s) continue;
-      const size_t o = base + (size_t)x * N + y;
-      const float2 sp = c.w.prSP32[o];
-      const float S = sp.x, Pv = sp.y;
-      const float3 d = pos_diff(px, lx, P[y], PL[y]);
-      gx.add(2.0f * S * d.x);
-      gy.add(2.0f * S * d.y);
-      gz.add(2.0f * S * d.z);
-      if (Pv != 0.f) {
-        const float cw = T[y].w;  // sqrt(C6(q=0)) / r^3: C6(q=0) = w^2 r^6
-        const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-        const float D = Pv / (2.0f * (cw * cw) * (r2 * r2 * r2));
-        const float *A0y = c.w.A032 + a32_index(b, y, slot_x, 0, N, c.S);
-#pragma unroll
-        for (int w = 0; w < NFREQ; ++w) gacc[w] = fmaf(D, A0y[(size_t)w * N], gacc[w]);
-      }
-    }
-    const float mine = warp_reduce_scatter32(gacc);  // lane w: sum of gacc[w]
-    // chain rule to CN and q for this slot (lane = frequency)
-    if (lane < NFREQ) {
-      const size_t o = (ax * c.S + s) * NFREQ + lane;
-      const float g0w = mine;  // dE/dA'0_x
-      const float gw = c.w.G32[o];
-      const float *d = c.w.dA32 + 3 * o;
-      dcn_acc.add(gw * d[0]);
-      dcn_acc.add(g0w * d[2]);
-      dq_acc.add(gw * d[1]);
-    }
-  }
-  const Acc32 g0 = warp_sum_acc(gx), g1 = warp_sum_acc(gy), g2 = warp_sum_acc(gz);
-  const Acc32 dcn = warp_sum_acc(dcn_acc), dq = warp_sum_acc(dq_acc);
-  if (lane == 0) {
-    c.w.dEdcn[ax] = dcn.value();
-    c.w.dEdq[ax] = dq.value();
-    c.w.adj32[ax] = make_float4(dcn.hi + dcn.lo, 0.f, (float)c.w.q[ax], 0.f);
-    c.out.d_gradient[3 * ax] += g0.value();
-    c.out.d_gradient[3 * ax + 1] += g1.value();
-    c.out.d_gradient[3 * ax + 2] += g2.value();
-    c.out.d_energy[ax] += c.w.e3[ax];
-  }
-}
-
 // Forces through the D4 CN, the EEQ CN and the EEQ Coulomb matrix (FP32).
 __global__ void __launch_bounds__(256) pair_cn_bwd_mixed_kernel(Ctx c) {
   const int b = blockIdx.y;
@@ -1964,12 +1698,8 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   stage_begin(ST_PAIR_FWD, st);
   if (c.cfg.kind == D4_MODEL_D4)  // C6 on the tensor cores
     launch_pair_fwd_tc(c, st);
-  else if (pgrad)
-    pair_fwd_mixed_kernel<true, true><<<atoms, 256, 0, st>>>(c);
-  else if (grad)
-    pair_fwd_mixed_kernel<true, false><<<atoms, 256, 0, st>>>(c);
   else
-    pair_fwd_mixed_kernel<false, false><<<atoms, 256, 0, st>>>(c);
+    launch_pair_fwd_d4s32(c, st);
   stage_end(ST_PAIR_FWD, st);
   stage_begin(ST_ATM, st);
   if (pgrad)
@@ -1984,7 +1714,7 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
     if (pair_atm_bwd_tc_ok(c))  // C6(q=0) adjoint on the tensor cores
       launch_pair_atm_bwd_tc(c, st);
     else
-      pair_atm_bwd_mixed_kernel<<<atoms, 256, 0, st>>>(c);
+      launch_pair_bwd_d4s32(c, st);
     stage_end(ST_PAIR_ATM_BWD, st);
     if (eeq) {
       stage_begin(ST_EEQ_ADJ, st);
