@@ -22,31 +22,30 @@ constexpr int ATM_THREADS_PGRAD = 512;  // the parameter-gradient variant needs 
 
 // ---------------------------------------------------------------- weights
 
-// threads of tables32_kernel: the largest of its tables, 128 x 7 x 23
-constexpr int TABLES32_THREADS = ((MAX_ELEM_ID * NREF * NFREQ + 255) / 256) * 256;
-static_assert(TABLES32_THREADS >= MAX_ELEM_ID * MAX_ELEM_ID && TABLES32_THREADS >= ERF_TAB,
-              "tables32_kernel covers every table");
-
 // FP32 tables of the precision form, rebuilt on every call (20k values):
 // alpha32 [128][7][23]; ref32 [128][7] = (refcovcn, refq + zeff, Gaussians
 // per reference, zeta at q = 0 evaluated in FP64); el32 [128] = (zeff,
 // gam * gc); the erf nodes and 1/sqrt(rad_a^2 + rad_b^2) per element pair as
 // double-floats for the EEQ matrix.  Rows of elements without references are
 // zero.
-static __device__ __forceinline__ void tables32_entry(const Ctx &c, int t) {
+//
+// One table per CTA, FP64-heavy ones with few threads each: a warp's FP64
+// instruction takes 64 cycles of its sub-partition, and the tables ahead of the
+// structures spread over the SMs (all tables per thread, behind the structures:
+// 45 us for 1000 structures; now 11).
+constexpr int TC_PAIR = MAX_ELEM_ID * MAX_ELEM_ID / 256;  // CTAs of an element-pair table
+constexpr int TC_REF = MAX_ELEM_ID * NREF / 64, TC_ERF = (ERF_TAB + 127) / 128;
+constexpr int TC_ALPHA = (MAX_ELEM_ID * NREF * NFREQ + 255) / 256;
+constexpr int TABLE_CTAS = TC_REF + TC_ERF + 1 + 3 * TC_PAIR + TC_ALPHA;
+static_assert(MAX_ELEM_ID * NREF % 64 == 0 && MAX_ELEM_ID * MAX_ELEM_ID % 256 == 0 &&
+              MAX_ELEM_ID <= 256 && NFREQ <= 256, "the tables' CTAs cover them");
+
+static __device__ __forceinline__ void tables32(const Ctx &c, int cta) {
   const int nz = c.tab.n_ref_elem < MAX_ELEM_ID ? c.tab.n_ref_elem : MAX_ELEM_ID;
-  if (t < MAX_ELEM_ID * NREF * NFREQ) {
-    const int z = t / (NREF * NFREQ);
-    const dfl a = z < nz ? df_from(c.tab.alpha[t]) : dfl{0.f, 0.f};
-    c.w.alpha32[t] = a.hi;
-    c.w.alpha32lo[t] = a.lo;
-  }
-  if (t < NFREQ) {
-    const dfl f = df_from(sqrt(THOPI * c.tab.freq_weights[t]));
-    c.w.sfw[t] = make_float2(f.hi, f.lo);
-  }
-  if (t < MAX_ELEM_ID * NREF) {
-    const int z = t / NREF;
+  const int tid = threadIdx.x;
+  if (cta < TC_REF) {
+    if (tid >= 64) return;
+    const int t = cta * 64 + tid, z = t / NREF;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     float z0lo = 0.f;
     if (z < nz && z < c.tab.n_elem) {
@@ -60,65 +59,110 @@ static __device__ __forceinline__ void tables32_entry(const Ctx &c, int t) {
     }
     c.w.ref32[t] = v;
     c.w.z0lo[t] = z0lo;
+    return;
   }
-  if (t < MAX_ELEM_ID) {
-    float2 e = make_float2(0.f, 0.f);
-    if (t < nz && t < c.tab.n_elem)
-      e = make_float2((float)c.tab.zeff[t], (float)(c.tab.gam[t] * c.cfg.gc));
-    c.w.el32[t] = e;
-    dfl d = {0.f, 0.f};
-    if (t < c.tab.n_elem) d = df_from(c.tab.eeq_eta[t] + SQRT_2_OVER_PI / c.tab.eeq_rad[t]);
-    c.w.eeq_diag[t] = make_float2(d.hi, d.lo);
-  }
-  if (t < ERF_TAB) {  // nodes of the double-float erf
+  cta -= TC_REF;
+  if (cta < TC_ERF) {  // nodes of the double-float erf
+    const int t = cta * 128 + tid;
+    if (tid >= 128 || t >= ERF_TAB) return;
     const double x0 = (double)t / (double)ERF_SCALE;
     const dfl e = df_from(erf(x0)), d = df_from(2.0 / sqrt(M_PI) * exp(-x0 * x0));
     c.w.erf_tab[t] = make_float4(e.hi, e.lo, d.hi, d.lo);
+    return;
   }
-  if (t < MAX_ELEM_ID * MAX_ELEM_ID) {  // R0, qq, R0^6, R0^8 of the table r4r2 values
-    const int za = t / MAX_ELEM_ID, zb = t % MAX_ELEM_ID;
-    float4 A = make_float4(0.f, 0.f, 0.f, 0.f), Bq = A;
-    if (za < c.tab.n_elem && zb < c.tab.n_elem) {
-      const double qq = 3.0 * c.tab.r4r2[za] * c.tab.r4r2[zb];
-      const double R0 = c.par.a1 * sqrt(qq) + c.par.a2;
-      const double R02 = R0 * R0, R06 = R02 * R02 * R02;
-      const dfl r0 = df_from(R0), q = df_from(qq), r6 = df_from(R06), r8 = df_from(R06 * R02);
-      A = make_float4(r0.hi, r0.lo, q.hi, q.lo);
-      Bq = make_float4(r6.hi, r6.lo, r8.hi, r8.lo);
+  cta -= TC_ERF;
+  if (cta == 0) {
+    const int t = tid;
+    if (t < NFREQ) {
+      const dfl f = df_from(sqrt(THOPI * c.tab.freq_weights[t]));
+      c.w.sfw[t] = make_float2(f.hi, f.lo);
     }
-    c.w.pairA[t] = A;
-    c.w.pairB[t] = Bq;
+    if (t < MAX_ELEM_ID) {
+      float2 e = make_float2(0.f, 0.f);
+      if (t < nz && t < c.tab.n_elem)
+        e = make_float2((float)c.tab.zeff[t], (float)(c.tab.gam[t] * c.cfg.gc));
+      c.w.el32[t] = e;
+      dfl d = {0.f, 0.f};
+      if (t < c.tab.n_elem) d = df_from(c.tab.eeq_eta[t] + SQRT_2_OVER_PI / c.tab.eeq_rad[t]);
+      c.w.eeq_diag[t] = make_float2(d.hi, d.lo);
+    }
+    return;
   }
-  if (t < MAX_ELEM_ID * MAX_ELEM_ID) {  // CN pair constants in FP64, kept as double-floats
-    // (an FP32 rounding of them would shift every pair of an element pair the
-    // same way: a bias that adds up over the structure instead of averaging out)
+  cta -= 1;
+  if (cta < 3 * TC_PAIR) {
+    const int table = cta / TC_PAIR, t = (cta % TC_PAIR) * 256 + tid;
     const int za = t / MAX_ELEM_ID, zb = t % MAX_ELEM_ID;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (za < c.tab.n_elem && zb < c.tab.n_elem && za > 0 && zb > 0) {
-      const dfl a = df_from(1.0 / (c.tab.cov_d3[za] + c.tab.cov_d3[zb]));
-      const dfl e = df_from(en_factor(c.tab.en[za], c.tab.en[zb], c.par.k4, c.par.k5, c.par.k6));
-      v = make_float4(a.hi, a.lo, e.hi, e.lo);
+    const bool in = za < c.tab.n_elem && zb < c.tab.n_elem;
+    if (table == 0) {  // R0, qq, R0^6, R0^8 of the table r4r2 values
+      float4 A = make_float4(0.f, 0.f, 0.f, 0.f), Bq = A;
+      if (in) {
+        const double qq = 3.0 * c.tab.r4r2[za] * c.tab.r4r2[zb];
+        const double R0 = c.par.a1 * sqrt(qq) + c.par.a2;
+        const double R02 = R0 * R0, R06 = R02 * R02 * R02;
+        const dfl r0 = df_from(R0), q = df_from(qq), r6 = df_from(R06), r8 = df_from(R06 * R02);
+        A = make_float4(r0.hi, r0.lo, q.hi, q.lo);
+        Bq = make_float4(r6.hi, r6.lo, r8.hi, r8.lo);
+      }
+      c.w.pairA[t] = A;
+      c.w.pairB[t] = Bq;
+    } else if (table == 1) {  // CN pair constants in FP64, kept as double-floats
+      // (an FP32 rounding of them would shift every pair of an element pair the
+      // same way: a bias that adds up over the structure instead of averaging out)
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (in && za > 0 && zb > 0) {
+        const dfl a = df_from(1.0 / (c.tab.cov_d3[za] + c.tab.cov_d3[zb]));
+        const dfl e = df_from(en_factor(c.tab.en[za], c.tab.en[zb], c.par.k4, c.par.k5, c.par.k6));
+        v = make_float4(a.hi, a.lo, e.hi, e.lo);
+      }
+      c.w.cnpair[t] = v;
+    } else {  // 1 / sqrt(rad_a^2 + rad_b^2)
+      dfl g = {0.f, 0.f};
+      if (in) {
+        const double ra = c.tab.eeq_rad[za], rb = c.tab.eeq_rad[zb];
+        g = df_from(1.0 / sqrt(ra * ra + rb * rb));
+      }
+      c.w.igam[t] = make_float2(g.hi, g.lo);
     }
-    c.w.cnpair[t] = v;
+    return;
   }
-  if (t < MAX_ELEM_ID * MAX_ELEM_ID) {  // 1 / sqrt(rad_a^2 + rad_b^2)
-    const int za = t / MAX_ELEM_ID, zb = t % MAX_ELEM_ID;
-    dfl g = {0.f, 0.f};
-    if (za < c.tab.n_elem && zb < c.tab.n_elem) {
-      const double ra = c.tab.eeq_rad[za], rb = c.tab.eeq_rad[zb];
-      g = df_from(1.0 / sqrt(ra * ra + rb * rb));
-    }
-    c.w.igam[t] = make_float2(g.hi, g.lo);
+  const int t = (cta - 3 * TC_PAIR) * 256 + tid;
+  if (t < MAX_ELEM_ID * NREF * NFREQ) {
+    const dfl a = t / (NREF * NFREQ) < nz ? df_from(c.tab.alpha[t]) : dfl{0.f, 0.f};
+    c.w.alpha32[t] = a.hi;
+    c.w.alpha32lo[t] = a.lo;
   }
 }
 
-// The per-structure set-up (prep_structure: CTAs 0 .. B-1) and the per-call
-// FP32 tables (the other CTAs) in one launch: neither needs the other.
+// The per-call FP32 tables (the first CTAs) and the per-structure set-up
+// (prep_structure) in one launch: neither needs the other.
 __global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c) {
-  if ((int)blockIdx.x < c.B)
-    prep_structure(c, blockIdx.x);
+  if ((int)blockIdx.x < TABLE_CTAS)
+    tables32(c, blockIdx.x);
   else
-    tables32_entry(c, ((int)blockIdx.x - c.B) * 256 + threadIdx.x);
+    prep_structure(c, (int)blockIdx.x - TABLE_CTAS);
+}
+
+// exp(x), |x| <= 80, rounded once: reduction by ln 2 = 355/512 - 2.1e-4 (Cody and
+// Waite, Software Manual for the Elementary Functions, 1980) and the series, its first terms in double-float (within 1e-10 before the
+// rounding).  In place of an FP64 exp, whose 30 instructions for every reference of
+// every atom were most of the weights' time.
+__device__ __forceinline__ float exp_once(dfl x) {
+  const float n = rintf(x.hi * 1.44269504f);
+  const float ch = 2.1219444e-4f;
+  constexpr float cl = (float)(2.1219444005469058277e-4 - (double)2.1219444e-4f);
+  const float p = n * ch;
+  const dfl t = df_two_sum(fmaf(n, -0.693359375f, x.hi), p);  // (exact: few bits)
+  const dfl r = df_fast(t.hi, t.lo + (fmaf(n, ch, -p) + fmaf(n, cl, x.lo)));
+  const dfl r2 = df_mul(r, r);
+  const dfl r3 = df_mul(df_mul(r2, r), dfl{1.f / 6.f, (float)(1.0 / 6.0 - (double)(1.f / 6.f))});
+  const float q = fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, 1.f / 362880.f,
+                       1.f / 40320.f), 1.f / 5040.f), 1.f / 720.f), 1.f / 120.f), 1.f / 24.f);
+  const dfl tail = df_two_sum(r3.hi, r2.hi * r2.hi * q);
+  const dfl h = df_two_sum(0.5f * r2.hi, tail.hi);
+  const dfl u = df_two_sum(r.hi, h.hi);
+  const dfl v = df_two_sum(1.f, u.hi);
+  const float lo = v.lo + (u.lo + (r.lo + (h.lo + fmaf(0.5f, r2.lo, tail.lo + r3.lo))));
+  return (v.hi + lo) * __int_as_float(((int)n + 127) << 23);
 }
 
 // transposed index of (structure b, atom i, slot s, frequency w)
@@ -130,7 +174,10 @@ __device__ __forceinline__ size_t a32_index(int b, int i, int s, int w, int N, i
 // A_i(w) = sum_r gw_ir zeta_ir alpha_{Z_i r}(w) at q and at q = 0, with their
 // CN / q derivatives, in FP32 (model/d4.py:103-228, model/d4s.py:109-248).
 // One thread per (atom, slot); lanes over consecutive atoms, so that the
-// transposed A32 / A032 rows are stored coalesced.
+// transposed A32 / A032 rows are stored coalesced; the derivatives, a row per
+// atom, leave through shared memory (three words at stride 276 bytes per thread
+// were 32 sectors each).  With that and exp_once, 512 structures of 8..200 atoms
+// 74 -> 54 us, 256 of 20..150 68 -> 38, D4S of 96 structures 107 -> 75.
 //
 // The Gaussian exponents c k dcn_r^2 are taken relative to the nearest
 // reference (smallest c dcn^2), whose first Gaussian becomes exp(0) = 1:
@@ -148,15 +195,16 @@ __device__ __forceinline__ size_t a32_index(int b, int i, int s, int w, int N, i
 // zeta_n alpha_n + sum_{r != n} gw_r (zeta_r alpha_r - zeta_n alpha_n), the
 // first term as a double-float, the corrections in FP32 (exact in the limit
 // of one reference, no value near 1 rounded).
-__global__ void __launch_bounds__(128) weights_mixed_kernel(Ctx c) {
+constexpr int WEIGHT_ATOMS = 128;
+template <bool GRAD>
+__global__ void __launch_bounds__(WEIGHT_ATOMS) weights_mixed_kernel(Ctx c) {
   const int b = blockIdx.y;
   const int S = c.S, N = c.N;
   const int s = blockIdx.x % S;
-  const int i = (blockIdx.x / S) * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const size_t ai = (size_t)b * N + i;
-  const int zi = c.w.z[ai];
-  const bool grad = c.w.dA32 != nullptr;
+  const int i0 = (blockIdx.x / S) * WEIGHT_ATOMS, i = i0 + threadIdx.x;
+  __shared__ float s_d[GRAD ? WEIGHT_ATOMS * 3 * NFREQ : 1];
+  const size_t ai = (size_t)b * N + (i < N ? i : 0);
+  const int zi = i < N ? c.w.z[ai] : 0;
   const bool live = i < c.w.n_eff[b] && zi != 0 && s < c.w.n_slots[b];
   // gq / g0: coefficients of the corrections (gw_r zeta_r for r != n,
   // -G zeta_n with G = sum_{r != n} gw_r for the nearest reference n);
@@ -187,6 +235,7 @@ __global__ void __launch_bounds__(128) weights_mixed_kernel(Ctx c) {
     const double gam64 = c.tab.gam[zi] * c.cfg.gc;
     // one FP64 division per atom (GB300 runs FP64 at 1/64 of the FP32 rate)
     const double gq64 = qmod64 > 0.0 ? gam64 / qmod64 : 0.0;
+    const dfl gad = df_from(c.cfg.ga);
 #pragma unroll
     for (int r = 0; r < NREF; ++r) {
       rv[r] = R[r];
@@ -200,13 +249,17 @@ __global__ void __launch_bounds__(128) weights_mixed_kernel(Ctx c) {
       y64[r] = cfr * d * d;
       dcn[r] = (float)d;
       cf[r] = (float)cfr;
-      // zeta(q) = exp(-ga expm1(u)) with the outer exponential in FP64,
+      // zeta(q) = exp(-ga expm1(u)) with the outer exponential
       // rounded once: FP32 expf carries a mean relative error of ~+5e-9,
       // which C6 ~ zeta_i zeta_j would double into a bias shared by every pair
       // of the structure (expm1f's error is scaled down by u ~ 0.1 there)
       const double u64 = gq64 * (q - c.tab.refq[zi * NREF + r]);
       ua[r] = (float)u64;
-      zq[r] = (float)exp(-c.cfg.ga * (double)expm1f((float)u64));
+      const float em1 = expm1f((float)u64), ex = -gad.hi * em1;
+      if (fabsf(ex) <= 80.f)
+        zq[r] = exp_once(df_fast(ex, fmaf(-gad.hi, em1, -ex) - gad.lo * em1));
+      else
+        zq[r] = (float)exp(-c.cfg.ga * (double)em1);
       if (y64[r] < best) {
         best = y64[r];
         rn = r;
@@ -305,14 +358,23 @@ __global__ void __launch_bounds__(128) weights_mixed_kernel(Ctx c) {
     const dfl A0 = df_two_sum(b0h, a0);
     const float A0l = A0.lo + (fmaf(z0n, vn, -b0h) + fmaf(z0nl, vn, fmaf(z0n, vnl, al0)));
     const float2 f = c.w.sfw[w];
-    const size_t t = a32_index(b, i, s, w, N, S);
-    c.w.A32[t] = fmaf(A.hi, f.x, fmaf(A.hi, f.y, Al * f.x));
-    c.w.A032[t] = fmaf(A0.hi, f.x, fmaf(A0.hi, f.y, A0l * f.x));
-    if (grad) {
-      float *d = c.w.dA32 + 3 * ((ai * S + s) * NFREQ + w);
+    if (i < N) {
+      const size_t t = a32_index(b, i, s, w, N, S);
+      c.w.A32[t] = fmaf(A.hi, f.x, fmaf(A.hi, f.y, Al * f.x));
+      c.w.A032[t] = fmaf(A0.hi, f.x, fmaf(A0.hi, f.y, A0l * f.x));
+    }
+    if (GRAD) {
+      float *d = s_d + (threadIdx.x * NFREQ + w) * 3;
       d[0] = da_dcn * f.x;
       d[1] = da_dq * f.x;
       d[2] = da0_dcn * f.x;
+    }
+  }
+  if (GRAD) {  // a row of 69 derivatives per atom, written along the rows
+    __syncthreads();
+    for (int t = threadIdx.x; t < min(WEIGHT_ATOMS, N - i0) * 3 * NFREQ; t += WEIGHT_ATOMS) {
+      const int a = t / (3 * NFREQ), k = t % (3 * NFREQ);
+      c.w.dA32[((size_t)((size_t)b * N + i0 + a) * S + s) * 3 * NFREQ + k] = s_d[t];
     }
   }
 }
@@ -1658,7 +1720,7 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
     if (out.d_cn) c.out.d_cn = c.w.zs_ocn;
     if (out.d_cn_eeq) c.out.d_cn_eeq = c.w.zs_ocnq;
   }
-  prep_tables_kernel<<<B + TABLES32_THREADS / 256, 256, 0, st>>>(c);
+  prep_tables_kernel<<<TABLE_CTAS + B, 256, 0, st>>>(c);
   {
     int P = 1;
     while (P < B && P < SORDER_MAX) P <<= 1;
@@ -1693,7 +1755,11 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   }
   stage_end(ST_EEQ, st);
   stage_begin(ST_WEIGHTS, st);
-  weights_mixed_kernel<<<dim3((unsigned)(((N + 127) / 128) * c.S), B), 128, 0, st>>>(c);
+  const dim3 wgrid((unsigned)(((N + WEIGHT_ATOMS - 1) / WEIGHT_ATOMS) * c.S), B);
+  if (c.w.dA32 != nullptr)
+    weights_mixed_kernel<true><<<wgrid, WEIGHT_ATOMS, 0, st>>>(c);
+  else
+    weights_mixed_kernel<false><<<wgrid, WEIGHT_ATOMS, 0, st>>>(c);
   stage_end(ST_WEIGHTS, st);
   stage_begin(ST_PAIR_FWD, st);
   if (c.cfg.kind == D4_MODEL_D4)  // C6 on the tensor cores
