@@ -83,7 +83,7 @@ template <bool GRAD, bool PGRAD>
 __global__ void __launch_bounds__(TC_THREADS, 2) pair_fwd_tc_kernel(Ctx c) {
   extern __shared__ __align__(128) unsigned char s_raw[];
   TcSmem &S = *reinterpret_cast<TcSmem *>(s_raw);
-  const int b = blockIdx.y;
+  const int b = c.w.sorder[blockIdx.y];  // largest structures first
   const int N = c.N;
   const int n = c.w.n_eff[b];
   const int i0 = blockIdx.x * TC_M;
@@ -588,7 +588,7 @@ __device__ __forceinline__ void split_tf32(float *hi, float *lo, int off, float 
 __global__ void __launch_bounds__(BW_THREADS) pair_atm_bwd_tc_kernel(Ctx c) {
   extern __shared__ __align__(128) unsigned char s_raw[];
   BwSmem &S = *reinterpret_cast<BwSmem *>(s_raw);
-  const int b = blockIdx.y;
+  const int b = c.w.sorder[blockIdx.y];  // largest structures first
   const int N = c.N;
   const int n = c.w.n_eff[b];
   const int x0 = blockIdx.x * TC_M;
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(BW_THREADS) pair_atm_bwd_tc_kernel(Ctx c) {
 // Chain rule of the split tensor-core adjoint (thread per atom): dE/dCN and
 // dE/dq from G (pair kernel) and the accumulated G0, and E2 + E3.
 __global__ void __launch_bounds__(256) pair_atm_bwd_finish_kernel(Ctx c) {
-  const int b = blockIdx.y;
+  const int b = c.w.sorder[blockIdx.y];  // largest structures first
   const int N = c.N;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= N) return;
