@@ -29,6 +29,8 @@ constexpr int A3_THREADS = 128;
 constexpr int A3_ROW = 10;        // row and group strides of the (i, j) sums in shared memory
 constexpr int A3_GROUP = 88;      // (float2; no bank conflicts)
 constexpr int A3_STAGES = 3;      // staged chunks of eight inner atoms per warp
+constexpr int A3_REC = 2 * A3 + 1;  // float4 per staged row: the four groups' broadcasts in
+                                    // different banks
 
 // Halving exchanges over the lane bits H, H/2, ... (STEPS of them): v[p]
 // for p < NV >> STEPS ends as the sum over the 2^STEPS lanes that differ in
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(1024) atm32_plan_kernel(Ctx c, int s) {
 template <bool GRAD, bool PGRAD>
 __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c, int s) {
   __shared__ float s_c[A3_THREADS / 32][A3 * 32];
-  __shared__ float4 s_rec[A3_THREADS / 32][A3_STAGES][8 * 2 * A3];
+  __shared__ float4 s_rec[A3_THREADS / 32][A3_STAGES][8 * A3_REC];
   __shared__ __align__(16) float2 s_sum[A3_THREADS / 32][4 * A3_GROUP];
   const int lane = threadIdx.x & 31, q = lane >> 3;
   const int N = c.N;
@@ -350,9 +352,9 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
       for (int tt = 0; tt < A3; ++tt) cj[32 * tt] = 0.f;
     }
     A3Pg pg;
-    // records of eight inner atoms at a time: entry 16 r + t is (i, j0 + t),
-    // 16 r + 8 + t is (i, kc + t), i = first + r; copied two chunks ahead
-    float4(*stage)[8 * 2 * A3] = s_rec[threadIdx.x >> 5];
+    // records of eight inner atoms at a time: entry t of row r is (i, j0 + t),
+    // 8 + t (i, kc + t), i = first + r; copied two chunks ahead
+    float4(*stage)[8 * A3_REC] = s_rec[threadIdx.x >> 5];
     float2 *red = s_sum[threadIdx.x >> 5] + A3_GROUP * q;
     auto fetch = [&](int first_i, int st) {
       if (first_i < iend) {
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
           const int i = first_i + r, x = col < A3 ? j0 + col : kc + col - A3;
           const bool ok = i < iend && x > i && (col < A3 ? ((jmask >> col) & 1u) != 0u : x < n) &&
                           (!gaps || (Z[i] != 0 && Z[x] != 0));
-          copy16(&stage[st][slot], a.T + (ok ? (size_t)i * N + x : 0), ok);
+          copy16(&stage[st][A3_REC * r + col], a.T + (ok ? (size_t)i * N + x : 0), ok);
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
         const int i = ib + 4 * half + q;
         if (ib + 4 * half >= iend) break;
         const bool iok = i < iend && (!gaps || Z[i] != 0);
-        const float4 *rec = stage[st] + 2 * A3 * (4 * half + q);
+        const float4 *rec = stage[st] + A3_REC * (4 * half + q);
         const bool mask =
             task_far || (any_far && __any_sync(0xffffffffu, iok && far2[i] > a.cut2));
         if (mask)
