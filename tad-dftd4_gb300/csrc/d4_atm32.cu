@@ -672,6 +672,8 @@ __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float
   int ti, tj;  // rows ti, columns tj >= ti
   tri_entry(blockIdx.x, tj, ti);
   if (tj * 32 >= n) return;
+  // the sides of a triple with weight are within twice the cutoff
+  if (c.far_skip && block_gap_sq(c, b, ti, tj) > 4.f * c.pf.cut3 * c.pf.cut3) return;
   float2 *SP = c.w.prSP32 + (size_t)b * N * N;
   double *e3 = c.w.e3 + (size_t)b * N;
   const float cut2 = c.pf.cut3 * c.pf.cut3;

@@ -189,6 +189,7 @@ struct Workspace {
   int64_t *zs_num;    // [B*N]
   double *zs_pos, *zs_q, *zs_r4, *zs_w;           // [B*N*3], [B*N] each
   double *zs_e, *zs_g, *zs_oq, *zs_ocn, *zs_ocnq;  // [B*N], [B*N*3], [B*N] each
+  float4 *zs_box;     // [B][(N + 31) / 32][2] bounding boxes of 32 consecutive atoms
   int *sorder;      // [B] structures by decreasing n_eff (launch order of the
                     // per-structure kernels of the precision form)
   unsigned *atm_rowmax;  // [B*N] largest r^2 over the real pairs of each atom (FP32
@@ -327,6 +328,7 @@ inline Workspace carve_workspace(void *base, int B, int N, int S, uint32_t flags
       w.zs_oq = (double *)take(8 * BN);
       w.zs_ocn = (double *)take(8 * BN);
       w.zs_ocnq = (double *)take(8 * BN);
+      w.zs_box = (float4 *)take(32 * (size_t)B * ((N + 31) / 32));
     }
     if (!atm_smem_fits(N)) {
       w.nbr = (int *)take(sizeof(int) * BNN);
@@ -363,6 +365,7 @@ struct Ctx {
   int B, N, S;
   uint32_t flags;
   int zsorted;    // the atoms are in spatial order (set by launch_mixed)
+  int far_skip;   // pair kernels pass over far blocks of it (D4; set by launch_mixed)
   int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
   int pair64;     // the pair stages of d4_pair64.cu run (set by launch_fp64)
   double cut2_sq, cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp2, cut_disp3 (likewise)
@@ -434,6 +437,50 @@ __device__ __forceinline__ void zeta_and_deriv(double gam, double qref, double q
 __device__ __forceinline__ double pair_t(double log_t) {
   const double t = exp(log_t);
   return t > PAIR_T_MAX ? PAIR_T_MAX : t;
+}
+
+// Square of a lower bound of the distance of atoms in blocks A and B of 32
+// consecutive atoms of structure b (structures in spatial order; infinite where
+// a block has no atoms): the boxes' gap, less the rounding of the FP32 positions
+// (a box's .w) and a relative 1e-5, beyond that of any kernel's distances.
+__device__ __forceinline__ float block_gap_sq(const Ctx &c, int b, int A, int B) {
+  const float4 *x = c.w.zs_box + 2 * (size_t)b * ((c.N + 31) / 32);
+  const float4 la = x[2 * A], ha = x[2 * A + 1], lb = x[2 * B], hb = x[2 * B + 1];
+  const float slack = la.w + lb.w;
+  const float dx = fmaxf(fmaxf(la.x - hb.x, lb.x - ha.x) - slack, 0.f);
+  const float dy = fmaxf(fmaxf(la.y - hb.y, lb.y - ha.y) - slack, 0.f);
+  const float dz = fmaxf(fmaxf(la.z - hb.z, lb.z - ha.z) - slack, 0.f);
+  // (no contraction: the same value in every kernel)
+  const float s = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+  return __fmul_rn(0.99998f, s);
+}
+
+// First atoms of the blocks of 32 that a warp has to visit for an atom of block
+// A: all blocks in turn, or those not farther than cut_sq of a structure in
+// spatial order (32 tests at a time, a lane each).
+struct NearBlocks {
+  const Ctx &c;
+  int b, A, n, base;
+  float cut_sq;
+  unsigned mask;
+  // the next block's first atom, or n and beyond at the end (all lanes)
+  __device__ __forceinline__ int next() {
+    if (!c.zsorted) return base += 32;
+    while (mask == 0u) {
+      base += 32 * 32;
+      if (base >= n) return n;
+      const int k = base / 32 + (threadIdx.x & 31);
+      mask = __ballot_sync(0xffffffffu,
+                           32 * k < n && !(block_gap_sq(c, b, A, k) > cut_sq));
+    }
+    const int k = __ffs(mask) - 1;
+    mask &= mask - 1u;
+    return base + 32 * k;
+  }
+};
+__device__ __forceinline__ NearBlocks near_blocks(const Ctx &c, int b, int A, int n,
+                                                  float cut_sq) {
+  return {c, b, A, n, c.zsorted ? -32 * 32 : -32, cut_sq, 0u};
 }
 
 // (row, col), col <= row, of entry t of a packed lower triangle

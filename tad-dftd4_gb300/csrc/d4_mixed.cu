@@ -133,6 +133,30 @@ static __device__ __forceinline__ void tables32(const Ctx &c, int cta) {
   }
 }
 
+// Bounding boxes of 32 consecutive atoms each (block_gap_sq), a warp per block.
+__global__ void __launch_bounds__(256) block_boxes_kernel(Ctx c) {
+  const int b = blockIdx.y, k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int nb = (c.N + 31) / 32, i = 32 * k + lane;
+  if (k >= nb) return;
+  const size_t a = (size_t)b * c.N + (i < c.N ? i : 0);
+  const bool real = i < c.N && c.w.z[a] != 0;
+  const float4 p = c.w.pos32[a];
+  const float lo[3] = {real ? p.x : INFINITY, real ? p.y : INFINITY, real ? p.z : INFINITY};
+  const float hi[3] = {real ? p.x : -INFINITY, real ? p.y : -INFINITY, real ? p.z : -INFINITY};
+  float l[3], h[3], far = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    l[d] = -warp_maxf(-lo[d]);
+    h[d] = warp_maxf(hi[d]);
+    if (l[d] <= h[d]) far = fmaxf(far, fmaxf(fabsf(l[d]), fabsf(h[d])));
+  }
+  if (lane == 0) {
+    float4 *o = c.w.zs_box + 2 * ((size_t)b * nb + k);
+    o[0] = make_float4(l[0], l[1], l[2], 1e-6f * far);
+    o[1] = make_float4(h[0], h[1], h[2], 0.f);
+  }
+}
+
 // The per-call FP32 tables (the first CTAs) and the per-structure set-up
 // (prep_structure) in one launch: neither needs the other.
 __global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c) {
@@ -388,6 +412,8 @@ __global__ void __launch_bounds__(WEIGHT_ATOMS) weights_mixed_kernel(Ctx c) {
 // factor as a double-float per element pair (no FP32-rounded constant), and
 // compensated per-lane sums; FP64 per-atom totals and the smooth EEQ cap in
 // FP64.
+// SORTED: structures in spatial order, whose far blocks are passed over.
+template <bool SORTED>
 __global__ void __launch_bounds__(256) cn_mixed_kernel(Ctx c) {
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -414,8 +440,11 @@ __global__ void __launch_bounds__(256) cn_mixed_kernel(Ctx c) {
   const float cut_cn = c.pf.cut_cn, cut_q = c.pf.cut_q;
   const float4 *CP = c.w.cnpair + (size_t)zi * MAX_ELEM_ID;
   Acc32 s_d4, s_q;
-  for (int j = lane; j < n; j += 32) {
-    const int zj = c.w.z[(size_t)b * N + j];
+  const float cut = fmaxf(cut_cn, cut_q);
+  NearBlocks near = near_blocks(c, b, i >> 5, n, cut * cut);
+  for (int j0 = SORTED ? near.next() : 0; j0 < n; j0 = SORTED ? near.next() : j0 + 32) {
+    const int j = j0 + lane;
+    const int zj = j < n ? c.w.z[(size_t)b * N + j] : 0;
     if (j == i || zj == 0) continue;
     const float4 pj = P[j];
     const float4 cp = CP[zj];
@@ -829,7 +858,8 @@ __global__ void __launch_bounds__(256) atm_nbr_kernel(Ctx c) {
   int *L = c.w.nbr + (bN + j) * N;
   const int *Z = c.w.z + bN;
   int base = 0;
-  for (int k0 = 0; k0 < n; k0 += 32) {
+  auto near = near_blocks(c, b, j >> 5, n, cut2);
+  for (int k0 = near.next(); k0 < n; k0 = near.next()) {
     const int k = k0 + lane;
     bool ok = false;
     if (k < n && k != j && Z[k] != 0) ok = T[k].x <= cut2;
@@ -1694,6 +1724,11 @@ static void launch_atm(const Ctx &c, cudaStream_t st) {
     launch_atm_mirror(c, st, tiled, tiled && PGRAD ? c.pf.s9 : 1.f);
 }
 
+// Pair kernels pass over far blocks from this size (C6 and two-body term + ATM
+// adjoints, us, at cutoffs 50 and 25: 16000 atoms 7139 -> 5558, 8000 1977 -> 1725,
+// 6000 1176 -> 1061, but 4000 521 -> 526: too few blocks are far).
+constexpr int FAR_MIN = 5000;
+
 int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   Ctx c = c_in;
   const int B = c.B, N = c.N;
@@ -1721,6 +1756,10 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
     if (out.d_cn_eeq) c.out.d_cn_eeq = c.w.zs_ocnq;
   }
   prep_tables_kernel<<<TABLE_CTAS + B, 256, 0, st>>>(c);
+  if (c.zsorted) {
+    block_boxes_kernel<<<dim3(((N + 31) / 32 + 7) / 8, B), 256, 0, st>>>(c);
+    c.far_skip = c.cfg.kind == D4_MODEL_D4 && N >= FAR_MIN;
+  }
   {
     int P = 1;
     while (P < B && P < SORDER_MAX) P <<= 1;
@@ -1731,7 +1770,10 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
   }
   stage_end(ST_PREP, st);
   stage_begin(ST_CN, st);
-  cn_mixed_kernel<<<atoms, 256, 0, st>>>(c);
+  if (c.zsorted)
+    cn_mixed_kernel<true><<<atoms, 256, 0, st>>>(c);
+  else
+    cn_mixed_kernel<false><<<atoms, 256, 0, st>>>(c);
   stage_end(ST_CN, st);
   const size_t vec_bytes = 4 * eeq_mixed_vec_floats(N);
   const size_t tri_bytes = (size_t)4 * ((size_t)N * (N + 1) / 2);
