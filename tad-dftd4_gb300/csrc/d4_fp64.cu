@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
   const double *P = c.positions + 3 * ab;
   const int *Z = c.w.z + ab;
   const float kcn32 = (float)c.par.kcn;
+  const double ik6 = 1.0 / c.par.k6;
   auto evaluate = [&](int i, int j) {
     const int zi = Z[i], zj = Z[j];
     const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
@@ -51,8 +52,8 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
     const double x = r * rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     const double cf = 0.5 * erfc(c.par.kcn * (x - 1.0));
     if (r <= c.par.cut_cn) {
-      const double v =
-          cf * en_factor(c.tab.en[zi], c.tab.en[zj], c.par.k4, c.par.k5, c.par.k6);
+      const double t = fabs(c.tab.en[zi] - c.tab.en[zj]) + c.par.k5;
+      const double v = cf * (c.par.k4 * exp(-(t * t) * ik6));  // en_factor with 1 / k6
       atomicAdd(&c.w.cn[ab + i], v);
       atomicAdd(&c.w.cn[ab + j], v);
     }

@@ -12,8 +12,8 @@
 // Measured, 64 structures of 8..200 atoms / 360 of 30 atoms / 57 atoms (us;
 // before: a warp per atom over ordered pairs, d4_fp64.cu):
 //   C6, two-body term, records   566 / 337 / 58 -> 197 / 71 / 17
-//   C6 adjoints, chain rule      189 / 188 / 30 -> 133 / 94 / 15
-//   CN / EEQ adjoints, forces    455 / 153 / 35 -> 197 / 98 / 21
+//   C6 adjoints, chain rule      189 / 188 / 30 -> 133 / 71 / 14
+//   CN / EEQ adjoints, forces    455 / 153 / 35 -> 186 / 92 / 20
 #include "d4_common.cuh"
 #include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
@@ -225,6 +225,7 @@ constexpr int BX = 4;  // atoms (warps) per CTA of pair64_bwd_kernel
 template <bool D4S>
 __global__ void __launch_bounds__(32 * BX) pair64_bwd_kernel(Ctx c) {
   __shared__ double s_a[D4S ? 1 : 32 * 2 * NFREQ];
+  __shared__ double2 s_kd[D4S ? 1 : BX][32];  // dE/dC6 and its like at q = 0 of the partners
   const int b = blockIdx.y, N = c.N, n = c.w.n_eff[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int x = blockIdx.x * BX + warp;
@@ -239,51 +240,89 @@ __global__ void __launch_bounds__(32 * BX) pair64_bwd_kernel(Ctx c) {
   const int nslot = D4S ? c.w.n_slots[b] : 1;
   const int slot_x = D4S ? c.w.slot[ax] : 0;
   double psum = 0.0, dcn = 0.0, dq = 0.0;
-  for (int s = 0; s < nslot; ++s) {
-    double g[24], g0[24];
-#pragma unroll
-    for (int w = 0; w < 24; ++w) g[w] = g0[w] = 0.0;
+  // Few partners: a lane per frequency, the partners in turn (two FMAs each);
+  // else a lane per partner (46 FMAs per 32 of them and 48 additions to sum up).
+  if (!D4S && 2 * n <= 46 * ((n + 31) / 32) + 48) {
+    double g = 0.0, g0 = 0.0;
     for (int y0 = 0; y0 < n; y0 += 32) {
-      if (!D4S) {
-        __syncthreads();
-        const int ny = min(32, n - y0);
-        for (int t = threadIdx.x; t < ny * NFREQ; t += 32 * BX) {
-          const int k = t / NFREQ, w = t % NFREQ;
-          s_a[2 * k * NFREQ + w] = c.w.A[(ab + y0 + k) * NFREQ + w];
-          s_a[(2 * k + 1) * NFREQ + w] = c.w.A0[(ab + y0 + k) * NFREQ + w];
-        }
-        __syncthreads();
+      __syncthreads();
+      const int ny = min(32, n - y0), y = y0 + lane;
+      for (int t = threadIdx.x; t < ny * NFREQ; t += 32 * BX) {
+        const int k = t / NFREQ, w = t % NFREQ;
+        s_a[2 * k * NFREQ + w] = c.w.A[(ab + y0 + k) * NFREQ + w];
+        s_a[(2 * k + 1) * NFREQ + w] = c.w.A0[(ab + y0 + k) * NFREQ + w];
       }
-      const int y = y0 + lane;
-      if (!live || y >= n || y == x || c.w.z[ab + y] == 0) continue;
-      if (D4S && c.w.slot[ab + y] != s) continue;
-      const size_t lo = (size_t)min(x, y), hi = (size_t)max(x, y);
-      const double K = c.w.pr_S[base + hi * N + lo];
-      const double Pv = c.w.pr_P[base + lo * N + hi];
-      const double D = Pv != 0.0 ? Pv * c.w.pr_P[base + hi * N + lo] : 0.0;
-      psum += Pv;
-      const double *A, *A0;
-      if (D4S) {
-        const size_t o = ((ab + y) * c.S + slot_x) * NFREQ;
-        A = c.w.A + o;
-        A0 = c.w.A0 + o;
-      } else {
-        A = s_a + 2 * lane * NFREQ;
-        A0 = A + NFREQ;
+      double2 kd = make_double2(0.0, 0.0);
+      if (live && y < n && y != x && c.w.z[ab + y] != 0) {
+        const size_t lo = (size_t)min(x, y), hi = (size_t)max(x, y);
+        const double Pv = c.w.pr_P[base + lo * N + hi];
+        kd.x = c.w.pr_S[base + hi * N + lo];
+        kd.y = Pv != 0.0 ? Pv * c.w.pr_P[base + hi * N + lo] : 0.0;
+        psum += Pv;
       }
-#pragma unroll
-      for (int w = 0; w < NFREQ; ++w) {
-        g[w] = fma(K, A[w], g[w]);
-        g0[w] = fma(D, A0[w], g0[w]);
+      s_kd[warp][lane] = kd;
+      __syncthreads();
+      const double *A = s_a + min(lane, NFREQ - 1);
+#pragma unroll 8
+      for (int k = 0; k < ny; ++k) {
+        const double2 v = s_kd[warp][k];
+        g = fma(v.x, A[2 * k * NFREQ], g);
+        g0 = fma(v.y, A[(2 * k + 1) * NFREQ], g0);
       }
     }
-    const double gw = reduce_scatter24(g), gw0 = reduce_scatter24(g0);
-    const int w = reduce_scatter24_index();
-    if (live && w >= 0 && w < NFREQ) {
-      const size_t o = (ax * c.S + s) * NFREQ + w;
-      const double f = THOPI * c.tab.freq_weights[w];
-      dcn += f * (gw * c.w.dA_dcn[o] + gw0 * c.w.dA0_dcn[o]);
-      dq += f * gw * c.w.dA_dq[o];
+    if (live && lane < NFREQ) {
+      const size_t o = ax * NFREQ + lane;
+      const double f = THOPI * c.tab.freq_weights[lane];
+      dcn = f * (g * c.w.dA_dcn[o] + g0 * c.w.dA0_dcn[o]);
+      dq = f * g * c.w.dA_dq[o];
+    }
+  } else {
+    for (int s = 0; s < nslot; ++s) {
+      double g[24], g0[24];
+#pragma unroll
+      for (int w = 0; w < 24; ++w) g[w] = g0[w] = 0.0;
+      for (int y0 = 0; y0 < n; y0 += 32) {
+        if (!D4S) {
+          __syncthreads();
+          const int ny = min(32, n - y0);
+          for (int t = threadIdx.x; t < ny * NFREQ; t += 32 * BX) {
+            const int k = t / NFREQ, w = t % NFREQ;
+            s_a[2 * k * NFREQ + w] = c.w.A[(ab + y0 + k) * NFREQ + w];
+            s_a[(2 * k + 1) * NFREQ + w] = c.w.A0[(ab + y0 + k) * NFREQ + w];
+          }
+          __syncthreads();
+        }
+        const int y = y0 + lane;
+        if (!live || y >= n || y == x || c.w.z[ab + y] == 0) continue;
+        if (D4S && c.w.slot[ab + y] != s) continue;
+        const size_t lo = (size_t)min(x, y), hi = (size_t)max(x, y);
+        const double K = c.w.pr_S[base + hi * N + lo];
+        const double Pv = c.w.pr_P[base + lo * N + hi];
+        const double D = Pv != 0.0 ? Pv * c.w.pr_P[base + hi * N + lo] : 0.0;
+        psum += Pv;
+        const double *A, *A0;
+        if (D4S) {
+          const size_t o = ((ab + y) * c.S + slot_x) * NFREQ;
+          A = c.w.A + o;
+          A0 = c.w.A0 + o;
+        } else {
+          A = s_a + 2 * lane * NFREQ;
+          A0 = A + NFREQ;
+        }
+#pragma unroll
+        for (int w = 0; w < NFREQ; ++w) {
+          g[w] = fma(K, A[w], g[w]);
+          g0[w] = fma(D, A0[w], g0[w]);
+        }
+      }
+      const double gw = reduce_scatter24(g), gw0 = reduce_scatter24(g0);
+      const int w = reduce_scatter24_index();
+      if (live && w >= 0 && w < NFREQ) {
+        const size_t o = (ax * c.S + s) * NFREQ + w;
+        const double f = THOPI * c.tab.freq_weights[w];
+        dcn += f * (gw * c.w.dA_dcn[o] + gw0 * c.w.dA0_dcn[o]);
+        dq += f * gw * c.w.dA_dq[o];
+      }
     }
   }
   dcn = warp_sum(dcn);
@@ -320,8 +359,9 @@ __global__ void __launch_bounds__(PT) pair64_cn_bwd_kernel(Ctx c, int rounds) {
     const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
                  dz = P[3 * i + 2] - P[3 * j + 2];
     r2 = dx * dx + dy * dy + dz * dz;
-    ir = rsqrt(r2);
+    ir = r2 > 0.0 ? rsqrt_pos(r2) : INFINITY;
   };
+  const double ik6 = 1.0 / p.k6;
   auto charges = [&](int i, int j) {
     return c.w.eeq_w[ab + i] * c.w.q[ab + j] + c.w.eeq_w[ab + j] * c.w.q[ab + i];
   };
@@ -330,20 +370,22 @@ __global__ void __launch_bounds__(PT) pair64_cn_bwd_kernel(Ctx c, int rounds) {
     geometry(i, j, r2, ir);
     const double r = r2 * ir;
     const int zi = Z[i], zj = Z[j];
-    const double r0 = c.tab.cov_d3[zi] + c.tab.cov_d3[zj];
+    const double ir0 = rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     double dEdr = 0.0;
     double gcn = 0.0;
-    if (r <= p.cut_cn)
-      gcn = (c.w.dEdcn[ab + i] + c.w.dEdcn[ab + j]) *
-            en_factor(c.tab.en[zi], c.tab.en[zj], p.k4, p.k5, p.k6);
+    if (r <= p.cut_cn) {  // (en_factor with 1 / k6)
+      const double t = fabs(c.tab.en[zi] - c.tab.en[zj]) + p.k5;
+      gcn = (c.w.dEdcn[ab + i] + c.w.dEdcn[ab + j]) * (p.k4 * exp(-(t * t) * ik6));
+    }
     if (eeq) {
       if (r <= p.cut_cn_eeq) gcn += c.w.dEdcnq[ab + i] + c.w.dEdcnq[ab + j];
       const double ra = c.tab.eeq_rad[zi], rb = c.tab.eeq_rad[zj];
-      const double g = rsqrt(ra * ra + rb * rb), gr = g * r;
+      const double g = rsqrt_pos(ra * ra + rb * rb), gr = g * r;
       const double dA = (2.0 * INV_SQRT_PI * exp(-gr * gr) * gr - erf(gr)) * (ir * ir);
       dEdr = -charges(i, j) * dA;
     }
-    dEdr = fma(gcn, erf_count_dr(r, r0, p.kcn), dEdr);
+    const double x = p.kcn * (r * ir0 - 1.0);  // erf_count_dr with 1 / r0
+    dEdr = fma(gcn, -p.kcn * ir0 * INV_SQRT_PI * exp(-x * x), dEdr);
     S[(size_t)i * N + j] += 0.5 * dEdr * ir;
   };
   int queued = 0;
