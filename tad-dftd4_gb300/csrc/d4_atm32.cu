@@ -472,13 +472,14 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
 // its smallest atom (j < i).  A warp task is 32 neighbours k, a lane each with
 // its (j, k) record and sums in registers, against up to 64 neighbours i, four
 // rows' (i, k) records in flight: the (i, k) sums leave by one reduction at L2
-// each, the (i, j) sums of four rows cross lanes through shared memory.  Atom
+// each, the (i, j) sums of four rows cross lanes by halving exchanges (9 shuffles;
+// through shared memory they took 22 of its wavefronts, and the kernel is bound by
+// those, 0.80 of their rate: 16000 atoms, cutoff 25 Bohr, 8.0 -> 7.1 ms).  Atom
 // energies come from the pair sums (atm_mirror_kernel); only the energies e_w
 // of the centre's 1/3 triples, which it gets nothing of, leave here as -e_w /
 // 3 (see a3_step).  Energies without gradient have no pair sums and add up
 // atom energies instead, in units of eu / 6.
 constexpr int SP_THREADS = 512, SP_ROWS = 4, SP_BLOCK = 64;
-constexpr int SP_ROW = 40;  // float2 stride of the row sums (8 lanes and 2 of padding each)
 
 // Tasks of the first m chunks: chunk ec has ec / 2 + 1 blocks of rows.
 __device__ __forceinline__ int sp_tasks(int m) { return (m + 1) * (m + 1) / 4; }
@@ -489,7 +490,6 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
   float2 *s_SP = reinterpret_cast<float2 *>(s_rec + ATM_SPARSE_DMAX);  // their sums
   int *s_L = reinterpret_cast<int *>(s_SP + ATM_SPARSE_DMAX);
   float *s_W = reinterpret_cast<float *>(s_L + ATM_SPARSE_DMAX);  // PGRAD: damping sums
-  __shared__ __align__(16) float2 s_row[SP_THREADS / 32][SP_ROWS * SP_ROW];
   __shared__ float s_red[SP_THREADS / 32];
   __shared__ int s_next;
   const int b = blockIdx.y, N = c.N, n = c.w.n_eff[b];
@@ -515,7 +515,6 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
   __syncthreads();
   const float cut2 = c.pf.cut3 * c.pf.cut3, alp3h = 0.5f * c.pf.alp3;
   const float s9 = (GRAD && !PGRAD) ? c.pf.s9 : 1.f;  // PGRAD, energies: at the end
-  float2 *rowbuf = s_row[warp];
   float Cj = 0.f;
   A3Pg pg;
   const int nch = (d + 31) / 32, tasks = sp_tasks(nch);
@@ -541,6 +540,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
         pik[r] = ok ? T[(size_t)s_L[ok ? a : 0] * N + k] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       float wij[PGRAD ? SP_ROWS : 1];
+      float v[GRAD ? 2 * SP_ROWS : SP_ROWS];  // the rows' sums (S, P), or energies
 #pragma unroll
       for (int r = 0; r < SP_ROWS; ++r) {
         const int a = a0 + r;
@@ -584,26 +584,32 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
             Cj += in ? 2.0f * eu : 0.f;
           }
         }
-        rowbuf[SP_ROW * r + lane + 2 * (lane >> 3)] = out;
+        if (GRAD) {
+          v[2 * r] = out.x;
+          v[2 * r + 1] = out.y;
+        } else {
+          v[r] = out.x;
+        }
         if (PGRAD) wij[r] = wv;
       }
-      __syncwarp();
-      // (i, j) sums: eight lanes per row, four entries each
+      // (i, j) sums: halving exchanges leave value lane >> 2 (2 r + component of
+      // row r; energies lane >> 3, row r) to the lanes of a group
+      float sum;
+      if (GRAD) {
+        float (&v8)[8] = *reinterpret_cast<float(*)[8]>(&v[0]);
+        halving<8, 16, 3>(v8);
+        sum = v8[0];
+      } else {
+        float (&v4)[4] = *reinterpret_cast<float(*)[4]>(&v[0]);
+        halving<4, 16, 2>(v4);
+        sum = v4[0] + __shfl_xor_sync(0xffffffffu, v4[0], 4);
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       {
-        const int r = lane >> 3, q = lane & 7;  // entries 4 q .. 4 q + 3
-        const float4 *p4 =
-            reinterpret_cast<const float4 *>(rowbuf + SP_ROW * r + 4 * q + 2 * (q >> 1));
-        const float4 v0 = p4[0], v1 = p4[1];
-        float sv = (v0.x + v0.z) + (v1.x + v1.z), ev = (v0.y + v0.w) + (v1.y + v1.w);
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
-          sv += __shfl_xor_sync(0xffffffffu, sv, o);
-          if (GRAD) ev += __shfl_xor_sync(0xffffffffu, ev, o);
-        }
-        if (q == 0 && a0 + r < a_end) {
-          if (sv != 0.f) atomicAdd(&s_SP[a0 + r].x, sv);
-          if (GRAD && ev != 0.f) atomicAdd(&s_SP[a0 + r].y, ev);
-        }
+        const int row = a0 + (lane >> 3), comp = GRAD ? (lane >> 2) & 1 : 0;
+        if ((lane & (GRAD ? 3 : 7)) == 0 && row < a_end && sum != 0.f)
+          atomicAdd(comp ? &s_SP[row].y : &s_SP[row].x, sum);
       }
       if (PGRAD) {
 #pragma unroll
@@ -612,7 +618,6 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
           if (lane == 0 && wv != 0.f) atomicAdd(&s_W[a0 + r], wv);
         }
       }
-      __syncwarp();
     }
     if (eok) {
       if (GRAD && Sjk != 0.f) atomicAdd(&s_SP[e].x, Sjk);
