@@ -1015,6 +1015,16 @@ __global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint
     s_b[warp] = sb;
   }
   __syncthreads();
+  if (warp == 0) {  // (32 warps)
+    sa = warp_sum(s_a[lane]);
+    sb = warp_sum(s_b[lane]);
+    __syncwarp();
+    if (lane == 0) {
+      s_a[0] = sa;
+      s_b[0] = sb;
+    }
+    __syncwarp();
+  }
   if (tid == 0) {
     // final refinement residual: that of the first iteration below the
     // tolerance (later iterations were skipped), else of the last one
@@ -1024,11 +1034,7 @@ __global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint
       if (fin < BIG_TOL) break;
     }
     if (lead) c.w.eeq_final[2 * b + (adjoint ? 1 : 0)] = fin;
-    double ta = 0.0, tb = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      ta += s_a[w];
-      tb += s_b[w];
-    }
+    double ta = s_a[0], tb = s_b[0];
     if (adjoint) {
       s_par = m > 0 ? ta / c.w.eeq_sum[2 * b] : 0.0;
     } else {
@@ -1042,7 +1048,9 @@ __global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint
   }
   __syncthreads();
   const double par = s_par;
-  const int g0 = blockIdx.x * blockDim.x + tid, gs = gridDim.x * blockDim.x;
+  // atoms of this CTA, every FIN_CTAS-th: FP64 divisions and roots spread over
+  // the CTAs for a few hundred atoms too (997 atoms 14 -> 10 us)
+  const int g0 = blockIdx.x + FIN_CTAS * tid, gs = gridDim.x * blockDim.x;
   for (int i = g0; i < N; i += gs) {
     if (c.w.cidx[(size_t)b * N + i] >= 0) continue;  // a real atom: written below
     if (adjoint) {

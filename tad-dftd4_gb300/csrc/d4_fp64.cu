@@ -20,7 +20,9 @@ namespace d4 {
 // ---------------------------------------------------------------- prep
 
 // n_eff, input validation, D4S element slots, zeroing of accumulators.
-__global__ void __launch_bounds__(256) prep_kernel(Ctx c) { prep_structure(c, blockIdx.x); }
+__global__ void __launch_bounds__(256) prep_kernel(Ctx c, int parts) {
+  prep_structure(c, blockIdx.x / parts, blockIdx.x % parts, parts);
+}
 
 // ---------------------------------------------------------------- CN
 
@@ -1093,7 +1095,8 @@ int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_
 
 void launch_prep(const Ctx &c, cudaStream_t st) {
   launch_prep_memsets(c, st);
-  prep_kernel<<<c.B, 256, 0, st>>>(c);
+  const int parts = prep_parts(c);
+  prep_kernel<<<c.B * parts, 256, 0, st>>>(c, parts);
 }
 
 void launch_prep_memsets(const Ctx &c, cudaStream_t st) {

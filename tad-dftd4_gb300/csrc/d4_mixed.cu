@@ -159,11 +159,12 @@ __global__ void __launch_bounds__(256) block_boxes_kernel(Ctx c) {
 
 // The per-call FP32 tables (the first CTAs) and the per-structure set-up
 // (prep_structure) in one launch: neither needs the other.
-__global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c) {
+__global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c, int parts) {
   if ((int)blockIdx.x < TABLE_CTAS)
     tables32(c, blockIdx.x);
   else
-    prep_structure(c, (int)blockIdx.x - TABLE_CTAS);
+    prep_structure(c, ((int)blockIdx.x - TABLE_CTAS) / parts,
+                   ((int)blockIdx.x - TABLE_CTAS) % parts, parts);
 }
 
 // exp(x), |x| <= 80, rounded once: reduction by ln 2 = 355/512 - 2.1e-4 (Cody and
@@ -971,6 +972,7 @@ __global__ void __launch_bounds__(1024) atm_order_kernel(Ctx c) {
   const int b = blockIdx.x;
   const int n = c.w.n_eff[b];
   const size_t bN = (size_t)b * c.N;
+  if (!atm_sparse_mode(c, b, n)) return;  // all triples: nothing reads the order
   if (n > ATM_ORDER_MAX) {
     for (int t = threadIdx.x; t < n; t += blockDim.x) c.w.atm_order[bN + t] = t;
     return;
@@ -1755,7 +1757,8 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
     if (out.d_cn) c.out.d_cn = c.w.zs_ocn;
     if (out.d_cn_eeq) c.out.d_cn_eeq = c.w.zs_ocnq;
   }
-  prep_tables_kernel<<<TABLE_CTAS + B, 256, 0, st>>>(c);
+  const int parts = prep_parts(c);
+  prep_tables_kernel<<<TABLE_CTAS + B * parts, 256, 0, st>>>(c, parts);
   if (c.zsorted) {
     block_boxes_kernel<<<dim3(((N + 31) / 32 + 7) / 8, B), 256, 0, st>>>(c);
     c.far_skip = c.cfg.kind == D4_MODEL_D4 && N >= FAR_MIN;

@@ -10,22 +10,36 @@ namespace d4 {
 // cleared by memsets instead of by the prep kernel.
 constexpr int PREP_ZERO_MAX_N = 256;
 
+// CTAs of prep_structure per structure: one per 256 atoms of few large
+// structures (every CTA scans the atomic numbers; 16000 atoms 273 -> 28 us).
+inline int prep_parts(const Ctx &c) {
+  const int most = (c.N + 255) / 256;
+  return c.N <= 512 ? 1 : (c.B >= 304 ? 1 : (most < 304 / c.B ? most : 304 / c.B));
+}
+
 // n_eff, input validation, D4S element slots, zeroing of accumulators of
-// structure b, by one CTA of 256 threads (all of which call it).
-static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
+// structure b, by ``parts`` CTAs of 256 threads (all of which call it): each finds
+// the structure's figures and sets up its part of the atoms.
+static __device__ __forceinline__ void prep_structure(const Ctx &c, int b, int part, int parts) {
   const int N = c.N;
   const int64_t *Z = c.numbers + (size_t)b * N;
-  __shared__ int s_neff, s_first;
+  // this CTA's atoms: whole blocks of 32
+  const int blocks = (N + 31) / 32;
+  const int beg = 32 * (int)((long long)blocks * part / parts);
+  const int end = min(N, 32 * (int)((long long)blocks * (part + 1) / parts));
+  __shared__ int s_neff, s_first, s_before, s_real;
   __shared__ int s_present[MAX_ELEM_ID];
   __shared__ int s_slot_of[MAX_ELEM_ID];
   if (threadIdx.x == 0) {
     s_neff = 0;
     s_first = N;
+    s_before = s_real = 0;
     c.w.eeq_final[2 * b] = 0.f;  // stays 0 where no refinement runs
     c.w.eeq_final[2 * b + 1] = 0.f;
   }
   for (int e = threadIdx.x; e < MAX_ELEM_ID; e += blockDim.x) s_present[e] = 0;
   __syncthreads();
+  int real = 0, before = 0;
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const int64_t z = Z[i];
     if (z == 0) continue;
@@ -36,9 +50,18 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
     atomicMax(&s_neff, i + 1);
     atomicMin(&s_first, i);
     s_present[z] = 1;
+    if (parts > 1) {
+      ++real;
+      before += i < beg;
+      if (i < beg || i >= end) continue;
+    }
     const double *r = c.positions + ((size_t)b * N + i) * 3;
     if (!isfinite(r[0]) || !isfinite(r[1]) || !isfinite(r[2]))
       set_status(c.w.status, D4_ERR_NONFINITE);
+  }
+  if (real > 0) {
+    atomicAdd(&s_real, real);
+    atomicAdd(&s_before, before);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -48,7 +71,7 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
       for (int e = 0; e < MAX_ELEM_ID; ++e) {
         s_slot_of[e] = s_present[e] ? ns : 0;
         if (s_present[e]) {
-          if (ns < c.S) c.w.slot_elem[b * MAX_ELEM_ID + ns] = e;
+          if (ns < c.S && part == 0) c.w.slot_elem[b * MAX_ELEM_ID + ns] = e;
           ++ns;
         }
       }
@@ -66,7 +89,7 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
   const int n = s_neff;
   // FP32 positions are taken relative to the first real atom
   const double *p0 = c.positions + ((size_t)b * N + (s_first < N ? s_first : 0)) * 3;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+  for (int i = beg + threadIdx.x; i < end; i += blockDim.x) {
     const size_t a = (size_t)b * N + i;
     const int64_t z = Z[i];
     const bool ok = z > 0 && z < c.tab.n_ref_elem && z < MAX_ELEM_ID;
@@ -97,8 +120,8 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
   }
   // index of every real atom among the real atoms (EEQ matrix rows)
   if (threadIdx.x < 32) {
-    int base = 0;
-    for (int i0 = 0; i0 < N; i0 += 32) {
+    int base = parts > 1 ? s_before : 0;
+    for (int i0 = beg; i0 < end; i0 += 32) {
       const int i = i0 + threadIdx.x;
       const int64_t z = i < N ? Z[i] : 0;
       const bool real = i < N && z > 0 && z < c.tab.n_ref_elem && z < MAX_ELEM_ID;
@@ -108,10 +131,11 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b) {
       if (real && c.w.ridx) c.w.ridx[(size_t)b * N + k] = i;
       base += __popc(mask);
     }
-    if (threadIdx.x == 0 && c.w.n_real) c.w.n_real[b] = base;
+    if (threadIdx.x == 0 && part == 0 && c.w.n_real) c.w.n_real[b] = parts > 1 ? s_real : base;
   }
-  if (threadIdx.x < D4_PARAM_GRAD_STRIDE) c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + threadIdx.x] = 0.0;
-  if (b == 0 && threadIdx.x < NFREQ)
+  if (part == 0 && threadIdx.x < D4_PARAM_GRAD_STRIDE)
+    c.w.pgrad[b * D4_PARAM_GRAD_STRIDE + threadIdx.x] = 0.0;
+  if (b == 0 && part == 0 && threadIdx.x < NFREQ)
     c.w.fw32[threadIdx.x] = (float)(THOPI * c.tab.freq_weights[threadIdx.x]);
   if (c.w.pr_S && c.N <= PREP_ZERO_MAX_N && !c.pair64) {
     for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
