@@ -1370,7 +1370,7 @@ __device__ __forceinline__ dfl df_warp_sum(dfl a) {
 // (FP64-accurate, on the FP32 pipe): a warp takes four rows at a time, lanes
 // over columns (coalesced), so that 32 independent loads per lane are in
 // flight (one row at a time left the warp waiting on L2 latency row after
-// row).  r is rounded to FP32 into vf, the right-hand side of the next
+// row; loads under a condition 5 % of the solves).  r is rounded to FP32 into vf, the right-hand side of the next
 // correction; returns max |r| over the block.
 __device__ float eeq_residual_df(const float *Hi, const float *Lo, const float2 *X,
                                  const float2 *BB, float *vf, int m, int N, int nr,
@@ -1380,20 +1380,23 @@ __device__ float eeq_residual_df(const float *Hi, const float *Lo, const float2 
   float mx = 0.f;
   for (int k0 = warp * RW; k0 < m; k0 += nw * RW) {
     dfl a0[RW], a1[RW];
+    const float *hr[RW], *lr[RW];  // rows beyond the matrix repeat the last one
 #pragma unroll
-    for (int q = 0; q < RW; ++q) a0[q] = a1[q] = dfl{0.f, 0.f};
+    for (int q = 0; q < RW; ++q) {
+      a0[q] = a1[q] = dfl{0.f, 0.f};
+      const size_t o = (size_t)min(k0 + q, m - 1) * N;
+      hr[q] = Hi + o;
+      lr[q] = Lo + o;
+    }
     for (int l0 = lane; l0 < m; l0 += 128) {
       float h[RW][4], lo[RW][4];
 #pragma unroll
-      for (int q = 0; q < RW; ++q) {
-        const int k = k0 + q;
-        const float *hr = Hi + (size_t)(k < m ? k : 0) * N, *lr = Lo + (size_t)(k < m ? k : 0) * N;
+      for (int u = 0; u < 4; ++u) {  // (unconditional: all loads leave at once)
+        const int l = min(l0 + 32 * u, m - 1);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int l = l0 + 32 * u;
-          const bool ok = k < m && l < m;
-          h[q][u] = ok ? hr[l] : 0.f;
-          lo[q][u] = ok ? lr[l] : 0.f;
+        for (int q = 0; q < RW; ++q) {
+          h[q][u] = hr[q][l];
+          lo[q][u] = lr[q][l];
         }
       }
 #pragma unroll
