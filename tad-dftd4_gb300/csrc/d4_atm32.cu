@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
     const float s9q = (GRAD && !PGRAD) ? c.pf.s9 : 1.f;
     float zjk[A3], izjk[A3], ejk[A3], qjk[A3], Sjk[A3], Pjk[A3], Wjk[A3];
     unsigned jmask = 0u;
-    bool far = kok && far2[k] > a.cut2;
+    bool far = kok && far2[k] > a.cut2, task_far = false;
 #pragma unroll
     for (int tt = 0; tt < A3; ++tt) {
       const int jt = j0 + tt;
@@ -341,8 +341,9 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
       qjk[tt] = s9q * r.w;   // 0 where (j, k) is not a pair: every product vanishes
       Sjk[tt] = Pjk[tt] = Wjk[tt] = 0.f;
       far |= jok && far2[jt] > a.cut2;
+      task_far |= r.x > a.cut2;
     }
-    const bool task_far = __any_sync(0xffffffffu, far);
+    task_far = __any_sync(0xffffffffu, task_far);  // a (j, k) beyond the cutoff
     for (int ib = ib0 + lane; ib < iend; ib += 32) far |= far2[ib] > a.cut2;
     const bool any_far = __any_sync(0xffffffffu, far);
     float Ek = 0.f;
@@ -383,8 +384,11 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
         if (ib + 4 * half >= iend) break;
         const bool iok = i < iend && (!gaps || Z[i] != 0);
         const float4 *rec = stage[st] + A3_REC * (4 * half + q);
-        const bool mask =
-            task_far || (any_far && __any_sync(0xffffffffu, iok && far2[i] > a.cut2));
+        // a pair of the step beyond the cutoff (any_far: an atom of the task has one;
+        // by atoms alone nearly all steps of 997 atoms took their masks)
+        const bool mask = any_far && (task_far || __any_sync(0xffffffffu,
+                                                             rec[lane & 7].x > a.cut2 ||
+                                                                 rec[A3 + (lane & 7)].x > a.cut2));
         if (mask)
           a3_step<GRAD, PGRAD, true>(a, rec, j0, jmask, k, kok, i, iok, zjk, izjk, ejk, qjk, Sjk,
                                      Pjk, Wjk, Ek, cj, red, pg);

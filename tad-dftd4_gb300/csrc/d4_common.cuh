@@ -72,8 +72,10 @@ constexpr int ATM_SPARSE_DMAX = 2048;
 // (one shared-memory sort per structure); larger ones keep index order.
 constexpr int ATM_ORDER_MAX = 16384;
 // The precision form takes structures of this size range in spatial order
-// throughout (d4_mixed.cu, zsort_kernel).
-constexpr int ZSORT_MIN = 1536;
+// throughout (d4_mixed.cu, zsort_kernel): the sort and the copies cost 26 us, and
+// blocks of atoms then rarely straddle the three-body cutoff, which takes 8 %
+// off the ATM over all triples (997 atoms 546 -> 503 us, 600 atoms 178 -> 155).
+constexpr int ZSORT_MIN = 896;
 __host__ __device__ inline bool zsort_fits(int N) { return N >= ZSORT_MIN && N <= ATM_ORDER_MAX; }
 
 
