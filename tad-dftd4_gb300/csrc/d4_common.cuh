@@ -75,7 +75,9 @@ constexpr int ATM_ORDER_MAX = 16384;
 // throughout (d4_mixed.cu, zsort_kernel): the sort and the copies cost 26 us, and
 // blocks of atoms then rarely straddle the three-body cutoff, which takes 8 %
 // off the ATM over all triples (997 atoms 546 -> 503 us, 600 atoms 178 -> 155).
-constexpr int ZSORT_MIN = 896;
+// Above what the static scratch of d4_dispersion_noalloc takes (932 atoms), whose
+// limit the copies would lower.
+constexpr int ZSORT_MIN = 960;
 __host__ __device__ inline bool zsort_fits(int N) { return N >= ZSORT_MIN && N <= ATM_ORDER_MAX; }
 
 
