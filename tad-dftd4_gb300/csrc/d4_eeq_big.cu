@@ -1195,6 +1195,20 @@ static bool converged_on_host(const Ctx &c, cudaStream_t st, int it) {
   return true;
 }
 
+// x += v and the residual of refinement iteration ``it``.
+static void launch_refine(const Ctx &c, cudaStream_t st, int it, bool adjoint) {
+  const int B = c.B, N = c.N;
+  eeq_big_update_kernel<<<dim3((N + 255) / 256, B), 256, 0, st>>>(c, it, adjoint ? 1 : 2);
+  const dim3 rg((N + 8 * RS_ROWS - 1) / (8 * RS_ROWS), B);
+  if (N % 4 == 0) {
+    if (!adjoint) eeq_big_residual_kernel<2, true><<<rg, 256, 0, st>>>(c, it);
+    else eeq_big_residual_kernel<1, true><<<rg, 256, 0, st>>>(c, it);
+  } else {
+    if (!adjoint) eeq_big_residual_kernel<2, false><<<rg, 256, 0, st>>>(c, it);
+    else eeq_big_residual_kernel<1, false><<<rg, 256, 0, st>>>(c, it);
+  }
+}
+
 // Forward (adjoint = 0: factorisation, two right-hand sides, charges) or
 // adjoint (reuses the factor; one right-hand side dE/dq) multi-CTA EEQ.
 // Refinement iterations after the second are launched only while some
@@ -1240,27 +1254,13 @@ void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint) {
         eeq_sweep_above_kernel<<<dim3((s0 + AB_COLS - 1) / AB_COLS, B), 256, 0, st>>>(c, sb, it,
                                                                                      nr);
     }
-    launch_eeq_big_refine(c, st, it, adjoint);
+    launch_refine(c, st, it, adjoint);
   }
   launch_eeq_big_finish(c, st, adjoint);
 }
 
 void launch_eeq_big_rhs(const Ctx &c, cudaStream_t st, bool adjoint) {
   eeq_big_rhs_kernel<<<dim3((c.N + 255) / 256, c.B), 256, 0, st>>>(c, adjoint ? 1 : 0);
-}
-
-// x += v and the residual of refinement iteration ``it``.
-void launch_eeq_big_refine(const Ctx &c, cudaStream_t st, int it, bool adjoint) {
-  const int B = c.B, N = c.N;
-  eeq_big_update_kernel<<<dim3((N + 255) / 256, B), 256, 0, st>>>(c, it, adjoint ? 1 : 2);
-  const dim3 rg((N + 8 * RS_ROWS - 1) / (8 * RS_ROWS), B);
-  if (N % 4 == 0) {
-    if (!adjoint) eeq_big_residual_kernel<2, true><<<rg, 256, 0, st>>>(c, it);
-    else eeq_big_residual_kernel<1, true><<<rg, 256, 0, st>>>(c, it);
-  } else {
-    if (!adjoint) eeq_big_residual_kernel<2, false><<<rg, 256, 0, st>>>(c, it);
-    else eeq_big_residual_kernel<1, false><<<rg, 256, 0, st>>>(c, it);
-  }
 }
 
 void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint) {

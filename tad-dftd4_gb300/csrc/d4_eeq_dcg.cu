@@ -8,12 +8,11 @@
 // vectors Z of the blocks (K <= 256 of them) hold those modes: CG on
 // P A, P = 1 - A Z (Z^T A Z)^-1 Z^T, gains five digits in 14 iterations at 6000
 // atoms and 17 at 16000, where plain CG takes 32 at 6000.  As in d4_eeq_cg.cu the FP32 solve is the
-// inner one of a refinement whose residuals are taken in double-float
-// (eeq_big_residual_kernel).
+// inner one of a refinement whose residuals are taken in double-float.
 //
-// Measured at 16000 atoms, charges + adjoint: 21.9 (factorisation) -> 11.6 ms,
-// of it 7.7 the solves, 2.0 the residuals, 1.2 the matrix, 0.5 Z^T A Z, its
-// inverse and G.  A product takes 93 us with one right-hand side (5.5 TB/s of the
+// Measured at 16000 atoms, charges + adjoint: 21.9 (factorisation) -> 10.8 ms,
+// of it 7.7 the solves, 1.5 the residuals, 1.0 the matrix, 0.4 Z^T A Z, its
+// inverse and G (2.0, 1.2 and 0.5 over the whole matrix).  A product takes 93 us with one right-hand side (5.5 TB/s of the
 // half matrix), 122 with two; the rest of an iteration (two exchanges, three
 // barriers) 12 to 14 us.
 //
@@ -40,7 +39,7 @@ namespace {
 
 constexpr int DC_BLOCK = 64;  // atoms per block vector
 constexpr int DC_K = 256;     // blocks at most
-constexpr int DC_TILE = 128;
+constexpr int DC_TILE = EEQ_HALF_TILE;
 constexpr int DC_THREADS = 512, DC_WARPS = DC_THREADS / 32, DC_ROWS = DC_TILE / DC_WARPS;
 constexpr int DC_SLICE = DC_THREADS / 4;  // rows of a CTA's slice at most (four lanes each)
 constexpr int DC_LDG = DC_K + 16;         // row stride of G in shared memory (no bank conflicts)
@@ -288,24 +287,49 @@ __device__ __forceinline__ void dc_cta_sum(float (&v)[V], DcSmem &sm) {
 
 }  // namespace
 
-// A Z: sums of A over the columns of each block, a warp per row; clears the
-// barrier counters.
+// A Z: sums of A over the columns of each block.  A CTA per pair of blocks on or
+// below the diagonal: its row sums, and its column sums for the mirrored pair.
 __global__ void __launch_bounds__(256) dcg_az_kernel(Ctx c) {
+  constexpr int ROWS = DC_BLOCK / 8;  // of a warp
+  __shared__ float s_col[8][DC_BLOCK];
   const int b = blockIdx.y, m = c.w.n_real[b], N = c.N;
+  int I, J;
+  tri_entry(blockIdx.x, I, J);
+  if (DC_BLOCK * I >= m) return;
   const DcArea ar = dc_area(c, b);
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= m) return;
-  const float *h = c.w.eeq_hi + ((size_t)b * N + row) * N;
-  const int K = (m + DC_BLOCK - 1) / DC_BLOCK;
-#pragma unroll 4
-  for (int k = 0; k < DC_K; ++k) {
-    if (k >= K) break;
-    const int l = DC_BLOCK * k + lane;
-    const float a0 = l < m ? __ldg(h + l) : 0.f, a1 = l + 32 < m ? __ldg(h + l + 32) : 0.f;
-    const float s = warp_sumf(a0 + a1);
-    if (lane == 0) ar.AZ[(size_t)row * DC_K + k] = s;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = DC_BLOCK * I + ROWS * warp, l = DC_BLOCK * J + lane;
+  const float *h = c.w.eeq_hi + (size_t)b * N * N;
+  float a[ROWS][2], s[2] = {0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const bool ok = row0 + r < m && l + 32 * e < m;
+      a[r][e] = ok ? __ldg(h + (size_t)(row0 + r) * N + l + 32 * e) : 0.f;
+    }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    s[0] += a[r][0];
+    s[1] += a[r][1];
+    const float v = warp_sumf(a[r][0] + a[r][1]);
+    if (lane == 0 && row0 + r < m) ar.AZ[(size_t)(row0 + r) * DC_K + J] = v;
   }
-  for (int k = K + lane; k < DC_K; k += 32) ar.AZ[(size_t)row * DC_K + k] = 0.f;
+  if (I != J) {  // (J < I: whole columns)
+    s_col[warp][lane] = s[0];
+    s_col[warp][lane + 32] = s[1];
+    __syncthreads();
+    if (threadIdx.x < DC_BLOCK) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v += s_col[w][threadIdx.x];
+      ar.AZ[(size_t)(DC_BLOCK * J + threadIdx.x) * DC_K + I] = v;
+    }
+  } else {
+    const int K = (m + DC_BLOCK - 1) / DC_BLOCK;
+    for (int r = row0; r < min(row0 + ROWS, m); ++r)
+      for (int k = K + lane; k < DC_K; k += 32) ar.AZ[(size_t)r * DC_K + k] = 0.f;
+  }
 }
 
 // Z^T A Z, a CTA per block.
@@ -697,6 +721,196 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
   }
 }
 
+// x += v in double-float; clears the sums of the residual (FP64, in the room of
+// the products w).
+__global__ void __launch_bounds__(256) dcg_update_kernel(Ctx c, int it, int nr) {
+  const int b = blockIdx.y, N = c.N, k = blockIdx.x * 256 + threadIdx.x;
+  if (k >= c.w.n_real[b] || dc_skip(c, b, it)) return;
+  double *sums = reinterpret_cast<double *>(dc_area(c, b).w[0]);
+  for (int q = 0; q < nr; ++q) {
+    const size_t o = (size_t)b * 2 * N + (size_t)q * N + k;
+    const float2 x = c.w.eeq_X[o];
+    const dfl s = df_add(dfl{x.x, x.y}, dfl{c.w.eeq_V[o], 0.f});
+    c.w.eeq_X[o] = make_float2(s.hi, s.lo);
+    sums[q * dc_pad(N) + k] = 0.0;
+  }
+}
+
+struct DrSmem {
+  float2 z[2][2][DC_WARPS][DC_TILE];  // [turn][right-hand side][warp]: a tile's column sums
+  float2 xj[2][2][DC_TILE], xi[2][DC_TILE];  // x of a tile's columns, rows
+};
+
+// (hi + lo) x in double-float, summed in FP64 at L2, over the stored half of the
+// matrix: dc_product's tiles, each for both of its products, with four of a
+// warp's eight rows of both planes in flight.  Bound by the latency of its FP32
+// sums (12 instructions per entry, product and right-hand side): 16000 atoms, two
+// right-hand sides 0.37 ms (2.8 TB/s), one 0.21 ms (4.8 TB/s); the five of charges +
+// adjoint 1.5 ms against 2.0 over the whole matrix.  256 threads with eight rows in
+// flight 0.38 and 0.22, two rows of 16 warps 0.39 and 0.24.
+template <int NR, bool VEC>
+__global__ void __launch_bounds__(DC_THREADS, 1) dcg_residual_kernel(Ctx c, int it) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  DrSmem &sm = *reinterpret_cast<DrSmem *>(s_raw);
+  const int b = blockIdx.y, N = c.N, m = c.w.n_real[b];
+  if (m == 0 || dc_skip(c, b, it)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int NB = (m + DC_TILE - 1) / DC_TILE;
+  const long long tiles = (long long)NB * (NB + 1) / 2;
+  const int t0 = (int)(tiles * blockIdx.x / gridDim.x);
+  const int t1 = (int)(tiles * (blockIdx.x + 1) / gridDim.x);
+  if (t0 >= t1) return;
+  const float *Hi = c.w.eeq_hi + (size_t)b * N * N, *Lo = c.w.eeq_lo + (size_t)b * N * N;
+  const float2 *X = c.w.eeq_X + (size_t)b * 2 * N;
+  double *sums = reinterpret_cast<double *>(dc_area(c, b).w[0]);
+  const size_t us = dc_pad(N);
+  constexpr int W = 4;  // rows in flight
+  static_assert(DC_ROWS % W == 0 && NR * DC_TILE <= DC_THREADS, "the warp's rows");
+  auto col = [&](int J, int e) { return DC_TILE * J + (VEC ? 4 * lane + e : lane + 32 * e); };
+  auto load_row = [&](float (&h)[4], float (&g)[4], int I, int J, int r) {  // as in dc_product
+    const size_t o = (size_t)min(DC_TILE * I + DC_ROWS * warp + r, m - 1) * N;
+    if (VEC) {
+      const size_t p = o + min(col(J, 0), N - 4);
+      const float4 v = dc_stream4(Hi + p), w = dc_stream4(Lo + p);
+      h[0] = v.x, h[1] = v.y, h[2] = v.z, h[3] = v.w;
+      g[0] = w.x, g[1] = w.y, g[2] = w.z, g[3] = w.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const size_t p = o + min(col(J, e), m - 1);
+        h[e] = __ldg(Hi + p), g[e] = __ldg(Lo + p);
+      }
+    }
+  };
+  const int xq = tid / DC_TILE, xk = tid % DC_TILE;  // an x entry per thread
+  auto load_x = [&](int J) {
+    const int k = DC_TILE * J + xk;
+    return xq < NR && k < m ? __ldg(X + (size_t)xq * N + k) : make_float2(0.f, 0.f);
+  };
+  // acc += (h + g) x, the low part unnormalised
+  auto add = [](dfl &acc, float h, float g, float2 x) {
+    const float p = h * x.x;
+    const float e = fmaf(h, x.y, fmaf(g, x.x, fmaf(h, x.x, -p)));
+    const dfl s = df_two_sum(acc.hi, p);
+    acc = {s.hi, acc.lo + (s.lo + e)};
+  };
+  int I, J;
+  tri_entry(t0, I, J);
+  float h[W][4], g[W][4];
+  dfl y[DC_ROWS][NR];
+#pragma unroll
+  for (int r = 0; r < W; ++r) load_row(h[r], g[r], I, J, r);
+  if (xq < NR) sm.xj[0][xq][xk] = load_x(J);
+  bool first = true;
+  int turn = 0;
+  for (int t = t0; t < t1; ++t) {
+    if (first || J == 0) {  // a new row of tiles
+      first = false;
+      const float2 xi = load_x(I);
+      __syncthreads();
+      if (xq < NR) sm.xi[xq][xk] = xi;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < DC_ROWS; ++r)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) y[r][q] = {0.f, 0.f};
+    }
+    const bool diag = J == I, more = t + 1 < t1;
+    const int In = diag ? I + 1 : I, Jn = diag ? 0 : J + 1;
+    const float2 xn = load_x(more ? Jn : J);
+    float2 xj[NR][4];
+    dfl z[NR][4];
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        xj[q][e] = sm.xj[turn][q][VEC ? 4 * lane + e : lane + 32 * e];
+        z[q][e] = {0.f, 0.f};
+      }
+    const bool edge = DC_TILE * (J + 1) > m;
+#pragma unroll
+    for (int r = 0; r < DC_ROWS; ++r) {
+      float (&hr)[4] = h[r % W], (&gr)[4] = g[r % W];
+      if (edge) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (col(J, e) >= m) hr[e] = gr[e] = 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const float2 xi = sm.xi[q][DC_ROWS * warp + r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          add(y[r][q], hr[e], gr[e], xj[q][e]);
+          add(z[q][e], hr[e], gr[e], xi);
+        }
+      }
+      if (r + W < DC_ROWS) load_row(hr, gr, I, J, r + W);
+      else if (more) load_row(hr, gr, In, Jn, r + W - DC_ROWS);
+    }
+    if (xq < NR) sm.xj[turn ^ 1][xq][xk] = xn;
+    if (!diag) {  // the mirrored tile's product, summed over the warps
+#pragma unroll
+      for (int q = 0; q < NR; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          sm.z[turn][q][warp][VEC ? 4 * lane + e : lane + 32 * e] =
+              make_float2(z[q][e].hi, z[q][e].lo);
+      __syncthreads();
+      if (xq < NR) {
+        dfl s = {0.f, 0.f};
+#pragma unroll
+        for (int v = 0; v < DC_WARPS; ++v) {
+          const float2 a = sm.z[turn][xq][v][xk];
+          const dfl n = df_two_sum(s.hi, a.x);
+          s = {n.hi, s.lo + (n.lo + a.y)};
+        }
+        atomicAdd(sums + xq * us + DC_TILE * J + xk, (double)s.hi + (double)s.lo);
+      }
+    }
+    if (diag || !more) {  // the row of tiles ends
+#pragma unroll
+      for (int r = 0; r < DC_ROWS; ++r)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          dfl a = y[r][q];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const float oh = __shfl_xor_sync(0xffffffffu, a.hi, o);
+            const float ol = __shfl_xor_sync(0xffffffffu, a.lo, o);
+            const dfl s = df_two_sum(a.hi, oh);
+            a = df_fast(s.hi, s.lo + (a.lo + ol));
+          }
+          const int row = DC_TILE * I + DC_ROWS * warp + r;
+          if (lane == 0 && row < m) atomicAdd(sums + q * us + row, (double)a.hi + (double)a.lo);
+        }
+    }
+    turn ^= 1;
+    I = In;
+    J = Jn;
+  }
+}
+
+// v <- FP32 r = b - A x and the structure's max |r| of the iteration.
+__global__ void __launch_bounds__(256) dcg_rest_kernel(Ctx c, int it, int nr) {
+  const int b = blockIdx.y, N = c.N, k = blockIdx.x * 256 + threadIdx.x;
+  const int m = c.w.n_real[b];
+  if (blockIdx.x * 256 >= m || dc_skip(c, b, it)) return;
+  const double *sums = reinterpret_cast<const double *>(dc_area(c, b).w[0]);
+  float mx = 0.f;
+  if (k < m)
+    for (int q = 0; q < nr; ++q) {
+      const size_t o = (size_t)b * 2 * N + (size_t)q * N + k;
+      const float2 bb = c.w.eeq_B[o];
+      const float r = (float)((double)bb.x - sums[q * dc_pad(N) + k] + (double)bb.y);
+      c.w.eeq_V[o] = r;
+      mx = fmaxf(mx, fabsf(r));
+    }
+  mx = warp_maxf(mx);
+  if ((threadIdx.x & 31) == 0)
+    atomicMax(&c.w.eeq_res[b * EEQ_BIG_REFINE + it], __float_as_uint(mx));
+}
+
 namespace {
 
 int dc_sms() {
@@ -726,14 +940,24 @@ bool launch_solve(const Ctx &c, cudaStream_t st, int it) {
   return true;
 }
 
+template <int NR, bool VEC>
+void launch_residual(const Ctx &c, cudaStream_t st, int it) {
+  const dim3 rows((c.N + 255) / 256, c.B);
+  dcg_update_kernel<<<rows, 256, 0, st>>>(c, it, NR);
+  ensure_smem(dcg_residual_kernel<NR, VEC>, (int)sizeof(DrSmem));
+  dcg_residual_kernel<NR, VEC><<<dim3(dc_sms(), c.B), DC_THREADS, sizeof(DrSmem), st>>>(c, it);
+  dcg_rest_kernel<<<rows, 256, 0, st>>>(c, it, NR);
+}
+
 }  // namespace
 
 // Whether deflated conjugate gradients solve the batch: one or two structures
 // in spatial order whose matrices outgrow L2.  Charges + adjoint in us, against
 // plain conjugate gradients (d4_eeq_cg.cu) 1 x 4500 atoms 2007 / 1906, 1 x 5000
-// 2063 / 3799; against the factorisation 1 x 6001 2697 / 5559, 1 x 16000 11635 /
+// 2063 / 3799; against the factorisation 1 x 6001 2697 / 5559, 1 x 16000 10830 /
 // 21870, 2 x 4000 3291 / 3910, 2 x 6001 5255 / 6709, but 4 x 5000 7276 / 6425
-// (structures run one after the other here).
+// (structures run one after the other here; all but 1 x 16000's 10.8 ms now with
+// the residuals over the whole matrix).
 bool eeq_dcg_takes(const Ctx &c) {
   if (!c.zsorted || c.B > 2 || c.N > DC_K * DC_BLOCK) return false;
   if ((size_t)4 * c.B * c.N * c.N <= (size_t)84 << 20) return false;
@@ -745,8 +969,9 @@ bool eeq_dcg_takes(const Ctx &c) {
 bool launch_eeq_dcg(const Ctx &c, cudaStream_t st, bool adjoint) {
   const int B = c.B, N = c.N;
   if (!adjoint) {
-    dcg_az_kernel<<<dim3((N + 7) / 8, B), 256, 0, st>>>(c);
-    dcg_a0_kernel<<<dim3((N + DC_BLOCK - 1) / DC_BLOCK, B), DC_K, 0, st>>>(c);
+    const unsigned nk = (N + DC_BLOCK - 1) / DC_BLOCK;
+    dcg_az_kernel<<<dim3(nk * (nk + 1) / 2, B), 256, 0, st>>>(c);
+    dcg_a0_kernel<<<dim3(nk, B), DC_K, 0, st>>>(c);
     dcg_inverse_kernel<<<B, 1024, 0, st>>>(c);
     dcg_g_kernel<<<dim3((N + DG_ROWS - 1) / DG_ROWS, B), DC_K, 0, st>>>(c);
   }
@@ -757,7 +982,9 @@ bool launch_eeq_dcg(const Ctx &c, cudaStream_t st, bool adjoint) {
     auto solve = adjoint ? (vec ? &launch_solve<1, true> : &launch_solve<1, false>)
                          : (vec ? &launch_solve<2, true> : &launch_solve<2, false>);
     if (!solve(c, st, it)) return false;
-    launch_eeq_big_refine(c, st, it, adjoint);
+    auto residual = adjoint ? (vec ? &launch_residual<1, true> : &launch_residual<1, false>)
+                            : (vec ? &launch_residual<2, true> : &launch_residual<2, false>);
+    residual(c, st, it);
   }
   launch_eeq_big_finish(c, st, adjoint);
   return true;

@@ -42,10 +42,10 @@ int launch_fp64(const Ctx &c, cudaStream_t st);
 int launch_mixed(const Ctx &c, cudaStream_t st);
 void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint);
 void launch_eeq_big_rhs(const Ctx &c, cudaStream_t st, bool adjoint);
-void launch_eeq_big_refine(const Ctx &c, cudaStream_t st, int it, bool adjoint);
 void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint);
 bool eeq_cg_takes(const Ctx &c);  // conjugate gradients instead (d4_eeq_cg.cu)
 bool launch_eeq_cg(const Ctx &c, cudaStream_t st, bool adjoint);
+constexpr int EEQ_HALF_TILE = 128;  // the tiles of a matrix stored in half (below)
 bool eeq_dcg_takes(const Ctx &c);  // deflated, large structures (d4_eeq_dcg.cu)
 bool launch_eeq_dcg(const Ctx &c, cudaStream_t st, bool adjoint);
 void launch_pair_fwd_tc(const Ctx &c, cudaStream_t st);  // D4, precision form (d4_c6tc.cu)

@@ -1253,8 +1253,10 @@ __global__ void __launch_bounds__(256) pair_cn_bwd_mixed_kernel(Ctx c) {
 // all structures; a tile and its mirror are both stored coalesced (the
 // mirror through shared memory).  ``factor``: the lower tiles' hi part also goes
 // to the multi-CTA factorisation's matrix F (row stride eeq_ldf(N)), which
-// reads nothing above the diagonal.
-__global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c, bool factor) {
+// reads nothing above the diagonal.  ``half``: of the upper triangle only what
+// lies in the diagonal tiles of EEQ_HALF_TILE is stored (all that the deflated
+// conjugate gradients read).
+__global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c, bool factor, bool half) {
   __shared__ float4 s_erf[ERF_TAB];
   __shared__ float s_hi[32][33], s_lo[32][33];
   for (int k = threadIdx.x; k < ERF_TAB; k += blockDim.x) s_erf[k] = c.w.erf_tab[k];
@@ -1316,7 +1318,8 @@ __global__ void __launch_bounds__(256) eeq_build_df_kernel(Ctx c, bool factor) {
       s_hi[rr][tx] = v.hi;
       s_lo[rr][tx] = v.lo;
     }
-    if (ti != tj) {
+    constexpr int HT = EEQ_HALF_TILE / 32;
+    if (ti != tj && (!half || ti / HT == tj / HT)) {
       __syncthreads();
 #pragma unroll 1
       for (int kk = 0; kk < 4; ++kk) {
@@ -1792,9 +1795,9 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
       eeq_mixed_kernel<true><<<B, EEQ_THREADS, vec_bytes + pt_bytes + tri_bytes, st>>>(c);
     } else {
       const bool iterate = eeq_dcg_takes(c) || eeq_cg_takes(c);
-      eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, !iterate);
+      eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, !iterate, eeq_dcg_takes(c));
       if (!iterate || !launch_eeq_iterative(c, st, false)) {
-        if (iterate) eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true);
+        if (iterate) eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true, false);
         launch_eeq_big(c, st, false);
       }
     }
@@ -1839,7 +1842,7 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
         if (!eeq_dcg_takes(c) && !eeq_cg_takes(c)) {
           launch_eeq_big(c, st, true);
         } else if (!launch_eeq_iterative(c, st, true)) {  // the factor is needed after all
-          eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true);
+          eeq_build_df_kernel<<<build_blocks(c), 256, 0, st>>>(c, true, false);
           launch_eeq_big(c, st, false);
           launch_eeq_big(c, st, true);
         }
