@@ -13,8 +13,8 @@
 // 664 us, and so were direct loads instead of staged copies, 563.
 // Measured, ATM stage, against a tile kernel with the sums in shared memory
 // (N <= 234; no parameter gradients) and the per-triple kernel elsewhere: 512
-// structures of 8..200 atoms 572 -> 503 us; 256 of 20..150 with parameter
-// gradients 793 -> 249; 997 atoms 2115 -> 562; 1000 of 5..60, energies only,
+// structures of 8..200 atoms 572 -> 481 us; 256 of 20..150 with parameter
+// gradients 793 -> 245; 997 atoms 2115 -> 503; 1000 of 5..60, energies only,
 // 110 -> 55.
 #include "d4_atm.cuh"
 #include "d4_common.cuh"
@@ -673,7 +673,9 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
 // shared memory.  After the unit-weight kernels also the atom energies from the row sums
 // (every triple reaches an atom through two of its pairs, a third of its
 // energy each; a pair beyond the cutoff counts twice, see a3_step) and, with
-// parameter gradients, the factor s9.
+// parameter gradients, the factor s9.  Bound by latency: loads carry no condition and a
+// warp's eight sums leave by one exchange (512 structures of 8..200 atoms 42 -> 24 us;
+// 16000 atoms 496 -> 341 us).
 __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float s9) {
   __shared__ float2 s_t[32][33];
   __shared__ float s_e[32][33];
@@ -690,40 +692,48 @@ __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float
   const float4 *T = c.w.ptf + (size_t)b * N * N;
   const int *Z = c.w.z + (size_t)b * N;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int jr = tj * 32 + tx;
-  const bool jok = jr < n && Z[jr] != 0;
-  const bool far_j = rows && jok && far2[jr] > cut2;
+  const int jr = tj * 32 + tx, jc = min(jr, N - 1);
+  float2 v[4];
+  int zi[4];
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int i = ti * 32 + r;
-    float2 v = make_float2(0.f, 0.f);
-    if (jok && jr > i && Z[i] != 0) {
-      v = SP[(size_t)i * N + jr];
-      if (s9 != 1.f) {
-        v.x *= s9;
-        v.y *= s9;
-        SP[(size_t)i * N + jr] = v;
-      }
+  for (int q = 0; q < 4; ++q) {  // (unconditional, so that all loads are in flight)
+    const int i = ti * 32 + ty + 8 * q, ic = min(i, N - 1);
+    zi[q] = Z[ic];
+    v[q] = SP[(size_t)ic * N + jc];
+  }
+  const bool jok = jr < n && Z[jc] != 0;
+  const bool far_j = rows && jok && far2[jc] > cut2;
+  float e[8];  // row sums' terms, then those of the mirrored rows
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = ty + 8 * q, i = ti * 32 + r;
+    const bool ok = jok && jr > i && zi[q] != 0;  // (i < jr < n)
+    if (!ok) v[q] = make_float2(0.f, 0.f);
+    if (ok && s9 != 1.f) {
+      v[q].x *= s9;
+      v[q].y *= s9;
+      SP[(size_t)i * N + jr] = v[q];
     }
-    float ev = v.y;
-    if (far_j && ev != 0.f && T[(size_t)i * N + jr].x > cut2) ev += ev;
-    s_t[r][tx] = v;
-    s_e[r][tx] = ev;
-    if (rows) {
-      const float e = warp_sumf(ev);
-      if (tx == 0 && e != 0.f) atomicAdd(&e3[i], (double)e * (1.0 / 6.0));
-    }
+    e[q] = v[q].y;
+    if (far_j && e[q] != 0.f && T[(size_t)i * N + jr].x > cut2) e[q] += e[q];
+    s_t[r][tx] = v[q];
+    if (rows) s_e[r][tx] = e[q];
   }
   __syncthreads();
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
+  for (int q = 0; q < 4; ++q) {
+    const int r = ty + 8 * q;
     const int i = tj * 32 + r, j = ti * 32 + tx;  // destination (i > j)
-    const float2 v = s_t[tx][r];
-    if (i < n && j < n && i > j) SP[(size_t)i * N + j] = v;
-    if (rows) {
-      const float e = warp_sumf(s_e[tx][r]);
-      if (tx == 0 && e != 0.f) atomicAdd(&e3[i], (double)e * (1.0 / 6.0));
-    }
+    if (i < n && j < n && i > j) SP[(size_t)i * N + j] = s_t[tx][r];
+    if (rows) e[4 + q] = s_e[tx][r];
+  }
+  if (rows) {
+    halving<8, 16, 3>(e);
+    e[0] += __shfl_xor_sync(0xffffffffu, e[0], 2);
+    e[0] += __shfl_xor_sync(0xffffffffu, e[0], 1);
+    const int q = tx >> 2;  // the sum that the lane ends with: bits 16, 8, 4
+    const int i = (q < 4 ? ti : tj) * 32 + ty + 8 * (q & 3);
+    if ((tx & 3) == 0 && e[0] != 0.f) atomicAdd(&e3[i], (double)e[0] * (1.0 / 6.0));
   }
 }
 
