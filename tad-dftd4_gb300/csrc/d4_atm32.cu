@@ -674,11 +674,12 @@ __global__ void __launch_bounds__(SP_THREADS, 2) atm_sparse32_kernel(Ctx c) {
 // (every triple reaches an atom through two of its pairs, a third of its
 // energy each; a pair beyond the cutoff counts twice, see a3_step) and, with
 // parameter gradients, the factor s9.  Bound by latency: loads carry no condition and a
-// warp's eight sums leave by one exchange (512 structures of 8..200 atoms 42 -> 24 us;
-// 16000 atoms 496 -> 341 us).
+// warp's eight sums leave by one exchange (512 structures of 8..200 atoms 42 -> 23 us;
+// 16000 atoms 496 -> 335 us).
 __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float s9) {
   __shared__ float2 s_t[32][33];
   __shared__ float s_e[32][33];
+  __shared__ float s_sum[64];
   const int b = blockIdx.y, N = c.N, n = c.w.n_eff[b];
   int ti, tj;  // rows ti, columns tj >= ti
   tri_entry(blockIdx.x, tj, ti);
@@ -732,8 +733,13 @@ __global__ void __launch_bounds__(256) atm_mirror_kernel(Ctx c, bool rows, float
     e[0] += __shfl_xor_sync(0xffffffffu, e[0], 2);
     e[0] += __shfl_xor_sync(0xffffffffu, e[0], 1);
     const int q = tx >> 2;  // the sum that the lane ends with: bits 16, 8, 4
-    const int i = (q < 4 ? ti : tj) * 32 + ty + 8 * (q & 3);
-    if ((tx & 3) == 0 && e[0] != 0.f) atomicAdd(&e3[i], (double)e[0] * (1.0 / 6.0));
+    if ((tx & 3) == 0) s_sum[(q < 4 ? 0 : 32) + ty + 8 * (q & 3)] = e[0];
+    __syncthreads();
+    if (threadIdx.x < 64) {  // (FP64 instructions of two warps, not eight)
+      const float es = s_sum[threadIdx.x];
+      if (es != 0.f)
+        atomicAdd(&e3[(threadIdx.x < 32 ? ti : tj) * 32 + tx], (double)es * (1.0 / 6.0));
+    }
   }
 }
 
