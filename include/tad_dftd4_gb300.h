@@ -18,11 +18,12 @@
  * size comes from ``d4_workspace_size``.  All pointers named ``d_*`` or
  * documented as "device" are device pointers.  ``stream`` is a
  * ``cudaStream_t`` passed as ``void*``; work is enqueued on it and every
- * call returns without synchronising, with one exception: for structures
- * padded beyond 3584 atoms the precision form's EEQ solves wait once each
- * for ``stream`` (after their second refinement iteration, to launch a
- * third only if a residual asks for it), unless the stream is being
- * captured or the call sets D4_FLAG_NO_HOST_WAIT.  Calls on different
+ * call returns without synchronising, with one exception: where the
+ * precision form factorises the EEQ matrices of structures padded beyond
+ * 3584 atoms (batches that its conjugate gradients do not take), the
+ * solves wait once each for ``stream`` (after their second refinement
+ * iteration, to launch a third only if a residual asks for it), unless the
+ * stream is being captured or the call sets D4_FLAG_NO_HOST_WAIT.  Calls on different
  * streams with different workspaces are independent.
  *
  * Errors: every entry point returns a ``d4_status`` code.  Input problems

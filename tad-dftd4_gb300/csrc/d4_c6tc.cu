@@ -17,8 +17,8 @@
 // evaluates the rational damping, the energy, the direct gradient, the C6
 // adjoint dE/dA'_i and the ATM pair record of every pair (i, j) -- the C6
 // matrices never reach global memory.  Everything after the contraction is
-// the arithmetic of pair_fwd_mixed_kernel (the D4S model keeps that kernel:
-// its C6 does not factorise into one product).
+// the arithmetic of the D4S kernels (d4_d4s32.cu: D4S C6 does not factorise
+// into one product).
 #include <float.h>
 
 #include "d4_common.cuh"
@@ -593,7 +593,7 @@ namespace d4 {
 // ---------------------------------------------------------------- ATM / C6(q=0) adjoint
 
 // ATM forces, the C6(q=0) adjoint and the chain rule to dE/dCN and dE/dq of
-// the D4 precision form (the work of pair_atm_bwd_mixed_kernel), with the
+// the D4 precision form (the work of pair_bwd_d4s32_kernel), with the
 // C6(q=0) adjoint on the tensor cores:
 //   G0_x(w) = sum_y D_xy A0'_y(w),  D_xy = P_xy / (2 C6(q=0)_xy),
 // P_xy = the weighted triple energies of the pair, C6(q=0)_xy = c_xy^2 from

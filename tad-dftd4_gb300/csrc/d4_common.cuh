@@ -139,7 +139,7 @@ struct Workspace {
   double *f3x;      // [B*N*3] ATM part of dE/dR
   double *eeq_L;    // [B*N*(N+1)/2] packed Cholesky factor (FP64 method) or
                     // packed FP64 EEQ matrix (precision form)
-  float4 *pos32;    // [B*N] positions relative to the structure's first slot, FP32,
+  float4 *pos32;    // [B*N] positions relative to one of the structure's atoms, FP32,
                     // with sqrt(r4r2) in .w (both methods)
   float4 *aux32;    // [B*N] (cov_d3, en, eeq_rad, 0) in FP32 (both methods)
   int *cidx;        // [B*N] index among the real atoms of the structure, -1 padding
@@ -152,7 +152,7 @@ struct Workspace {
   float *eeq_lo;    //         double-float hi + lo
   int *ridx;        // [B*N] atom index of the k-th real atom
   int *n_real;      // [B] real atoms
-  float4 *pos32lo;  // [B*N] low parts of the positions: pos32 + pos32lo = r - r_first
+  float4 *pos32lo;  // [B*N] low parts of the positions: pos32 + pos32lo = r - r_origin
   float4 *erf_tab;  // [ERF_TAB] (erf(x0) hi, lo, 2/sqrt(pi) exp(-x0^2) hi, lo), x0 = k/256
   float2 *igam;     // [MAX_ELEM_ID^2] 1/sqrt(rad_a^2 + rad_b^2) as double-float
   float2 *eeq_diag; // [MAX_ELEM_ID] eta + sqrt(2/pi)/rad as double-float
@@ -500,7 +500,7 @@ __host__ __device__ inline size_t tri_index(int i, int j) {  // packed lower, j 
   return (size_t)i * (i + 1) / 2 + j;
 }
 
-// r_i - r_j from the FP32 positions relative to the structure's first atom
+// r_i - r_j from the FP32 positions relative to one of the structure's atoms
 // (pos32) and their low parts (pos32lo): the high parts of nearby atoms
 // subtract exactly, the low parts restore what rounding the absolute
 // positions to FP32 lost (about 4e-6 Bohr at 60 Bohr from the origin).

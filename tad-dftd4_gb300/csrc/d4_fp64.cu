@@ -5,7 +5,8 @@
 // quantities live in dense per-structure N x N blocks, only the leading
 // n_eff x n_eff part of which is touched.  Every "atom-owned" kernel maps one
 // warp to one atom i and loops its lanes over partners j, so per-atom sums
-// need no atomics.  The general ATM kernel maps a CTA to a tile of pairs (j, k)
+// need no atomics; the coordination numbers go over unordered pairs and add
+// both ends' sums by reductions at L2.  The general ATM kernel maps a CTA to a tile of pairs (j, k)
 // and loops over the third atom i < j.
 #include <float.h>
 #include <math.h>
