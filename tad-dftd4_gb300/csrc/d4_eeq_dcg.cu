@@ -7,14 +7,15 @@
 // consecutive atoms are compact in space (Z-order), so the piecewise constant
 // vectors Z of the blocks (K <= 256 of them) hold those modes: CG on
 // P A, P = 1 - A Z (Z^T A Z)^-1 Z^T, gains five digits in 14 iterations at 6000
-// atoms and 17 at 16000, where plain CG takes 32 at 6000.  As in d4_eeq_cg.cu the FP32 solve is the
-// inner one of a refinement whose residuals are taken in double-float.
+// atoms and 17 at 16000, where plain CG takes 32 at 6000.  As in d4_eeq_cg.cu the
+// FP32 solve is the inner one of a refinement whose residuals are taken in
+// double-float.
 //
 // Measured at 16000 atoms, charges + adjoint: 21.9 (factorisation) -> 10.8 ms,
 // of it 7.7 the solves, 1.5 the residuals, 1.0 the matrix, 0.4 Z^T A Z, its
-// inverse and G (2.0, 1.2 and 0.5 over the whole matrix).  A product takes 93 us with one right-hand side (5.5 TB/s of the
-// half matrix), 122 with two; the rest of an iteration (two exchanges, three
-// barriers) 12 to 14 us.
+// inverse and G (2.0, 1.2 and 0.5 over the whole matrix).  A product takes 93 us
+// with one right-hand side (5.5 TB/s of the half matrix), 122 with two; the rest
+// of an iteration (two exchanges, three barriers) 12 to 14 us.
 //
 // An iteration is one product with A, bound by reading the matrix: only tiles
 // on and below the diagonal are read, each for both of its products (rows from

@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c, int parts) {
 }
 
 // exp(x), |x| <= 80, rounded once: reduction by ln 2 = 355/512 - 2.1e-4 (Cody and
-// Waite, Software Manual for the Elementary Functions, 1980) and the series, its first terms in double-float (within 1e-10 before the
-// rounding).  In place of an FP64 exp, whose 30 instructions for every reference of
+// Waite, Software Manual for the Elementary Functions, 1980) and the series, its
+// first terms in double-float (within 1e-10 before the rounding).  In place of an FP64 exp, whose 30 instructions for every reference of
 // every atom were most of the weights' time.
 __device__ __forceinline__ float exp_once(dfl x) {
   const float n = rintf(x.hi * 1.44269504f);
@@ -1395,8 +1395,8 @@ __device__ __forceinline__ dfl df_warp_sum(dfl a) {
 // (FP64-accurate, on the FP32 pipe): a warp takes four rows at a time, lanes
 // over columns (coalesced), so that 32 independent loads per lane are in
 // flight (one row at a time left the warp waiting on L2 latency row after
-// row; loads under a condition 5 % of the solves).  r is rounded to FP32 into vf, the right-hand side of the next
-// correction; returns max |r| over the block.
+// row; loads under a condition 5 % of the solves).  r is rounded to FP32 into
+// vf, the right-hand side of the next correction; returns max |r| over the block.
 __device__ float eeq_residual_df(const float *Hi, const float *Lo, const float2 *X,
                                  const float2 *BB, float *vf, int m, int N, int nr,
                                  float *s_red) {
