@@ -112,7 +112,10 @@ def _atoms(numbers: torch.Tensor, N: int, device) -> torch.Tensor:
 
 
 def _structures(positions: torch.Tensor, N: int) -> torch.Tensor:
-    """Positions as (B, N, 3)."""
+    """Positions as (B, N, 3); the kernels read three coordinates per atom."""
+    if positions.shape[-1] != 3:
+        raise RuntimeError(f"positions of shape {tuple(positions.shape)}: the last dimension "
+                           "has to hold the three coordinates")
     return positions if positions.dim() == 3 else positions.reshape(-1, N, 3)
 
 
@@ -663,7 +666,7 @@ def hessian(numbers: torch.Tensor, positions: torch.Tensor, charge, param: Param
     N = shape[-1]
     nums = numbers.reshape(-1, N)
     B = nums.shape[0]
-    pos = positions.reshape(-1, N, 3)
+    pos = _structures(positions, N)
     chg = _as_tensor(charge, positions.device, torch.float64)
     chg = chg.expand(B) if chg.dim() == 0 else chg.reshape(-1)
     if chg.numel() != B:
@@ -713,7 +716,7 @@ def get_properties(numbers: torch.Tensor, positions: torch.Tensor, charge=None,
     N = shape[-1]
     nums = numbers.reshape(-1, N).to(device=device, dtype=torch.int64).contiguous()
     B = nums.shape[0]
-    pos = positions.reshape(-1, N, 3).detach().to(torch.float64).contiguous()
+    pos = _structures(positions, N).detach().to(torch.float64).contiguous()
     charge = 0.0 if charge is None else charge
     chg = _as_tensor(charge, device, torch.float64)
     chg = (chg.expand(B) if chg.dim() == 0 else chg.reshape(-1)).contiguous()
