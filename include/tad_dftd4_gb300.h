@@ -314,6 +314,14 @@ int d4_probe_fma(int32_t fp64, int32_t n_blocks, int32_t iters, double *d_sink,
 int d4_selftest_wait(int32_t *d_result, uint64_t limit_ns, void *stream);
 
 /*
+ * Self-test of the error report: a launch that the runtime refuses (more
+ * shared memory than a CTA can have; nothing runs), followed by the set-up of
+ * another kernel as inside a call.  Returns D4_ERR_CUDA, or D4_OK if the
+ * error was lost on the way.  No counterpart in the reference.
+ */
+int d4_selftest_launch_error(void *stream);
+
+/*
  * Allocation-free variant of d4_dispersion.  This entry point has no
  * counterpart in the reference (tad-dftd4 allocates tensors on every call).
  *

@@ -171,6 +171,7 @@ SIGNATURES = {
          ctypes.POINTER(Params), c_void_p, c_size_t, ctypes.POINTER(Properties), c_void_p],
     ),
     "d4_selftest_wait": (c_int, [c_void_p, ctypes.c_uint64, c_void_p]),
+    "d4_selftest_launch_error": (c_int, [c_void_p]),
     "d4_dispersion_noalloc": (
         c_int,
         [ctypes.POINTER(Tables), ctypes.POINTER(ModelCfg), ctypes.POINTER(Batch),

@@ -11,6 +11,21 @@
 
 namespace d4 {
 
+// The first error of this thread's current call (d4_common.cuh).
+static thread_local cudaError_t g_kept = cudaSuccess;
+
+void keep_error() {
+  const cudaError_t e = cudaGetLastError();
+  if (g_kept == cudaSuccess) g_kept = e;
+}
+
+cudaError_t take_error() {
+  keep_error();
+  const cudaError_t e = g_kept;
+  g_kept = cudaSuccess;
+  return e;
+}
+
 // (device, kernel) -> dynamic shared-memory limit already set
 void ensure_smem_impl(const void *func, size_t bytes) {
   static std::mutex mu;
@@ -18,16 +33,20 @@ void ensure_smem_impl(const void *func, size_t bytes) {
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
+  std::pair<std::pair<int, const void *>, size_t> *at = nullptr;
   for (auto &e : done)
-    if (e.first.first == dev && e.first.second == func) {
-      if (bytes > e.second) {
-        cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        e.second = bytes;
-      }
-      return;
-    }
-  cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  done.push_back({{dev, func}, bytes});
+    if (e.first.first == dev && e.first.second == func) at = &e;
+  if (at && bytes <= at->second) return;
+  keep_error();
+  if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+      cudaSuccess) {
+    keep_error();
+    return;
+  }
+  if (at)
+    at->second = bytes;
+  else
+    done.push_back({{dev, func}, bytes});
 }
 
 }  // namespace d4
@@ -83,7 +102,7 @@ int d4_prepare_alpha(const d4_tables_t *tables, const d4_model_cfg_t *cfg,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   d4::launch_prepare_alpha(*tables, *cfg, d_refalpha, d_refascale, d_refscount, d_refsys,
                            d_secscale, d_secalpha, n_sec, d_refh, d_alpha_out, st);
-  return check_cuda(cudaGetLastError());
+  return check_cuda(d4::take_error());
 }
 
 size_t d4_workspace_size(int32_t n_struct, int32_t n_pad, int32_t n_slots, uint32_t flags) {
@@ -149,7 +168,7 @@ int d4_dispersion(const d4_tables_t *tables, const d4_model_cfg_t *cfg,
     d4::launch_mixed(c, st);
   else
     d4::launch_fp64(c, st);
-  return check_cuda(cudaGetLastError());
+  return check_cuda(d4::take_error());
 }
 
 int d4_properties(const d4_tables_t *tables, const d4_model_cfg_t *cfg,
@@ -185,7 +204,7 @@ int d4_properties(const d4_tables_t *tables, const d4_model_cfg_t *cfg,
           (float)pp.cn_eeq_max, (float)cfg->wf,        (float)cfg->ga};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   d4::launch_properties(c, out->d_c6, out->d_alpha, out->d_charges, st);
-  return check_cuda(cudaGetLastError());
+  return check_cuda(d4::take_error());
 }
 
 int d4_status_async(void *d_workspace, int32_t *h_status, void *stream) {

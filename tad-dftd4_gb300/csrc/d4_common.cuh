@@ -204,6 +204,13 @@ struct Workspace {
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// The runtime's last error is what tells a call that one of its launches was
+// refused, and some runtime calls that succeed reset it (cudaFuncSetAttribute on a
+// kernel does): keep_error() before such a call sets it aside, and take_error()
+// at the end of an entry point gives the first one of the thread's call.
+void keep_error();
+cudaError_t take_error();
+
 // Raise a kernel's dynamic shared-memory limit once per device and size:
 // cudaFuncSetAttribute costs microseconds of host time, which every call of
 // the library would otherwise pay again (d4_api.cu).

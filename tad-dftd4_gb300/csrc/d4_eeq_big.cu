@@ -1097,6 +1097,7 @@ SideStream *side_stream_for_device() {
   SideStream &ss = g_side[dev & 63];
   if (!ss.tried) {
     ss.tried = true;
+    keep_error();
     int lo = 0, hi = 0;
     bool ok = cudaDeviceGetStreamPriorityRange(&lo, &hi) == cudaSuccess &&
               cudaStreamCreateWithPriority(&ss.s, cudaStreamNonBlocking, hi) == cudaSuccess;

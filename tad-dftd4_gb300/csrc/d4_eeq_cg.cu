@@ -420,6 +420,7 @@ bool launch_cg(const Ctx &c, cudaStream_t st) {
   const void *f = pick(&eeq_cg_kernel<CG_MANY, NR, true>, &eeq_cg_kernel<CG_MANY, NR, false>,
                        &eeq_cg_kernel<CG_FEW, NR, true>, &eeq_cg_kernel<CG_FEW, NR, false>);
   ensure_smem_impl(f, smem);
+  keep_error();  // (a refused launch of this kernel itself is no error of the call)
   if (cudaLaunchCooperativeKernel(f, dim3((unsigned)(p.G * p.groups)),
                                   dim3(few ? CG_FEW : CG_MANY), args, smem, st) != cudaSuccess) {
     cudaGetLastError();

@@ -933,6 +933,7 @@ bool launch_solve(const Ctx &c, cudaStream_t st, int it) {
   void *args[] = {&cc, &it};
   const void *f = reinterpret_cast<const void *>(&eeq_dcg_kernel<NR, VEC>);
   ensure_smem_impl(f, sizeof(DcSmem));
+  keep_error();  // (a refused launch of this kernel itself is no error of the call)
   if (cudaLaunchCooperativeKernel(f, dim3((unsigned)dc_sms()), dim3(DC_THREADS), args,
                                   sizeof(DcSmem), st) != cudaSuccess) {
     cudaGetLastError();

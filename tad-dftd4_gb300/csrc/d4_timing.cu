@@ -72,9 +72,19 @@ __global__ void selftest_wait_kernel(int32_t *result, unsigned long long limit_n
   *result = tc::mbar_wait(mbar, 0u, limit_ns) ? D4_OK : D4_ERR_DEVICE_TIMEOUT;
 }
 
+// Two kernels that do nothing, for d4_selftest_launch_error.
+__global__ void selftest_refused_kernel() {}
+__global__ void selftest_next_kernel() {}
+
 }  // namespace d4
 
 extern "C" {
+
+int d4_selftest_launch_error(void *stream) {
+  d4::selftest_refused_kernel<<<1, 1, 1 << 20, static_cast<cudaStream_t>(stream)>>>();
+  d4::ensure_smem(d4::selftest_next_kernel, 64 * 1024);
+  return d4::take_error() == cudaSuccess ? D4_OK : D4_ERR_CUDA;
+}
 
 int d4_selftest_wait(int32_t *d_result, uint64_t limit_ns, void *stream) {
   if (!d_result || limit_ns > 1000000000ull) return D4_ERR_ARGUMENT;
