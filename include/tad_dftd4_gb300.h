@@ -87,6 +87,10 @@ typedef enum d4_model_kind { D4_MODEL_D4 = 0, D4_MODEL_D4S = 1 } d4_model_kind;
    in flight, tensor memory released, early return).  Results of such a call
    are incomplete; the next call is unaffected. */
 #define D4_FLAG_TEST_TIMEOUT 0x80000000u
+/* Test hook of the paths for what usually does not happen at small sizes: the
+   FP64 EEQ solves keep their vectors in global memory (as for structures padded
+   beyond 14080 atoms).  Results are those of a call without it. */
+#define D4_FLAG_TEST_FALLBACK 0x40000000u
 
 /* Entries per structure of d_param_grad: dE_b / d(s6, s8, s10, a1, a2, s9,
    alp, rs6, rs8, bet), then two unused entries. */

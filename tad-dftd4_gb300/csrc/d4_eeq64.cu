@@ -342,7 +342,7 @@ __device__ double eeq64_dot(const double *x, const double *y, int m, SolveSmem &
 // q = A^-1 (b - lambda 1) = L^-T (z_b - lambda z_1) takes one right-hand side.
 // By the whole CTA; z_1 stays for the adjoint (eeq_y, compact order).
 __device__ void eeq64_charges(const Ctx &c, int b, const double *L, const InvAt &inv, double *v,
-                              int ldv, int m, SolveSmem &sm) {
+                              ptrdiff_t ldv, int m, SolveSmem &sm) {
   const double sx = eeq64_dot(v, v + ldv, m, sm), sy = eeq64_dot(v + ldv, v + ldv, m, sm);
   const double lam = m > 0 ? (sx - c.charge[b]) / sy : 0.0;
   if (threadIdx.x == 0) {
@@ -551,19 +551,26 @@ __global__ void __launch_bounds__(128) eeq64_update_kernel(Ctx c, int k0) {
                         t0, m);
 }
 
-// Backward solve, charges, and the block inverses into the factor.
+// Backward solve, charges, and the block inverses into the factor.  SMEM: the
+// vectors in shared memory, else where they are (eeq64_vec_fits).
+template <bool SMEM>
 __global__ void __launch_bounds__(256) eeq64_finish_kernel(Ctx c) {
   extern __shared__ double s_dyn[];
   __shared__ SolveSmem ss;
   const int b = blockIdx.x, N = c.N;
   const int m = eeq64_order(c, b);
   double *L = eeq64_factor(c, b), *X = eeq64_inv(c, b);
-  for (int t = threadIdx.x; t < m; t += blockDim.x) {
-    s_dyn[t] = eeq64_rhs(c, b, 0)[t];
-    s_dyn[N + t] = eeq64_rhs(c, b, 1)[t];
+  double *v0 = eeq64_rhs(c, b, 0), *v1 = eeq64_rhs(c, b, 1);
+  if (SMEM) {
+    for (int t = threadIdx.x; t < m; t += blockDim.x) {
+      s_dyn[t] = v0[t];
+      s_dyn[N + t] = v1[t];
+    }
+    v0 = s_dyn;
+    v1 = s_dyn + N;
   }
   __syncthreads();
-  eeq64_charges(c, b, L, InvAt{L, X}, s_dyn, N, m, ss);
+  eeq64_charges(c, b, L, InvAt{L, X}, v0, v1 - v0, m, ss);
   if (c.flags & D4_FLAG_GRADIENT)
     for (int t = threadIdx.x; t < m * EB; t += blockDim.x) {
       const int i = t / EB, cc = t % EB, k0 = i & ~(EB - 1);
@@ -573,37 +580,45 @@ __global__ void __launch_bounds__(256) eeq64_finish_kernel(Ctx c) {
 
 // Adjoint of the constrained EEQ solve: w = A^-1 (g - nu 1) with sum(w) = 0,
 // g = dE/dq; as for the charges, nu = z_1 . z_g / z_1 . z_1 and w = L^-T (z_g -
-// nu z_1).  Then dE/d(raw EEQ CN) = w kcn / (2 sqrt(cn)) dcap.
+// nu z_1).  Then dE/d(raw EEQ CN) = w kcn / (2 sqrt(cn)) dcap.  SMEM: the vector
+// in shared memory, else in the room of the pair records, whose readers are done.
+template <bool SMEM>
 __global__ void __launch_bounds__(ES_THREADS) eeq64_adjoint_kernel(Ctx c) {
   extern __shared__ double s_dyn[];
   __shared__ SolveSmem ss;
   const int b = blockIdx.x, N = c.N;
   const int m = eeq64_order(c, b);
   const double *L = eeq64_factor(c, b), *z1 = c.w.eeq_y + (size_t)b * N;
+  double *v = SMEM ? s_dyn : c.w.pr_r + (size_t)b * N;
   for (int i = threadIdx.x; i < N; i += ES_THREADS) {
     const int k = c.w.cidx[(size_t)b * N + i];
-    if (k >= 0) s_dyn[k] = c.w.dEdq[(size_t)b * N + i];
+    if (k >= 0) v[k] = c.w.dEdq[(size_t)b * N + i];
   }
   __syncthreads();
   const InvAt inv{L, nullptr};
-  eeq64_solve<true>(L, inv, s_dyn, m, ss);
-  const double su = eeq64_dot(s_dyn, z1, m, ss);
+  eeq64_solve<true>(L, inv, v, m, ss);
+  const double su = eeq64_dot(v, z1, m, ss);
   const double nu = m > 0 ? su / c.w.eeq_sum[2 * b] : 0.0;
-  for (int k = threadIdx.x; k < m; k += ES_THREADS) s_dyn[k] = fma(-nu, z1[k], s_dyn[k]);
+  for (int k = threadIdx.x; k < m; k += ES_THREADS) v[k] = fma(-nu, z1[k], v[k]);
   __syncthreads();
-  eeq64_solve<false>(L, inv, s_dyn, m, ss);
+  eeq64_solve<false>(L, inv, v, m, ss);
   for (int i = threadIdx.x; i < N; i += ES_THREADS) {
     const size_t a = (size_t)b * N + i;
     const int k = c.w.cidx[a];
     double w = 0.0, d = 0.0;
     if (k >= 0) {
-      w = s_dyn[k];
+      w = v[k];
       const double cq = c.w.cnq[a];
       d = cq > 0.0 ? w * c.tab.eeq_kcn[c.w.z[a]] * 0.5 / sqrt(cq) * c.w.dcnq[a] : 0.0;
     }
     c.w.eeq_w[a] = w;
     c.w.dEdcnq[a] = d;
   }
+}
+
+// Whether the final solves' vectors fit a CTA's shared memory (N <= 14080).
+static bool eeq64_vec_fits(const Ctx &c) {
+  return !(c.flags & D4_FLAG_TEST_FALLBACK) && 16 * (size_t)c.N <= 220 * 1024;
 }
 
 template <int S>
@@ -654,13 +669,21 @@ void launch_eeq64(const Ctx &c, cudaStream_t st) {
     else
       eeq64_update_kernel<8><<<dim3((unsigned)(tiles * 4 + 3) / 4, B), 128, 0, st>>>(c, k0);
   }
-  ensure_smem(eeq64_finish_kernel, 16 * (size_t)N);
-  eeq64_finish_kernel<<<B, ES_THREADS, 16 * (size_t)N, st>>>(c);
+  if (eeq64_vec_fits(c)) {
+    ensure_smem(eeq64_finish_kernel<true>, 16 * (size_t)N);
+    eeq64_finish_kernel<true><<<B, ES_THREADS, 16 * (size_t)N, st>>>(c);
+  } else {
+    eeq64_finish_kernel<false><<<B, ES_THREADS, 0, st>>>(c);
+  }
 }
 
 void launch_eeq64_adjoint(const Ctx &c, cudaStream_t st) {
-  ensure_smem(eeq64_adjoint_kernel, 8 * (size_t)c.N);
-  eeq64_adjoint_kernel<<<c.B, ES_THREADS, 8 * (size_t)c.N, st>>>(c);
+  if (eeq64_vec_fits(c)) {
+    ensure_smem(eeq64_adjoint_kernel<true>, 8 * (size_t)c.N);
+    eeq64_adjoint_kernel<true><<<c.B, ES_THREADS, 8 * (size_t)c.N, st>>>(c);
+  } else {
+    eeq64_adjoint_kernel<false><<<c.B, ES_THREADS, 0, st>>>(c);
+  }
 }
 
 }  // namespace d4
