@@ -326,6 +326,14 @@ int d4_selftest_wait(int32_t *d_result, uint64_t limit_ns, void *stream);
 int d4_selftest_launch_error(void *stream);
 
 /*
+ * The numbering of the tasks of the precision form's ATM (host code, nothing
+ * runs): task ``task`` of a structure of ``n`` atoms whose tasks cover 8 ``s``
+ * inner atoms each goes to ``out`` as (range of inner atoms, tile of middle
+ * atoms, chunk of outer atoms).  Returns the number of tasks.
+ */
+int64_t d4_selftest_atm_task(int32_t n, int32_t s, int64_t task, int32_t *out);
+
+/*
  * Allocation-free variant of d4_dispersion.  This entry point has no
  * counterpart in the reference (tad-dftd4 allocates tensors on every call).
  *

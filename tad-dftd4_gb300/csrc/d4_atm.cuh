@@ -82,4 +82,39 @@ __device__ __forceinline__ bool atm_sparse_mode(const Ctx &c, int b, int n) {
   return dmax <= (unsigned long long)ATM_SPARSE_DMAX && 2 * visits < all;
 }
 
+// ---------------------------------------------------------------- tasks of atm32_kernel
+
+constexpr int A3 = 8;  // middle atoms per lane, and outer atoms per task
+
+// Number of tasks of a structure of n atoms whose tasks cover 8 s inner atoms
+// each.  Tiles of middle atoms are counted from the last (n - 9 .. n - 2), so
+// that all chunks of outer atoms are full and the lowest tile, with the fewest
+// inner atoms, takes what does not divide by eight (its first j may be < 1).
+// Tile g from below has NG - g chunks of outer atoms and g / s + 1 ranges of
+// inner atoms.
+__host__ __device__ inline long long a3_tasks(int n, int s) {
+  const long long ng = n < 3 ? 0 : (n - 2 + A3 - 1) / A3;
+  long long t = 0;
+  for (long long m = ng; m > 0; m -= s) t += m * (m + 1) / 2;
+  return t;
+}
+
+// Task t of them: the inner range ip, tile u (from the top) and chunk ch of
+// outer atoms.  (All of it in 64 bits: 47300 atoms have 2^31 tasks.)
+struct A3Task {
+  int ip, u, ch;
+};
+__host__ __device__ inline A3Task a3_task(long long t, int n, int s) {
+  A3Task r;
+  r.ip = 0;
+  long long m = (n - 2 + A3 - 1) / A3;
+  while (t >= m * (m + 1) / 2) {
+    t -= m * (m + 1) / 2;
+    m -= s;
+    ++r.ip;
+  }
+  tri_entry(t, r.u, r.ch);
+  return r;
+}
+
 }  // namespace d4

@@ -24,7 +24,6 @@ namespace d4 {
 
 namespace {
 
-constexpr int A3 = 8;             // middle atoms per lane, and outer atoms per task
 constexpr int A3_THREADS = 128;
 constexpr int A3_ROW = 10;        // row and group strides of the (i, j) sums in shared memory
 constexpr int A3_GROUP = 88;      // (float2; no bank conflicts)
@@ -196,19 +195,6 @@ __device__ __forceinline__ void a3_step(const A3Pair &a, const float4 *rec, int 
   }
 }
 
-// Number of tasks of a structure of n atoms whose tasks cover 8 s inner atoms
-// each.  Tiles of middle atoms are counted from the last (n - 9 .. n - 2), so
-// that all chunks of outer atoms are full and the lowest tile, with the fewest
-// inner atoms, takes what does not divide by eight (its first j may be < 1).
-// Tile g from below has NG - g chunks of outer atoms and g / s + 1 ranges of
-// inner atoms.
-__device__ __forceinline__ long long a3_tasks(int n, int s) {
-  const long long ng = n < 3 ? 0 : (n - 2 + A3 - 1) / A3;
-  long long t = 0;
-  for (long long m = ng; m > 0; m -= s) t += m * (m + 1) / 2;
-  return t;
-}
-
 }  // namespace
 
 // Running task counts of the structures in launch order (largest first),
@@ -295,18 +281,9 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
     const int b = c.w.sorder[at];
     const int n = c.w.n_eff[b];
     // tile, chunk and inner range
-    const int ng = (n - 2 + A3 - 1) / A3;
-    int t = (int)(task - first[at]);
-    int ip = 0, m = ng;
-    while (t >= m * (m + 1) / 2) {
-      t -= m * (m + 1) / 2;
-      m -= s;
-      ++ip;
-    }
-    int u, ch;
-    tri_entry(t, u, ch);
-    const int j0 = n - 1 - A3 * (u + 1), kc = j0 + 1 + A3 * ch, jend = j0 + A3;
-    const int ib0 = ip * A3 * s, iend = min(ib0 + A3 * s, jend - 1);
+    const A3Task at3 = a3_task(task - first[at], n, s);
+    const int j0 = n - 1 - A3 * (at3.u + 1), kc = j0 + 1 + A3 * at3.ch, jend = j0 + A3;
+    const int ib0 = at3.ip * A3 * s, iend = min(ib0 + A3 * s, jend - 1);
     const size_t bN = (size_t)b * N;
     A3Pair a;
     a.T = c.w.ptf + bN * N;
@@ -795,3 +772,14 @@ void launch_atm32(const Ctx &c, cudaStream_t st) {
 }
 
 }  // namespace d4
+
+extern "C" int64_t d4_selftest_atm_task(int32_t n, int32_t s, int64_t task, int32_t *out) {
+  if (n < 3 || s < 1 || !out) return -1;
+  const long long total = d4::a3_tasks(n, s);
+  if (task < 0 || task >= total) return total;
+  const d4::A3Task t = d4::a3_task(task, n, s);
+  out[0] = t.ip;
+  out[1] = t.u;
+  out[2] = t.ch;
+  return total;
+}

@@ -495,7 +495,7 @@ __device__ __forceinline__ NearBlocks near_blocks(const Ctx &c, int b, int A, in
 }
 
 // (row, col), col <= row, of entry t of a packed lower triangle
-__device__ __forceinline__ void tri_entry(long long t, int &row, int &col) {
+__host__ __device__ __forceinline__ void tri_entry(long long t, int &row, int &col) {
   int r = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
   while ((long long)(r + 1) * (r + 2) / 2 <= t) ++r;
   while ((long long)r * (r + 1) / 2 > t) --r;
