@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(256, 3) eeq_big_residual_kernel(Ctx c, int it)
 // padding slots zeroed -- disjoint sets, so the CTAs never write the same
 // entry).
 constexpr int FIN_CTAS = 16;
-__global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint) {
+__global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint, bool last) {
   __shared__ double s_a[32], s_b[32];
   __shared__ double s_par;
   const int b = blockIdx.y;
@@ -1027,11 +1027,12 @@ __global__ void __launch_bounds__(1024) eeq_big_finish_kernel(Ctx c, int adjoint
   }
   if (tid == 0) {
     // final refinement residual: that of the first iteration below the
-    // tolerance (later iterations were skipped), else of the last one
+    // tolerance (later iterations were skipped), else (or with ``last``, where the
+    // entries of skipped ones repeat it) of the last one
     float fin = 0.f;
     for (int it = 0; it < EEQ_BIG_REFINE; ++it) {
       fin = __uint_as_float(c.w.eeq_res[b * EEQ_BIG_REFINE + it]);
-      if (fin < BIG_TOL) break;
+      if (fin < BIG_TOL && !last) break;
     }
     if (lead) c.w.eeq_final[2 * b + (adjoint ? 1 : 0)] = fin;
     double ta = s_a[0], tb = s_b[0];
@@ -1257,15 +1258,15 @@ void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint) {
     }
     launch_refine(c, st, it, adjoint);
   }
-  launch_eeq_big_finish(c, st, adjoint);
+  launch_eeq_big_finish(c, st, adjoint, false);
 }
 
 void launch_eeq_big_rhs(const Ctx &c, cudaStream_t st, bool adjoint) {
   eeq_big_rhs_kernel<<<dim3((c.N + 255) / 256, c.B), 256, 0, st>>>(c, adjoint ? 1 : 0);
 }
 
-void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint) {
-  eeq_big_finish_kernel<<<dim3(FIN_CTAS, c.B), 1024, 0, st>>>(c, adjoint ? 1 : 0);
+void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint, bool last) {
+  eeq_big_finish_kernel<<<dim3(FIN_CTAS, c.B), 1024, 0, st>>>(c, adjoint ? 1 : 0, last);
 }
 
 }  // namespace d4

@@ -38,7 +38,7 @@ namespace {
 // 251 / 186, 11 (4 x 400) 173 / 125 and 174 / 123, 14 (1 x 2000) 404 / 329 and
 // 392 / 302, 57 (16 x 512) 293 / 227 and 266 / 192.
 constexpr int CG_FEW = 256, CG_MANY = 512, CG_FEW_ROWS = 10;
-constexpr float CG_TOL = 1e-10f;     // max |b - A x|
+constexpr float CG_TOL = 1e-10f;     // max |b - A x| that converges
 constexpr float CG_GAIN = 1e-12f;    // of (r, r / diag) per FP32 solve
 constexpr int CG_OUTER = 16;         // refinements at most
 constexpr int CG_INNER = 500;        // iterations of one FP32 solve at most
@@ -104,6 +104,18 @@ __device__ __forceinline__ dfl cg_warp_sum(dfl a) {
   }
   return a;
 }
+
+// The factorisation's corrections overshoot CG_TOL: they leave 1e-11 (charges; what
+// the residuals of a double-float solution resolve) and 1e-13 (adjoint).  So
+// that these solves leave no more, one more correction follows where the first
+// residual below CG_TOL is above cg_goal, and a correction after the first solve
+// ends at cg_end, not at CG_TOL.  Residuals of charges / adjoint, ending at a
+// quarter of CG_TOL and now: 997 atoms 1.8e-11 / 2.5e-11 and 7.8e-12 / 8e-14, 16000
+// (d4_eeq_dcg.cu) 2.1e-11 / 2.4e-11 and 7.8e-12 / 1e-13, for 4 % of such calls' time.
+template <int NR>
+__device__ __forceinline__ float cg_goal() { return NR == 1 ? 3e-13f : 1.2e-11f; }
+template <int NR>
+__device__ __forceinline__ float cg_end() { return NR == 1 ? 1e-13f : 9e-12f; }
 
 __host__ __device__ inline int cg_pad(int m) { return (m + 3) & ~3; }
 // floats of the vectors of NR right-hand sides and of R rows of solution
@@ -177,7 +189,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
           rows[(size_t)i * ms + k] = k < m ? Hi[(size_t)(row0 + i) * N + k] : 0.f;
     for (int t = tid; t < NR * RS; t += NT) x[t] = make_float2(0.f, 0.f);
     __syncthreads();
-    bool alive = true;
+    bool alive = true, below = false;
     for (int outer = 0;; ++outer) {
       // the FP32 solve A d = r, from u = r / diag, p = s = 0
       float g[NR], mx[NR], beta[NR], alpha[NR];
@@ -205,14 +217,16 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
       }
       res = mx[0];
       if (NR == 2) res = fmaxf(res, mx[NR - 1]);
-      if (res < CG_TOL || outer == CG_OUTER) break;
+      if (res <= cg_goal<NR>() || below || outer == CG_OUTER) break;
+      below = res < CG_TOL;  // (then this correction is the last)
       float stop[NR];
       bool on[NR];
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
         stop[q] = CG_GAIN * g[q];
-        on[q] = mx[q] >= CG_TOL;
+        on[q] = mx[q] > cg_goal<NR>();
       }
+      const float end = outer == 0 ? 0.f : cg_end<NR>();
       for (int it = 0; it < CG_INNER; ++it) {
         // own rows of A u
         float *w = cg_exchange(c, b, par);
@@ -318,7 +332,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
         for (int q = 0; q < NR; ++q) {
           beta[q] = on[q] ? n[q] / g[q] : 0.f;
           g[q] = n[q];
-          on[q] = on[q] && n[q] > stop[q] && n[NR + q] > 0.25f * CG_TOL;
+          on[q] = on[q] && n[q] > stop[q] && n[NR + q] > end;
           more |= on[q];
         }
         if (!more) break;
@@ -447,7 +461,7 @@ bool eeq_cg_takes(const Ctx &c) {
 bool launch_eeq_cg(const Ctx &c, cudaStream_t st, bool adjoint) {
   cg_rhs_kernel<<<dim3((c.N + 255) / 256, c.B), 256, 0, st>>>(c, adjoint ? 1 : 0);
   if (!(adjoint ? launch_cg<1>(c, st) : launch_cg<2>(c, st))) return false;
-  launch_eeq_big_finish(c, st, adjoint);
+  launch_eeq_big_finish(c, st, adjoint, true);
   return true;
 }
 

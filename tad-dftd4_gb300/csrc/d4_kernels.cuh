@@ -42,7 +42,7 @@ int launch_fp64(const Ctx &c, cudaStream_t st);
 int launch_mixed(const Ctx &c, cudaStream_t st);
 void launch_eeq_big(const Ctx &c, cudaStream_t st, bool adjoint);
 void launch_eeq_big_rhs(const Ctx &c, cudaStream_t st, bool adjoint);
-void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint);
+void launch_eeq_big_finish(const Ctx &c, cudaStream_t st, bool adjoint, bool last);
 bool eeq_cg_takes(const Ctx &c);  // conjugate gradients instead (d4_eeq_cg.cu)
 bool launch_eeq_cg(const Ctx &c, cudaStream_t st, bool adjoint);
 constexpr int EEQ_HALF_TILE = 128;  // the tiles of a matrix stored in half (below)
