@@ -190,6 +190,7 @@ struct Workspace {
   // spatially sorted copies (precision form, zsort_fits(N)): perm[k] = input
   // index of sorted atom k, then inputs and outputs in sorted order
   int *zs_perm;       // [B*N]
+  int *zs_first;      // [B] place of the input's first atom in the sorted order
   int64_t *zs_num;    // [B*N]
   double *zs_pos, *zs_q, *zs_r4, *zs_w;           // [B*N*3], [B*N] each
   double *zs_e, *zs_g, *zs_oq, *zs_ocn, *zs_ocnq;  // [B*N], [B*N*3], [B*N] each
@@ -329,6 +330,7 @@ inline Workspace carve_workspace(void *base, int B, int N, int S, uint32_t flags
     }
     if (zsort_fits(N)) {
       w.zs_perm = (int *)take(sizeof(int) * BN);
+      w.zs_first = (int *)take(sizeof(int) * (size_t)B);
       w.zs_num = (int64_t *)take(8 * BN);
       w.zs_pos = (double *)take(24 * BN);
       w.zs_q = (double *)take(8 * BN);

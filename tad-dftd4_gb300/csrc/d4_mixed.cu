@@ -1005,8 +1005,19 @@ __global__ void __launch_bounds__(1024) zsort_kernel(Ctx c) {
         return make_float3((float)P[3 * t], (float)P[3 * t + 1], (float)P[3 * t + 2]);
       },
       [&](int t) { return c.numbers[bN + t] != 0; });
+  __shared__ int s_first;  // the input's first atom
+  if (threadIdx.x == 0) s_first = N;
+  __syncthreads();
+  for (int t = threadIdx.x; t < N; t += blockDim.x)
+    if (c.numbers[bN + t] != 0) {
+      atomicMin(&s_first, t);
+      break;
+    }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_first == N) c.w.zs_first[blockIdx.x] = 0;
   for (int t = threadIdx.x; t < N; t += blockDim.x) {
     const int a = (int)(s_key[t] & 0xFFFFFFFFu);
+    if (a == s_first) c.w.zs_first[blockIdx.x] = t;
     c.w.zs_perm[bN + t] = a;
     c.w.zs_num[bN + t] = c.numbers[bN + a];
     for (int d = 0; d < 3; ++d) c.w.zs_pos[3 * (bN + t) + d] = P[3 * a + d];

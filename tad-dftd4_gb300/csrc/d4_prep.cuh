@@ -87,10 +87,9 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b, int p
   }
   __syncthreads();
   const int n = s_neff;
-  // FP32 positions are taken relative to the first real atom; in spatial order,
-  // where that is a corner, to the middle one (16000 atoms: 3.2e-8 -> 2.5e-8 Eh
-  // from the FP64 energy, whatever the order of the input)
-  const int first = c.zsorted ? n / 2 : s_first;
+  // FP32 positions are taken relative to the first real atom of the input, whatever
+  // order the kernels run in (the energy error of FP32 depends on that atom)
+  const int first = c.zsorted ? c.w.zs_first[b] : s_first;
   const double *p0 = c.positions + ((size_t)b * N + (first < N ? first : 0)) * 3;
   for (int i = beg + threadIdx.x; i < end; i += blockDim.x) {
     const size_t a = (size_t)b * N + i;
