@@ -531,6 +531,11 @@ __device__ __forceinline__ float warp_maxf(float v) {
   return v;
 }
 
+// A power of two that brings a vector of largest entry m to [1, 2).
+__device__ __forceinline__ float scale_to_one(float m) {
+  return ldexpf(1.f, -max(-126, min(126, ilogbf(m))));
+}
+
 // Compensated FP32 accumulator (Knuth two-sum): value = hi + lo.
 struct Acc32 {
   float hi = 0.0f, lo = 0.0f;

@@ -24,6 +24,9 @@
 // 997 atoms 1099 / 184 -> 223 / 167 us; the rule below has other sizes.  Of an
 // iteration's 8200 cycles there, 2700 go to the barrier, 1450 to the product,
 // 1480 to reading the exchanged rows and 2500 to the updates and reductions.
+#include <float.h>
+#include <math_constants.h>
+
 #include "d4_common.cuh"
 #include "d4_group.cuh"
 #include "d4_kernels.cuh"
@@ -108,14 +111,24 @@ __device__ __forceinline__ dfl cg_warp_sum(dfl a) {
 // The factorisation's corrections overshoot CG_TOL: they leave 1e-11 (charges; what
 // the residuals of a double-float solution resolve) and 1e-13 (adjoint).  So
 // that these solves leave no more, one more correction follows where the first
-// residual below CG_TOL is above cg_goal, and a correction after the first solve
-// ends at cg_end, not at CG_TOL.  Residuals of charges / adjoint, ending at a
+// residual below CG_TOL is above ``goal``, and a correction after the first solve
+// ends at ``end``, not at CG_TOL.  Residuals of charges / adjoint, ending at a
 // quarter of CG_TOL and now: 997 atoms 1.8e-11 / 2.5e-11 and 7.8e-12 / 8e-14, 16000
 // (d4_eeq_dcg.cu) 2.1e-11 / 2.4e-11 and 7.8e-12 / 1e-13, for 4 % of such calls' time.
-template <int NR>
-__device__ __forceinline__ float cg_goal() { return NR == 1 ? 3e-13f : 1.2e-11f; }
-template <int NR>
-__device__ __forceinline__ float cg_end() { return NR == 1 ? 1e-13f : 9e-12f; }
+//
+// The adjoint's right-hand side is as large or small as the energies' weights make
+// it.  It is solved times the power of two ``sc`` that brings its largest entry to
+// ``top`` in [1, 2), so that no product of two residuals leaves FP32's range, and the
+// bars follow it: those above for entries up to 1, relative beyond, and never
+// above what the factorisation left of a small one (2e-7).
+struct CgBars {
+  float tol, goal, end;
+};
+__device__ __forceinline__ CgBars cg_charge_bars() { return {CG_TOL, 1.2e-11f, 9e-12f}; }
+__device__ __forceinline__ CgBars cg_adjoint_bars(float sc, float top) {
+  const float one = fmaxf(sc, top);
+  return {CG_TOL * one, fminf(3e-13f * one, 2e-7f * top), fminf(1e-13f * one, 5e-8f * top)};
+}
 
 __host__ __device__ inline int cg_pad(int m) { return (m + 3) & ~3; }
 // floats of the vectors of NR right-hand sides and of R rows of solution
@@ -188,6 +201,24 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
         for (int k = lane; k < ms; k += 32)
           rows[(size_t)i * ms + k] = k < m ? Hi[(size_t)(row0 + i) * N + k] : 0.f;
     for (int t = tid; t < NR * RS; t += NT) x[t] = make_float2(0.f, 0.f);
+    float sc = 1.f;
+    CgBars bars = cg_charge_bars();
+    if (NR == 1) {
+      float top[1] = {0.f};
+      bool finite = true;
+      for (int k = tid; k < ms; k += NT) {
+        top[0] = fmaxf(top[0], fabsf(r[k]));
+        finite = finite && fabsf(r[k]) <= FLT_MAX;
+      }
+      if (__syncthreads_or(!finite)) {  // every entry of the solution depends on all of them
+        for (int t = tid; t < R; t += NT) X[row0 + t] = make_float2(CUDART_NAN_F, 0.f);
+        continue;
+      }
+      cg_reduce<NT, 1, 0>(top, sm, turn);
+      sc = scale_to_one(top[0]);
+      bars = cg_adjoint_bars(sc, top[0] * sc);
+      for (int k = tid; k < ms; k += NT) r[k] *= sc;
+    }
     __syncthreads();
     bool alive = true, below = false;
     for (int outer = 0;; ++outer) {
@@ -217,16 +248,16 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
       }
       res = mx[0];
       if (NR == 2) res = fmaxf(res, mx[NR - 1]);
-      if (res <= cg_goal<NR>() || below || outer == CG_OUTER) break;
-      below = res < CG_TOL;  // (then this correction is the last)
+      if (res <= bars.goal || below || outer == CG_OUTER) break;
+      below = res < bars.tol;  // (then this correction is the last)
       float stop[NR];
       bool on[NR];
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
         stop[q] = CG_GAIN * g[q];
-        on[q] = mx[q] > cg_goal<NR>();
+        on[q] = mx[q] > bars.goal;
       }
-      const float end = outer == 0 ? 0.f : cg_end<NR>();
+      const float end = outer == 0 ? 0.f : bars.end;
       for (int it = 0; it < CG_INNER; ++it) {
         // own rows of A u
         float *w = cg_exchange(c, b, par);
@@ -372,7 +403,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
         for (int q = 0; q < NR; ++q) {
           const dfl t = cg_warp_sum(a[q]);
           const float2 bv = B[q * N + row];
-          const dfl v = df_add(dfl{bv.x, bv.y}, df_neg(t));
+          const dfl v = df_add(dfl{bv.x * sc, bv.y * sc}, df_neg(t));
           if (lane == 0) __stcg(&w[q * N + row], v.hi);
         }
       }
@@ -385,8 +416,10 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
       __syncthreads();
     }
     if (!alive) return;
+    if (NR == 1)  // (the exchanged solution was the scaled one)
+      for (int t = tid; t < R; t += NT) X[row0 + t] = make_float2(x[t].x / sc, x[t].y / sc);
     if (rank == 0 && tid < EEQ_BIG_REFINE)
-      c.w.eeq_res[b * EEQ_BIG_REFINE + tid] = __float_as_uint(res);
+      c.w.eeq_res[b * EEQ_BIG_REFINE + tid] = __float_as_uint(res / sc);
   }
 }
 

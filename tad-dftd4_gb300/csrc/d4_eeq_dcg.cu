@@ -62,6 +62,7 @@ struct DcArea {
   float2 *dot;                // [ranks][2] partial (A u, u), (r, u)
   float4 *norm;               // [ranks][2] partial (r, u), max |r|, (b, b / diag)
   unsigned *counter;          // [EEQ_BIG_REFINE] barriers of each solve
+  float *top;                 // [1] largest entry of the adjoint's right-hand side
 };
 constexpr size_t DC_RANKS = 512;
 constexpr int DC_COPIES = 8;  // of the sums that every CTA adds to at once (same L2 lines)
@@ -97,21 +98,31 @@ __device__ __forceinline__ DcArea dc_area(const Ctx &c, int b) {
   a.dot = reinterpret_cast<float2 *>(a.tr + EEQ_BIG_REFINE * 2 * DC_K);
   a.norm = reinterpret_cast<float4 *>(a.dot + 2 * DC_RANKS);
   a.counter = reinterpret_cast<unsigned *>(a.norm + 2 * DC_RANKS);
+  a.top = reinterpret_cast<float *>(a.counter + EEQ_BIG_REFINE);
   return a;
 }
 
-// The residual that a solve aims at, and where a correction after the first solve
-// ends: see cg_goal (d4_eeq_cg.cu).
-__device__ __forceinline__ float dc_goal(int nr) { return nr == 1 ? 3e-13f : 1.2e-11f; }
-__device__ __forceinline__ float dc_end(int nr) { return nr == 1 ? 1e-13f : 9e-12f; }
+// The bars of a solve, as in d4_eeq_cg.cu (CgBars): the residual that converges, the
+// one it aims at, and where a correction after the first solve ends.  top: the
+// largest entry of the adjoint's right-hand side.
+struct DcBars {
+  float tol, goal, end;
+};
+__device__ __forceinline__ DcBars dc_bars(const Ctx &c, int b, int nr) {
+  if (nr == 2) return {DC_TOL, 1.2e-11f, 9e-12f};
+  const float top = *dc_area(c, b).top, one = fmaxf(1.f, top);
+  return {DC_TOL * one, fminf(3e-13f * one, 2e-7f * top), fminf(1e-13f * one, 5e-8f * top)};
+}
 
 // Whether iteration ``it`` has nothing to do: the goal is reached, or the last one
-// was the one that may follow a residual below DC_TOL.  Its entry of eeq_res
+// was the one that may follow a residual below ``tol``.  Its entry of eeq_res
 // then repeats the last one's (dcg_rest_kernel).
 __device__ __forceinline__ bool dc_skip(const Ctx &c, int b, int it, int nr) {
+  if (it == 0) return false;
   const unsigned *res = c.w.eeq_res + b * EEQ_BIG_REFINE + it;
-  return (it > 0 && __uint_as_float(res[-1]) <= dc_goal(nr)) ||
-         (it > 1 && __uint_as_float(res[-2]) < DC_TOL);
+  const DcBars bars = dc_bars(c, b, nr);
+  return __uint_as_float(res[-1]) <= bars.goal ||
+         (it > 1 && __uint_as_float(res[-2]) < bars.tol);
 }
 
 __device__ __forceinline__ float4 dc_stream4(const float *p) {
@@ -488,16 +499,29 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
       *reinterpret_cast<float4 *>(&sm.G[r * DC_LDG + k]) =
           *reinterpret_cast<const float4 *>(&ar.G[(size_t)(k0 + r) * DC_K + k]);
     }
+    float top = 0.f;
     for (int k = warp; k < DC_K; k += DC_WARPS) {  // Z^T b
       const int l = DC_BLOCK * k + lane;
 #pragma unroll
       for (int p = 0; p < NR; ++p) {
         const float *Vp = V + (size_t)p * N;
-        const float s = warp_sumf((l < m ? __ldcg(Vp + l) : 0.f) +
-                                  (l + 32 < m ? __ldcg(Vp + l + 32) : 0.f));
+        const float v0 = l < m ? __ldcg(Vp + l) : 0.f;
+        const float v1 = l + 32 < m ? __ldcg(Vp + l + 32) : 0.f;
+        top = fmaxf(top, fmaxf(fabsf(v0), fabsf(v1)));
+        const float s = warp_sumf(v0 + v1);
         if (lane == 0) sm.tb[p][k] = s;
       }
     }
+    // The solve runs on b times a power of two: no product of two residuals leaves
+    // FP32's range then, whatever the energies' weights.
+    top = warp_maxf(top);
+    if (lane == 0) sm.red[warp][0] = top;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < DC_WARPS; ++w) top = fmaxf(top, sm.red[w][0]);
+    const float sc = scale_to_one(top);
+    if (NR == 1 && it == 0 && rank == 0 && tid == 0) *ar.top = top;
+    for (int k = tid; k < NR * DC_K; k += DC_THREADS) sm.tb[k / DC_K][k % DC_K] *= sc;
     // G t of the thread's row and right-hand side: four lanes share a row
     auto project = [&](const float (&tv)[2][DC_K]) {
       float s[NR];
@@ -575,7 +599,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
       }
     };
     __syncthreads();
-    const float bv = own ? __ldcg(V + oV) : 0.f;
+    const float bv = own ? __ldcg(V + oV) * sc : 0.f;
     const float dinv = own ? 1.0f / __ldg(Hi + (size_t)row * N + row) : 0.f;
     float r = bv - project(sm.tb), p = 0.f, s = 0.f, x = 0.f;
     if (!own) r = 0.f;
@@ -616,7 +640,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
     float g[NR], mx[NR], bb[NR], stop[NR], alpha[NR], beta[NR];
     bool on[NR], more = false;
     norms(g, mx, bb);
-    const float end = it == 0 ? 0.f : dc_end(NR);
+    const float end = it == 0 ? 0.f : dc_bars(c, b, NR).end * sc;
 #pragma unroll
     for (int e = 0; e < NR; ++e) {
       stop[e] = fmaxf(DC_GAIN * g[e], DC_FLOOR * bb[e]);
@@ -730,7 +754,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
       if (lane == 0) sm.y[e][warp & 3] = a;
     }
     __syncthreads();
-    if (own) V[oV] = x + sm.y[q][row / DC_BLOCK - kb];
+    if (own) V[oV] = (x + sm.y[q][row / DC_BLOCK - kb]) / sc;
   }
 }
 
