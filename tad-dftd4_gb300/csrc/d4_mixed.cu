@@ -1747,7 +1747,9 @@ static void launch_atm(const Ctx &c, cudaStream_t st) {
       atm_order_kernel<<<c.B, 1024, osm, st>>>(c);
     }
   }
-  const bool tiled = c.weights == nullptr;
+  // (the register-tiled kernels multiply records of pairs by the zeros of others: up
+  // to alp = 48, (R0/r)^(alp/3) of any two pairs stays finite until R0/r = 15)
+  const bool tiled = c.weights == nullptr && c.par.alp >= 0.0 && c.par.alp <= 48.0;
   if (tiled)
     launch_atm32(c, st);
   else if (big)
