@@ -382,6 +382,7 @@ struct Ctx {
   int atm64;      // the register-tiled FP64 ATM runs (set by launch_fp64)
   int pair64;     // the pair stages of d4_pair64.cu run (set by launch_fp64)
   double cut2_sq, cut3_sq;  // largest r^2 with sqrt(r^2) <= cut_disp2, cut_disp3 (likewise)
+  double cutcn_sq, cutq_sq;  // the same of cut_cn, cut_cn_eeq
   Workspace w;
   d4_outputs_t out;
 };

@@ -54,13 +54,13 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
     const double r = r2 > 0.0 ? r2 * rsqrt_pos(r2) : r2;
     const double x = r * rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     const double cf = 0.5 * erfc(c.par.kcn * (x - 1.0));
-    if (r <= c.par.cut_cn) {
+    if (r2 <= c.cutcn_sq) {
       const double t = fabs(c.tab.en[zi] - c.tab.en[zj]) + c.par.k5;
       const double v = cf * (c.par.k4 * exp(-(t * t) * ik6));  // en_factor with 1 / k6
       atomicAdd(&c.w.cn[ab + i], v);
       atomicAdd(&c.w.cn[ab + j], v);
     }
-    if (r <= c.par.cut_cn_eeq) {
+    if (r2 <= c.cutq_sq) {
       atomicAdd(&c.w.cnq[ab + i], cf);  // capped with the EEQ right-hand sides (eeq64_cap)
       atomicAdd(&c.w.cnq[ab + j], cf);
     }
@@ -953,6 +953,11 @@ static double cutoff_sq(double cut) {
   return x;
 }
 
+static void set_cn_cutoffs(Ctx &c) {
+  c.cutcn_sq = cutoff_sq(c.par.cut_cn);
+  c.cutq_sq = cutoff_sq(c.par.cut_cn_eeq);
+}
+
 int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   Ctx c = c_in;
   const int B = c.B, N = c.N;
@@ -963,6 +968,7 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
             c.par.alp <= 100.0;
   c.cut2_sq = cutoff_sq(c.par.cut_disp2);
   c.cut3_sq = cutoff_sq(c.par.cut_disp3);
+  set_cn_cutoffs(c);
   // With the rational damping on top, the pair stages of d4_pair64.cu, which
   // write the energies and parameter gradients to the outputs directly.
   c.pair64 = c.atm64 && c.par.damping == D4_DAMP_RATIONAL;
@@ -1082,8 +1088,10 @@ __global__ void __launch_bounds__(256) props_kernel(Ctx c, double *c6out, double
   }
 }
 
-int launch_properties(const Ctx &c, double *c6out, double *alpha_out, double *q_out,
+int launch_properties(const Ctx &c_in, double *c6out, double *alpha_out, double *q_out,
                       cudaStream_t st) {
+  Ctx c = c_in;
+  set_cn_cutoffs(c);
   const int B = c.B, N = c.N;
   const dim3 atoms((N + 7) / 8, B);
   launch_prep(c, st);

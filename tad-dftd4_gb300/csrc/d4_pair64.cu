@@ -373,12 +373,12 @@ __global__ void __launch_bounds__(PT) pair64_cn_bwd_kernel(Ctx c, int rounds) {
     const double ir0 = rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     double dEdr = 0.0;
     double gcn = 0.0;
-    if (r <= p.cut_cn) {  // (en_factor with 1 / k6)
+    if (r2 <= c.cutcn_sq) {  // (en_factor with 1 / k6)
       const double t = fabs(c.tab.en[zi] - c.tab.en[zj]) + p.k5;
       gcn = (c.w.dEdcn[ab + i] + c.w.dEdcn[ab + j]) * (p.k4 * exp(-(t * t) * ik6));
     }
     if (eeq) {
-      if (r <= p.cut_cn_eeq) gcn += c.w.dEdcnq[ab + i] + c.w.dEdcnq[ab + j];
+      if (r2 <= c.cutq_sq) gcn += c.w.dEdcnq[ab + i] + c.w.dEdcnq[ab + j];
       const double ra = c.tab.eeq_rad[zi], rb = c.tab.eeq_rad[zj];
       const double g = rsqrt_pos(ra * ra + rb * rb), gr = g * r;
       const double dA = (2.0 * INV_SQRT_PI * exp(-gr * gr) * gr - erf(gr)) * (ir * ir);
