@@ -406,6 +406,12 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Terms of the FP64 coordination numbers (D4, EEQ) of the pairs i < j at [j][i], in
+// the room of the pair records, which are written later.
+__device__ __forceinline__ double2 *cn64_terms(const Ctx &c, int b) {
+  return reinterpret_cast<double2 *>(c.w.pr4) + (size_t)b * c.N * c.N;
+}
+
 __device__ __forceinline__ void set_status(int *status, int code) {
   atomicCAS(status, 0, code);
 }

@@ -5,9 +5,9 @@
 // quantities live in dense per-structure N x N blocks, only the leading
 // n_eff x n_eff part of which is touched.  Every "atom-owned" kernel maps one
 // warp to one atom i and loops its lanes over partners j, so per-atom sums
-// need no atomics; the coordination numbers go over unordered pairs and add
-// both ends' sums by reductions at L2.  The general ATM kernel maps a CTA to a tile of pairs (j, k)
-// and loops over the third atom i < j.
+// need no atomics; the coordination numbers' terms go over unordered pairs and are
+// added up per atom afterwards.  The general ATM kernel maps a CTA to a tile of pairs
+// (j, k) and loops over the third atom i < j.
 #include <float.h>
 #include <math.h>
 
@@ -27,10 +27,12 @@ __global__ void __launch_bounds__(256) prep_kernel(Ctx c, int parts) {
 
 // ---------------------------------------------------------------- CN
 
-// D4 and EEQ coordination numbers, once per pair i < j: pairs with a counting
-// function left (kcn (r / r0 - 1) <= 9: 1/2 erfc(9) < 1e-36), found in FP32, are
-// queued per warp and evaluated 32 at a time, added to both atoms (cleared by
-// the prep kernel).  Bound by the FP64 pipe, ~100 instructions per pair.  Measured
+// Terms of the D4 and EEQ coordination numbers, once per pair i < j: pairs with a
+// counting function left (kcn (r / r0 - 1) <= 9: 1/2 erfc(9) < 1e-36), found in
+// FP32, are queued per warp and evaluated 32 at a time; zeros elsewhere.  The
+// terms leave as numbers per pair (cn64_terms) that cn64_sum adds up in a fixed
+// order, so that a call repeats itself to the last bit (reductions at L2 to both
+// atoms do not).  Bound by the FP64 pipe, ~100 instructions per pair.  Measured
 // against a warp per atom over ordered pairs: 360 structures of 30 atoms 99 ->
 // 29 us, 64 of 8..200 atoms 71 -> 41.
 constexpr int CN_T = 128;
@@ -46,6 +48,7 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
   const int *Z = c.w.z + ab;
   const float kcn32 = (float)c.par.kcn;
   const double ik6 = 1.0 / c.par.k6;
+  double2 *terms = cn64_terms(c, b);
   auto evaluate = [&](int i, int j) {
     const int zi = Z[i], zj = Z[j];
     const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
@@ -54,16 +57,13 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
     const double r = r2 > 0.0 ? r2 * rsqrt_pos(r2) : r2;
     const double x = r * rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     const double cf = 0.5 * erfc(c.par.kcn * (x - 1.0));
+    double2 v = make_double2(0.0, 0.0);
     if (r2 <= c.cutcn_sq) {
       const double t = fabs(c.tab.en[zi] - c.tab.en[zj]) + c.par.k5;
-      const double v = cf * (c.par.k4 * exp(-(t * t) * ik6));  // en_factor with 1 / k6
-      atomicAdd(&c.w.cn[ab + i], v);
-      atomicAdd(&c.w.cn[ab + j], v);
+      v.x = cf * (c.par.k4 * exp(-(t * t) * ik6));  // en_factor with 1 / k6
     }
-    if (r2 <= c.cutq_sq) {
-      atomicAdd(&c.w.cnq[ab + i], cf);  // capped with the EEQ right-hand sides (eeq64_cap)
-      atomicAdd(&c.w.cnq[ab + j], cf);
-    }
+    if (r2 <= c.cutq_sq) v.y = cf;  // capped with the EEQ right-hand sides (eeq64_cap)
+    terms[(size_t)j * N + i] = v;
   };
   int queued = 0;
   for (int k = 0; k < rounds; ++k, t += 32) {
@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
         const float r32 = sqrtf(ex * ex + ey * ey + ez * ez);
         near = kcn32 * (r32 / (c.w.aux32[ab + i].x + c.w.aux32[ab + j].x) - 1.0f) <= 9.0f;
       }
+      if (!near) terms[(size_t)j * N + i] = make_double2(0.0, 0.0);
     }
     const unsigned m = __ballot_sync(0xffffffffu, near);
     if (near) {
@@ -107,8 +108,6 @@ static void launch_cn(const Ctx &c, cudaStream_t st) {
   const long long per = (long long)CN_T * rounds;
   if (pairs > 0)
     cn_kernel<<<dim3((unsigned)((pairs + per - 1) / per), c.B), CN_T, 0, st>>>(c, rounds);
-  if (c.out.d_cn)
-    cudaMemcpyAsync(c.out.d_cn, c.w.cn, 8 * (size_t)c.B * c.N, cudaMemcpyDeviceToDevice, st);
 }
 
 // ---------------------------------------------------------------- weights
@@ -992,6 +991,7 @@ int launch_fp64(const Ctx &c_in, cudaStream_t st) {
   } else {
     const size_t total = (size_t)B * N;
     charges_in_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(c);
+    launch_cn64_sum(c, st);
     if (c.out.d_cn_eeq) launch_eeq64_cap(c, st, false);
   }
   stage_end(ST_EEQ, st);

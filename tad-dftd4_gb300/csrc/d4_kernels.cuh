@@ -60,7 +60,8 @@ void launch_atm_mirror(const Ctx &c, cudaStream_t st, bool rows, float s9);
 void launch_pair64(const Ctx &c, cudaStream_t st);  // FP64 pair stages (d4_pair64.cu)
 void launch_pair64_bwd(const Ctx &c, cudaStream_t st);
 void launch_pair64_forces(const Ctx &c, cudaStream_t st);
-void launch_eeq64(const Ctx &c, cudaStream_t st);  // FP64 EEQ charges (d4_eeq64.cu)
+void launch_eeq64(const Ctx &c, cudaStream_t st);  // FP64 EEQ charges (d4_eeq64.cu), and
+void launch_cn64_sum(const Ctx &c, cudaStream_t st);  // coordination numbers without them
 void launch_eeq64_cap(const Ctx &c, cudaStream_t st, bool eeq);
 void launch_eeq64_adjoint(const Ctx &c, cudaStream_t st);
 void launch_atm_exact(const Ctx &c, cudaStream_t st);  // exact C9, FP64 (d4_exact.cu)

@@ -101,7 +101,7 @@ static __device__ __forceinline__ void prep_structure(const Ctx &c, int b, int p
     c.w.slot[a] = s < c.S ? s : c.S - 1;
     c.w.e3[a] = 0.0;
     if (c.pair64) c.w.rowmax[a] = 0.0;
-    if ((c.flags & D4_FLAG_MIXED) == 0) c.w.cn[a] = c.w.cnq[a] = c.w.dcnq[a] = 0.0;
+    if ((c.flags & D4_FLAG_MIXED) == 0) c.w.dcnq[a] = 0.0;
     if (ok) {
       const double *p = c.positions + 3 * a;
       const double dx = p[0] - p0[0], dy = p[1] - p0[1], dz = p[2] - p0[2];
