@@ -326,6 +326,13 @@ int d4_selftest_wait(int32_t *d_result, uint64_t limit_ns, void *stream);
 int d4_selftest_launch_error(void *stream);
 
 /*
+ * The library's own elementary functions at ``n`` arguments: ``which`` 0 the FP64
+ * reciprocal, 1 the FP64 inverse square root, 2 the FP32 exponential (of a
+ * double-float; |x| <= 80).  Device pointers.
+ */
+int d4_selftest_math(int32_t which, const double *d_x, double *d_y, int32_t n, void *stream);
+
+/*
  * The numbering of the tasks of the precision form's ATM (host code, nothing
  * runs): task ``task`` of a structure of ``n`` atoms whose tasks cover 8 ``s``
  * inner atoms each goes to ``out`` as (range of inner atoms, tile of middle

@@ -104,7 +104,7 @@ __device__ __forceinline__ void eeq64_pivot(double a, int c, PanelSmem &sm, int 
     d = 1.0;
   }
   if (lane == c) a = d;
-  const double inv = rsqrt_pos(d);
+  const double inv = rsqrt_pos<false>(d);  // (finite: a matrix with an infinite entry has NaN)
   sm.L[c * EB + lane] = lane >= c ? a * inv : 0.0;
   if (lane == c) sm.inv[c] = inv;
 }

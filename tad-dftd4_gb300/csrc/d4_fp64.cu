@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
     const double dx = P[3 * i] - P[3 * j], dy = P[3 * i + 1] - P[3 * j + 1],
                  dz = P[3 * i + 2] - P[3 * j + 2];
     const double r2 = dx * dx + dy * dy + dz * dz;
-    const double r = r2 > 0.0 ? r2 * rsqrt_pos(r2) : r2;
+    const double r = r2 > 1e-300 ? r2 * rsqrt_pos(r2) : 0.0;
     const double x = r * rcp_pos(c.tab.cov_d3[zi] + c.tab.cov_d3[zj]);
     const double cf = 0.5 * erfc(c.par.kcn * (x - 1.0));
     double2 v = make_double2(0.0, 0.0);

@@ -10,6 +10,7 @@
 #include "d4_atm.cuh"
 #include "d4_common.cuh"
 #include "d4_chol.cuh"
+#include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
 #include "d4_prep.cuh"
 
@@ -165,29 +166,6 @@ __global__ void __launch_bounds__(256) prep_tables_kernel(Ctx c, int parts) {
   else
     prep_structure(c, ((int)blockIdx.x - TABLE_CTAS) / parts,
                    ((int)blockIdx.x - TABLE_CTAS) % parts, parts);
-}
-
-// exp(x), |x| <= 80, rounded once: reduction by ln 2 = 355/512 - 2.1e-4 (Cody and
-// Waite, Software Manual for the Elementary Functions, 1980) and the series, its
-// first terms in double-float (within 1e-10 before the rounding).  In place of an FP64 exp, whose 30 instructions for every reference of
-// every atom were most of the weights' time.
-__device__ __forceinline__ float exp_once(dfl x) {
-  const float n = rintf(x.hi * 1.44269504f);
-  const float ch = 2.1219444e-4f;
-  constexpr float cl = (float)(2.1219444005469058277e-4 - (double)2.1219444e-4f);
-  const float p = n * ch;
-  const dfl t = df_two_sum(fmaf(n, -0.693359375f, x.hi), p);  // (exact: few bits)
-  const dfl r = df_fast(t.hi, t.lo + (fmaf(n, ch, -p) + fmaf(n, cl, x.lo)));
-  const dfl r2 = df_mul(r, r);
-  const dfl r3 = df_mul(df_mul(r2, r), dfl{1.f / 6.f, (float)(1.0 / 6.0 - (double)(1.f / 6.f))});
-  const float q = fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, fmaf(r.hi, 1.f / 362880.f,
-                       1.f / 40320.f), 1.f / 5040.f), 1.f / 720.f), 1.f / 120.f), 1.f / 24.f);
-  const dfl tail = df_two_sum(r3.hi, r2.hi * r2.hi * q);
-  const dfl h = df_two_sum(0.5f * r2.hi, tail.hi);
-  const dfl u = df_two_sum(r.hi, h.hi);
-  const dfl v = df_two_sum(1.f, u.hi);
-  const float lo = v.lo + (u.lo + (r.lo + (h.lo + fmaf(0.5f, r2.lo, tail.lo + r3.lo))));
-  return (v.hi + lo) * __int_as_float(((int)n + 127) << 23);
 }
 
 // transposed index of (structure b, atom i, slot s, frequency w)

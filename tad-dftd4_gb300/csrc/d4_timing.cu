@@ -2,6 +2,7 @@
 #include <vector>
 
 #include "d4_common.cuh"
+#include "d4_fpmath.cuh"
 #include "d4_kernels.cuh"
 #include "d4_tc.cuh"
 
@@ -72,6 +73,14 @@ __global__ void selftest_wait_kernel(int32_t *result, unsigned long long limit_n
   *result = tc::mbar_wait(mbar, 0u, limit_ns) ? D4_OK : D4_ERR_DEVICE_TIMEOUT;
 }
 
+// The functions of d4_fpmath.cuh, one value per thread.
+__global__ void selftest_math_kernel(int which, const double *x, double *y, int n) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  y[t] = which == 0 ? rcp_pos(x[t]) : which == 1 ? rsqrt_pos(x[t])
+                                                 : (double)exp_once(df_from(x[t]));
+}
+
 // Two kernels that do nothing, for d4_selftest_launch_error.
 __global__ void selftest_refused_kernel() {}
 __global__ void selftest_next_kernel() {}
@@ -79,6 +88,13 @@ __global__ void selftest_next_kernel() {}
 }  // namespace d4
 
 extern "C" {
+
+int d4_selftest_math(int32_t which, const double *d_x, double *d_y, int32_t n, void *stream) {
+  if (which < 0 || which > 2 || !d_x || !d_y || n <= 0) return D4_ERR_ARGUMENT;
+  d4::selftest_math_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      which, d_x, d_y, n);
+  return d4::take_error() == cudaSuccess ? D4_OK : D4_ERR_CUDA;
+}
 
 int d4_selftest_launch_error(void *stream) {
   d4::selftest_refused_kernel<<<1, 1, 1 << 20, static_cast<cudaStream_t>(stream)>>>();
