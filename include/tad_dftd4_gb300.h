@@ -60,7 +60,8 @@ typedef enum d4_status {
   D4_ERR_EEQ_SINGULAR = 5,     /* EEQ matrix not positive definite */
   D4_ERR_NONFINITE = 6,        /* non-finite position or charge */
   D4_ERR_TOO_MANY_ELEMENTS = 7, /* D4S: more distinct elements than slots */
-  D4_ERR_DEVICE_TIMEOUT = 8     /* an on-device wait for the tensor cores ran out */
+  D4_ERR_DEVICE_TIMEOUT = 8     /* an on-device wait (tensor cores or the
+                                  barrier of an EEQ solve) ran out */
 } d4_status;
 
 /* Model variants (tad_dftd4.model): D4Model and D4SModel. */
@@ -316,6 +317,16 @@ int d4_probe_fma(int32_t fp64, int32_t n_blocks, int32_t iters, double *d_sink,
  * reference.
  */
 int d4_selftest_wait(int32_t *d_result, uint64_t limit_ns, void *stream);
+
+/*
+ * Self-test of the barrier between the CTAs of an EEQ solve: a cooperative launch of
+ * ``ctas`` CTAs (1 to 64) passes one barrier, then one that expects ``extra``
+ * arrivals more than there are, limited to ``limit_ns`` nanoseconds of the global
+ * timer.  ``d_result`` (device, 2 + ``ctas`` ints, cleared by the call): the status
+ * word, the arrivals, and per CTA the barriers passed.
+ */
+int d4_selftest_barrier(int32_t *d_result, int32_t ctas, int32_t extra, uint64_t limit_ns,
+                        void *stream);
 
 /*
  * Self-test of the error report: a launch that the runtime refuses (more

@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
   const int N = c.N;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x % G;
+  if (group_gave_up(c.w.status)) return;
   if (tid == 0) sm.dead = 0;
   int turn = 0;
   for (int b = blockIdx.x / G; b < c.B; b += groups) {

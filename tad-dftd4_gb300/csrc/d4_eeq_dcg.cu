@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
   const int N = c.N, ranks = gridDim.x, rank = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int i = tid >> 2, q = tid & 3;  // row of the slice, quarter of a G row / right-hand side
+  if (group_gave_up(c.w.status)) return;
   if (tid == 0) sm.dead = 0;
   for (int b = 0; b < c.B; ++b) {
     const int m = c.w.n_real[b];

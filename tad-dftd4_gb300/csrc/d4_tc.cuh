@@ -28,7 +28,8 @@
 namespace d4 {
 namespace tc {
 
-// Bound of every wait on the tensor cores (nanoseconds of %globaltimer).
+// Bound of every wait on the tensor cores and of the barriers of the EEQ solves
+// (nanoseconds of %globaltimer).
 constexpr unsigned long long WAIT_LIMIT_NS = 1000000000ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {

@@ -3,6 +3,7 @@
 
 #include "d4_common.cuh"
 #include "d4_fpmath.cuh"
+#include "d4_group.cuh"
 #include "d4_kernels.cuh"
 #include "d4_tc.cuh"
 
@@ -73,6 +74,21 @@ __global__ void selftest_wait_kernel(int32_t *result, unsigned long long limit_n
   *result = tc::mbar_wait(mbar, 0u, limit_ns) ? D4_OK : D4_ERR_DEVICE_TIMEOUT;
 }
 
+// Two barriers of the launch's CTAs; the second waits for ``extra`` arrivals that
+// nobody makes.
+__global__ void __launch_bounds__(128) selftest_barrier_kernel(int32_t *result, int extra,
+                                                               unsigned long long limit_ns) {
+  __shared__ int dead;
+  if (threadIdx.x == 0) dead = 0;
+  unsigned *counter = reinterpret_cast<unsigned *>(result + 1);
+  int passed = 0;
+  if (group_barrier(counter, gridDim.x, dead, result, limit_ns)) {
+    passed = 1;
+    if (group_barrier(counter, 2 * gridDim.x + extra, dead, result, limit_ns)) passed = 2;
+  }
+  if (threadIdx.x == 0) result[2 + blockIdx.x] = passed;
+}
+
 // The functions of d4_fpmath.cuh, one value per thread.
 __global__ void selftest_math_kernel(int which, const double *x, double *y, int n) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,6 +104,19 @@ __global__ void selftest_next_kernel() {}
 }  // namespace d4
 
 extern "C" {
+
+int d4_selftest_barrier(int32_t *d_result, int32_t ctas, int32_t extra, uint64_t limit_ns,
+                        void *stream) {
+  if (!d_result || ctas < 1 || ctas > 64 || extra < 0 || extra > 1 || limit_ns > 1000000000ull)
+    return D4_ERR_ARGUMENT;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaMemsetAsync(d_result, 0, sizeof(int32_t) * (2 + (size_t)ctas), st);
+  unsigned long long limit = limit_ns;
+  void *args[] = {&d_result, &extra, &limit};
+  cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&d4::selftest_barrier_kernel),
+                              dim3((unsigned)ctas), dim3(128), args, 0, st);
+  return d4::take_error() == cudaSuccess ? D4_OK : D4_ERR_CUDA;
+}
 
 int d4_selftest_math(int32_t which, const double *d_x, double *d_y, int32_t n, void *stream) {
   if (which < 0 || which > 2 || !d_x || !d_y || n <= 0) return D4_ERR_ARGUMENT;
