@@ -90,7 +90,9 @@ typedef enum d4_model_kind { D4_MODEL_D4 = 0, D4_MODEL_D4S = 1 } d4_model_kind;
 #define D4_FLAG_TEST_TIMEOUT 0x80000000u
 /* Test hook of the paths for what usually does not happen at small sizes: the
    FP64 EEQ solves keep their vectors in global memory (as for structures padded
-   beyond 14080 atoms).  Results are those of a call without it. */
+   beyond 14080 atoms), and the precision form's conjugate gradients take
+   their cooperative launches as refused and factorise instead.  Results are those of
+   a call without it, to the solvers' bar. */
 #define D4_FLAG_TEST_FALLBACK 0x40000000u
 
 /* Entries per structure of d_param_grad: dE_b / d(s6, s8, s10, a1, a2, s9,
@@ -307,6 +309,18 @@ const char *d4_stage_name(int32_t stage);
  */
 int d4_probe_fma(int32_t fp64, int32_t n_blocks, int32_t iters, double *d_sink,
                  float *ms_out, void *stream);
+
+/* EEQ solvers of the precision form. */
+typedef enum d4_eeq_solver_kind {
+  D4_EEQ_ONE_CTA = 0,       /* factorisation in a CTA's shared memory (n_pad <= 296) */
+  D4_EEQ_CG = 1,            /* conjugate gradients */
+  D4_EEQ_DEFLATED_CG = 2,   /* the same, deflated, over half of the matrix */
+  D4_EEQ_FACTORISATION = 3  /* by several CTAs */
+} d4_eeq_solver_kind;
+
+/* Which of them takes a batch of ``n_struct`` structures padded to ``n_pad`` atoms on
+   the current device (a d4_eeq_solver_kind; -1: bad sizes). */
+int32_t d4_eeq_solver(int32_t n_struct, int32_t n_pad);
 
 /*
  * Self-test of the bounded waits every tensor-core kernel uses: one CTA

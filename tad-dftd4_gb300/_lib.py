@@ -173,6 +173,7 @@ SIGNATURES = {
     ),
     "d4_selftest_wait": (c_int, [c_void_p, ctypes.c_uint64, c_void_p]),
     "d4_selftest_launch_error": (c_int, [c_void_p]),
+    "d4_eeq_solver": (c_int32, [c_int32, c_int32]),
     "d4_selftest_barrier": (c_int, [c_void_p, c_int32, c_int32, ctypes.c_uint64, c_void_p]),
     "d4_selftest_math": (c_int, [c_int32, c_void_p, c_void_p, c_int32, c_void_p]),
     "d4_selftest_atm_task": (ctypes.c_int64, [c_int32, c_int32, ctypes.c_int64,

@@ -455,6 +455,7 @@ CgPlan cg_plan(const Ctx &c, int nr) {
 
 template <int NR>
 bool launch_cg(const Ctx &c, cudaStream_t st) {
+  if (c.flags & D4_FLAG_TEST_FALLBACK) return false;
   CgPlan p = cg_plan(c, NR);
   const bool rows = p.full <= CG_SMEM;
   const size_t smem = rows ? p.full : p.vec;

@@ -970,6 +970,7 @@ int dc_sms() {
 
 template <int NR, bool VEC>
 bool launch_solve(const Ctx &c, cudaStream_t st, int it) {
+  if (c.flags & D4_FLAG_TEST_FALLBACK) return false;
   Ctx cc = c;
   void *args[] = {&cc, &it};
   const void *f = reinterpret_cast<const void *>(&eeq_dcg_kernel<NR, VEC>);

@@ -1675,11 +1675,13 @@ __global__ void __launch_bounds__(EEQ_THREADS, 2) eeq_adjoint_mixed_kernel(Ctx c
 
 // ---------------------------------------------------------------- launch
 
-// persistent grid of the EEQ build: 4 blocks per SM, at most one per tile
+// The conjugate gradients that take the batch; false: a launch was refused (their
+// cooperative launches need all their CTAs resident at once).
 static bool launch_eeq_iterative(const Ctx &c, cudaStream_t st, bool adjoint) {
   return eeq_dcg_takes(c) ? launch_eeq_dcg(c, st, adjoint) : launch_eeq_cg(c, st, adjoint);
 }
 
+// persistent grid of the EEQ build: 4 blocks per SM, at most one per tile
 static unsigned build_blocks(const Ctx &c) {
   static int sms[64] = {0};
   int dev = 0;
@@ -1875,3 +1877,14 @@ int launch_mixed(const Ctx &c_in, cudaStream_t st) {
 }
 
 }  // namespace d4
+
+extern "C" int32_t d4_eeq_solver(int32_t n_struct, int32_t n_pad) {
+  if (n_struct <= 0 || n_pad <= 0) return -1;
+  if (d4::eeq_small_fits(n_pad)) return D4_EEQ_ONE_CTA;
+  d4::Ctx c{};
+  c.B = n_struct;
+  c.N = n_pad;
+  c.zsorted = d4::zsort_fits(n_pad);
+  return d4::eeq_dcg_takes(c) ? D4_EEQ_DEFLATED_CG
+         : d4::eeq_cg_takes(c) ? D4_EEQ_CG : D4_EEQ_FACTORISATION;
+}
