@@ -45,6 +45,12 @@ __device__ __forceinline__ int sl_first(int lane) {
   return 12 * ((lane >> 2) & 1) + 6 * ((lane >> 1) & 1) + 3 * (lane & 1);
 }
 
+// Slots that a structure can have, for everything in shared memory: a caller's S may
+// be larger.
+__host__ __device__ inline int sl_slots(const Ctx &c) {
+  return c.S < MAX_ELEM_ID ? c.S : MAX_ELEM_ID;
+}
+
 __host__ __device__ inline int sl_entries(int S) { return SL_TILE + 8 * S; }
 // shared memory: the list, slots of its groups and of the tile's atoms, run
 // starts (in whole float4), then ``warp_floats`` per warp
@@ -132,11 +138,12 @@ __global__ void __launch_bounds__(256, 2) pair_fwd_d4s32_kernel(Ctx c) {
   const int i = blockIdx.x * (blockDim.x >> 5) + warp;
   const int N = c.N, n = c.w.n_eff[b], nslot = c.w.n_slots[b];
   extern __shared__ float4 s_dyn[];
-  const SlotList list = slot_list_smem(s_dyn, c.S);
+  const int SS = sl_slots(c);
+  const SlotList list = slot_list_smem(s_dyn, SS);
   // atom i's A at q and at q = 0 by slot, the adjoint sums by group and slot
-  float *wa = reinterpret_cast<float *>(reinterpret_cast<char *>(s_dyn) + sl_list_bytes(c.S)) +
-              (size_t)warp * fwd_floats(c.S);
-  float *wa0 = wa + c.S * SL_WA, *sums = wa0 + c.S * SL_WA;
+  float *wa = reinterpret_cast<float *>(reinterpret_cast<char *>(s_dyn) + sl_list_bytes(SS)) +
+              (size_t)warp * fwd_floats(SS);
+  float *wa0 = wa + SS * SL_WA, *sums = wa0 + SS * SL_WA;
   const size_t ai = (size_t)b * N + (i < N ? i : 0);
   const int zi = i < n ? c.w.z[ai] : 0;
   const bool live = zi != 0;
@@ -187,7 +194,7 @@ __global__ void __launch_bounds__(256, 2) pair_fwd_d4s32_kernel(Ctx c) {
       }
     }
     if (GRAD)
-      for (int k = lane; k < 4 * c.S * SL_W; k += 32) sums[k] = 0.f;
+      for (int k = lane; k < 4 * SS * SL_W; k += 32) sums[k] = 0.f;
   }
   const float *Ab = c.w.A32 + a32_at(c, b, 0, slot_i, 0);
   const float *A0b = c.w.A032 + a32_at(c, b, 0, slot_i, 0);
@@ -293,7 +300,7 @@ __global__ void __launch_bounds__(256, 2) pair_fwd_d4s32_kernel(Ctx c) {
         for (int w = 0; w < SL_W; ++w) v[w] = w < NFREQ ? K * Ajr[w < NFREQ ? w : 0] : 0.f;
         group_sums(v);
         if (e < entries) {
-          float *o = sums + ((lane >> 3) * c.S + sg) * SL_W + sl_first(lane);
+          float *o = sums + ((lane >> 3) * SS + sg) * SL_W + sl_first(lane);
           o[0] += v[0];
           o[1] += v[1];
           o[2] += v[2];
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(256, 2) pair_fwd_d4s32_kernel(Ctx c) {
       for (int s = 0; s < c.S; ++s) {
         float g = 0.f;
         if (s < nslot)
-          for (int k = 0; k < 4; ++k) g += sums[(k * c.S + s) * SL_W + lane];
+          for (int k = 0; k < 4; ++k) g += sums[(k * SS + s) * SL_W + lane];
         c.w.G32[(ai * c.S + s) * NFREQ + lane] = g;
       }
   }
@@ -346,9 +353,10 @@ __global__ void __launch_bounds__(256) pair_bwd_d4s32_kernel(Ctx c) {
   const int x = blockIdx.x * (blockDim.x >> 5) + warp;
   const int N = c.N, n = c.w.n_eff[b], nslot = c.w.n_slots[b];
   extern __shared__ float4 s_dyn[];
-  const SlotList list = slot_list_smem(s_dyn, c.S);
-  float *sums = reinterpret_cast<float *>(reinterpret_cast<char *>(s_dyn) + sl_list_bytes(c.S)) +
-                (size_t)warp * bwd_floats(c.S);  // by group and slot
+  const int SS = sl_slots(c);
+  const SlotList list = slot_list_smem(s_dyn, SS);
+  float *sums = reinterpret_cast<float *>(reinterpret_cast<char *>(s_dyn) + sl_list_bytes(SS)) +
+                (size_t)warp * bwd_floats(SS);  // by group and slot
   const size_t ax = (size_t)b * N + (x < N ? x : 0);
   const bool live = x < n && c.w.z[ax] != 0;
   if (!live && x < N && lane == 0) {
@@ -366,7 +374,7 @@ __global__ void __launch_bounds__(256) pair_bwd_d4s32_kernel(Ctx c) {
   Acc32 gx, gy, gz;
   Acc32 dcn_acc, dq_acc;
   if (live)
-    for (int k = lane; k < 4 * c.S * SL_W; k += 32) sums[k] = 0.f;
+    for (int k = lane; k < 4 * SS * SL_W; k += 32) sums[k] = 0.f;
   for (int t0 = 0; t0 < n; t0 += SL_TILE) {
     const int entries = make_slot_list(c, b, t0, min(SL_TILE, n - t0), nslot, list);
     if (!live) continue;
@@ -395,7 +403,7 @@ __global__ void __launch_bounds__(256) pair_bwd_d4s32_kernel(Ctx c) {
       }
       group_sums(v);
       if (e < entries) {
-        float *o = sums + ((lane >> 3) * c.S + sg) * SL_W + sl_first(lane);
+        float *o = sums + ((lane >> 3) * SS + sg) * SL_W + sl_first(lane);
         o[0] += v[0];
         o[1] += v[1];
         o[2] += v[2];
@@ -409,7 +417,7 @@ __global__ void __launch_bounds__(256) pair_bwd_d4s32_kernel(Ctx c) {
     for (int s = 0; s < nslot; ++s) {
       const size_t o = (ax * c.S + s) * NFREQ + lane;
       float g0w = 0.f;  // dE/dA'0_x
-      for (int k = 0; k < 4; ++k) g0w += sums[(k * c.S + s) * SL_W + lane];
+      for (int k = 0; k < 4; ++k) g0w += sums[(k * SS + s) * SL_W + lane];
       const float gw = c.w.G32[o];
       const float *d = c.w.dA32 + 3 * o;
       dcn_acc.add(gw * d[0]);
@@ -434,7 +442,7 @@ namespace {
 // Eight warps per CTA share a list; fewer where many slots would not fit.
 template <typename K>
 void launch_slots(const Ctx &c, cudaStream_t st, K kernel, size_t warp_floats) {
-  const size_t fixed = sl_list_bytes(c.S), most = 200 * 1024;
+  const size_t fixed = sl_list_bytes(sl_slots(c)), most = 200 * 1024;
   int warps = 8;
   while (warps > 1 && fixed + 4 * warps * warp_floats > most) --warps;
   const size_t smem = fixed + 4 * warps * warp_floats;
@@ -445,7 +453,7 @@ void launch_slots(const Ctx &c, cudaStream_t st, K kernel, size_t warp_floats) {
 }  // namespace
 
 void launch_pair_fwd_d4s32(const Ctx &c, cudaStream_t st) {
-  const size_t f = fwd_floats(c.S);
+  const size_t f = fwd_floats(sl_slots(c));
   if (c.flags & D4_FLAG_PARAM_GRAD)
     launch_slots(c, st, pair_fwd_d4s32_kernel<true, true>, f);
   else if (c.flags & D4_FLAG_GRADIENT)
@@ -455,7 +463,7 @@ void launch_pair_fwd_d4s32(const Ctx &c, cudaStream_t st) {
 }
 
 void launch_pair_bwd_d4s32(const Ctx &c, cudaStream_t st) {
-  launch_slots(c, st, pair_bwd_d4s32_kernel, bwd_floats(c.S));
+  launch_slots(c, st, pair_bwd_d4s32_kernel, bwd_floats(sl_slots(c)));
 }
 
 }  // namespace d4
