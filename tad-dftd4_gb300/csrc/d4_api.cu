@@ -2,6 +2,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -24,6 +25,20 @@ cudaError_t take_error() {
   const cudaError_t e = g_kept;
   g_kept = cudaSuccess;
   return e;
+}
+
+int sm_count() {
+  static std::atomic<int> sms[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int> &n = sms[dev & 63];
+  int v = n.load(std::memory_order_relaxed);
+  if (v == 0) {
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1)
+      v = 1;
+    n.store(v, std::memory_order_relaxed);
+  }
+  return v;
 }
 
 // (device, kernel) -> dynamic shared-memory limit already set

@@ -743,15 +743,7 @@ void launch_atm_sparse32(const Ctx &c, cudaStream_t st) {
 
 void launch_atm32(const Ctx &c, cudaStream_t st) {
   if (c.N < 3) return;
-  static int sms[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &nsm = sms[dev & 63];
-  if (nsm == 0) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    nsm = v > 0 ? v : 1;
-  }
+  const int nsm = sm_count();
   const bool grad = (c.flags & D4_FLAG_GRADIENT) != 0;
   const bool pgrad = (c.flags & D4_FLAG_PARAM_GRAD) != 0;
   // inner atoms per task: 128 (finding, loading and flushing a task takes as

@@ -373,10 +373,10 @@ static void launch_tiled64(const Ctx &c, cudaStream_t st) {
   // (57 atoms 30 -> 20; 360 x 30, which has more, loses by it: 325)
   int il = 32;
   auto count = [&]() { return tasks * c.B * ((N + il - 1) / il); };
-  while (il > 8 && count() < 128LL * 152) il >>= 1;
-  if (count() < 32LL * 152) il = 4;
+  while (il > 8 && count() < 128LL * sm_count()) il >>= 1;
+  if (count() < 32LL * sm_count()) il = 4;
   // one warp per CTA spreads few tasks over the SMs; four where there are many
-  const int warps = count() < 64LL * 152 ? 1 : 4;
+  const int warps = count() < 64LL * sm_count() ? 1 : 4;
   const dim3 grid((unsigned)((tasks + warps - 1) / warps), (unsigned)((N + il - 1) / il),
                   (unsigned)c.B);
   atm_tiled64_kernel<J, GRAD, PGRAD><<<grid, 32 * warps, 0, st>>>(c, il);

@@ -541,17 +541,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) pair_fwd_tc_kernel(Ctx c) {
 // Few tiles (large structures): the partners of a tile are split over
 // several CTAs so that every SM gets about four CTAs.
 static int pair_tc_splits(const Ctx &c) {
-  static int sms[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &nsm = sms[dev & 63];
-  if (nsm == 0) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    nsm = v > 0 ? v : 1;
-  }
   const long long tiles = (long long)((c.N + TC_M - 1) / TC_M) * c.B;
-  const long long want = 4LL * nsm;
+  const long long want = 4LL * sm_count();
   if (tiles >= want) return 1;
   const long long chunks = (c.N + TC_NJ - 1) / TC_NJ;
   const long long s = (want + tiles - 1) / tiles;
@@ -883,11 +874,8 @@ void launch_pair_atm_bwd_tc(const Ctx &c, cudaStream_t st) {
   ensure_smem(pair_atm_bwd_tc_kernel, smem);
   // few tiles (large structures): a tile's partners are split over several
   // CTAs so that every SM gets about four
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)((c.N + TC_M - 1) / TC_M) * c.B;
-  const long long want = 4LL * (nsm > 0 ? nsm : 1);
+  const long long want = 4LL * sm_count();
   const long long chunks = (c.N + BW_K - 1) / BW_K;
   int nsplit = 1;
   if (tiles < want) {

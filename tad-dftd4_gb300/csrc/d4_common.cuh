@@ -205,6 +205,9 @@ struct Workspace {
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Multiprocessors of the current device (152 on GB300), for launch rules.
+int sm_count();
+
 // The runtime's last error is what tells a call that one of its launches was
 // refused, and some runtime calls that succeed reset it (cudaFuncSetAttribute on a
 // kernel does): keep_error() before such a call sets it aside, and take_error()

@@ -725,7 +725,7 @@ void launch_eeq64(const Ctx &c, cudaStream_t st) {
   const int B = c.B, N = c.N;
   const long long pairs = (long long)N * (N - 1) / 2;
   // eight pairs per thread fill the queues of a batch, one spreads few pairs
-  const int rounds = B * pairs <= 4LL * 152 * 128 ? 1 : 8;
+  const int rounds = B * pairs <= 4LL * sm_count() * 128 ? 1 : 8;
   const int ctas = (int)((pairs + 128 * rounds - 1) / (128 * rounds));
   eeq64_build_kernel<<<dim3(ctas + (N + CS_ATOMS - 1) / CS_ATOMS, B), 128, 0, st>>>(c, rounds,
                                                                                    ctas);
@@ -745,14 +745,14 @@ void launch_eeq64(const Ctx &c, cudaStream_t st) {
     const int T = (left + 31) / 32;
     // 32 rows per CTA while that leaves SMs idle, 128 once the CTAs' own
     // diagonal factors would crowd the pipe
-    if ((long long)B * ((rows + 31) / 32) <= 4 * 152)
+    if ((long long)B * ((rows + 31) / 32) <= 4 * sm_count())
       eeq64_panel_kernel<1><<<dim3((rows + 31) / 32, B), 256, 0, st>>>(c, k0);
     else
       eeq64_panel_kernel<4><<<dim3((rows + 127) / 128, B), 256, 0, st>>>(c, k0);
     if (T == 0) break;
     const long long tiles = (long long)T * (T + 1) / 2;
     // four columns per warp while that leaves sub-partitions idle
-    if (B * tiles * 8 <= 4 * 152 * 4)
+    if (B * tiles * 8 <= 4 * sm_count() * 4)
       eeq64_update_kernel<4><<<dim3((unsigned)(tiles * 8 + 3) / 4, B), 128, 0, st>>>(c, k0);
     else
       eeq64_update_kernel<8><<<dim3((unsigned)(tiles * 4 + 3) / 4, B), 128, 0, st>>>(c, k0);

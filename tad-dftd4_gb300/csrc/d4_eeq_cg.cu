@@ -432,15 +432,7 @@ struct CgPlan {
 };
 
 CgPlan cg_plan(const Ctx &c, int nr) {
-  static int sms[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &nsm = sms[dev & 63];
-  if (nsm == 0) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    nsm = v > 0 ? v : 1;
-  }
+  const int nsm = sm_count();
   // all SMs shared by the batch, at least eight rows each
   CgPlan p;
   const int most = (c.N + 7) / 8;

@@ -956,15 +956,7 @@ __global__ void __launch_bounds__(256) dcg_rest_kernel(Ctx c, int it, int nr) {
 namespace {
 
 int dc_sms() {
-  static int sms[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &n = sms[dev & 63];
-  if (n == 0) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    n = v > 0 ? v : 1;
-  }
+  const int n = sm_count();
   return n < (int)DC_RANKS ? n : (int)DC_RANKS;
 }
 

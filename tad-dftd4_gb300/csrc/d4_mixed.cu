@@ -1683,18 +1683,9 @@ static bool launch_eeq_iterative(const Ctx &c, cudaStream_t st, bool adjoint) {
 
 // persistent grid of the EEQ build: 4 blocks per SM, at most one per tile
 static unsigned build_blocks(const Ctx &c) {
-  static int sms[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &n = sms[dev & 63];
-  if (n == 0) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    n = v > 0 ? v : 1;
-  }
   const size_t T = (size_t)(c.N + 31) / 32;
   const size_t tiles = (size_t)c.B * T * (T + 1) / 2;
-  const size_t want = (size_t)4 * n;
+  const size_t want = (size_t)4 * sm_count();
   return (unsigned)(tiles < want ? (tiles > 0 ? tiles : 1) : want);
 }
 

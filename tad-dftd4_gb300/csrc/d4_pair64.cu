@@ -466,7 +466,7 @@ void launch_pair64(const Ctx &c, cudaStream_t st) {
   const long long nb = (N + TB - 1) / TB, tiles = nb * (nb + 1) / 2;
   // a pair per thread while that leaves sub-partitions idle, else four
   const long long pairs = (long long)B * N * (N - 1) / 2;
-  const int per = pairs <= 4LL * 152 * PT ? PT : 4 * PT;
+  const int per = pairs <= 4LL * sm_count() * PT ? PT : 4 * PT;
   const int most = N <= TB ? N * (N - 1) / 2 : TB * TB;
   const int parts = most > per ? (most + per - 1) / per : 1;
   const dim3 grid((unsigned)(tiles * parts), B);
@@ -490,7 +490,7 @@ void launch_pair64_bwd(const Ctx &c, cudaStream_t st) {
 void launch_pair64_forces(const Ctx &c, cudaStream_t st) {
   const int B = c.B, N = c.N;
   const long long pairs = (long long)N * (N - 1) / 2;
-  const int rounds = B * pairs <= 4LL * 152 * PT ? 1 : 8;
+  const int rounds = B * pairs <= 4LL * sm_count() * PT ? 1 : 8;
   const long long per = (long long)PT * rounds;
   if (pairs > 0)
     pair64_cn_bwd_kernel<<<dim3((unsigned)((pairs + per - 1) / per), B), PT, 0, st>>>(c, rounds);

@@ -14,7 +14,8 @@ constexpr int PREP_ZERO_MAX_N = 256;
 // structures (every CTA scans the atomic numbers; 16000 atoms 273 -> 28 us).
 inline int prep_parts(const Ctx &c) {
   const int most = (c.N + 255) / 256;
-  return c.N <= 512 ? 1 : (c.B >= 304 ? 1 : (most < 304 / c.B ? most : 304 / c.B));
+  const int ctas = 2 * sm_count();
+  return c.N <= 512 ? 1 : (c.B >= ctas ? 1 : (most < ctas / c.B ? most : ctas / c.B));
 }
 
 // n_eff, input validation, D4S element slots, zeroing of accumulators of
