@@ -40,7 +40,7 @@ __host__ __device__ inline size_t eeq_small_bytes(int N) {
               (size_t)N * (N + 1) / 2);
 }
 // Structures padded to N are solved by one CTA each when everything fits in
-// shared memory (N <= 290), else by the multi-CTA path.
+// shared memory (N <= 296), else by one of the multi-CTA solvers.
 __host__ __device__ inline bool eeq_small_fits(int N) { return eeq_small_bytes(N) <= 220 * 1024; }
 constexpr int EEQ_BIG_REFINE = 4;  // refinement iterations of the multi-CTA path at most
 constexpr int EEQ_SB = 512;        // diagonal blocks inverted for the multi-CTA solves
@@ -55,10 +55,11 @@ constexpr size_t EEQ_OPND_BLOCK = (size_t)8 * 2 * 8192;
 
 // ---------------------------------------------------------------- ATM sizes
 
-// The precision-form ATM accumulates a structure's pair adjoints in shared
-// memory (upper triangle + atoms, FP32) when the padded size allows it
-// (N <= 234); larger structures accumulate in global memory and get
-// neighbour lists for the neighbour-triple variant.
+// The precision form's general ATM (energy weights, unusual exponents) accumulates
+// a structure's pair adjoints in shared memory (upper triangle + atoms, FP32) when
+// the padded size allows it (N <= 234), in global memory beyond.  Structures
+// beyond get neighbour lists, and run over neighbour triples where that pays, with
+// either kind of ATM.
 __host__ __device__ inline size_t atm_smem_bytes(int N) {
   return (size_t)4 * ((size_t)N * (N - 1) + N);
 }

@@ -1,5 +1,5 @@
 // Multi-CTA EEQ solve of the precision form, for structures too large for
-// one CTA's shared memory (N > 290): blocked right-looking FP32 Cholesky of
+// one CTA's shared memory (N > 296): blocked right-looking FP32 Cholesky of
 // the dense matrix in panels of 128 columns, blocked triangular solves and
 // double-float refinement residuals, every stage spread over all SMs.
 //

@@ -1,5 +1,5 @@
 // EEQ solves of the precision form for structures beyond the one-CTA solver
-// (N > 290) and few or small enough: conjugate gradients instead of a
+// (N > 296) and few or small enough: conjugate gradients instead of a
 // factorisation (eeq_cg_takes).
 //
 // The Coulomb matrix is positive definite and well conditioned (its smallest
@@ -9,7 +9,7 @@
 // pays ~75 us per 128 columns in dependent steps.  The solve is the same
 // refinement as before with CG in the factor's place: the residual b - A x in
 // double-float (hi + lo matrix) is corrected by an FP32 solve, until it is
-// below 1e-10.
+// where the factorisation left it (CgBars).
 //
 // One cooperative launch per solve.  A group of G CTAs shares a structure;
 // each holds its rows of the matrix in shared memory when they fit and keeps
@@ -21,7 +21,7 @@
 // Bound by the barrier and the L2 round trips of the exchange.
 //
 // Measured, charges / adjoint, against the factorisation (d4_eeq_big.cu):
-// 997 atoms 1099 / 184 -> 223 / 167 us; the rule below has other sizes.  Of an
+// 997 atoms 1113 / 178 -> 226 / 188 us; the rule below has other sizes.  Of an
 // iteration's 8200 cycles there, 2700 go to the barrier, 1450 to the product,
 // 1480 to reading the exchanged rows and 2500 to the updates and reductions.
 #include <float.h>
@@ -475,9 +475,9 @@ bool launch_cg(const Ctx &c, cudaStream_t st) {
 // Whether conjugate gradients solve the batch: when every CTA holds its matrix
 // rows in shared memory, or when all SMs share few structures whose matrices
 // stay in L2.  Charges + adjoint against the factorisation, us: 1 x 300 atoms
-// 241 / 600, 1 x 2000 694 / 2184, 1 x 4000 1710 / 3621, 16 x 512 458 / 937;
-// but 1 x 6001 7429 / 5621 (matrix from HBM) and 160 x 320 2875 / 1779 (a CTA
-// per structure, matrix from L2).
+// 253 / 597, 1 x 997 413 / 1291, 1 x 2000 731 / 2170, 1 x 4000 1822 / 3616, 16 x
+// 512 470 / 931; but 1 x 6001 8032 / 5645 (matrix from HBM) and 160 x 320 3032 /
+// 1803 (a CTA per structure, matrix from L2).
 bool eeq_cg_takes(const Ctx &c) {
   if (eeq_small_fits(c.N)) return false;
   const CgPlan p = cg_plan(c, 2);

@@ -989,11 +989,11 @@ void launch_residual(const Ctx &c, cudaStream_t st, int it) {
 
 // Whether deflated conjugate gradients solve the batch: one or two structures
 // in spatial order whose matrices outgrow L2.  Charges + adjoint in us, against
-// plain conjugate gradients (d4_eeq_cg.cu) 1 x 4500 atoms 2007 / 1906, 1 x 5000
-// 2063 / 3799; against the factorisation 1 x 6001 2697 / 5559, 1 x 16000 10830 /
-// 21870, 2 x 4000 3291 / 3910, 2 x 6001 5255 / 6709, but 4 x 5000 7276 / 6425
-// (structures run one after the other here; all but 1 x 16000's 10.8 ms now with
-// the residuals over the whole matrix).
+// plain conjugate gradients (d4_eeq_cg.cu) 1 x 4000 atoms 2129 / 1822, 1 x 4500
+// 2249 / 2019 and 1 x 5000 2378 / 4419; against the factorisation 1 x 6001 3042 /
+// 5645, 1 x 16000 12087 / 22010, 2 x 4000 3768 / 3983, 2 x 6001 5696 / 6729, but 3 x
+// 5000 6462 / 5845 and 4 x 5000 8473 / 6456 (structures run one after the other
+// here).
 bool eeq_dcg_takes(const Ctx &c) {
   if (!c.zsorted || c.B > 2 || c.N > DC_K * DC_BLOCK) return false;
   if ((size_t)4 * c.B * c.N * c.N <= (size_t)84 << 20) return false;

@@ -45,8 +45,8 @@ __device__ __forceinline__ double rsqrt_pos(double d) {
 
 // exp(x), |x| <= 80, rounded once: reduction by ln 2 = 355/512 - 2.1e-4 (Cody and
 // Waite, Software Manual for the Elementary Functions, 1980) and the series, its
-// first terms in double-float: within 0.502 ulp of exp (0.501 measured), as the rounding of an FP64 exp
-// is within 0.5 (tests/test_gpu_fpmath.py).  In place of that, whose 30 FP64
+// first terms in double-float: within 0.502 ulp of exp (0.501 measured), where an
+// FP64 exp rounded to FP32 is within 0.5.  In place of that, whose 30 FP64
 // instructions for every reference of every atom were most of the weights' time.
 __device__ __forceinline__ float exp_once(dfl x) {
   const float n = rintf(x.hi * 1.44269504f);

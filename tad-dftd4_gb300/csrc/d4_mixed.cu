@@ -1,8 +1,9 @@
 // Precision form of the D4 path: FP32 coordination numbers, reference
-// weights, pair and triple arithmetic with compensated accumulation, FP32
-// Cholesky of the EEQ matrix recovered by FP64 iterative refinement; FP64 for
-// the EEQ matrix and residuals and the final per-atom / per-structure
-// reductions.
+// weights, pair and triple arithmetic with compensated accumulation; EEQ matrix
+// and residuals in double-float, solved in FP32 (a Cholesky factor in one CTA up
+// to 296 atoms, beyond it conjugate gradients or a factorisation by several
+// CTAs: d4_eeq_cg.cu, d4_eeq_dcg.cu, d4_eeq_big.cu) and refined; FP64 for the
+// final per-atom / per-structure reductions.
 //
 // Shared stages (prep, finish) are the FP64 ones.
 #include <float.h>
@@ -457,8 +458,9 @@ __global__ void __launch_bounds__(256) cn_mixed_kernel(Ctx c) {
 
 // ---------------------------------------------------------------- launch order
 
-// Structures by decreasing size (n_eff), ties by index: the per-structure
-// kernels (EEQ solves, shared-memory ATM) take structure sorder[blockIdx],
+// Structures by decreasing size (n_eff), ties by index: the kernels that map CTAs
+// to structures (EEQ solves, tensor-core pair kernels, ATM tasks) take them in
+// this order,
 // so that the largest structures start first and the small ones fill the
 // last wave (longest-processing-time-first).  One CTA, bitonic sort of
 // (size, index) keys in shared memory; batches above SORDER_MAX keep index
