@@ -366,89 +366,57 @@ __device__ void eeq64_charges(const Ctx &c, int b, const double *L, const InvAt 
 
 namespace {
 
-constexpr int CS_ATOMS = 8;  // atoms of a CTA of 128 threads
+constexpr int CS_ATOMS = 16;  // atoms of a group of four warps
 
-// Coordination numbers (D4; EEQ, not capped yet) of atoms 8 block .. 8 block + 7 from
-// the pairs' terms (cn_kernel), always in the same order: terms of the later atoms by
-// columns (a lane per atom and one of four rows at a time), those of the earlier
-// atoms by rows (two atoms per warp).
-__device__ __forceinline__ void cn64_sum(const Ctx &c, int b, int block) {
-  __shared__ double2 s_col[4][CS_ATOMS], s_row[CS_ATOMS];
+// Coordination numbers (D4; EEQ, not capped yet) from the pairs' terms (cn_kernel),
+// always in the same order: 16 atoms from ``first`` on per group of four warps (of
+// GROUPS in the CTA), two lanes per atom and warp, every eighth partner each, then
+// the sums of lanes and warps.  (A lane per partner and sums across all lanes take
+// four times the FP64 instructions for small structures.)
+template <int GROUPS>
+__device__ __forceinline__ void cn64_sum(const Ctx &c, int b, int first) {
+  __shared__ double2 s_part[GROUPS][4][CS_ATOMS];
   const int N = c.N, n = c.w.n_eff[b];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int a0 = CS_ATOMS * block, a = a0 + (lane & 7);
+  const int group = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int a = first + CS_ATOMS * group + (lane & 15);
   const double2 *M = cn64_terms(c, b);
-  double2 col = make_double2(0.0, 0.0);
+  double2 s = make_double2(0.0, 0.0);
 #pragma unroll 4
-  for (int j = a0 + 1 + 4 * warp + (lane >> 3); j < n; j += 16)
-    if (j > a) {
-      const double2 v = M[(size_t)j * N + a];
-      col.x += v.x;
-      col.y += v.y;
+  for (int j = 2 * warp + (lane >> 4); j < n; j += 8)
+    if (a < n && j != a) {
+      const double2 v = M[(size_t)max(a, j) * N + min(a, j)];
+      s.x += v.x;
+      s.y += v.y;
     }
-#pragma unroll
-  for (int h = 8; h <= 16; h <<= 1) {
-    col.x += __shfl_xor_sync(FULL, col.x, h);
-    col.y += __shfl_xor_sync(FULL, col.y, h);
-  }
-  if (lane < CS_ATOMS) s_col[warp][lane] = col;
-  double v[4] = {0.0, 0.0, 0.0, 0.0};  // of two atoms: (D4, EEQ) each
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int r = a0 + 2 * warp + q;
-    if (r < n)
-#pragma unroll 4
-      for (int i = lane; i < r; i += 32) {
-        const double2 t = M[(size_t)r * N + i];
-        v[2 * q] += t.x;
-        v[2 * q + 1] += t.y;
-      }
-  }
-  // two halving exchanges leave value lane / 8 to a lane, three more add it up
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const int m = 2 >> s, h = 16 >> s;
-    const bool up = (lane & h) != 0;
-#pragma unroll
-    for (int q = 0; q < m; ++q) {
-      const double keep = up ? v[q + m] : v[q], send = up ? v[q] : v[q + m];
-      v[q] = keep + __shfl_xor_sync(FULL, send, h);
-    }
-  }
-#pragma unroll
-  for (int h = 4; h >= 1; h >>= 1) v[0] += __shfl_xor_sync(FULL, v[0], h);
-  if ((lane & 7) == 0) {
-    double2 &o = s_row[2 * warp + (lane >> 4)];
-    ((lane >> 3) & 1 ? o.y : o.x) = v[0];
-  }
+  s.x += __shfl_xor_sync(FULL, s.x, 16);
+  s.y += __shfl_xor_sync(FULL, s.y, 16);
+  if (lane < CS_ATOMS) s_part[group][warp][lane] = s;
   __syncthreads();
-  const int t = threadIdx.x;
-  if (t < CS_ATOMS && a0 + t < N) {
-    const size_t at = (size_t)b * N + a0 + t;
-    double x = s_row[t].x, y = s_row[t].y;
+  if (warp == 0 && lane < CS_ATOMS && a < N) {
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      x += s_col[w][t].x;
-      y += s_col[w][t].y;
+    for (int w = 1; w < 4; ++w) {
+      s.x += s_part[group][w][lane].x;
+      s.y += s_part[group][w][lane].y;
     }
-    c.w.cn[at] = x;
-    c.w.cnq[at] = y;
-    if (c.out.d_cn) c.out.d_cn[at] = x;
+    const size_t at = (size_t)b * N + a;
+    c.w.cn[at] = s.x;
+    c.w.cnq[at] = s.y;
+    if (c.out.d_cn) c.out.d_cn[at] = s.x;
   }
 }
 
 }  // namespace
 
 __global__ void __launch_bounds__(128) cn64_sum_kernel(Ctx c) {
-  cn64_sum(c, blockIdx.y, blockIdx.x);
+  cn64_sum<1>(c, blockIdx.y, CS_ATOMS * blockIdx.x);
 }
 
 void launch_cn64_sum(const Ctx &c, cudaStream_t st) {
   cn64_sum_kernel<<<dim3((c.N + CS_ATOMS - 1) / CS_ATOMS, c.B), 128, 0, st>>>(c);
 }
 
-// Off-diagonal Coulomb matrix of the real atoms (packed lower rows); CTAs beyond
-// ``ctas`` add up the coordination numbers meanwhile.  A thread
+// Off-diagonal Coulomb matrix of the real atoms (packed lower rows); CTAs from
+// ``ctas`` on add up the coordination numbers.  A thread
 // per pair of the flattened triangle, so that small structures fill their
 // warps; pairs with g r < 6.6 (beyond, erf = 1 to the last bit) are queued per
 // warp and evaluated 32 at a time, so that erf runs with full warps.
@@ -456,7 +424,7 @@ __global__ void __launch_bounds__(128) eeq64_build_kernel(Ctx c, int rounds, int
   __shared__ int s_i[4][64], s_j[4][64];
   const int b = blockIdx.y;
   if ((int)blockIdx.x >= ctas) {
-    cn64_sum(c, b, (int)blockIdx.x - ctas);
+    cn64_sum<1>(c, b, CS_ATOMS * ((int)blockIdx.x - ctas));
     return;
   }
   const int N = c.N, n = c.w.n_eff[b];
@@ -569,7 +537,10 @@ __global__ void __launch_bounds__(256) eeq64_small_kernel(Ctx c) {
   const int tri_m = m * (m + 1) / 2;
   double *G = eeq64_factor(c, b);
   for (int t = threadIdx.x; t < tri_m; t += blockDim.x) L[t] = G[t];  // (diagonal: below)
-  __syncthreads();
+  for (int a = 0; a < N; a += 2 * CS_ATOMS) {
+    cn64_sum<2>(c, b, a);
+    __syncthreads();
+  }
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     const size_t a = (size_t)b * N + i;
     const int k = c.w.cidx[a];
@@ -727,8 +698,11 @@ void launch_eeq64(const Ctx &c, cudaStream_t st) {
   // eight pairs per thread fill the queues of a batch, one spreads few pairs
   const int rounds = B * pairs <= 4LL * sm_count() * 128 ? 1 : 8;
   const int ctas = (int)((pairs + 128 * rounds - 1) / (128 * rounds));
-  eeq64_build_kernel<<<dim3(ctas + (N + CS_ATOMS - 1) / CS_ATOMS, B), 128, 0, st>>>(c, rounds,
-                                                                                   ctas);
+  // (the one-CTA solver adds up its structure's coordination numbers itself: beside
+  // the pairs of many small structures their CTAs cost 12 us of 360 x 30 atoms)
+  const int sums = N <= EEQ64_SMALL ? 0 : (N + CS_ATOMS - 1) / CS_ATOMS;
+  if (ctas + sums > 0)
+    eeq64_build_kernel<<<dim3(ctas + sums, B), 128, 0, st>>>(c, rounds, ctas);
   if (N <= EEQ64_SMALL) {
     const int rows = EB + 2 + (N > EB ? N - EB : 0);  // beside the first diagonal block
     if (rows <= 64)
