@@ -454,8 +454,9 @@ __global__ void __launch_bounds__(A3_THREADS, PGRAD ? 3 : 4) atm32_kernel(Ctx c,
 // its (j, k) record and sums in registers, against up to 64 neighbours i, four
 // rows' (i, k) records in flight: the (i, k) sums leave by one reduction at L2
 // each, the (i, j) sums of four rows cross lanes by halving exchanges (9 shuffles;
-// through shared memory they took 22 of its wavefronts, and the kernel is bound by
-// those, 0.80 of their rate: 16000 atoms, cutoff 25 Bohr, 8.0 -> 7.1 ms).  Atom
+// through shared memory they took 22 of its wavefronts and those bound the kernel at
+// 0.80 of their rate; now it is issue, 0.80: 16000 atoms, cutoff 25 Bohr, 8.0 -> 7.1
+// ms).  Atom
 // energies come from the pair sums (atm_mirror_kernel); only the energies e_w
 // of the centre's 1/3 triples, which it gets nothing of, leave here as -e_w /
 // 3 (see a3_step).  Energies without gradient have no pair sums and add up

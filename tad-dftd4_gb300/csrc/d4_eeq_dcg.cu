@@ -11,9 +11,9 @@
 // FP32 solve is the inner one of a refinement whose residuals are taken in
 // double-float.
 //
-// Measured at 16000 atoms, charges + adjoint: 21.9 (factorisation) -> 10.8 ms,
-// of it 7.7 the solves, 1.5 the residuals, 1.0 the matrix, 0.4 Z^T A Z, its
-// inverse and G (2.0, 1.2 and 0.5 over the whole matrix).  A product takes 93 us
+// Measured at 16000 atoms, charges + adjoint: 22.0 (factorisation) -> 12.0 ms, of
+// it 8.8 the solves (73 products), 1.7 the residuals, 1.0 the matrix, 0.4 Z^T A Z,
+// its inverse and G.  A product takes 93 us
 // with one right-hand side (5.5 TB/s of the half matrix), 122 with two; the rest
 // of an iteration (two exchanges, three barriers) 12 to 14 us.
 //
@@ -783,8 +783,8 @@ struct DrSmem {
 // matrix: dc_product's tiles, each for both of its products, with four of a
 // warp's eight rows of both planes in flight.  Bound by the latency of its FP32
 // sums (12 instructions per entry, product and right-hand side): 16000 atoms, two
-// right-hand sides 0.37 ms (2.8 TB/s), one 0.21 ms (4.8 TB/s); the five of charges +
-// adjoint 1.5 ms against 2.0 over the whole matrix.  256 threads with eight rows in
+// right-hand sides 0.37 ms (2.8 TB/s), one 0.21 ms (4.8 TB/s); five of them 1.5 ms
+// against 2.0 over the whole matrix.  256 threads with eight rows in
 // flight 0.38 and 0.22, two rows of 16 warps 0.39 and 0.24.
 template <int NR, bool VEC>
 __global__ void __launch_bounds__(DC_THREADS, 1) dcg_residual_kernel(Ctx c, int it) {
