@@ -43,6 +43,7 @@ namespace {
 constexpr int CG_FEW = 256, CG_MANY = 512, CG_FEW_ROWS = 10;
 constexpr float CG_TOL = 1e-10f;     // max |b - A x| that converges
 constexpr float CG_GAIN = 1e-12f;    // of (r, r / diag) per FP32 solve
+constexpr float CG_LAST = 1e-10f;    // of it: FP32 may be at its end
 constexpr int CG_OUTER = 16;         // refinements at most
 constexpr int CG_INNER = 500;        // iterations of one FP32 solve at most
 constexpr size_t CG_SMEM = 200 * 1024;
@@ -251,10 +252,11 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
       if (NR == 2) res = fmaxf(res, mx[NR - 1]);
       if (res <= bars.goal || below || outer == CG_OUTER) break;
       below = res < bars.tol;  // (then this correction is the last)
-      float stop[NR];
+      float stop[NR], g0[NR];
       bool on[NR];
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
+        g0[q] = g[q];
         stop[q] = CG_GAIN * g[q];
         on[q] = mx[q] > bars.goal;
       }
@@ -327,9 +329,11 @@ __global__ void __launch_bounds__(NT, 1) eeq_cg_kernel(Ctx c, int G, int groups)
             continue;
           }
           const float den = it == 0 ? v[q] : v[q] - beta[q] * g[q] / alpha[q];
-          if (!(den > 0.f)) {  // (p, A p): not positive definite, or FP32 at its end
+          // (p, A p): not positive definite, or FP32 at its end, where the residual
+          // of a definite matrix is
+          if (!(den > 0.f)) {
             bad = true;
-            definite = definite && it > 0 && v[q] > 0.f;
+            definite = definite && it > 0 && v[q] > 0.f && g[q] <= CG_LAST * g0[q];
           }
           alpha[q] = g[q] / den;
         }

@@ -47,6 +47,7 @@ constexpr int DC_LDG = DC_K + 16;         // row stride of G in shared memory (n
 constexpr float DC_TOL = 1e-10f;          // max |b - A x| that converges
 constexpr float DC_GAIN = 3e-9f;          // of (r, r / diag) per FP32 solve (1e-8 to 1e-9 alike;
                                           // 1e-11 takes 2 % more of a call of 16000 atoms)
+constexpr float DC_LAST = 1e-8f;          // of it: FP32 may be at its end
 constexpr float DC_FLOOR = 1e-14f;        // of (b, b / diag): FP32 rounding of r
 constexpr int DC_ITS = 100;               // iterations of one FP32 solve at most
 
@@ -638,12 +639,13 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
         for (int e = 0; e < NR; ++e) __stcg(ar.u + e * dc_pad(N) + k, 0.f);
     publish(r * u, fabsf(r), bv * dinv * bv);
     if (!group_barrier(counter, (unsigned)ranks * ++passed, sm.dead, c.w.status)) return;
-    float g[NR], mx[NR], bb[NR], stop[NR], alpha[NR], beta[NR];
+    float g[NR], g0[NR], mx[NR], bb[NR], stop[NR], alpha[NR], beta[NR];
     bool on[NR], more = false;
     norms(g, mx, bb);
     const float end = it == 0 ? 0.f : dc_bars(c, b, NR).end * sc;
 #pragma unroll
     for (int e = 0; e < NR; ++e) {
+      g0[e] = g[e];
       stop[e] = fmaxf(DC_GAIN * g[e], DC_FLOOR * bb[e]);
       on[e] = g[e] > stop[e] && mx[e] > end;
       more |= on[e];
@@ -710,9 +712,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) eeq_dcg_kernel(Ctx c, int it) {
         beta[e] = n == 0 ? 0.f : ru / g[e];
         g[e] = ru;
         const float den = n == 0 ? d : d - beta[e] * ru / alpha[e];
-        if (!(den > 0.f)) {  // (p, P A p): not positive definite, or FP32 at its end
+        if (!(den > 0.f)) {  // (p, P A p): as in d4_eeq_cg.cu
           bad = true;
-          definite = definite && n > 0 && d > 0.f;
+          definite = definite && n > 0 && d > 0.f && ru <= DC_LAST * g0[e];
         }
         alpha[e] = ru / den;
       }
