@@ -145,7 +145,8 @@ __device__ __forceinline__ void a6_step(const A6 &a, int j0, int k, bool kok, in
     const double A = d + z, B = fma(2.0, x, -A), C = z - d;
     const double AB = A * B;
     const double g = fma(AB * C, w, 1.0);
-    const double fd = rcp_pos<false>(fma(ij.t, ik.t * tjk[t], 1.0));  // (1 .. 6e300; tjk carries the 6)
+    // (tjk carries the factor 6: 1 .. 6e300)
+    const double fd = rcp_pos<false>(fma(ij.t, ik.t * tjk[t], 1.0));
     const double D = q * (ik.q * qjk[t]) * fd;
     const double e = D * g;
     if (!GRAD) {

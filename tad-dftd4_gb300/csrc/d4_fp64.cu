@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(CN_T) cn_kernel(Ctx c, int rounds) {
 
 static void launch_cn(const Ctx &c, cudaStream_t st) {
   const long long pairs = (long long)c.N * (c.N - 1) / 2;
-  const int rounds = c.B * pairs <= 4LL * sm_count() * CN_T ? 1 : 8;  // few pairs: spread over the SMs
+  // (few pairs: spread over the SMs)
+  const int rounds = c.B * pairs <= 4LL * sm_count() * CN_T ? 1 : 8;
   const long long per = (long long)CN_T * rounds;
   if (pairs > 0)
     cn_kernel<<<dim3((unsigned)((pairs + per - 1) / per), c.B), CN_T, 0, st>>>(c, rounds);

@@ -19,8 +19,9 @@ __device__ __forceinline__ bool fp64_edge(double y) {
 
 // 1 / d for d >= 0: the PTX approximation (20 bits and more) and one third-order
 // step, y (1 + e + e^2) with e = 1 - d y (Householder's method), whose error is
-// below 0.01 of its last FMA's rounding (0.504 ulp measured).  d beyond 2^1022 and infinity give 0, 0
-// and subnormals infinity.  EDGE false: d is normal and below 2^1022.
+// below 0.01 of its last FMA's rounding (0.504 ulp measured).  d beyond 2^1022 and
+// infinity give 0, 0 and subnormals infinity.  EDGE false: d is normal and below
+// 2^1022.
 template <bool EDGE = true>
 __device__ __forceinline__ double rcp_pos(double d) {
   double y;

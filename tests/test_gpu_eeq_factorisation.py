@@ -59,7 +59,7 @@ def test_which_solver_takes_a_batch(d4):
     solver = d4._lib.load().d4_eeq_solver
     assert [solver(*x) for x in ((1, 296), (1, 297), (1, 4000), (16, 512), (1, 5000), (1, 16384),
                                  (2, 4000))] == [ONE_CTA, CG, CG, CG, DEFLATED, DEFLATED, DEFLATED]
-    assert [solver(*x) for x in ((80, 303), (12, 1003), (3, 5000), (1, 16385))] == [FACTORISATION] * 4
+    assert {solver(*x) for x in ((80, 303), (12, 1003), (3, 5000), (1, 16385))} == {FACTORISATION}
     assert solver(0, 5) == -1 and solver(5, 0) == -1
 
 
